@@ -189,6 +189,10 @@ struct KmeansDev {
 };
 cudaError_t launch_kmeans(const uint32_t* d_list, KmeansDev* d_km, int pixfmt, unsigned long long nmax,
                           int iters, cudaStream_t s);
+// Expand a monotone table given by its runs (value val[j] from entry start[j]
+// on, start[0] = 0, m runs) into fwd[n]; rev (may be null) gets it mirrored.
+cudaError_t launch_expand_runs(const int* d_start, const int* d_val, int m, int n, int* d_fwd, int* d_rev,
+                               cudaStream_t s);
 cudaError_t launch_build_graph(const GridDev& g, const void* d_img, const uint8_t* d_seeds,
                                const BuildModelDev& m, const int* d_lut_xy, const int* d_lut_z,
                                const int* d_lut_s, const int* d_lut_t,

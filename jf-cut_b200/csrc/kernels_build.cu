@@ -358,6 +358,23 @@ __device__ __forceinline__ void tlinks(const BuildModelDev& m, const int* __rest
   ct = lut_t[q];
 }
 
+// Table entry t takes the value of the last run that starts at or before it
+// (a bisection of the few hundred starts, which stay in L1).
+__global__ void __launch_bounds__(256) k_expand_runs(const int* __restrict__ start, const int* __restrict__ val, int m,
+                                                     int n, int* __restrict__ fwd, int* __restrict__ rev) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  int lo = 0, hi = m;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (start[mid] <= t) lo = mid;
+    else hi = mid;
+  }
+  const int v = val[lo];
+  fwd[t] = v;
+  if (rev) rev[n - 1 - t] = v;
+}
+
 // One pass over the padded grid: n-links (both directions of every pair, from
 // the contrast table), t-links, e = cs - ct, label = 0; padding is zeroed.
 template <int PF, int DIMS>
@@ -529,6 +546,14 @@ cudaError_t launch_kmeans(const uint32_t* d_list, KmeansDev* d_km, int pixfmt, u
       default: return cudaErrorInvalidValue;
     }
   }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_expand_runs(const int* d_start, const int* d_val, int m, int n, int* d_fwd, int* d_rev,
+                               cudaStream_t s) {
+  if (n <= 0 || m <= 0) return cudaErrorInvalidValue;
+  jfc_note_launch();
+  k_expand_runs<<<(n + 255) / 256, 256, 0, s>>>(d_start, d_val, m, n, d_fwd, d_rev);
   return cudaGetLastError();
 }
 
