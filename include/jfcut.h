@@ -228,7 +228,7 @@ int jfc_graph_edit_seeds(jfc_graph* g, const uint32_t* idx, const uint8_t* new_s
  * when they need a cut (real-time frame loops that must not stall on the
  * allocator, hosts that hand the library a fixed memory budget up front).
  * The working set lives in one fixed file-scope device array of about
- * 13.2 MB that every GPU loading the library holds until exit; grids are
+ * 13.5 MB that every GPU loading the library holds until exit; grids are
  * limited to 524,288 nodes after padding (width to a multiple of 32, height
  * to a multiple of 16), larger ones return JFC_ERR_INVALID_ARG.
  * Inputs d_excess and d_ncap[4] (reference channel order, dense w*h int32)

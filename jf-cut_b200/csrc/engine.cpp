@@ -159,9 +159,11 @@ static bool encode_pr_maps(const GridDev& g, int ty, int tz, CUtensorMap* out) {
   return true;
 }
 
-// Carve the control block for cap_tiles tiles / cap_grids grids.
+// Carve the control block for cap_tiles tiles / cap_grids grids (and, in 2D
+// sets, cap_rw row words and cap_reg regions of the global relabel).
 static void tileset_carve(TileSet& ts, char* blk, size_t* total) {
   const size_t nt = (size_t)ts.cap_tiles, ng = (size_t)ts.cap_grids;
+  const size_t nr = (size_t)ts.cap_reg;
   size_t off = 0;
   auto take = [&](size_t bytes) { const size_t o = off; off = align_up(off + bytes, 256); return o; };
   const size_t o_desc = take(sizeof(GridDev) * ng);
@@ -181,6 +183,11 @@ static void tileset_carve(TileSet& ts, char* blk, size_t* total) {
   const size_t o_ring = take(sizeof(unsigned long long) * nt * 2);   // work items: halves of split tiles
   const size_t o_lock = take(sizeof(int) * nt * 2);
   const size_t o_tmap = take(kTmapBytes * ng);
+  const size_t o_dirty = take(nt);
+  const size_t o_vf = take(sizeof(uint4) * (size_t)ts.cap_rw);
+  const size_t o_reg = take(sizeof(int4) * nr);
+  const size_t o_rrec = take(sizeof(unsigned) * nr);
+  const size_t o_rf0 = take(nr), o_rf1 = take(nr);
   *total = off;
   if (!blk) return;
   ts.d_desc = (GridDev*)(blk + o_desc);
@@ -199,6 +206,12 @@ static void tileset_carve(TileSet& ts, char* blk, size_t* total) {
   ts.d_pr_ring = (unsigned long long*)(blk + o_ring);
   ts.d_pr_lock = (int*)(blk + o_lock);
   ts.tmap_slot = blk + o_tmap;
+  ts.d_dirty = (uint8_t*)(blk + o_dirty);
+  ts.d_vf = (uint4*)(blk + o_vf);
+  ts.d_reg = (int4*)(blk + o_reg);
+  ts.d_rrec = (unsigned*)(blk + o_rrec);
+  ts.d_rflag[0] = (uint8_t*)(blk + o_rf0);
+  ts.d_rflag[1] = (uint8_t*)(blk + o_rf1);
 }
 
 int tileset_build(TileSet& ts, int dims, int tile_rows, int tile_depth, const std::vector<GridDev>& grids_in,
@@ -224,10 +237,23 @@ int tileset_build(TileSet& ts, int dims, int tile_rows, int tile_depth, const st
     base += g.tiles_x * g.tiles_y * g.tiles_z;
   }
   const int ntiles = base, ngrids = (int)grids.size();
+  // regions and row words of the 2D global relabel
+  std::vector<int4> regs;
+  long long nrw = 0;
+  if (dims == 2) {
+    nrw = (long long)ntiles * TY;
+    for (int gi = 0; gi < ngrids; ++gi) {
+      const GridDev& g = grids[gi];
+      const int rx = (g.tiles_x + JFC_WAVE_WORDS - 1) / JFC_WAVE_WORDS, first = (int)regs.size();
+      const int n = wave_regions(g.tiles_x, g.Hp);
+      for (int k = 0; k < n; ++k) regs.push_back(make_int4(gi, k % rx, k / rx, first));
+    }
+  }
+  const int nreg = (int)regs.size();
   // reuse the control block while it is large enough (the server re-forms its
   // tile sets between relabels); otherwise allocate with headroom when asked
   // to stage asynchronously
-  if (!ts.d_block || ts.cap_tiles < ntiles || ts.cap_grids < ngrids) {
+  if (!ts.d_block || ts.cap_tiles < ntiles || ts.cap_grids < ngrids || ts.cap_rw < nrw || ts.cap_reg < nreg) {
     if (s) {
       // stream-ordered: the old block goes back to the pool when `s` reaches
       // the free, and nothing waits for the other streams' work (the server
@@ -240,6 +266,8 @@ int tileset_build(TileSet& ts, int dims, int tile_rows, int tile_depth, const st
     }
     ts.cap_tiles = s ? ntiles + ntiles / 4 + 64 : ntiles;
     ts.cap_grids = s ? ngrids + ngrids / 4 + 8 : ngrids;
+    ts.cap_rw = s ? nrw + nrw / 4 : nrw;
+    ts.cap_reg = s ? nreg + nreg / 4 : nreg;
     if (ts.cap_tiles < 1) ts.cap_tiles = 1;
     if (ts.cap_grids < 1) ts.cap_grids = 1;
     size_t total = 0;
@@ -262,10 +290,13 @@ int tileset_build(TileSet& ts, int dims, int tile_rows, int tile_depth, const st
   ts.pr_split = pr_split && dims == 2 && TY == 16 ? 1 : 0;
   ts.ngrids = ngrids;
   ts.ntiles = ntiles;
+  ts.nreg = nreg;
   const size_t desc_bytes = sizeof(GridDev) * (size_t)ngrids, info_bytes = sizeof(int4) * (size_t)ntiles;
   const size_t tmap_bytes = kTmapBytes * (size_t)ngrids;
   const size_t o_maps = align_up(align_up(desc_bytes, 256) + info_bytes, 256);
-  const size_t stage = o_maps + tmap_bytes;
+  const size_t reg_bytes = sizeof(int4) * (size_t)nreg;
+  const size_t o_regs = align_up(o_maps + tmap_bytes, 256);
+  const size_t stage = o_regs + reg_bytes;
   int4* info;
   if (s) {
     if (ts.h_stage_bytes < stage) {
@@ -314,10 +345,16 @@ int tileset_build(TileSet& ts, int dims, int tile_rows, int tile_depth, const st
     if (desc_bytes) JFC_CUDA(cudaMemcpyAsync(ts.d_desc, ts.h_stage, desc_bytes, cudaMemcpyHostToDevice, s));
     if (info_bytes) JFC_CUDA(cudaMemcpyAsync(ts.d_info, info, info_bytes, cudaMemcpyHostToDevice, s));
     if (tma) JFC_CUDA(cudaMemcpyAsync((void*)ts.d_tmap, maps, tmap_bytes, cudaMemcpyHostToDevice, s));
+    if (reg_bytes) {
+      std::memcpy((char*)ts.h_stage + o_regs, regs.data(), reg_bytes);
+      JFC_CUDA(cudaMemcpyAsync(ts.d_reg, (char*)ts.h_stage + o_regs, reg_bytes, cudaMemcpyHostToDevice, s));
+    }
+    JFC_CUDA(launch_mark_dirty(ts, s));
   } else {
     if (desc_bytes) JFC_CUDA(cudaMemcpy(ts.d_desc, grids.data(), desc_bytes, cudaMemcpyHostToDevice));
     if (info_bytes) JFC_CUDA(cudaMemcpy(ts.d_info, info, info_bytes, cudaMemcpyHostToDevice));
     if (tma) JFC_CUDA(cudaMemcpy((void*)ts.d_tmap, maps, tmap_bytes, cudaMemcpyHostToDevice));
+    if (reg_bytes) JFC_CUDA(cudaMemcpy(ts.d_reg, regs.data(), reg_bytes, cudaMemcpyHostToDevice));
   }
   return JFC_OK;
 }
@@ -350,6 +387,12 @@ static size_t pin_need_cycle(const TileSet& ts) { return (pin_need(ts) + 255) / 
 static cudaError_t enqueue_bfs(TileSet& ts, bool cut, int max_passes, cudaStream_t s, void* pin) {
   cudaError_t e;
 #define JFC_E(call) do { e = (call); if (e != cudaSuccess) return e; } while (0)
+  if (!cut && ts.dims == 2) {
+    JFC_E(launch_wave_relabel(ts, s));
+    JFC_E(cudaMemcpyAsync(pin, ts.d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s));
+    return cudaMemcpyAsync((char*)pin + sizeof(DevCounters), ts.d_grid_active, sizeof(int) * ts.ngrids,
+                           cudaMemcpyDeviceToHost, s);
+  }
   JFC_E(cudaMemsetAsync(ts.d_flag_bfs[0], 0, sizeof(int) * (size_t)ts.ntiles, s));
   JFC_E(cudaMemsetAsync(ts.d_flag_bfs[1], 0, sizeof(int) * (size_t)ts.ntiles, s));
   if (!cut) JFC_E(cudaMemsetAsync(ts.d_grid_active, 0, sizeof(int) * ts.ngrids, s));
@@ -599,6 +642,7 @@ int engine_solve(jfc_ctx* ctx, TileSet& ts, const jfc_params& p_in, std::vector<
       cudaEvent_t f0 = ev[2], f1 = ev[3];
       JFC_CUDA(cudaEventRecord(f0, s));
       for (int it = 0; it < interval; ++it) JFC_CUDA(launch_fast_iteration(*fast_grid, &ts.d_ctr->fast_moved, s));
+      JFC_CUDA(launch_mark_dirty(ts, s));
       JFC_CUDA(cudaEventRecord(f1, s));
       rc = engine_bfs(ctx, ts, p, false, st.bfs_passes, &active, nullptr, nullptr);
       if (rc) return rc;

@@ -24,6 +24,11 @@
 #define JFC_PAD_Z3 4        // 3D z padding (tile depths 1, 2, 4)
 #define JFC_MAX_K 32        // k-means clusters per class
 #define JFC_TQ 65536        // t-link probability quantisation
+// Regions of the 2D global relabel (kernels_wave.cu): interior rows and
+// 32-node words, levels per phase (the halo)
+#define JFC_WAVE_ROWS 64
+#define JFC_WAVE_WORDS 6
+#define JFC_WAVE_T 32
 
 // Device-side descriptor of one grid instance.
 struct GridDev {
@@ -69,10 +74,9 @@ struct DevCounters {
   unsigned pr_head;          // push-relabel worklist: tickets taken
   unsigned pr_tail;          // push-relabel worklist: ring positions reserved
   int pr_out;                // push-relabel worklist: items queued and not yet fully visited
-  unsigned wl_head;          // 2D relabel worklist: tickets taken
-  unsigned long long wl_tail_out;  // 2D relabel worklist, updated together: ring positions
-                                   // reserved (high 32 bits) and items queued and not yet fully
-                                   // visited (low 32 bits)
+  // 2D global relabel (kernels_wave.cu)
+  unsigned long long wave_bar; // barrier arrivals (low 40 bits), CTAs that flagged a region (high bits)
+  unsigned long long wave_q; // active items queued so far: parity 0 low, parity 1 high 32 bits
 };
 
 // A set of grids tiled with one tile shape: the unit every launch works on
@@ -93,6 +97,13 @@ struct TileSet {
   int* d_q_bfs[2] = {nullptr, nullptr};     // [buffer] BFS frontiers
   uint8_t* d_act = nullptr;          // [ntiles] bits 0-1: tile (half) held an active node at its last
                                      // relabel visit
+  // 2D global relabel (kernels_wave.cu; null in 3D sets)
+  uint4* d_vf = nullptr;             // [row words] two buffers of level-set state
+  int4* d_reg = nullptr;             // [nreg] {grid, region x, region y, first region of the grid}
+  unsigned* d_rrec = nullptr;        // [nreg] phase << 1 | buffer that holds the region's state
+  uint8_t* d_rflag[2] = {nullptr, nullptr};   // [phase & 1][nreg] the region takes part in the phase
+  uint8_t* d_dirty = nullptr;        // [ntiles] e or a residual arc changed since the last relabel
+  int nreg = 0;
   int* d_grid_active = nullptr;      // [ngrids] active tiles after global relabel
   unsigned long long* d_pr_ring = nullptr;  // [work items] push-relabel worklist ring (null: sweeps only)
   int* d_pr_lock = nullptr;          // [work items] a visit of the item is in progress
@@ -106,6 +117,8 @@ struct TileSet {
   void* d_block = nullptr;           // single allocation backing the above
   size_t block_bytes = 0;
   int cap_tiles = 0, cap_grids = 0;  // capacity of d_block (reused while it fits)
+  long long cap_rw = 0;              // row words
+  int cap_reg = 0;                   // regions
   void* h_stage = nullptr;           // pinned staging of d_desc / d_info uploads
   size_t h_stage_bytes = 0;
   void* gcache = nullptr;            // captured relabel-cycle graphs (engine.cpp)
@@ -143,11 +156,21 @@ cudaError_t launch_prepush(const TileSet& ts, cudaStream_t s);
 // global relabel (cut = false; also refills the push-relabel queues) or the
 // source-side cut (cut = true)
 cudaError_t launch_bfs(const TileSet& ts, bool cut, int max_passes, cudaStream_t s);
+// (kernels_wave.cu) the global relabel of a 2D tile set; resets its own queues
+// and counters
+cudaError_t launch_wave_relabel(const TileSet& ts, cudaStream_t s);
+// regions of a 2D grid in that relabel
+inline int wave_regions(int tiles_x, int Hp) {
+  return (tiles_x + JFC_WAVE_WORDS - 1) / JFC_WAVE_WORDS * ((Hp + JFC_WAVE_ROWS - 1) / JFC_WAVE_ROWS);
+}
 // (kernels_bfs.cu) tag post-process: bit 1 of each label byte = object node
 // connected through object nodes to a foreground seed (dense d_seeds)
 cudaError_t launch_tag(const TileSet& ts, const uint8_t* d_seeds, int max_passes, cudaStream_t s);
 cudaError_t launch_grid_sums(const TileSet& ts, cudaStream_t s);
+// Start of a solve: counters zero, every tile marked changed.
 cudaError_t launch_clear_counters(const TileSet& ts, cudaStream_t s);
+// Every tile changed: the next global relabel reads all of e and the arcs.
+cudaError_t launch_mark_dirty(const TileSet& ts, cudaStream_t s);
 // Polls before the device-side waits of later launches give up (0: default)
 // and the distance cap of the global relabels (0: none).
 cudaError_t launch_set_limits(const TileSet& ts, unsigned long long polls, int h_cap, cudaStream_t s);

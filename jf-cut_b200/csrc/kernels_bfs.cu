@@ -58,52 +58,6 @@ __device__ __forceinline__ void flush_staged(const BfsQ& Q, int lane) {
   for (int i = lane; i < cnt; i += 32) Q.q[base + i] = Q.sbuf[i];
 }
 
-// Worklist of the asynchronous 2D relabel: a ring of `cap` tile slots (-1 =
-// empty) with the queued flags of BfsQ, a tail counter and the count of
-// items queued and not yet fully visited (zero = the relaxation is done).
-struct RlRing {
-  int* ring;
-  unsigned cap;
-  unsigned long long* tail_out;   // ring positions reserved (high 32 bits), items outstanding (low 32)
-  int* err;
-  unsigned long long max_spins;   // polls before a wait gives up
-};
-
-// Append the tiles offered by the lanes of a warp that win their queued
-// flag: count them as outstanding first (so the count never reaches zero
-// while one is on its way), then reserve ring positions and claim each slot
-// (free, or freed by its reader within a few polls; bounded: after
-// W.max_spins polls the error flag is raised).  Returns false after an error.
-// Returns false after an error.  `folded` tells whether the appending visit's
-// own completion was counted in the same update (it appended something): the
-// update adds m positions and m - 1 outstanding items, made before the items
-// are published, so the count cannot reach zero while they wait.
-__device__ __forceinline__ bool ring_append(bool want, int tile, int* flags, const RlRing& W, bool& folded) {
-  bool won = false;
-  if (want) won = atomicExch(flags + tile, 1) == 0;
-  const unsigned m = __ballot_sync(jfc::FULL, won);
-  folded = m != 0;
-  if (!m) return true;
-  const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
-  unsigned base = 0;
-  if (lane == leader) {
-    const unsigned c = (unsigned)__popc(m);
-    base = (unsigned)(atomicAdd(W.tail_out, ((unsigned long long)c << 32) + (c - 1u)) >> 32);
-  }
-  base = __shfl_sync(jfc::FULL, base, leader);
-  bool ok = true;
-  if (won) {
-    int* slot = W.ring + (base + __popc(m & ((1u << lane) - 1u))) % W.cap;
-    __threadfence();
-    unsigned long long spins = 0;
-    while (atomicCAS(slot, -1, tile) != -1) {
-      if (++spins > W.max_spins || *(volatile int*)W.err) { atomicExch(W.err, 1); ok = false; break; }
-      __nanosleep(64);
-    }
-  }
-  return __all_sync(jfc::FULL, ok);
-}
-
 template <int DIMS>
 struct Dirs {
   static constexpr int XP = 0, YP = 1;
@@ -448,141 +402,6 @@ __global__ void __launch_bounds__(256) k_cut(TileSet ts, int max_passes, const u
 }
 
 // ------------------------------------------------------------ global relabel
-template <int DIMS, int TY, int TZ>
-using RTile = jfc::CtaTile<DIMS, TY, TZ>;
-
-template <int DIMS, int TY, int TZ>
-struct RlSmem {
-  int h[RTile<DIMS, TY, TZ>::HN];
-  uint8_t arc[RTile<DIMS, TY, TZ>::NT];
-  int ntile;
-  int face[6];
-  int folded;   // worklist: the visit's completion was counted with its appends
-};
-
-// One frontier visit, one CTA per tile, one thread per node (the reference's
-// work-group layout, graphcut_global_relabel.cl:50-124): stage the tile's
-// heights and the halo, close the in-tile distances (relax_cta), write the
-// heights that fell, queue the neighbours whose halo fell and the tile itself
-// when its fixpoint was not reached.
-// W.ring non-null: the asynchronous worklist (neighbours go to the ring).
-template <int DIMS, int TY, int TZ>
-__device__ __forceinline__ void relabel_visit(const TileSet& ts, int tid, RlSmem<DIMS, TY, TZ>& s,
-                                              const BfsQ& Q, int& cur_grid, int& delta,
-                                              const RlRing& W = RlRing{nullptr, 0, nullptr, nullptr, 0}) {
-  using T = RTile<DIMS, TY, TZ>;
-  using D = Dirs<DIMS>;
-  const int t = threadIdx.x;
-  const int x = t & 31, row = t >> 5, y = row % TY, z = row / TY;
-  const int4 ti = ts.d_info[tid];
-  const GridDev& g = ts.d_desc[ti.x];
-  const int pitch = g.pitch;
-  const long long slab = (long long)g.pitch * g.Hp;
-  const int x0 = ti.y * 32, y0 = ti.z * TY, z0 = ti.w * TZ;
-  const long long tbase = (long long)x0 + (long long)y0 * pitch + (long long)z0 * slab;
-  const long long n = tbase + x + (long long)y * pitch + (long long)z * slab;
-  const int hi = T::hidx(x, y, z);
-  // residual-arc bits and the excess sign, written by the first pass
-  const unsigned ab = g.label[n];
-  const unsigned arcs = ab & 63u;
-  const bool pos = (ab & 128u) != 0;
-  s.arc[t] = (uint8_t)arcs;
-  // heights other CTAs write while the worklist runs are read from L2 (the
-  // SM's L1 may hold an older copy of the line)
-  const bool fresh = W.ring != nullptr;
-  // (thread 0) the tile's activity byte as its last visit left it, read early
-  unsigned act_old = 0;
-  if (t == 0) act_old = fresh ? __ldcg(ts.d_act + tid) : ts.d_act[tid];
-  const int hstart = fresh ? __ldcg(g.h + n) : g.h[n];
-  s.h[hi] = hstart;
-  for (int c = t; c < T::NHALO; c += T::NT) {
-    int hx, hy, hz, f;
-    T::halo_cell(c, hx, hy, hz, f);
-    const int gx = x0 + hx, gy = y0 + hy, gz = z0 + hz;
-    int v = JFC_INF;
-    if (gx >= 0 && gx < pitch && gy >= 0 && gy < g.Hp && gz >= 0 && gz < g.Dp) {
-      const int* p = g.h + (long long)gx + (long long)gy * pitch + (long long)gz * slab;
-      v = fresh ? __ldcg(p) : *p;
-    }
-    s.h[T::hidx(hx, hy, hz)] = v;
-  }
-  if (t < 6) s.face[t] = 0;
-  __syncthreads();
-  // a tile is queued when a neighbour's boundary heights changed, which may
-  // not lower anything here: relax only when some residual arc (in the tile
-  // or into the halo) still offers a shorter distance
-  int m = JFC_INF;
-  if (arcs & jfc::A_XP) m = min(m, s.h[hi + 1]);
-  if (arcs & jfc::A_XM) m = min(m, s.h[hi - 1]);
-  if (arcs & jfc::A_YP) m = min(m, s.h[hi + T::SY]);
-  if (arcs & jfc::A_YM) m = min(m, s.h[hi - T::SY]);
-  if constexpr (DIMS == 3) {
-    if (arcs & jfc::A_ZP) m = min(m, s.h[hi + T::SZ]);
-    if (arcs & jfc::A_ZM) m = min(m, s.h[hi - T::SZ]);
-  }
-  const int cap = jfc::cap_of(g, ts.d_ctr);
-  const bool need = __syncthreads_or(m + 1 < hstart && m + 1 < cap);
-  const bool converged = need ? jfc::relax_cta<DIMS, TY, TZ>(s.h, s.arc, 16) : true;
-  // distances at or above the cap stay unreachable (every stored height is
-  // below the cap or JFC_INF, so the capped closure is the closure clamped)
-  const int hf = s.h[hi] < cap ? s.h[hi] : hstart;
-  const bool changed = hf != hstart;
-  if (changed) {
-    g.h[n] = hf;
-    if (W.ring) __threadfence();   // visible before any neighbour is queued
-    if (x == 0) s.face[0] = 1;
-    if (x == 31) s.face[1] = 1;
-    if (y == 0) s.face[2] = 1;
-    if (y == TY - 1) s.face[3] = 1;
-    if (DIMS == 3 && z == 0) s.face[4] = 1;
-    if (DIMS == 3 && z == TZ - 1) s.face[5] = 1;
-  }
-  // activity per 8-row half of a 2D 32x16 tile (bit 0 rows 0-7, bit 1 rows
-  // 8-15: the push-relabel work items of split tile sets), else bit 0
-  const bool live = pos & (hf < JFC_INF);
-  bool act_lo, act_hi = false;
-  if constexpr (DIMS == 2 && TY == 16) {
-    act_lo = __syncthreads_or(live && y < 8);
-    act_hi = __syncthreads_or(live && y >= 8);
-  } else {
-    act_lo = __syncthreads_or(live);
-  }
-  const bool act = act_lo || act_hi;
-  if (t < 32) {
-    const int txs = g.tiles_x, tys = g.tiles_y;
-    bool want = false;
-    int nb = tid;
-    switch (t) {
-      case 0: want = s.face[0] && x0 > 0; nb = tid - 1; break;
-      case 1: want = s.face[1] && x0 + 32 < pitch; nb = tid + 1; break;
-      case 2: want = s.face[2] && y0 > 0; nb = tid - txs; break;
-      case 3: want = s.face[3] && y0 + TY < g.Hp; nb = tid + txs; break;
-      case 4: want = DIMS == 3 && s.face[4] && z0 > 0; nb = tid - txs * tys; break;
-      case 5: want = DIMS == 3 && s.face[5] && z0 + TZ < g.Dp; nb = tid + txs * tys; break;
-      case 6: want = !converged; nb = tid; break;
-      default: break;
-    }
-    if (W.ring) {
-      bool folded = false;
-      ring_append(want, nb, Q.flags, W, folded);
-      if (t == 0) s.folded = folded ? 1 : 0;
-    } else {
-      jfc::warp_append(want, nb, Q.flags, Q.q, Q.qn);
-    }
-    if (t == 0) {
-      const int old = (act_old & 3u) != 0 ? 1 : 0;
-      ts.d_act[tid] = (uint8_t)((act_lo ? 1 : 0) | (act_hi ? 2 : 0));
-      if (ti.x != cur_grid) {
-        if (delta && cur_grid >= 0) atomicAdd(&ts.d_grid_active[cur_grid], delta);
-        delta = 0;
-        cur_grid = ti.x;
-      }
-      delta += (act ? 1 : 0) - old;
-    }
-  }
-  __syncthreads();
-}
-
 // x-direction closure of one tile row (lane = x): h(p) = min(h(p), h(q) + |p - q|)
 // over the runs of residual arcs p -> p+1 -> ... -> q (axp) and p -> p-1 ->
 // ... -> q (axm), by doubling.  The arc runs are read from the row's arc
@@ -661,9 +480,10 @@ __device__ __forceinline__ void tile_close(int (&hv)[TY * TZ], const unsigned (&
 // (h = 0 in this pass); everything later passes refine.  (A min-plus closure
 // of the tile instead of the level steps measured slower here: the deficits
 // lie close, so few levels run, and the pass streams its loads.)
-template <int DIMS, int TY, int TZ>
+template <int TY, int TZ>
 __device__ __forceinline__ void relabel_first_warp(const TileSet& ts, int tid, const BfsQ& Q, int& cur_grid,
                                                    int& delta) {
+  constexpr int DIMS = 3;
   using D = Dirs<DIMS>;
   constexpr int R = TY * TZ;
   const int lane = threadIdx.x & 31;
@@ -802,162 +622,6 @@ __device__ __forceinline__ void relabel_first_warp(const TileSet& ts, int tid, c
   flag_neighbours<DIMS, TY, TZ>(g, a, tid, rows_fin, c0 != 0, c31 != 0, false, Q);
 }
 
-// Frontier visit, one warp per tile: a level BFS over the tile (bit-parallel
-// rows as in the first pass) seeded by the halo heights, keeping only strict
-// improvements (heights only fall during a relabel, and a node is assigned
-// at the first level that reaches it).  Levels with an empty frontier jump
-// to the next halo seed that could improve its node, so a visit costs one
-// level per improved BFS layer plus one per distinct useful seed value:
-// bounded by the tile's nodes plus its halo cells.
-template <int DIMS, int TY, int TZ>
-__device__ __forceinline__ void relabel_frontier_warp(const TileSet& ts, int tid, const BfsQ& Q, int& cur_grid,
-                                                      int& delta) {
-  constexpr int R = TY * TZ;
-  constexpr int kMaxLevels = 4096;   // above the bound (nodes + halo cells); never reached
-  const int lane = threadIdx.x & 31;
-  const int4 ti = ts.d_info[tid];
-  const GridDev& g = ts.d_desc[ti.x];
-  const Addr a = make_addr<DIMS, TY, TZ>(g, ti, lane);
-  unsigned AXP[R], AXM[R], AYP[R], AYM[R];
-  unsigned AZP[DIMS == 3 ? R : 1], AZM[DIMS == 3 ? R : 1];
-  int hv[R];
-  unsigned posm = 0;
-#pragma unroll
-  for (int i = 0; i < R; ++i) {
-    const long long n = roff<TY>(a, i);
-    const unsigned b = g.label[n];   // arc byte written by the first pass
-    hv[i] = g.h[n];
-    AXP[i] = __ballot_sync(FULL, b & jfc::A_XP);
-    AXM[i] = __ballot_sync(FULL, b & jfc::A_XM);
-    AYP[i] = __ballot_sync(FULL, b & jfc::A_YP);
-    AYM[i] = __ballot_sync(FULL, b & jfc::A_YM);
-    if constexpr (DIMS == 3) {
-      AZP[i] = __ballot_sync(FULL, b & jfc::A_ZP);
-      AZM[i] = __ballot_sync(FULL, b & jfc::A_ZM);
-    }
-    if (b & 128u) posm |= 1u << i;
-  }
-  // halo heights: y faces per z slice (lane = x), z faces per row y, x faces
-  // in lanes r (left of row r) and 16 + r (right of row r)
-  int HT[TZ], HB[TZ];
-#pragma unroll
-  for (int z = 0; z < TZ; ++z) {
-    const long long n = roff<TY>(a, z * TY);
-    HT[z] = a.has_yT ? g.h[n - a.pitch] : JFC_INF;
-    HB[z] = a.has_yB ? g.h[n + (long long)TY * a.pitch] : JFC_INF;
-  }
-  int HZT[DIMS == 3 ? TY : 1], HZB[DIMS == 3 ? TY : 1];
-  if constexpr (DIMS == 3) {
-#pragma unroll
-    for (int y = 0; y < TY; ++y) {
-      const long long n = roff<TY>(a, y);
-      HZT[y] = a.has_zT ? g.h[n - a.slab] : JFC_INF;
-      HZB[y] = a.has_zB ? g.h[n + (long long)TZ * a.slab] : JFC_INF;
-    }
-  }
-  int HX = JFC_INF;
-  const int xrow = lane & 15;
-  {
-    const bool left = lane < 16;
-    if (xrow < R && (left ? a.has_xL : a.has_xR))
-      HX = g.h[(long long)(left ? a.x0 - 1 : a.x0 + 32) + (long long)(a.y0 + xrow % TY) * a.pitch +
-               (long long)(a.z0 + xrow / TY) * a.slab];
-  }
-  // smallest seed level above d that could still improve its node
-  auto next_level = [&](int d) -> int {
-    int c = JFC_INF;
-#pragma unroll
-    for (int z = 0; z < TZ; ++z) {
-      const int it = z * TY, ib = z * TY + TY - 1;
-      int v = HT[z] + 1;
-      if (v > d && v < hv[it] && ((AYM[it] >> lane) & 1u)) c = min(c, v);
-      v = HB[z] + 1;
-      if (v > d && v < hv[ib] && ((AYP[ib] >> lane) & 1u)) c = min(c, v);
-    }
-    if constexpr (DIMS == 3) {
-#pragma unroll
-      for (int y = 0; y < TY; ++y) {
-        const int it = y, ib = (TZ - 1) * TY + y;
-        int v = HZT[y] + 1;
-        if (v > d && v < hv[it] && ((AZM[it] >> lane) & 1u)) c = min(c, v);
-        v = HZB[y] + 1;
-        if (v > d && v < hv[ib] && ((AZP[ib] >> lane) & 1u)) c = min(c, v);
-      }
-    }
-    if (xrow < R && HX + 1 > d) c = min(c, HX + 1);
-    return __reduce_min_sync(FULL, c);
-  };
-  unsigned F[R];
-#pragma unroll
-  for (int i = 0; i < R; ++i) F[i] = 0u;
-  unsigned rows_changed = 0, c0 = 0, c31 = 0;
-  bool again = false;
-  const int cap = jfc::cap_of(g, ts.d_ctr);   // levels at or above it stay unreachable
-  int d = next_level(-1);
-  for (int level = 0; d < cap; ++level) {
-    if (level >= kMaxLevels) { again = true; break; }
-    const unsigned sx = __ballot_sync(FULL, HX + 1 == d);
-    unsigned N[R];
-    unsigned any = 0;
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const int y = i % TY, z = i / TY;
-      unsigned m = ((F[i] >> 1) & AXP[i]) | ((F[i] << 1) & AXM[i]);
-      if (y < TY - 1) m |= F[(i + 1 < R) ? i + 1 : i] & AYP[i];
-      if (y > 0) m |= F[(i > 0) ? i - 1 : 0] & AYM[i];
-      if constexpr (DIMS == 3) {
-        if (z < TZ - 1) m |= F[(i + TY < R) ? i + TY : i] & AZP[i];
-        if (z > 0) m |= F[(i >= TY) ? i - TY : 0] & AZM[i];
-        if (z == 0) m |= __ballot_sync(FULL, HZT[y] + 1 == d) & AZM[i];
-        if (z == TZ - 1) m |= __ballot_sync(FULL, HZB[y] + 1 == d) & AZP[i];
-      }
-      if (y == 0) m |= __ballot_sync(FULL, HT[z] + 1 == d) & AYM[i];
-      if (y == TY - 1) m |= __ballot_sync(FULL, HB[z] + 1 == d) & AYP[i];
-      m |= ((sx >> i) & 1u) & AXM[i];
-      m |= (((sx >> (16 + i)) & 1u) << 31) & AXP[i];
-      N[i] = m & __ballot_sync(FULL, hv[i] > d);
-      any |= N[i];
-    }
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      F[i] = N[i];
-      if (N[i]) {
-        rows_changed |= 1u << i;
-        c0 |= N[i] & 1u;
-        c31 |= N[i] >> 31;
-        if ((N[i] >> lane) & 1u) {
-          hv[i] = d;
-          g.h[roff<TY>(a, i)] = d;
-        }
-      }
-    }
-    d = any ? d + 1 : next_level(d);
-  }
-  // activity per 8-row half of a 2D 32x16 tile (bit 0 rows 0-7, bit 1 rows
-  // 8-15: the push-relabel work items of split tile sets), else bit 0
-  bool act_lo = false, act_hi = false;
-#pragma unroll
-  for (int i = 0; i < R; ++i) {
-    const bool live = ((posm >> i) & 1u) && hv[i] < JFC_INF;
-    if (DIMS == 2 && TY == 16 && i >= 8) act_hi |= live;
-    else act_lo |= live;
-  }
-  act_lo = __any_sync(FULL, act_lo);
-  act_hi = __any_sync(FULL, act_hi);
-  const bool act = act_lo || act_hi;
-  if (lane == 0) {
-    const int old = (__ldcg(ts.d_act + tid) & 3u) != 0 ? 1 : 0;
-    ts.d_act[tid] = (uint8_t)((act_lo ? 1 : 0) | (act_hi ? 2 : 0));
-    if (ti.x != cur_grid) {
-      if (delta && cur_grid >= 0) atomicAdd(&ts.d_grid_active[cur_grid], delta);
-      delta = 0;
-      cur_grid = ti.x;
-    }
-    delta += (act ? 1 : 0) - old;
-  }
-  flag_neighbours<DIMS, TY, TZ>(g, a, tid, rows_changed, c0 != 0, c31 != 0, again, Q);
-}
-
 // Frontier visit, one warp per tile, min-plus form: the tile's heights in
 // registers (lane = x, one register per row), lowered by the halo heights
 // across residual arcs, then closed in place: row closures by doubling
@@ -981,10 +645,11 @@ struct alignas(128) RlStage {
 
 // hb / lb non-null: the tile comes from a staged copy (RlStage) instead of
 // global loads.
-template <int DIMS, int TY, int TZ, bool STAGED = false>
+template <int TY, int TZ, bool STAGED = false>
 __device__ __forceinline__ void relabel_frontier_minplus(const TileSet& ts, int tid, int4 ti, const BfsQ& Q,
                                                          int& cur_grid, int& delta, const int* hb = nullptr,
                                                          const uint8_t* lb = nullptr) {
+  constexpr int DIMS = 3;
   constexpr int R = TY * TZ;
   using ST = jfc::CtaTile<3, TY, TZ, 40, 4>;
   const int lane = threadIdx.x & 31;
@@ -1114,15 +779,6 @@ __device__ __forceinline__ void relabel_frontier_minplus(const TileSet& ts, int 
   flag_neighbours<DIMS, TY, TZ>(g, a, tid, rows_changed, c0, c31, false, Q);
 }
 
-// 1: frontier visits of the warp form use the min-plus closure, 0: the level BFS
-#ifndef JFC_RELABEL_MINPLUS
-#define JFC_RELABEL_MINPLUS 1
-#endif
-
-#ifndef JFC_GR_ASYNC
-#define JFC_GR_ASYNC 1
-#endif
-
 // Refill of the push-relabel queues (buffer 0 of each parity) from the
 // active-tile bits, warp-aggregated.  Split tile sets queue the active 8-row
 // halves as work items 2 * tile + half, half 0 with the tile's checkerboard
@@ -1162,10 +818,8 @@ __device__ __forceinline__ void refill_pr_queues(const TileSet& ts, DevCounters*
 // Global relabel, pass 0: every tile, one warp per tile (bit-parallel level
 // BFS from the deficits, fused initialisation).  A plain launch: its many
 // registers do not limit the occupancy of the frontier kernel.
-// (32 x 8 2D tiles fit in 64 registers without spills: 4 CTAs per SM keep
-// twice the loads in flight of the 2-CTA bound the larger tiles need)
-template <int DIMS, int TY, int TZ>
-__global__ void __launch_bounds__(256, (DIMS == 3 && TY * TZ > 8) ? 1 : (DIMS == 2 && TY == 8) ? 4 : 2)
+template <int TY, int TZ>
+__global__ void __launch_bounds__(256, TY * TZ > 8 ? 1 : 2)
     k_relabel_first(TileSet ts) {
   DevCounters* ctr = ts.d_ctr;
   if (blockIdx.x == 0 && threadIdx.x == 0) ctr->t_gr_start = jfc::global_ns();
@@ -1177,7 +831,7 @@ __global__ void __launch_bounds__(256, (DIMS == 3 && TY * TZ > 8) ? 1 : (DIMS ==
   // slowest warp)
   BfsQ Q{ts.d_flag_bfs[1], ts.d_q_bfs[1], &ctr->qn_bfs[1]};
   int wgrid = -1, wdelta = 0;
-  relabel_first_warp<DIMS, TY, TZ>(ts, (int)w, Q, wgrid, wdelta);
+  relabel_first_warp<TY, TZ>(ts, (int)w, Q, wgrid, wdelta);
   if (lane == 0 && wdelta && wgrid >= 0) atomicAdd(&ts.d_grid_active[wgrid], wdelta);
 }
 
@@ -1188,13 +842,9 @@ __global__ void __launch_bounds__(256, (DIMS == 3 && TY * TZ > 8) ? 1 : (DIMS ==
 // graphcut_count_block.cl:19-65, as one warp-aggregated append).
 // Warp form of the frontier passes: one warp per queued tile (3D: many
 // tiles per pass, so the visit throughput counts).
-// (level-BFS form: one CTA per SM, its registers; min-plus form: 2 CTAs per
-// SM, the registers the two-ahead ticket pipeline holds without spills: 3
+// (2 CTAs per SM, the registers the two-ahead ticket pipeline holds without spills: 3
 // CTAs per SM spilled and measured slower, 116.5 vs 104-108.5 ms of frontier
 // per video solve)
-#ifndef JFC_RELABEL_WARP_MINB
-#define JFC_RELABEL_WARP_MINB 1
-#endif
 #ifndef JFC_RL3D_MINB
 #define JFC_RL3D_MINB 2
 #endif
@@ -1202,8 +852,8 @@ __global__ void __launch_bounds__(256, (DIMS == 3 && TY * TZ > 8) ? 1 : (DIMS ==
 #ifndef JFC_RL3D_STAGE
 #define JFC_RL3D_STAGE 1
 #endif
-template <int DIMS, int TY, int TZ>
-__global__ void __launch_bounds__(256, JFC_RELABEL_MINPLUS ? (TY * TZ > 8 ? 2 : JFC_RL3D_MINB) : JFC_RELABEL_WARP_MINB)
+template <int TY, int TZ>
+__global__ void __launch_bounds__(256, TY * TZ > 8 ? 2 : JFC_RL3D_MINB)
     k_relabel_warp(TileSet ts, int max_passes) {
   __shared__ int s_items[8][64];   // per-warp staged queue appends (at most 38 before a flush)
   __shared__ int s_cnt[8];
@@ -1211,7 +861,7 @@ __global__ void __launch_bounds__(256, JFC_RELABEL_MINPLUS ? (TY * TZ > 8 ? 2 : 
   // tensor copies into two buffers of its own (dynamic shared memory), the
   // next ticket's tile copied while the current one is visited
   using Stage = RlStage<TY, TZ>;
-  constexpr bool kStage = JFC_RL3D_STAGE && JFC_RELABEL_MINPLUS && DIMS == 3 && TY * TZ <= 8;
+  constexpr bool kStage = JFC_RL3D_STAGE && TY * TZ <= 8;
   __shared__ uint64_t s_bar[8][2];
   extern __shared__ __align__(128) unsigned char s_dyn[];
   DevCounters* ctr = ts.d_ctr;
@@ -1316,13 +966,11 @@ __global__ void __launch_bounds__(256, JFC_RELABEL_MINPLUS ? (TY * TZ > 8 ? 2 : 
           __syncwarp();
           break;   // the grid barrier below sees the error: every CTA leaves
         }
-        relabel_frontier_minplus<DIMS, TY, TZ, true>(ts, tt, ti, Q, cur_grid, delta, stage[buf].hb, stage[buf].lb);
+        relabel_frontier_minplus<TY, TZ, true>(ts, tt, ti, Q, cur_grid, delta, stage[buf].hb, stage[buf].lb);
         __syncwarp();   // every lane has read `buf` before it is refilled
         if (tnn >= 0) issue(tinn, buf);
-      } else if (JFC_RELABEL_MINPLUS) {
-        relabel_frontier_minplus<DIMS, TY, TZ>(ts, tt, ti, Q, cur_grid, delta);
       } else {
-        relabel_frontier_warp<DIMS, TY, TZ>(ts, tt, Q, cur_grid, delta);
+        relabel_frontier_minplus<TY, TZ>(ts, tt, ti, Q, cur_grid, delta);
       }
       buf ^= 1;
       ++visits;
@@ -1360,216 +1008,6 @@ __global__ void __launch_bounds__(256, JFC_RELABEL_MINPLUS ? (TY * TZ > 8 ? 2 : 
     ok = jfc::grid_sync(ctr, [&]() { ctr->ticket[0] = 0; });
   }
   // frontier visits are counted per warp (lane 0); pass 0 visited every tile
-  __shared__ unsigned long long s_vis;
-  if (threadIdx.x == 0) s_vis = 0;
-  __syncthreads();
-  if (lane == 0 && visits) atomicAdd(&s_vis, visits);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    if (s_vis) atomicAdd(&ctr->bfs_visits, s_vis);
-    if (blockIdx.x == 0) {
-      ctr->bfs_passes = pass;
-      ctr->bfs_visits += (unsigned long long)ts.ntiles;
-      if (ctr->bfs_status == 0) ctr->bfs_status = 1;
-      const unsigned long long t2 = jfc::global_ns();
-      ctr->ns_gr_first += t1 - ctr->t_gr_start;
-      ctr->ns_gr_frontier += t2 - t1;
-    }
-  }
-}
-
-// Global relabel, frontier passes (persistent, cooperative), CTA form: one
-// CTA per queued tile (2D: few tiles per pass, so the visit latency counts), grid barrier between passes, until a pass queues nothing; then
-// the push-relabel queues are refilled with every tile holding an active node
-// (the reference's graphcut_count_node + clogs scan + graphcut_scatter_node,
-// graphcut_count_block.cl:19-65, as one warp-aggregated append).
-// After the dense first pass every tile's heights are the exact in-tile
-// distances (halo unknown), so a tile can only fall through an arc leaving
-// it: one warp checks the tile's border nodes against the halo (2D) and
-// queues the tile for a full visit only when some residual arc u -> v out of
-// the tile has h(v) + 1 < h(u).
-template <int TY>
-__device__ __forceinline__ bool border_improvable(const TileSet& ts, int tid, int lane) {
-  const int4 ti = ts.d_info[tid];
-  const GridDev& g = ts.d_desc[ti.x];
-  const int cap = jfc::cap_of(g, ts.d_ctr);
-  const long long pitch = g.pitch;
-  const int x0 = ti.y * 32, y0 = ti.z * TY;
-  const long long base = (long long)x0 + (long long)y0 * pitch;
-  // a distance offered through the arc counts only below the relabel's cap
-  auto better = [&](long long n, long long m) { const int v = g.h[m] + 1; return v < g.h[n] && v < cap; };
-  bool imp = false;
-  if (y0 > 0) {   // top row, arcs -y
-    const long long n = base + lane;
-    if ((g.label[n] & jfc::A_YM) && better(n, n - pitch)) imp = true;
-  }
-  if (y0 + TY < g.Hp) {   // bottom row, arcs +y
-    const long long n = base + lane + (TY - 1) * pitch;
-    if ((g.label[n] & jfc::A_YP) && better(n, n + pitch)) imp = true;
-  }
-  if (lane < TY && x0 > 0) {   // left column, arcs -x
-    const long long n = base + lane * pitch;
-    if ((g.label[n] & jfc::A_XM) && better(n, n - 1)) imp = true;
-  } else if (lane >= 16 && lane < 16 + TY && x0 + 32 < pitch) {   // right column, arcs +x
-    const long long n = base + 31 + (lane - 16) * pitch;
-    if ((g.label[n] & jfc::A_XP) && better(n, n + 1)) imp = true;
-  }
-  return __any_sync(jfc::FULL, imp);
-}
-
-// (32 x 8 tiles: 6 CTAs per SM, the worklist's pollers and the border check's warps)
-#ifndef JFC_RL2D_MINB
-#define JFC_RL2D_MINB 6
-#endif
-template <int DIMS, int TY, int TZ>
-__global__ void __launch_bounds__(RTile<DIMS, TY, TZ>::NT,
-                                  (DIMS == 2 && TY == 8) ? JFC_RL2D_MINB : RTile<DIMS, TY, TZ>::NT > 256 ? 2 : 3)
-    k_relabel_cta(TileSet ts, int max_passes) {
-  __shared__ RlSmem<DIMS, TY, TZ> sm;
-  DevCounters* ctr = ts.d_ctr;
-  const int lane = threadIdx.x & 31;
-  unsigned long long visits = 0;
-  int cur_grid = -1, delta = 0;
-  bool ok = true;
-  int pass = 1;
-  bool to_worklist = false;
-  const unsigned long long t1 = jfc::global_ns();
-  for (pass = 1; ok; ++pass) {
-    const int cb = pass & 1;
-    const int n = jfc::vload(&ctr->qn_bfs[cb]);
-    if (n == 0) break;
-    if (pass > max_passes) {
-      if (blockIdx.x == 0 && threadIdx.x == 0) ctr->bfs_status = 2;
-      break;
-    }
-    BfsQ Q{ts.d_flag_bfs[cb ^ 1], ts.d_q_bfs[cb ^ 1], &ctr->qn_bfs[cb ^ 1]};
-    const int* queue = ts.d_q_bfs[cb];
-    int* fcur = ts.d_flag_bfs[cb];
-    to_worklist = JFC_GR_ASYNC && DIMS == 2 && pass == 1;
-    if (DIMS == 2 && pass == 1) {
-      // the tiles the dense pass queued: a warp-level border check, full
-      // visits from pass 2 on for the tiles that can fall
-      for (;;) {
-        const unsigned k = jfc::warp_ticket(&ctr->ticket[cb]);
-        if ((int)k >= n) break;
-        const int tt = queue[k];
-        if (lane == 0) fcur[tt] = 0;
-        const bool imp = border_improvable<TY>(ts, tt, lane);
-        jfc::warp_append(imp && lane == 0, tt, Q.flags, Q.q, Q.qn);
-      }
-    } else {
-      for (;;) {
-        if (threadIdx.x == 0) {
-          const unsigned k = atomicAdd(&ctr->ticket[cb], 1u);
-          sm.ntile = (int)k < n ? queue[k] : -1;
-          if ((int)k < n) fcur[sm.ntile] = 0;
-        }
-        __syncthreads();
-        const int tt = sm.ntile;
-        __syncthreads();
-        if (tt < 0) break;
-        relabel_visit<DIMS, TY, TZ>(ts, tt, sm, Q, cur_grid, delta);
-        if (threadIdx.x < 32) ++visits;
-      }
-    }
-    ok = jfc::grid_sync(ctr, [&]() {
-      ctr->ticket[cb] = 0;
-      ctr->qn_bfs[cb] = 0;
-      if (to_worklist) {
-        ctr->wl_head = 0;
-        const unsigned long long q = (unsigned)ctr->qn_bfs[cb ^ 1];
-        ctr->wl_tail_out = (q << 32) | q;
-      }
-    });
-    if (to_worklist) { ++pass; break; }
-  }
-  if (ok && to_worklist) {
-    // 2D passes 2..: an asynchronous worklist instead of barrier-separated
-    // passes.  A tile whose boundary fell queues its neighbours at once and
-    // any free CTA takes them, so a distance wave crosses one tile per visit
-    // instead of one tile per pass (the relaxation is monotone: any order
-    // reaches the same exact distances).  A per-tile lock keeps two visits of
-    // one tile apart; the work is done when no queued item is left.
-    const unsigned cap = (unsigned)ts.ntiles;
-    int* ring = ts.d_q_bfs[0];          // the border check queued into buffer 0
-    int* busy = ts.d_flag_bfs[1];       // free after the border check
-    const unsigned n0 = (unsigned)(*(volatile unsigned long long*)&ctr->wl_tail_out >> 32);
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < cap; i += (long long)gridDim.x * blockDim.x) {
-      if (i >= n0) ring[i] = -1;
-      busy[i] = 0;
-    }
-    ok = jfc::grid_sync(ctr, [&]() {});
-    const unsigned long long max_spins = jfc::spin_cap(ctr);
-    const RlRing W{ring, cap, &ctr->wl_tail_out, &ctr->error, max_spins};
-    const BfsQ Q{ts.d_flag_bfs[0], nullptr, nullptr};
-    while (ok) {
-      if (threadIdx.x == 0) {
-        int tile = -1;
-        const unsigned k = atomicAdd(&ctr->wl_head, 1u);
-        int* slot = ring + k % cap;
-        // bounded: the item arrives, or the work is done, or an error; the
-        // count measures a stall (it restarts whenever the worklist moves:
-        // items appended or finished), not the length of the relabel
-        unsigned long long spins = 0;
-        volatile unsigned long long* vto = &ctr->wl_tail_out;
-        unsigned long long seen = *vto;
-        for (;;) {
-          if (*(volatile int*)slot >= 0) {
-            const int v = atomicExch(slot, -1);
-            if (v >= 0) { tile = v; break; }
-          }
-          const unsigned long long to = *vto;
-          if ((unsigned)to == 0u || *(volatile int*)&ctr->error) break;
-          if (to != seen) {
-            seen = to;
-            spins = 0;
-          } else if (++spins > max_spins) {
-            atomicExch(&ctr->error, 1);
-            break;
-          }
-          __nanosleep(32);
-        }
-        if (tile >= 0) {
-          spins = 0;
-          while (atomicCAS(busy + tile, 0, 1) != 0) {
-            if (++spins > max_spins || *(volatile int*)&ctr->error) { atomicExch(&ctr->error, 1); tile = -1; break; }
-            __nanosleep(32);
-          }
-        }
-        if (tile >= 0) {
-          __threadfence();
-          atomicExch(Q.flags + tile, 0);   // dequeued before its heights are read
-          __threadfence();
-        }
-        sm.ntile = tile;
-      }
-      __syncthreads();
-      const int tt = sm.ntile;
-      __syncthreads();
-      if (tt < 0) break;
-      relabel_visit<DIMS, TY, TZ>(ts, tt, sm, Q, cur_grid, delta, W);   // ends with a block barrier
-      if (threadIdx.x == 0) {
-        __threadfence();
-        atomicExch(busy + tt, 0);
-        if (!sm.folded) atomicAdd(&ctr->wl_tail_out, ~0ull);   // - 1 outstanding
-      }
-      if (threadIdx.x < 32) ++visits;
-    }
-  }
-  // per-grid activity deltas: thread 0 holds the CTA visits', lane 0 of
-  // each warp the warp visits'
-  if (lane == 0 && delta && cur_grid >= 0) atomicAdd(&ts.d_grid_active[cur_grid], delta);
-  // refill the push-relabel queues (buffer 0 of each parity) from the
-  // active-tile flags
-  if (ok) ok = jfc::grid_sync(ctr, [&]() {
-    ctr->qn_pr[0][0] = ctr->qn_pr[0][1] = ctr->qn_pr[1][0] = ctr->qn_pr[1][1] = 0;
-    ctr->cur_pr[0] = ctr->cur_pr[1] = 0;
-  });
-  if (ok) {
-    refill_pr_queues(ts, ctr, lane);
-    ok = jfc::grid_sync(ctr, [&]() { ctr->ticket[0] = 0; });
-  }
-  // frontier visits are counted by warp 0 of each CTA; pass 0 visited every tile
   __shared__ unsigned long long s_vis;
   if (threadIdx.x == 0) s_vis = 0;
   __syncthreads();
@@ -1632,15 +1070,13 @@ __global__ void __launch_bounds__(256) k_grid_sums(const GridDev* __restrict__ g
 template <int DIMS, int TY, int TZ, int MODE>
 cudaError_t bfs_t(const TileSet& ts, int max_passes, const uint8_t* seeds, cudaStream_t s) {
   constexpr bool CUT = MODE != 0;
-  // global relabel frontier passes: CTA per tile in 2D, warp per tile in 3D
   const void* fn;
   if constexpr (MODE == 1) fn = (const void*)k_cut<DIMS, TY, TZ, false>;
   else if constexpr (MODE == 2) fn = (const void*)k_cut<DIMS, TY, TZ, true>;
-  else if constexpr (DIMS == 2) fn = (const void*)k_relabel_cta<DIMS, TY, TZ>;
-  else fn = (const void*)k_relabel_warp<DIMS, TY, TZ>;
-  const int nt = (CUT || DIMS == 3) ? 256 : RTile<DIMS, TY, TZ>::NT;
+  else fn = (const void*)k_relabel_warp<TY, TZ>;
+  const int nt = 256;
   // the 3D frontier's staging buffers: two per warp (dynamic shared memory)
-  const size_t dyn = (!CUT && DIMS == 3 && JFC_RL3D_STAGE && JFC_RELABEL_MINPLUS && TY * TZ <= 8)
+  const size_t dyn = (!CUT && JFC_RL3D_STAGE && TY * TZ <= 8)
                          ? 2 * 8 * sizeof(RlStage<TY, TZ>) + 128 : 0;
   if (dyn > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
@@ -1648,10 +1084,10 @@ cudaError_t bfs_t(const TileSet& ts, int max_passes, const uint8_t* seeds, cudaS
   }
   static int cache[64] = {0};
   const int blocks = persistent_blocks_cached(cache, fn, nt, dyn);
-  if (!CUT) {
+  if constexpr (!CUT) {
     const long long fb = ((long long)ts.ntiles * 32 + 255) / 256;
     jfc_note_launch();
-    k_relabel_first<DIMS, TY, TZ><<<(unsigned)fb, 256, 0, s>>>(ts);
+    k_relabel_first<TY, TZ><<<(unsigned)fb, 256, 0, s>>>(ts);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
@@ -1769,19 +1205,20 @@ int persistent_blocks_cached(int* cache, const void* kernel, int threads, size_t
 
 static cudaError_t bfs_dispatch(const TileSet& ts, int mode, int max_passes, const uint8_t* seeds, cudaStream_t s) {
 #define JFC_BFS(D, Y, Z)                                                       \
-  (mode == 1 ? bfs_t<D, Y, Z, 1>(ts, max_passes, seeds, s)                     \
-             : mode == 2 ? bfs_t<D, Y, Z, 2>(ts, max_passes, seeds, s)         \
-                         : bfs_t<D, Y, Z, 0>(ts, max_passes, seeds, s))
+  (mode == 1 ? bfs_t<D, Y, Z, 1>(ts, max_passes, seeds, s) : bfs_t<D, Y, Z, 2>(ts, max_passes, seeds, s))
+#define JFC_BFS3(Y, Z) (mode == 0 ? bfs_t<3, Y, Z, 0>(ts, max_passes, seeds, s) : JFC_BFS(3, Y, Z))
   if (ts.dims == 2) {
+    if (mode == 0) return launch_wave_relabel(ts, s);
     if (ts.TR == 8) return JFC_BFS(2, 8, 1);
     if (ts.TR == 16) return JFC_BFS(2, 16, 1);
     return cudaErrorInvalidValue;
   }
-  if (ts.TY == 4 && ts.TZ == 4) return JFC_BFS(3, 4, 4);
-  if (ts.TY == 4 && ts.TZ == 2) return JFC_BFS(3, 4, 2);
-  if (ts.TY == 16 && ts.TZ == 1) return JFC_BFS(3, 16, 1);
-  if (ts.TY == 8 && ts.TZ == 2) return JFC_BFS(3, 8, 2);
-  if (ts.TY == 8 && ts.TZ == 1) return JFC_BFS(3, 8, 1);
+  if (ts.TY == 4 && ts.TZ == 4) return JFC_BFS3(4, 4);
+  if (ts.TY == 4 && ts.TZ == 2) return JFC_BFS3(4, 2);
+  if (ts.TY == 16 && ts.TZ == 1) return JFC_BFS3(16, 1);
+  if (ts.TY == 8 && ts.TZ == 2) return JFC_BFS3(8, 2);
+  if (ts.TY == 8 && ts.TZ == 1) return JFC_BFS3(8, 1);
+#undef JFC_BFS3
 #undef JFC_BFS
   return cudaErrorInvalidValue;
 }
@@ -1810,8 +1247,13 @@ cudaError_t launch_grid_sums(const TileSet& ts, cudaStream_t s) {
   return cudaErrorInvalidValue;
 }
 
+cudaError_t launch_mark_dirty(const TileSet& ts, cudaStream_t s) {
+  return cudaMemsetAsync(ts.d_dirty, 1, (size_t)ts.ntiles, s);
+}
+
 cudaError_t launch_clear_counters(const TileSet& ts, cudaStream_t s) {
-  return cudaMemsetAsync(ts.d_ctr, 0, sizeof(DevCounters), s);
+  const cudaError_t e = cudaMemsetAsync(ts.d_ctr, 0, sizeof(DevCounters), s);
+  return e == cudaSuccess ? launch_mark_dirty(ts, s) : e;
 }
 
 namespace {

@@ -344,8 +344,13 @@ __device__ __forceinline__ int pr_visit(const TileSet& ts, int tid, int local_it
   if (t < 6) {
     const int nb = s.face[t] ? face_item<DIMS, TY, TZ, SPLIT>(ts, tid, t) : -1;
     s.q_nb[t] = nb;
+    // the global relabel reads the arcs and signs of these tiles again
+    if (nb >= 0) ts.d_dirty[SPLIT ? nb >> 1 : nb] = 1;
   }
-  if (t == 0) s.active = active ? 1 : 0;
+  if (t == 0) {
+    s.active = active ? 1 : 0;
+    ts.d_dirty[SPLIT ? tid >> 1 : tid] = 1;
+  }
   __syncthreads();
   JFC_PCLK(ts.d_ctr, 3);
   return rounds;

@@ -1,0 +1,481 @@
+// kernels_wave.cu — 2D global relabel by bit-parallel level sets.
+//
+// Reference: graphcut_init_global_relabel / graphcut_global_relabel
+// (graphcut_global_relabel.cl:19-124) driven by QGCWidget::globalRelabel
+// (QGCWidget.cpp:2208-2241): heights = exact BFS distance to the deficit nodes
+// (e < 0) over residual arcs.
+//
+// Layout.  32 neighbouring nodes of a row are one bit position each of a few
+// 32-bit words ("row words").  The label plane, one byte per node, is free
+// between the start of a solve and its cut, and holds eight words per row
+// segment of 32 nodes in its 32 bytes:
+//   0..3  residual arc +x, +y, -y, -x      4, 5  unused
+//   6     deficit (e < 0)                  7     excess (e > 0)
+// k_wave_bits writes them, from 20 bytes per node of e and the four residual
+// planes, for the tiles that something changed since the last relabel (a
+// byte per tile, set by the push-relabel visits; every tile at the start of a
+// solve).  All further work of a relabel is on words: 0.75 bytes per node.
+//
+// k_wave_relabel expands level sets: the nodes at distance d + 1 are those
+// with a residual arc into a node at distance d that have no distance yet, a
+// dozen word operations per 32 nodes.  A CTA takes a region of 64 rows x 6
+// words together with a halo of 32 rows and one word on each side into
+// registers and runs 32 levels on it with one block barrier each; what the
+// halo misses from farther out cannot reach the region's interior within 32
+// levels, so the interior is exact, and the interiors of all regions advance
+// 32 levels per grid barrier.  Only regions that a level set can reach take
+// part after the first phase.  Distances leave the words once per phase and
+// node, as 128-byte row writes of the height plane.
+//
+// Why: the height plane's relaxation by tiles that this replaces (one CTA per
+// queued 32 x 8 tile, asynchronous, after a dense pass over all planes) spent
+// its time in the latency of dependent tile visits, about 7 us per 8 or 32
+// nodes of distance.  A phase here takes 14 us while a few regions take part
+// (load 2, 32 levels 6, heights 3, the rest and the barrier 3).  Relabels of
+// one solve before / after: 15000 x 10000 RGB 37.2 / 11.5 ms, 1023 x 767 2.44
+// / 1.1 ms; a solve's last ones: 15000 x 10000 1.65 / 0.43 ms, 4096 x 3072 0.46
+// / 0.16 ms, 1023 x 767 0.139 / 0.045 ms.
+#include <algorithm>
+
+#include "jfc_sync.cuh"
+
+namespace {
+
+using jfc::FULL;
+
+constexpr int kT = JFC_WAVE_T;          // levels per phase = halo rows (<= 32, the word halo)
+constexpr int kIR = JFC_WAVE_ROWS;      // interior rows of a region
+constexpr int kIW = JFC_WAVE_WORDS;     // interior words of a region
+constexpr int kC = kIW + 2;             // columns (words) of a region with its halo
+constexpr int kS = (kIR + 2 * kT) / 4;  // strips of 4 rows
+constexpr int kThreads = kC * kS;
+constexpr int kList = 64;               // regions a CTA looks at in one go
+static_assert(kC == 8 && kThreads == 256 && kT % 16 == 0 && kT <= 32 && kIR >= kT && kIR % 16 == 0,
+              "a warp holds 8 columns x 4 strips of 4 rows");
+
+__device__ __forceinline__ uint32_t* seg_words(const GridDev& g, int y, int c) {
+  return reinterpret_cast<uint32_t*>(g.label + (long long)y * g.pitch + c * 32);
+}
+
+// Row words of the changed tiles, their heights (0 at deficits, else INF) and
+// empty level-set state; the relabel's queues, flags and counters reset.
+// One warp per changed tile; lane i of the tile's rows writes row i's words.
+template <int TY>
+__global__ void __launch_bounds__(256) k_wave_bits(TileSet ts) {
+  DevCounters* ctr = ts.d_ctr;
+  const int lane = threadIdx.x & 31;
+  const long long gt = blockIdx.x * (long long)blockDim.x + threadIdx.x, gn = (long long)gridDim.x * blockDim.x;
+  if (gt == 0) {
+    ctr->t_gr_start = jfc::global_ns();
+    ctr->bfs_status = 0;
+    ctr->wave_bar = ctr->wave_q = 0;
+  }
+  for (long long i = gt; i < ts.ngrids; i += gn) ts.d_grid_active[i] = 0;
+  for (long long i = gt; i < ts.nreg; i += gn) ts.d_rflag[0][i] = ts.d_rflag[1][i] = 0;
+  const long long nitems = ts.pr_split ? 2ll * ts.ntiles : ts.ntiles;
+  for (long long i = gt; i < nitems; i += gn) ts.d_flag_pr[i] = 0;
+  for (long long t0 = gt - lane; t0 < ts.ntiles; t0 += gn) {
+    unsigned todo = __ballot_sync(FULL, t0 + lane < ts.ntiles && ts.d_dirty[t0 + lane] != 0);
+    while (todo) {
+      const long long tid = t0 + __ffs(todo) - 1;
+      todo &= todo - 1;
+      const int4 ti = ts.d_info[tid];
+      const GridDev& g = ts.d_desc[ti.x];
+      const long long pitch = g.pitch;
+      const int y0 = ti.z * TY;
+      const long long n0 = (long long)ti.y * 32 + lane + (long long)y0 * pitch;
+      int e[TY], r[4][TY];
+#pragma unroll
+      for (int i = 0; i < TY; ++i) {
+        const long long n = n0 + i * pitch;
+        e[i] = g.e[n];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) r[k][i] = g.r[k][n];
+      }
+      uint4 arcs = make_uint4(0, 0, 0, 0), sign = make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int i = 0; i < TY; ++i) {
+        const unsigned xp = __ballot_sync(FULL, r[0][i] > 0), yp = __ballot_sync(FULL, r[1][i] > 0);
+        const unsigned ym = __ballot_sync(FULL, r[2][i] > 0), xm = __ballot_sync(FULL, r[3][i] > 0);
+        const unsigned neg = __ballot_sync(FULL, e[i] < 0), pos = __ballot_sync(FULL, e[i] > 0);
+        if (lane == i) {
+          arcs = make_uint4(xp, yp, ym, xm);
+          sign = make_uint4(0, 0, neg, pos);
+        }
+        g.h[n0 + i * pitch] = e[i] < 0 ? 0 : JFC_INF;
+      }
+      if (lane < TY) {
+        uint4* w = reinterpret_cast<uint4*>(seg_words(g, y0 + lane, ti.y));
+        w[0] = arcs;
+        w[1] = sign;
+        ts.d_vf[(long long)g.tile_base * TY + (long long)(y0 + lane) * g.tiles_x + ti.y] = make_uint4(0, 0, 0, 0);
+      }
+      if (lane == 0) ts.d_dirty[tid] = 0;
+    }
+  }
+}
+
+// Grid barrier of the relabel: one counter that only grows (zeroed by
+// k_wave_bits), so an arrival is also the release and nothing is reset; its
+// high bits count the CTAs that flagged a region for the next phase, which
+// makes "is there a next phase" part of the same poll.  (A CTA that sees
+// arrivals of the phase after it sees them because that phase exists.)
+// Bounded like jfc::grid_sync.  Returns -1 on error, else whether any region
+// was flagged since `seen` (updated).
+constexpr int kArriveBits = 40;   // low bits of the counter: arrivals; the rest: CTAs that flagged
+__device__ __forceinline__ int wave_sync(DevCounters* ctr, unsigned long long target, bool any, unsigned& seen) {
+  __shared__ int s_res;
+  __shared__ unsigned s_seen;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(&ctr->wave_bar, 1ull + (any ? 1ull << kArriveBits : 0ull));
+    unsigned long long spins = 0, v;
+    const unsigned long long cap = jfc::spin_cap(ctr);
+    int res = 0;
+    while (((v = *(volatile unsigned long long*)&ctr->wave_bar) & ((1ull << kArriveBits) - 1)) < target) {
+      if (jfc::vload(&ctr->error)) { res = -1; break; }
+      if (++spins > cap) { atomicExch(&ctr->error, 1); res = -1; break; }
+      if (spins > 16) __nanosleep(40);
+    }
+    __threadfence();
+    if (res == 0) {
+      res = (unsigned)(v >> kArriveBits) != seen;
+      s_seen = (unsigned)(v >> kArriveBits);
+    }
+    s_res = res;
+  }
+  __syncthreads();
+  if (s_res > 0) seen = s_seen;
+  return s_res;
+}
+
+// What a phase writes to the height plane for one row word.
+struct alignas(16) RowOut {
+  unsigned got;    // nodes that got a distance (until the levels are done: that had one)
+  unsigned gone;   // nodes set back to INF
+  unsigned p[5];   // level within the phase, bit by bit
+  unsigned pad;
+};
+
+// State of the level sets between phases, per row word: ts.d_vf = {V0, F0, V1,
+// F1}, two buffers of (nodes with a distance, nodes of the last level).  A
+// region rewrites the buffer that its record does not name and then names it,
+// with the phase: {phase << 1 | buffer}.  A neighbour that reads the record in
+// the same phase takes the other buffer, so all of a phase reads the state as
+// the phase before left it.
+//
+// A thread holds 4 rows of one word column, a warp 16 rows x 8 words.  A level
+// needs from elsewhere only edge bits (left and right words: the edge bytes of
+// 4 rows packed into one shuffle each way) and edge rows (two shuffles, and
+// shared memory between warps, every lane loading and storing some word so
+// that no lane diverges): 6 accesses of the shared-memory pipe a warp and
+// level.  The level of a node is kept as 5 bits in 5 words (P), updated two
+// bits a level and three bits every four levels.  Measured per level with one
+// CTA on an SM / four: 335 / 400 cycles, a chain of dependent word operations;
+// whole words exchanged through shared memory 510 / 607, diverging edge lanes
+// 590 / 680.
+template <int TY>
+__global__ void __launch_bounds__(kThreads, 4) k_wave_relabel(TileSet ts) {
+  __shared__ RowOut s_out[kIR * kIW];
+  __shared__ unsigned s_edge[2 * 256];                 // two buffers; see aout
+  __shared__ int s_list[kList];
+  __shared__ int4 s_reg[kList];
+  __shared__ int s_n;
+  __shared__ unsigned s_mask, s_new[2], s_tiles;
+  __shared__ unsigned long long s_base;
+  DevCounters* ctr = ts.d_ctr;
+  const unsigned long long t1 = jfc::global_ns();
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int c = t & (kC - 1), s = t >> 3, ws = s & 3;   // word column, strip of 4 rows, strip within the warp
+  const bool inner = c >= 1 && c <= kIW && s >= kT / 4 && s < (kT + kIR) / 4;
+  // edge words of a buffer: [warp + 1][first / last row][word column], zeros
+  // around them; from word 192 on, what lanes without an edge store
+  for (int i = t; i < 2 * 256; i += kThreads) s_edge[i] = 0;
+  const int ain = ws == 0 ? (2 * warp + 1) * kC + c : ws == 3 ? 2 * (warp + 2) * kC + c : 0;
+  const int aout = ws == 0 ? 2 * (warp + 1) * kC + c : ws == 3 ? (2 * (warp + 1) + 1) * kC + c : 192 + lane;
+  const unsigned ml = c == 0 ? 0u : ~0u, mr = c == kC - 1 ? 0u : ~0u;
+  RowOut* const mine = &s_out[inner ? (4 * (s - kT / 4)) * kIW + c - 1 : 0];   // (interior) rows kIW apart
+  unsigned long long visits = 0;
+  unsigned seen = 0;
+  int phase = 1;
+  for (;; ++phase) {
+    const bool first = phase == 1;
+    bool any_next = false;   // (thread 0) this CTA flagged a region for the next phase
+    for (int base = blockIdx.x; base < ts.nreg; base += gridDim.x * kList) {
+      // this CTA's regions of the phase (every gridDim-th, so neighbours fall
+      // to different CTAs): all in the first phase, then the flagged ones
+      if (t == 0) s_n = 0;
+      __syncthreads();
+      const long long cand = base + (long long)t * gridDim.x;
+      if (t < kList && cand < ts.nreg) {
+        const int4 ri = ts.d_reg[cand];   // (with the flag, not after it)
+        bool take = first;
+        if (!first && __ldcg(ts.d_rflag[phase & 1] + cand)) {
+          ts.d_rflag[phase & 1][cand] = 0;
+          take = true;
+        }
+        if (take) {
+          const int k = atomicAdd(&s_n, 1);
+          s_list[k] = (int)cand;
+          s_reg[k] = ri;
+        }
+      }
+      __syncthreads();
+      const int count = s_n;
+      for (int q = 0; q < count; ++q) {
+        const int reg = s_list[q];
+        const int4 ri = s_reg[q];   // {grid, region x, region y, first region of the grid}
+        const GridDev& g = ts.d_desc[ri.x];
+        const int cap = jfc::cap_of(g, ctr);
+        const int level0 = (phase - 1) * kT;   // the state holds distances up to here
+        const int rx = (g.tiles_x + kIW - 1) / kIW, ry = (g.Hp + kIR - 1) / kIR;
+        const int wc = ri.y * kIW - 1 + c, y0 = ri.z * kIR - kT + 4 * s;
+        const bool ok = wc >= 0 && wc < g.tiles_x && y0 >= 0 && y0 < g.Hp;   // (Hp is a multiple of 16)
+        const long long rw = (long long)g.tile_base * TY + (long long)y0 * g.tiles_x + wc;
+        if (t == 0) { s_mask = 0; s_new[0] = s_new[1] = 0; s_tiles = 0; }
+        // ---- load
+        uint4 arc[4];
+        unsigned V[4], F[4];
+        const unsigned own = __ldcg(ts.d_rrec + reg) & 1u;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          arc[i] = make_uint4(0, 0, 0, 0);
+          V[i] = F[i] = 0;
+        }
+        if (ok) {
+          unsigned rec = 0;
+          if (!first) {
+            const int dx = c == 0 ? -1 : c > kIW ? 1 : 0, dy = s < kT / 4 ? -1 : s >= (kT + kIR) / 4 ? 1 : 0;
+            rec = __ldcg(ts.d_rrec + ri.w + (ri.z + dy) * rx + ri.y + dx);
+          }
+          uint4 vf[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const uint32_t* w = seg_words(g, y0 + i, wc);
+            arc[i] = *reinterpret_cast<const uint4*>(w);
+            if (first) V[i] = w[6];
+            if (!first || inner) vf[i] = __ldcg(ts.d_vf + rw + (long long)i * g.tiles_x);
+          }
+          const bool second = ((rec & 1u) ^ ((int)(rec >> 1) == phase ? 1u : 0u)) != 0u;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (first) {
+              F[i] = V[i];
+              if (inner) mine[i * kIW].gone = own ? vf[i].z : vf[i].x;   // had a distance after the last relabel
+            } else {
+              V[i] = second ? vf[i].z : vf[i].x;
+              F[i] = second ? vf[i].w : vf[i].y;
+            }
+          }
+        }
+        if (inner) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) mine[i * kIW].got = V[i];
+        }
+        // ---- levels
+        unsigned P[5][4];
+#pragma unroll
+        for (int b = 0; b < 5; ++b)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) P[b][i] = 0;
+        s_edge[aout] = ws < 2 ? F[0] : F[3];
+        __syncthreads();
+        const int dmax = min(kT, cap - 1 - level0);
+#pragma unroll 1
+        for (int d = 0; d < dmax; d += 4) {
+          unsigned VG[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) VG[i] = V[i];
+          unsigned any = 0;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int bo = (j & 1) << 8;
+            const unsigned lim = d + j < dmax ? ~0u : 0u;   // (levels past the cap find nothing)
+            const unsigned edge = s_edge[bo + ain];
+            unsigned up = __shfl_up_sync(FULL, F[3], 8), dn = __shfl_down_sync(FULL, F[0], 8);
+            // the lowest bytes of the right words' rows, the highest of the left words'
+            const unsigned lo = __byte_perm(__byte_perm(F[0], F[1], 0x0040), __byte_perm(F[2], F[3], 0x0040), 0x5410);
+            const unsigned hi = __byte_perm(__byte_perm(F[0], F[1], 0x0073), __byte_perm(F[2], F[3], 0x0073), 0x5410);
+            const unsigned rb = __shfl_down_sync(FULL, lo, 1) & mr, lb = __shfl_up_sync(FULL, hi, 1) & ml;
+            up = ws == 0 ? edge : up;
+            dn = ws == 3 ? edge : dn;
+            unsigned N[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              unsigned m = __funnelshift_r(F[i], rb >> (8 * i), 1) & arc[i].x;
+              m |= __funnelshift_l(lb << (24 - 8 * i), F[i], 1) & arc[i].w;
+              m |= (i < 3 ? F[i < 3 ? i + 1 : 3] : dn) & arc[i].y;
+              m |= (i > 0 ? F[i > 0 ? i - 1 : 0] : up) & arc[i].z;
+              N[i] = m & ~V[i] & lim;
+            }
+            s_edge[(bo ^ 256) + aout] = ws < 2 ? N[0] : N[3];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              F[i] = N[i];
+              V[i] |= N[i];
+              if (j & 1) P[0][i] |= N[i];
+              if (j & 2) P[1][i] |= N[i];
+            }
+            any = N[0] | N[1] | N[2] | N[3];
+            if (j < 3) __syncthreads();
+          }
+#pragma unroll
+          for (int b = 0; b < 3; ++b) {
+            const unsigned bit = 0u - ((unsigned)(d >> (2 + b)) & 1u);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) P[2 + b][i] |= V[i] & ~VG[i] & bit;
+          }
+          // (the reducing barrier takes 60 cycles more than the plain one)
+          if (!__syncthreads_or(any)) break;
+        }
+        // ---- heights of the nodes that got a distance, INF where the last
+        //      relabel left one that this phase does not renew (a later phase
+        //      may): a warp takes 4 row words at a time, a lane 4 columns
+        unsigned pos[4] = {0, 0, 0, 0};
+        unsigned got[4] = {0, 0, 0, 0};
+        if (inner) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (ok) pos[i] = seg_words(g, y0 + i, wc)[7];
+            RowOut o;
+            got[i] = o.got = V[i] & ~mine[i * kIW].got;
+            o.gone = first && ok ? mine[i * kIW].gone & ~V[i] : 0u;
+#pragma unroll
+            for (int b = 0; b < 5; ++b) o.p[b] = P[b][i];
+            o.pad = 0;
+            mine[i * kIW] = o;
+          }
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int k0 = 4 * warp; k0 < kIR * kIW; k0 += 4 * (kThreads / 32)) {
+          const int k = k0 + (lane >> 3), sh = 4 * (lane & 7);
+          const RowOut o = s_out[k];
+          const unsigned gn = (o.got >> sh) & 15u, zn = (o.gone >> sh) & 15u;
+          if (!__any_sync(FULL, (gn | zn) != 0u)) continue;
+          unsigned v = 0;   // the 4 columns' levels, a byte each
+#pragma unroll
+          for (int b = 0; b < 5; ++b) v |= ((((o.p[b] >> sh) & 15u) * 0x00204081u) & 0x01010101u) << b;
+          int* h = g.h + (long long)(ri.z * kIR + k / kIW) * g.pitch + (ri.y * kIW + k % kIW) * 32 + sh;
+          const int l1 = level0 + 1;
+          const int4 w = make_int4(l1 + (int)(v & 255u), l1 + (int)((v >> 8) & 255u), l1 + (int)((v >> 16) & 255u),
+                                   l1 + (int)(v >> 24));
+          if (gn == 15u) {
+            *reinterpret_cast<int4*>(h) = w;
+          } else if (gn | zn) {
+            if ((gn | zn) & 1u) h[0] = gn & 1u ? w.x : JFC_INF;
+            if ((gn | zn) & 2u) h[1] = gn & 2u ? w.y : JFC_INF;
+            if ((gn | zn) & 4u) h[2] = gn & 4u ? w.z : JFC_INF;
+            if ((gn | zn) & 8u) h[3] = gn & 8u ? w.w : JFC_INF;
+          }
+        }
+        // ---- the state, and the tiles (push-relabel items) that became active
+        const bool had = !first && ((pos[0] & V[0] & ~got[0]) | (pos[1] & V[1] & ~got[1]) | (pos[2] & V[2] & ~got[2]) |
+                                    (pos[3] & V[3] & ~got[3])) != 0u;
+        const bool has = ((pos[0] & V[0]) | (pos[1] & V[1]) | (pos[2] & V[2]) | (pos[3] & V[3])) != 0u;
+        if (inner && ok) {
+          uint2* vf = reinterpret_cast<uint2*>(ts.d_vf + rw) + (own ^ 1u);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) vf[2ll * i * g.tiles_x] = make_uint2(V[i], F[i]);
+        }
+        const unsigned bh = __ballot_sync(FULL, inner && had), bn = __ballot_sync(FULL, inner && has);
+        // an item is 2 strips (8 rows), or 4 for whole 32 x 16 tiles
+        const bool halves = TY == 8 || ts.pr_split;
+        const unsigned whole = 0x01010101u << c, im = halves ? 0x101u << (lane & 23) : whole;
+        const bool item_new = inner && ok && (s & (halves ? 1 : 3)) == 0 && (bn & im) && !(bh & im);
+        const bool tile_new = TY == 8 ? item_new : inner && ok && ws == 0 && (bn & whole) && !(bh & whole);
+        const int par = halves ? (wc + (y0 >> 3)) & 1 : (wc + (y0 >> 4)) & 1;
+        int item = -1;
+        if (item_new) {
+          item = g.tile_base + y0 / TY * g.tiles_x + wc;
+          if (TY == 16 && halves) item = 2 * item + ((y0 >> 3) & 1);
+        }
+        const unsigned b0 = __ballot_sync(FULL, item >= 0 && par == 0), b1 = __ballot_sync(FULL, item >= 0 && par == 1);
+        const unsigned bt = __ballot_sync(FULL, tile_new);
+        unsigned slot0 = 0, slot1 = 0;
+        if (lane == 0) {
+          if (b0) slot0 = atomicAdd(&s_new[0], __popc(b0));
+          if (b1) slot1 = atomicAdd(&s_new[1], __popc(b1));
+          if (bt) atomicAdd(&s_tiles, __popc(bt));
+        }
+        slot0 = __shfl_sync(FULL, slot0, 0) + __popc(b0 & ((1u << lane) - 1u));
+        slot1 = __shfl_sync(FULL, slot1, 0) + __popc(b1 & ((1u << lane) - 1u));
+        // ---- regions that the last level reaches within the next phase
+        unsigned mask = 0;
+        if (inner && ok && cap - 1 > level0 + kT && (F[0] | F[1] | F[2] | F[3])) {
+          const int si = s - kT / 4;
+          const unsigned row = (si < kT / 4 ? 1u : 0u) | 2u | (si >= (kIR - kT) / 4 ? 4u : 0u);
+          const unsigned col = (c == 1 ? 1u : 0u) | 2u | (c == kIW ? 4u : 0u);
+          mask = (row & 1u ? col : 0u) | (col << 3) | (row & 4u ? col << 6 : 0u);
+        }
+        mask = __reduce_or_sync(FULL, mask);
+        if (lane == 0 && mask) atomicOr(&s_mask, mask);
+        __syncthreads();
+        const unsigned new0 = s_new[0], new1 = s_new[1], reach = s_mask;
+        if (t == 0) {
+          if (new0 | new1) s_base = atomicAdd(&ctr->wave_q, (unsigned long long)new1 << 32 | new0);
+          if (s_tiles) atomicAdd(&ts.d_grid_active[ri.x], (int)s_tiles);
+          any_next |= reach != 0;
+          ts.d_rrec[reg] = (unsigned)phase << 1 | (own ^ 1u);
+        } else if (t >= 32 && t < 41 && (reach >> (t - 32) & 1u)) {
+          const int nx = ri.y + (t - 32) % 3 - 1, ny = ri.z + (t - 32) / 3 - 1;
+          if (nx >= 0 && nx < rx && ny >= 0 && ny < ry) ts.d_rflag[(phase + 1) & 1][ri.w + ny * rx + nx] = 1;
+        }
+        if (new0 | new1) {
+          __syncthreads();
+          if (item >= 0) {
+            ts.d_q_pr[par][0][(unsigned)(s_base >> (par ? 32 : 0)) + (par ? slot1 : slot0)] = item;
+            ts.d_flag_pr[item] = 1;
+          }
+        }
+        ++visits;
+        __syncthreads();   // the shared state is free for the next region
+      }
+    }
+    if (wave_sync(ctr, (unsigned long long)phase * gridDim.x, any_next, seen) <= 0) break;
+  }
+  if (t == 0) {
+    atomicAdd(&ctr->bfs_visits, visits * (unsigned long long)(kIR / TY * kIW));
+    if (blockIdx.x == 0) {
+      // (behind the last barrier: every append is counted)
+      const unsigned long long q = *(volatile unsigned long long*)&ctr->wave_q;
+      ctr->qn_pr[0][0] = (int)(unsigned)q;
+      ctr->qn_pr[1][0] = (int)(q >> 32);
+      ctr->qn_pr[0][1] = ctr->qn_pr[1][1] = 0;
+      ctr->cur_pr[0] = ctr->cur_pr[1] = 0;
+      ctr->bfs_passes = phase;
+      ctr->bfs_status = 1;
+      const unsigned long long t2 = jfc::global_ns();
+      ctr->ns_gr_first += t1 - ctr->t_gr_start;
+      ctr->ns_gr_frontier += t2 - t1;
+    }
+  }
+}
+
+template <int TY>
+cudaError_t wave_t(const TileSet& ts, cudaStream_t s) {
+  static int cache_bits[64] = {0}, cache[64] = {0};
+  const void* fn = (const void*)k_wave_relabel<TY>;
+  const int nb = persistent_blocks_cached(cache_bits, (const void*)k_wave_bits<TY>, 256);
+  const int need = (int)std::min<long long>(nb, (2ll * ts.ntiles + 255) / 256);
+  jfc_note_launch();
+  k_wave_bits<TY><<<need, 256, 0, s>>>(ts);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  // no more CTAs than regions: the grid barrier's cost grows with them
+  const int blocks = std::min(persistent_blocks_cached(cache, fn, kThreads), ts.nreg);
+  TileSet arg = ts;
+  void* params[] = {(void*)&arg};
+  jfc_note_launch();
+  return cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(kThreads), params, 0, s);
+}
+
+}  // namespace
+
+cudaError_t launch_wave_relabel(const TileSet& ts, cudaStream_t s) {
+  if (ts.ntiles <= 0) return cudaSuccess;
+  if (ts.TR == 8) return wave_t<8>(ts, s);
+  if (ts.TR == 16) return wave_t<16>(ts, s);
+  return cudaErrorInvalidValue;
+}

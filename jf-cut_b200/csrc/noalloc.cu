@@ -17,7 +17,7 @@
 //    16) is at most kMaxNodes = 524,288 nodes — e.g. 1024 x 512 or the
 //    600 x 450 / 640 x 480 images that ship with the reference; larger grids
 //    are rejected with JFC_ERR_INVALID_ARG;
-//  * the array (about 13.2 MB) is held by every GPU that loads the library,
+//  * the array (about 13.5 MB) is held by every GPU that loads the library,
 //    until the process exits;
 //  * every call shares the array and it keeps the last call's contents (the
 //    solve clears what must start at zero); calls that overlap on the GPU —
@@ -53,7 +53,16 @@ constexpr size_t kOffAct = kOffQBfs + 2 * kTileI;
 constexpr size_t kOffGact = kOffAct + al(kMaxTiles);
 constexpr size_t kOffSum = kOffGact + 256;
 constexpr size_t kOffCtr = kOffSum + 256;
-constexpr size_t kOffBad = kOffCtr + al(sizeof(DevCounters));
+// regions of the global relabel: the most a grid of kMaxNodes padded nodes has
+// (kMaxNodes / 32 row words; one column of regions 1 word wide, or one row of
+// regions 16 rows high)
+constexpr int kMaxReg = kMaxNodes / (32 * 16) / JFC_WAVE_WORDS + kMaxNodes / 32 / JFC_WAVE_ROWS + 2;
+constexpr size_t kOffDirty = kOffCtr + al(sizeof(DevCounters));
+constexpr size_t kOffVf = kOffDirty + al(kMaxTiles);
+constexpr size_t kOffReg = kOffVf + al(sizeof(uint4) * (size_t)(kMaxNodes / 32));
+constexpr size_t kOffRrec = kOffReg + al(sizeof(int4) * (size_t)kMaxReg);
+constexpr size_t kOffRflag = kOffRrec + al(sizeof(unsigned) * (size_t)kMaxReg);   // 2 flag arrays
+constexpr size_t kOffBad = kOffRflag + 2 * al(kMaxReg);
 constexpr size_t kBytes = kOffBad + 256;
 
 std::mutex g_mu;
@@ -70,6 +79,12 @@ struct DeviceGuard {
 __global__ void k_na_tile_info(int4* info, int tiles_x, int ntiles) {
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += gridDim.x * blockDim.x)
     info[t] = make_int4(0, t % tiles_x, t / tiles_x, 0);
+}
+
+// region k of a single grid of rx regions a row: {grid 0, x, y, first region 0}
+__global__ void k_na_regions(int4* reg, int rx, int n) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
+    reg[k] = make_int4(0, k % rx, k / rx, 0);
 }
 
 }  // namespace
@@ -114,13 +129,14 @@ int na_read(void* host, const void* dev, size_t bytes, cudaStream_t s) {
 }
 
 int na_bfs(TileSet& ts, const jfc_params& p, bool cut, cudaStream_t s, int* active, int* cut_bad) {
-  JFC_CUDA(cudaMemsetAsync(ts.d_flag_bfs[0], 0, sizeof(int) * (size_t)ts.ntiles, s));
-  JFC_CUDA(cudaMemsetAsync(ts.d_flag_bfs[1], 0, sizeof(int) * (size_t)ts.ntiles, s));
-  if (!cut) JFC_CUDA(cudaMemsetAsync(ts.d_grid_active, 0, sizeof(int), s));
-  JFC_CUDA(cudaMemsetAsync(ts.d_ctr->ticket, 0, sizeof(ts.d_ctr->ticket), s));
-  JFC_CUDA(cudaMemsetAsync(ts.d_ctr->qn_bfs, 0, sizeof(ts.d_ctr->qn_bfs), s));
-  JFC_CUDA(cudaMemsetAsync(&ts.d_ctr->bfs_status, 0, sizeof(int), s));
-  if (cut) JFC_CUDA(cudaMemsetAsync(&ts.d_ctr->cut_bad, 0, sizeof(int), s));
+  if (cut) {
+    JFC_CUDA(cudaMemsetAsync(ts.d_flag_bfs[0], 0, sizeof(int) * (size_t)ts.ntiles, s));
+    JFC_CUDA(cudaMemsetAsync(ts.d_flag_bfs[1], 0, sizeof(int) * (size_t)ts.ntiles, s));
+    JFC_CUDA(cudaMemsetAsync(ts.d_ctr->ticket, 0, sizeof(ts.d_ctr->ticket), s));
+    JFC_CUDA(cudaMemsetAsync(ts.d_ctr->qn_bfs, 0, sizeof(ts.d_ctr->qn_bfs), s));
+    JFC_CUDA(cudaMemsetAsync(&ts.d_ctr->bfs_status, 0, sizeof(int), s));
+    JFC_CUDA(cudaMemsetAsync(&ts.d_ctr->cut_bad, 0, sizeof(int), s));
+  }
   JFC_CUDA(launch_bfs(ts, cut, p.max_bfs_passes, s));
   DevCounters hc;
   int rc = na_read(&hc, ts.d_ctr, sizeof(hc), s);
@@ -197,6 +213,13 @@ extern "C" int jfc_solve_grid2d_noalloc(int device, void* stream, const jfc_para
   ts.d_grid_active = (int*)(base + kOffGact);
   ts.d_grid_sum = (long long*)(base + kOffSum);
   ts.d_ctr = (DevCounters*)(base + kOffCtr);
+  ts.nreg = wave_regions(g.tiles_x, Hp);
+  ts.d_dirty = (uint8_t*)(base + kOffDirty);
+  ts.d_vf = (uint4*)(base + kOffVf);
+  ts.d_reg = (int4*)(base + kOffReg);
+  ts.d_rrec = (unsigned*)(base + kOffRrec);
+  ts.d_rflag[0] = (uint8_t*)(base + kOffRflag);
+  ts.d_rflag[1] = (uint8_t*)(base + kOffRflag + al(kMaxReg));
   int* d_bad = (int*)(base + kOffBad);
 
   // ---- stage the graph: clear the planes in use, copy the caller's arrays in,
@@ -211,6 +234,9 @@ extern "C" int jfc_solve_grid2d_noalloc(int device, void* stream, const jfc_para
   JFC_CUDA(cudaMemcpyAsync(ts.d_desc, &g, sizeof(g), cudaMemcpyHostToDevice, s));
   jfc_note_launch();
   k_na_tile_info<<<(ts.ntiles + 255) / 256, 256, 0, s>>>(ts.d_info, g.tiles_x, ts.ntiles);
+  JFC_CUDA(cudaGetLastError());
+  jfc_note_launch();
+  k_na_regions<<<(ts.nreg + 255) / 256, 256, 0, s>>>(ts.d_reg, (g.tiles_x + JFC_WAVE_WORDS - 1) / JFC_WAVE_WORDS, ts.nreg);
   JFC_CUDA(cudaGetLastError());
   int bad = 0;
   rc = na_read(&bad, d_bad, sizeof(int), s);
