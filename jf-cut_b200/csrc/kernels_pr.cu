@@ -9,17 +9,16 @@
 //
 // B200 design:
 //  * one CTA per tile of 32 x TY (x TZ) nodes, one thread per node, one warp per
-//    tile row (128-byte coalesced row loads / stores); excess, heights (with
-//    the halo) and residual arcs live in shared memory for the visit.  With 2D
-//    32 x 16 relabel tiles the visits work on their 32 x 8 halves (SPLIT),
-//    which keep a checkerboard parity of their own;
+//    tile row (128-byte coalesced row loads / stores); a node's excess, height
+//    and residual arcs live in its thread's registers for the visit, heights
+//    (with the halo) in shared memory too.  With 2D 32 x 16 relabel tiles the
+//    visits work on their 32 x 8 halves (SPLIT), which keep a checkerboard
+//    parity of their own;
 //  * a round = one relabel step and one push step for all nodes at once
-//    (two block barriers per round):
-//    under a fixed height vector two neighbours never push to each other, so a
-//    node's own arcs are only written by itself, the reverse arc of a push only
-//    by the pusher, and excess arrives through shared-memory atomics;
+//    (two block barriers per round): each node computes its pushes and
+//    gathers its neighbours';
 //  * rounds repeat until a round moves nothing (__syncthreads_or) or
-//    `local_iters` rounds ran; the visit then writes back only words that
+//    `local_iters` rounds ran; the visit then writes back only the sectors that
 //    changed and sends the flow pushed across the border with global atomics;
 //  * persistent cooperative launch: `sweeps` x (even tiles, odd tiles) with a
 //    grid barrier between parities; each parity drains a compact device queue
@@ -50,10 +49,9 @@ using Tile = jfc::CtaTile<DIMS, TY, TZ>;
 template <int DIMS, int TY, int TZ>
 using PrTile = jfc::CtaTile<DIMS, TY, TZ, 40, 4>;
 
-// Staging buffer of one visit, the working copy of the tile during it:
-// the tile's planes {e, h, r[0..K-1]} (plane-major, thread order) and the h
-// plane over the tile plus its one-cell halo.  The visit pushes and relabels
-// in place here.
+// Staging buffer of one visit:
+// the tile's planes {e, h, r[0..K-1]} (plane-major, thread order), as they were
+// when the visit began, and the h plane over the tile plus its one-cell halo.
 template <int DIMS, int TY, int TZ>
 struct alignas(128) PrStage {
   using T = PrTile<DIMS, TY, TZ>;
@@ -66,7 +64,7 @@ struct alignas(128) PrStage {
 template <int DIMS, int TY, int TZ>
 struct PrSmem {
   using T = PrTile<DIMS, TY, TZ>;
-  int out[T::NHALO];      // flow pushed into each halo cell during the visit
+  int d[2 * (T::D - 1)][T::NT];   // a round's pushes along +y, -y (, +z, -z)
   uint8_t arc[T::NT];     // residual-arc bits for the local relabel
   int tile;
   int buf;                // staging buffer of the item being visited
@@ -173,7 +171,6 @@ __device__ __forceinline__ int pr_visit(const TileSet& ts, int tid, int local_it
     const bool in = gx >= 0 && gx < pitch && gy >= 0 && gy < g.Hp && gz >= 0 && gz < g.Dp;
     if (!staged || !in)
       sh[T::hidx(hx, hy, hz)] = in ? g.h[(long long)gx + (long long)gy * pitch + (long long)gz * slab] : JFC_INF;
-    s.out[c] = 0;
   }
   if (t < 6) s.face[t] = 0;
   {
@@ -212,131 +209,127 @@ __device__ __forceinline__ int pr_visit(const TileSet& ts, int tid, int local_it
   __syncthreads();
   JFC_PCLK(ts.d_ctr, 1);
 
-  // in-tile neighbours, or the halo cell a push across the border lands in
-  const bool in_xp = x < 31, in_xm = x > 0, in_yp = y < TY - 1, in_ym = y > 0;
-  const bool in_zp = DIMS == 3 && z < TZ - 1, in_zm = DIMS == 3 && z > 0;
-  const int hc_xm = T::NHY + row, hc_xp = T::NHY + T::R + row;
-  const int hc_ym = z * 32 + x, hc_yp = TZ * 32 + z * 32 + x;
-  const int hc_zm = T::NHY + T::NHX + y * 32 + x, hc_zp = T::NHY + T::NHX + TY * 32 + y * 32 + x;
-
-  // push order: +x, +y, -y, (+z, -z,) -x; q is a constant after unrolling
-  constexpr int NP = DIMS == 3 ? 6 : 4;
-  auto slot = [](int q) { return q == 0 ? T::XP : q == 1 ? T::YP : q == 2 ? T::YM
-                                        : q == NP - 1 ? T::XM : q == 3 ? T::ZP : T::ZM; };
-  auto hoff = [](int q) { return q == 0 ? 1 : q == 1 ? T::HX : q == 2 ? -T::HX
-                                       : q == NP - 1 ? -1 : q == 3 ? T::HX * T::HY : -T::HX * T::HY; };
-  auto toff = [](int q) { return q == 0 ? 1 : q == 1 ? 32 : q == 2 ? -32
-                                       : q == NP - 1 ? -1 : q == 3 ? 32 * TY : -32 * TY; };
+  // Rounds, the node's excess, height and arcs in registers.  A push u -> v is
+  // computed by u and gathered by v: along x by shuffles (a warp holds a tile
+  // row), along y and z through s.d.  Under one height vector two neighbours
+  // never push to each other, so a node's arc changes by its own push or by
+  // its neighbour's.  Nothing diverges and nothing is atomic; a round is a
+  // chain of two block barriers and about 60 instructions per thread, 610-740
+  // cycles.  With the state in shared memory and the pushes as divergent
+  // shared-memory reductions a round took 1,000-1,230 cycles (push-relabel of
+  // a 15000 x 10000 solve 38.5 -> 33.4 ms, of a 2560 x 1440 x 50 video 60.9 ->
+  // 54.4 ms).
+  int e = e0, r[T::K], hn[T::K];
+#pragma unroll
+  for (int k = 0; k < T::K; ++k) r[k] = r0[k];
+  const int h_left = sh[hi - 1], h_right = sh[hi + 1];   // (halo cells for lanes 0 and 31)
+  auto heights = [&]() {
+    const int hr = __shfl_down_sync(FULL, hown, 1), hl = __shfl_up_sync(FULL, hown, 1);
+    hn[T::XP] = x == 31 ? h_right : hr;
+    hn[T::XM] = x == 0 ? h_left : hl;
+    hn[T::YP] = sh[hi + T::SY];
+    hn[T::YM] = sh[hi - T::SY];
+    if constexpr (DIMS == 3) {
+      hn[T::ZP] = sh[hi + T::SZ];
+      hn[T::ZM] = sh[hi - T::SZ];
+    }
+  };
+  heights();
+  // push order: +x, +y, -y, (+z, -z,) -x
+  constexpr int kOrder[6] = {T::XP, T::YP, T::YM, DIMS == 3 ? T::ZP : T::XM, T::ZM, T::XM};
+  constexpr int NP = T::K;
   int it = 0;
   for (; it < local_iters; ++it) {
-    bool did = false;
-    // the node's excess and residual arcs, read once per round: nothing
-    // changes them between the relabel step and the push step, and the
-    // credits neighbours add during the push step only raise them, so these
-    // values bound what the node may push from below
-    const int e = se[t];
+    // relabel every active node without an admissible arc
+    // (graphcut_push_relabel.cl:80-99 relabels two colours in turn): 1 + the
+    // lowest residual neighbour; heights only grow, so the labelling stays
+    // valid when neighbours do so at once
     const bool act = e > 0 && hown < JFC_INF;
-    int rk[NP];
-    // relabel every active node without an admissible arc, in place
-    // (graphcut_push_relabel.cl:80-99 relabels two colours in turn).  A node
-    // reading a neighbour that relabels in the same step sees its old or new
-    // height; heights only grow, so either value keeps the labelling valid.
-    if (act) {
-      int hn[NP];
+    bool adm = false;
+    int m = JFC_INF;
 #pragma unroll
-      for (int q = 0; q < NP; ++q) {
-        rk[q] = st.pl[2 + slot(q)][t];
-        hn[q] = sh[hi + hoff(q)];
-      }
-      const int hm = hown - 1;
-      bool adm = false;
-      int m = JFC_INF;
-#pragma unroll
-      for (int q = 0; q < NP; ++q) {
-        adm |= rk[q] > 0 && hn[q] == hm;
-        m = min(m, rk[q] > 0 ? hn[q] : JFC_INF);
-      }
-      if (!adm) {
-        hown = max(hown, min(m + 1, JFC_INF));
-        sh[hi] = hown;
-        did = true;
-      }
+    for (int k = 0; k < T::K; ++k) {
+      adm |= r[k] > 0 && hn[k] == hown - 1;
+      m = min(m, r[k] > 0 ? hn[k] : JFC_INF);
+    }
+    bool did = act && !adm;
+    if (did) {
+      hown = max(hown, min(m + 1, JFC_INF));
+      sh[hi] = hown;
     }
     __syncthreads();
-    // push: every node with excess, along admissible arcs in reference order.
-    // All operands are loaded first and the pushes are computed in registers,
-    // then issued as independent shared-memory updates: a push u->v needs
-    // h(u) = h(v) + 1, so in one step nothing else writes u's own arcs or the
-    // reverse arc v->u that u credits (the credits are reductions, no load).
-    {
-      if (act && hown < JFC_INF) {
-        const int hm = hown - 1;
-        const bool inside[6] = {in_xp, in_yp, in_ym, DIMS == 3 ? in_zp : in_xm, in_zm, in_xm};
-        const int hcell[6] = {hc_xp, hc_yp, hc_ym, DIMS == 3 ? hc_zp : hc_xm, hc_zm, hc_xm};
-        int hn[NP], d[NP];
+    heights();
+    // push along admissible arcs in the reference's order
+    int left = act && hown < JFC_INF ? e : 0, d[T::K];
 #pragma unroll
-        for (int q = 0; q < NP; ++q) hn[q] = sh[hi + hoff(q)];
-        int ex = e;
-#pragma unroll
-        for (int q = 0; q < NP; ++q) {
-          d[q] = (ex > 0 && rk[q] > 0 && hn[q] == hm) ? min(ex, rk[q]) : 0;
-          ex -= d[q];
-        }
-        if (ex != e) {
-#pragma unroll
-          for (int q = 0; q < NP; ++q) {
-            if (d[q]) {
-              st.pl[2 + slot(q)][t] = rk[q] - d[q];
-              if (inside[q == NP - 1 ? 5 : q]) {
-                atomicAdd(&se[t + toff(q)], d[q]);
-                atomicAdd(&st.pl[2 + T::K - 1 - slot(q)][t + toff(q)], d[q]);
-              } else {
-                s.out[hcell[q == NP - 1 ? 5 : q]] += d[q];
-              }
-            }
-          }
-          atomicAdd(&se[t], ex - e);
-          did = true;
-        }
-      }
+    for (int q = 0; q < NP; ++q) {
+      const int k = kOrder[q == NP - 1 ? 5 : q];
+      d[k] = hn[k] == hown - 1 ? min(left, r[k]) : 0;
+      left -= d[k];
     }
+    s.d[0][t] = d[T::YP];
+    s.d[1][t] = d[T::YM];
+    if constexpr (DIMS == 3) {
+      s.d[2][t] = d[T::ZP];
+      s.d[3][t] = d[T::ZM];
+    }
+    int in[T::K], out = 0;   // in[k]: pushed to this node by its neighbour in direction k
+    in[T::XP] = __shfl_down_sync(FULL, d[T::XM], 1);
+    in[T::XM] = __shfl_up_sync(FULL, d[T::XP], 1);
+    if (x == 31) in[T::XP] = 0;
+    if (x == 0) in[T::XM] = 0;
+#pragma unroll
+    for (int k = 0; k < T::K; ++k) out += d[k];
+    did |= out != 0;
     if (!__syncthreads_or(did)) break;
+    in[T::YP] = y < TY - 1 ? s.d[1][t + 32] : 0;
+    in[T::YM] = y > 0 ? s.d[0][t - 32] : 0;
+    if constexpr (DIMS == 3) {
+      in[T::ZP] = z < TZ - 1 ? s.d[3][t + 32 * TY] : 0;
+      in[T::ZM] = z > 0 ? s.d[2][t - 32 * TY] : 0;
+    }
+    e -= out;
+#pragma unroll
+    for (int k = 0; k < T::K; ++k) {
+      e += in[k];
+      r[k] += in[k] - d[k];
+    }
   }
   const int rounds = it < local_iters ? it + 1 : local_iters;
   JFC_PCLK(ts.d_ctr, 2);
 
-  // ---- write back: each row's 4-node groups holding a changed word, as
-  //      128-bit stores (nothing else writes the tile while it is visited, so
-  //      the unchanged words of a group are rewritten with their own values)
-  const int e1 = se[t], h1 = hown;
+  // ---- write back the 32-byte sectors of each row that hold a changed word
+  //      (nothing else writes the tile while it is visited, so the unchanged
+  //      words of a sector are rewritten with their own values)
+  const int e1 = e, h1 = hown;
   {
-    const long long nrow = n - x;
-    const int grp = x & ~3;
-    auto put = [&](int* gplane, const int* srow, bool changed) {
-      const unsigned m = __ballot_sync(jfc::FULL, changed);
-      if ((x & 3) == 0 && ((m >> grp) & 0xFu))
-        *reinterpret_cast<int4*>(gplane + nrow + grp) = *reinterpret_cast<const int4*>(srow + grp);
+    const int grp = x & ~7;
+    auto put = [&](int* gplane, int v, bool changed) {
+      if ((__ballot_sync(FULL, changed) >> grp) & 0xFFu) gplane[n] = v;
     };
-    put(g.e, se + row * 32, e1 != e0);
-    put(g.h, sh + T::hidx(0, y, z), h1 != h0);
+    put(g.e, e1, e1 != st.pl[0][t]);
+    put(g.h, h1, h1 != st.pl[1][t]);
 #pragma unroll
-    for (int k = 0; k < T::K; ++k) put(g.r[k], st.pl[2 + k] + row * 32, st.pl[2 + k][t] != r0[k]);
+    for (int k = 0; k < T::K; ++k) put(g.r[k], r[k], r[k] != st.pl[2 + k][t]);
   }
   // ---- send the flow pushed across the border into the neighbours' excess
-  //      and reverse arcs (only halo cells inside the grid can receive flow:
-  //      arcs leaving the grid are zero)
-  for (int c = t; c < T::NHALO; c += T::NT) {
-    const int v = s.out[c];
+  //      and reverse arcs: what a border arc lost (arcs leaving the grid are
+  //      zero, so only neighbours inside it can receive flow)
+  auto send = [&](bool border, int k, int face, long long off) {
+    const int v = border ? st.pl[2 + k][t] - r[k] : 0;
     if (v) {
-      int hx, hy, hz, f;
-      halo_cell<DIMS, TY, TZ>(c, hx, hy, hz, f);
-      const long long m = tbase + hx + (long long)hy * pitch + (long long)hz * slab;
-      // the halo node's arc pointing back into the tile
-      const int rev = f == 0 ? T::XP : f == 1 ? T::XM : f == 2 ? T::YP : f == 3 ? T::YM : f == 4 ? T::ZP : T::ZM;
-      atomicAdd(g.e + m, v);
-      atomicAdd(g.r[rev] + m, v);
-      s.face[f] = 1;
+      atomicAdd(g.e + n + off, v);
+      atomicAdd(g.r[T::K - 1 - k] + n + off, v);
+      s.face[face] = 1;
     }
+  };
+  send(x == 0, T::XM, 0, -1);
+  send(x == 31, T::XP, 1, 1);
+  send(y == 0, T::YM, 2, -(long long)pitch);
+  send(y == TY - 1, T::YP, 3, pitch);
+  if constexpr (DIMS == 3) {
+    send(z == 0, T::ZM, 4, -slab);
+    send(z == TZ - 1, T::ZP, 5, slab);
   }
   const bool active = __syncthreads_or((e1 > 0) & (h1 < JFC_INF));
   // flow crossed face f only toward an item inside the grid (arcs leaving
