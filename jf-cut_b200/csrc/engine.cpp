@@ -468,10 +468,9 @@ void tileset_drop_graphs(TileSet& ts) {
 
 static cudaError_t enqueue_cycle(TileSet& ts, const int* pin_sw, int local_iters, int max_passes, int sched,
                                  cudaStream_t s, void* pin) {
-  cudaError_t e = cudaMemsetAsync(ts.d_ctr->ticket, 0, sizeof(ts.d_ctr->ticket), s);
   static_assert(offsetof(DevCounters, h_cap) == offsetof(DevCounters, pr_sweeps) + sizeof(int),
                 "pr_sweeps and h_cap are copied together");
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&ts.d_ctr->pr_sweeps, pin_sw, 2 * sizeof(int), cudaMemcpyHostToDevice, s);
+  cudaError_t e = cudaMemcpyAsync(&ts.d_ctr->pr_sweeps, pin_sw, 2 * sizeof(int), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = launch_pr_phase(ts, 0, local_iters, s, sched);
   if (e == cudaSuccess) e = enqueue_bfs(ts, false, max_passes, s, pin);
   return e;

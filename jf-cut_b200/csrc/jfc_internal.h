@@ -48,6 +48,7 @@ struct GridDev {
 // Device-side control state of one tile set (persistent phase kernels).
 struct DevCounters {
   unsigned ticket[2];        // work tickets (alternate between phases)
+  unsigned long long pr_bar; // grid barrier of the push-relabel sweeps: arrivals
   unsigned bar_count;        // grid barrier arrivals
   unsigned bar_gen;          // grid barrier generation
   int error;                 // a barrier wait timed out: kernels leave, host reports
@@ -149,6 +150,7 @@ void jfc_note_launch(int n = 1);
 // serves every interval
 // sched 2: the asynchronous worklist (needs ts.d_pr_ring) instead of the
 // parity sweeps
+// (the launcher zeroes the phase's tickets and barrier counter first)
 cudaError_t launch_pr_phase(const TileSet& ts, int sweeps, int local_iters, cudaStream_t s, int sched = 1);
 // Local pre-push inside every tile before the first relabel of a solve.
 cudaError_t launch_prepush(const TileSet& ts, cudaStream_t s);

@@ -53,6 +53,31 @@ __device__ __forceinline__ bool grid_sync(DevCounters* ctr, F on_last) {
 
 __device__ __forceinline__ int vload(const int* p) { return *(const volatile int*)p; }
 
+// Grid barrier on a counter that only grows (zero at the kernel's start): an
+// arrival is also the release, so the waiting is one atomic and one poll, 1.6
+// us against 3 us of grid_sync with its generation word and its reset by the
+// last block.  `target`: blocks x barriers so far.  Bounded like grid_sync.
+__device__ __forceinline__ bool arrive_wait(DevCounters* ctr, unsigned long long* counter, unsigned long long target) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(counter, 1ull);
+    unsigned long long spins = 0;
+    const unsigned long long cap = spin_cap(ctr);
+    int ok = 1;
+    while (*(volatile unsigned long long*)counter < target) {
+      if (vload(&ctr->error)) { ok = 0; break; }
+      if (++spins > cap) { atomicExch(&ctr->error, 1); ok = 0; break; }
+      if (spins > 8) __nanosleep(64);
+    }
+    __threadfence();
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
 // Distance cap of the running global relabel: distances at or above it are
 // stored as unreachable (JFC_INF); no cap when ctr->h_cap is 0.
 // (set before the kernel that reads it runs, constant during it: an ordinary

@@ -67,6 +67,7 @@ struct PrSmem {
   int d[2 * (T::D - 1)][T::NT];   // a round's pushes along +y, -y (, +z, -z)
   unsigned run[2 * (T::D - 1)][T::R];   // (local relabel) per tile row: nodes with a residual arc +y, -y (, +z, -z)
   int tile;
+  int4 ti;                // its tile: {grid, x, y, z}
   int buf;                // staging buffer of the item being visited
   int gen;                // worklist: generation of the item being visited
   int face[6];            // any flow left through face: x-, x+, y-, y+, z-, z+
@@ -82,12 +83,23 @@ __device__ __forceinline__ void halo_cell(int c, int& x, int& y, int& z, int& fa
 // SPLIT: the work item `tid` is half `tid & 1` (rows 0-7 / 8-15) of the 2D
 // 32x16 tile `tid >> 1`, visited as a 32x8 tile; the halves keep their own
 // checkerboard parity, so the two halves of a tile never run at once.
-// The work items behind the faces of item `tid` (x-, x+, y-, y+, z-, z+),
-// -1 where the face is the grid's border.
+// Coordinates of work item `tid`: {grid, tile x, y, z} of its tile.  A set of
+// one grid computes them (a table look-up is a round trip to L2 in front of
+// the copies of the tile).
+template <bool SPLIT>
+__device__ __forceinline__ int4 item_tile(const TileSet& ts, int tid) {
+  const int tile = SPLIT ? tid >> 1 : tid;
+  if (ts.ngrids != 1) return ts.d_info[tile];
+  const GridDev& g = ts.d_desc[0];
+  const unsigned row = (unsigned)tile / (unsigned)g.tiles_x;
+  return make_int4(0, tile - (int)row * g.tiles_x, (int)(row % (unsigned)g.tiles_y), (int)(row / (unsigned)g.tiles_y));
+}
+
+// The work item behind face f of item `tid` (x-, x+, y-, y+, z-, z+; ti: its
+// tile), -1 where the face is the grid's border.
 template <int DIMS, int TY, int TZ, bool SPLIT>
-__device__ __forceinline__ int face_item(const TileSet& ts, int tid, int f) {
+__device__ __forceinline__ int face_item(const TileSet& ts, int tid, const int4& ti, int f) {
   const int tile = SPLIT ? tid >> 1 : tid, half = SPLIT ? tid & 1 : 0;
-  const int4 ti = ts.d_info[tile];
   const GridDev& g = ts.d_desc[ti.x];
   const int txs = g.tiles_x, tys = g.tiles_y, tzs = g.tiles_z;
   switch (f) {
@@ -102,11 +114,10 @@ __device__ __forceinline__ int face_item(const TileSet& ts, int tid, int f) {
   }
 }
 
-// Tile origin of work item `tid` (elements) and its grid.
+// Grid and origin (elements) of work item `tid` in tile ti.
 template <int DIMS, int TY, int TZ, bool SPLIT>
-__device__ __forceinline__ int4 item_origin(const TileSet& ts, int tid) {
-  const int tile = SPLIT ? tid >> 1 : tid, half = SPLIT ? tid & 1 : 0;
-  const int4 ti = ts.d_info[tile];
+__device__ __forceinline__ int4 item_origin(int tid, const int4& ti) {
+  const int half = SPLIT ? tid & 1 : 0;
   return make_int4(ti.x, ti.y * 32, SPLIT ? (2 * ti.z + half) * TY : ti.z * TY, ti.w * TZ);
 }
 
@@ -115,9 +126,9 @@ __device__ __forceinline__ int4 item_origin(const TileSet& ts, int tid) {
 // `bar`.  Issued by one thread.  Box cells outside the grid arrive as zeros;
 // the visit sets the halo ones to INF.
 template <int DIMS, int TY, int TZ, bool SPLIT>
-__device__ __forceinline__ void pr_stage_issue(const TileSet& ts, int tid, PrStage<DIMS, TY, TZ>& st, uint64_t* bar,
-                                               int& acquired_grid) {
-  const int4 o = item_origin<DIMS, TY, TZ, SPLIT>(ts, tid);
+__device__ __forceinline__ void pr_stage_issue(const TileSet& ts, int tid, const int4& ti, PrStage<DIMS, TY, TZ>& st,
+                                               uint64_t* bar, int& acquired_grid) {
+  const int4 o = item_origin<DIMS, TY, TZ, SPLIT>(tid, ti);
   const char* maps = (const char*)ts.d_tmap + (size_t)o.x * 384;   // three maps per grid
   if (o.x != acquired_grid) {
     jfc::fence_tmap_acquire(maps);
@@ -229,18 +240,20 @@ __device__ __forceinline__ bool local_distance(Smem& s, const int* sh, int hi, c
   return false;
 }
 
-// One visit of work item `tid` on staging buffer `st`; staged: the tensor
-// copies already filled it, otherwise the visit loads the tile itself.  On
+// One visit of work item `tid` (in tile ti) on staging buffer `st`; staged: the
+// tensor copies already filled it, otherwise the visit loads the tile itself.
+// failed: a staging copy never completed for this thread; the visit then
+// returns -1 to every thread of the CTA and changes nothing.  On
 // return s.active tells whether the item still holds an active node and
 // s.q_nb[f] the item behind each face f that received flow (-1: none).  The
 // caller queues them.
 template <int DIMS, int TY, int TZ, bool SPLIT>
-__device__ __forceinline__ int pr_visit(const TileSet& ts, int tid, int local_iters, bool local_relabel,
-                                        PrSmem<DIMS, TY, TZ>& s, PrStage<DIMS, TY, TZ>& st, bool staged) {
+__device__ __forceinline__ int pr_visit(const TileSet& ts, int tid, const int4& ti, int local_iters, bool local_relabel,
+                                        PrSmem<DIMS, TY, TZ>& s, PrStage<DIMS, TY, TZ>& st, bool staged, bool failed) {
   using T = PrTile<DIMS, TY, TZ>;
   const int t = threadIdx.x;
   const int x = t & 31, row = t >> 5, y = row % TY, z = row / TY;
-  const int4 o = item_origin<DIMS, TY, TZ, SPLIT>(ts, tid);
+  const int4 o = item_origin<DIMS, TY, TZ, SPLIT>(tid, ti);
   const GridDev& g = ts.d_desc[o.x];
   const int pitch = g.pitch;
   const long long slab = (long long)g.pitch * g.Hp;
@@ -248,7 +261,6 @@ __device__ __forceinline__ int pr_visit(const TileSet& ts, int tid, int local_it
   const long long tbase = (long long)x0 + (long long)y0 * pitch + (long long)z0 * slab;
   const long long n = tbase + x + (long long)y * pitch + (long long)z * slab;
   const int hi = T::hidx(x, y, z);
-  int* const se = st.pl[0];
   int* const sh = st.hb;
   JFC_PCLK_DECL
 
@@ -272,7 +284,7 @@ __device__ __forceinline__ int pr_visit(const TileSet& ts, int tid, int local_it
       sh[T::hidx(hx, hy, hz)] = in ? g.h[(long long)gx + (long long)gy * pitch + (long long)gz * slab] : JFC_INF;
   }
   if (t < 6) s.face[t] = 0;
-  __syncthreads();
+  if (__syncthreads_or(failed)) return -1;
   JFC_PCLK(ts.d_ctr, 0);
   // the node's own height lives in a register (only its owner writes it); the
   // shared copy is what the neighbours read
@@ -421,7 +433,7 @@ __device__ __forceinline__ int pr_visit(const TileSet& ts, int tid, int local_it
   // flow crossed face f only toward an item inside the grid (arcs leaving
   // the grid are zero)
   if (t < 6) {
-    const int nb = s.face[t] ? face_item<DIMS, TY, TZ, SPLIT>(ts, tid, t) : -1;
+    const int nb = s.face[t] ? face_item<DIMS, TY, TZ, SPLIT>(ts, tid, ti, t) : -1;
     s.q_nb[t] = nb;
     // the global relabel reads the arcs and signs of these tiles again
     if (nb >= 0) ts.d_dirty[SPLIT ? nb >> 1 : nb] = 1;
@@ -436,9 +448,18 @@ __device__ __forceinline__ int pr_visit(const TileSet& ts, int tid, int local_it
 }
 
 // Persistent push-relabel phase: 2*sweeps alternating parity sweeps separated
-// by grid barriers.  Sweep s of parity p drains queue q_pr[p][cur_pr[p]] one
-// tile per CTA ticket; tiles still active go to q_pr[p][1-cur], neighbours
-// that received flow to the other parity's pending buffer.
+// by grid barriers.  Sweep s of parity p drains queue q_pr[p][cur[p]], a CTA's
+// first item at its block index, the others by ticket; tiles still active go
+// to q_pr[p][1-cur], neighbours that received flow to the other parity's
+// pending buffer.
+//
+// In the tail of a solve a sweep holds a few items and its time is a chain of
+// latencies, so the chain is kept short: which buffer a parity is on follows
+// from the sweep index; the queue's length and the CTA's own entry are one
+// round trip to L2; the barrier is one growing counter (pr_bar, zeroed with
+// the tickets before the phase) whose arrivals are also its release; the
+// counters that a sweep leaves are reset by block 0 during the next one.
+// 26 us a sweep before, 19.5 now (4096 x 3072, 200-1,000 active tiles).
 //
 // Staging (ts.d_tmap set): tensor copies fill one of two staging buffers in
 // dynamic shared memory.  While a visit runs, the CTA's next ticket is
@@ -477,92 +498,123 @@ __global__ void __launch_bounds__(Tile<DIMS, TY, TZ>::NT,
   int next_buf = 0;         // thread 0: buffer of the next fill
   int s = 0;
   const int npairs = sweeps > 0 ? sweeps : jfc::vload(&ctr->pr_sweeps);
+  const int own = min((int)blockIdx.x, ts.ntiles - 1);   // (a parity's queue holds at most ntiles items)
+  int cur[2] = {0, 0};   // pending buffer per parity (0 after a global relabel)
+  bool failed = false;   // a staging copy never completed (error raised): leave
   for (; s < 2 * npairs; ++s) {
-    const int p = s & 1;
-    const int b = jfc::vload(&ctr->cur_pr[p]);
-    const int bo = jfc::vload(&ctr->cur_pr[p ^ 1]);
-    const int n = jfc::vload(&ctr->qn_pr[p][b]);
-    if (n == 0 && jfc::vload(&ctr->qn_pr[p ^ 1][bo]) == 0) break;  // nothing left anywhere
-    const int* queue = ts.d_q_pr[p][b];
-    // the previous sweep's writes (seen through the grid barrier) come before
-    // this sweep's tensor reads
-    if (tma && threadIdx.x == 0) jfc::fence_async_global();
-    int pre = -1, pre_buf = 0;   // thread 0: the prefetched item and its buffer
-    unsigned pre_k = 0;
-    bool failed = false;
-    for (;;) {
+    const int p = s & 1, b = cur[p], bo = cur[p ^ 1];
+    int* const queue = ts.d_q_pr[p][b];
+    const int n = jfc::vload(&ctr->qn_pr[p][b]), n_other = jfc::vload(&ctr->qn_pr[p ^ 1][bo]);
+    const int mine = jfc::vload(queue + own);
+    if (n == 0 && n_other == 0) break;   // nothing left anywhere
+    if (threadIdx.x == 0) {
+      // the previous sweep's writes (seen through the grid barrier) come before
+      // this sweep's tensor reads
+      if (tma) jfc::fence_async_global();
+      if (blockIdx.x == 0) {
+        // what the previous sweep used up: next touched after this sweep's barrier
+        ctr->ticket[p ^ 1] = 0;
+        if (s > 0) ctr->qn_pr[p ^ 1][bo ^ 1] = 0;
+      }
+    }
+    int pre = -1, pre_buf = 0;   // thread 0: the prefetched item, its tile and its buffer
+    int4 pre_ti = make_int4(0, 0, 0, 0);
+    long long k = blockIdx.x;    // thread 0: ticket of the current item
+    bool more = (long long)blockIdx.x < n;
+    for (bool first = true; more; first = false) {
       if (threadIdx.x == 0) {
-        int item, buf = 0;
-        unsigned k;
+        int item = -1, buf = 0;
+        int4 ti = make_int4(0, 0, 0, 0);
+        auto issue = [&](int it, const int4& t4) {
+          const int bf = next_buf;
+          ts.d_flag_pr[it] = 0;
+          if (tma) {
+            next_buf ^= 1;
+            pr_stage_issue<DIMS, TY, TZ, SPLIT>(ts, it, t4, stage[bf], &s_bar[bf], acquired_grid);
+            return bf;
+          }
+          return 0;
+        };
+        auto next_ticket = [&]() { return (long long)gridDim.x + atomicAdd(&ctr->ticket[p], 1u); };
         if (pre >= 0) {
-          item = pre; buf = pre_buf; k = pre_k; pre = -1;
+          item = pre; ti = pre_ti; buf = pre_buf; pre = -1;
         } else {
-          k = atomicAdd(&ctr->ticket[s & 1], 1u);
-          item = (int)k < n ? queue[k] : -1;
-          if (item >= 0) {
-            ts.d_flag_pr[item] = 0;
-            if (tma) {
-              buf = next_buf; next_buf ^= 1;
-              pr_stage_issue<DIMS, TY, TZ, SPLIT>(ts, item, stage[buf], &s_bar[buf], acquired_grid);
-            }
+          if (!first) k = next_ticket();
+          if (k < n) {
+            item = first ? mine : queue[k];
+            ti = item_tile<SPLIT>(ts, item);
+            buf = issue(item, ti);
           }
         }
-        if (tma && item >= 0 && (long long)k + gridDim.x < n) {
-          const unsigned k2 = atomicAdd(&ctr->ticket[s & 1], 1u);
-          if ((int)k2 < n) {
+        if (tma && item >= 0 && k + gridDim.x < n) {
+          const long long k2 = next_ticket();
+          if (k2 < n) {
             pre = queue[k2];
-            pre_k = k2;
-            ts.d_flag_pr[pre] = 0;
-            pre_buf = next_buf; next_buf ^= 1;
-            pr_stage_issue<DIMS, TY, TZ, SPLIT>(ts, pre, stage[pre_buf], &s_bar[pre_buf], acquired_grid);
+            pre_ti = item_tile<SPLIT>(ts, pre);
+            k = k2;
+            pre_buf = issue(pre, pre_ti);
           }
         }
         sm.tile = item;
+        sm.ti = ti;
         sm.buf = buf;
       }
       __syncthreads();
       const int tid = sm.tile, buf = sm.buf;
+      const int4 ti = sm.ti;
       if (tid < 0) break;
+      bool late = false;
       if (tma) {
-        const bool ok = jfc::mbar_wait(&s_bar[buf], (parity >> buf) & 1u, cap);
+        late = !jfc::mbar_wait(&s_bar[buf], (parity >> buf) & 1u, cap);
         parity ^= 1u << buf;
-        if (__syncthreads_or(!ok)) {
-          if (threadIdx.x == 0) {
-            atomicExch(&ctr->error, 1);
-            // copies still in flight land before the CTA leaves its shared
-            // memory: bounded by a fixed poll count of its own, not by the
-            // (possibly tiny) spin limit that gave up above
-            constexpr unsigned long long kDrainPolls = 1ull << 26;
-            jfc::mbar_wait(&s_bar[buf], ((parity >> buf) & 1u) ^ 1u, kDrainPolls);
-            if (pre >= 0) jfc::mbar_wait(&s_bar[pre_buf], (parity >> pre_buf) & 1u, kDrainPolls);
-          }
-          failed = true;
-          break;
-        }
       }
       // first sweep of a phase: nothing moved since the exact global relabel
       // (the halo tiles have the other parity), so the local relabel would
       // reproduce the heights it finds
-      rounds += pr_visit<DIMS, TY, TZ, SPLIT>(ts, tid, local_iters, s > 0, sm, stage[buf], tma);
+      const int rd = pr_visit<DIMS, TY, TZ, SPLIT>(ts, tid, ti, local_iters, s > 0, sm, stage[buf], tma, late);
+      if (rd < 0) {
+        if (threadIdx.x == 0) {
+          atomicExch(&ctr->error, 1);
+          // copies still in flight land before the CTA leaves its shared
+          // memory: bounded by a fixed poll count of its own, not by the
+          // (possibly tiny) spin limit that gave up above
+          constexpr unsigned long long kDrainPolls = 1ull << 26;
+          jfc::mbar_wait(&s_bar[buf], ((parity >> buf) & 1u) ^ 1u, kDrainPolls);
+          if (pre >= 0) jfc::mbar_wait(&s_bar[pre_buf], (parity >> pre_buf) & 1u, kDrainPolls);
+        }
+        failed = true;
+        break;
+      }
+      rounds += rd;
       ++visits;
-      // queue: myself for my parity's next sweep, neighbours for the other parity
+      // queue: neighbours for the other parity (lanes 0-5), myself for my
+      // parity's next sweep (lane 6), both counters at once
       if (threadIdx.x < 32) {
         const int lane = threadIdx.x;
         const int nb = lane < 6 ? sm.q_nb[lane] : -1;
-        jfc::warp_append(nb >= 0, nb, ts.d_flag_pr, ts.d_q_pr[p ^ 1][bo], &ctr->qn_pr[p ^ 1][bo]);
-        const bool active = sm.active != 0;
-        if (active && lane == 0) ts.d_flag_pr[tid] = 1;
-        jfc::warp_append(active && lane == 0, tid, nullptr, ts.d_q_pr[p][b ^ 1], &ctr->qn_pr[p][b ^ 1]);
+        bool won = false;
+        if (nb >= 0) won = atomicExch(ts.d_flag_pr + nb, 1) == 0;
+        if (lane == 6 && sm.active) {
+          ts.d_flag_pr[tid] = 1;
+          won = true;
+        }
+        const unsigned m = __ballot_sync(FULL, won), mn = m & 63u;
+        int at = 0;
+        if (lane == 0 && mn) at = atomicAdd(&ctr->qn_pr[p ^ 1][bo], __popc(mn));
+        if (lane == 6 && won) at = atomicAdd(&ctr->qn_pr[p][b ^ 1], 1);
+        const int at0 = __shfl_sync(FULL, at, 0);
+        if (won) {
+          if (lane == 6) ts.d_q_pr[p][b ^ 1][at] = tid;
+          else ts.d_q_pr[p ^ 1][bo][at0 + __popc(mn & ((1u << lane) - 1u))] = nb;
+        }
       }
-      __syncthreads();
+      more = n > (int)gridDim.x;   // otherwise every item had its CTA
+      if (more) __syncthreads();
     }
-    if (failed) break;   // a staging copy never completed (error raised): leave
+    if (failed) break;
+    cur[p] = b ^ 1;
     JFC_PCLK_DECL
-    const bool ok = jfc::grid_sync(ctr, [&]() {
-      ctr->ticket[s & 1] = 0;
-      ctr->qn_pr[p][b] = 0;
-      ctr->cur_pr[p] = b ^ 1;
-    });
+    const bool ok = jfc::arrive_wait(ctr, &ctr->pr_bar, (unsigned long long)(s + 1) * gridDim.x);
     JFC_PCLK(ctr, 4);
     if (!ok) break;
   }
@@ -684,12 +736,14 @@ __global__ void __launch_bounds__(Tile<DIMS, TY, TZ>::NT)
         item = (int)(unsigned)(v & 0xffffffffu);
         gen = (int)(v >> 32);
         // neighbour exclusion (see above)
+        const int4 ti = item_tile<SPLIT>(ts, item);
+        sm.ti = ti;
         bool conflict = atomicCAS(lock + item, 0, 1) != 0;
         if (!conflict) {
           asm volatile("fence.sc.gpu;" ::: "memory");
 #pragma unroll
           for (int f = 0; f < (DIMS == 3 ? 6 : 4); ++f) {
-            const int nb = face_item<DIMS, TY, TZ, SPLIT>(ts, item, f);
+            const int nb = face_item<DIMS, TY, TZ, SPLIT>(ts, item, ti, f);
             if (nb >= 0 && jfc::vload(lock + nb) != 0) conflict = true;
           }
           if (conflict) atomicExch(lock + item, 0);
@@ -717,7 +771,7 @@ __global__ void __launch_bounds__(Tile<DIMS, TY, TZ>::NT)
     // generation 0: nothing around the item moved since the exact global
     // relabel unless a neighbour was visited first; the local relabel is an
     // improvement only, so skipping it is safe either way
-    rounds += pr_visit<DIMS, TY, TZ, SPLIT>(ts, item, local_iters, gen > 0, sm, stage, false);
+    rounds += pr_visit<DIMS, TY, TZ, SPLIT>(ts, item, sm.ti, local_iters, gen > 0, sm, stage, false, false);
     ++visits;
     maxgen = max(maxgen, gen);
     // release the item (its writes visible first), then queue what it fed
@@ -778,6 +832,10 @@ cudaError_t launch_t(const TileSet& ts, int sweeps, int local_iters, cudaStream_
     if (e != cudaSuccess) return e;
   }
   const int blocks = persistent_blocks_cached(async ? cache_async : cache_sweeps, fn, NT, dyn);
+  static_assert(offsetof(DevCounters, ticket) == 0 && offsetof(DevCounters, pr_bar) == sizeof(unsigned) * 2,
+                "tickets and barrier counter are zeroed together");
+  const cudaError_t z = cudaMemsetAsync(ts.d_ctr, 0, offsetof(DevCounters, pr_bar) + sizeof(unsigned long long), st);
+  if (z != cudaSuccess) return z;
   TileSet arg = ts;
   void* params[] = {(void*)&arg, (void*)&sweeps, (void*)&local_iters};
   jfc_note_launch();

@@ -272,7 +272,6 @@ int lane_cycle(jfc_server* S, Lane& L, int lane_id, int max_interval = 1 << 30) 
     for (size_t i = 0; i < L.mem[k].size(); ++i)
       if (!L.mem[k][i].done) a += L.active[k][i];
     if (a == 0) continue;
-    cudaMemsetAsync(L.ts[k].d_ctr->ticket, 0, sizeof(L.ts[k].d_ctr->ticket), ctx->stream);
     const cudaError_t e = launch_pr_phase(L.ts[k], std::min(L.interval, max_interval), p.local_iters, ctx->stream);
     if (e != cudaSuccess) return cuda_status(e, "push-relabel phase");
     ran_pr[k] = true;
