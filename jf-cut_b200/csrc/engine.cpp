@@ -393,6 +393,11 @@ static cudaError_t enqueue_bfs(TileSet& ts, bool cut, int max_passes, cudaStream
     return cudaMemcpyAsync((char*)pin + sizeof(DevCounters), ts.d_grid_active, sizeof(int) * ts.ngrids,
                            cudaMemcpyDeviceToHost, s);
   }
+  if (cut && ts.dims == 2) {
+    JFC_E(cudaMemsetAsync(&ts.d_ctr->bfs_status, 0, sizeof(int), s));
+    JFC_E(launch_wave_cut(ts, max_passes, s));
+    return cudaMemcpyAsync(pin, ts.d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s);
+  }
   JFC_E(cudaMemsetAsync(ts.d_flag_bfs[0], 0, sizeof(int) * (size_t)ts.ntiles, s));
   JFC_E(cudaMemsetAsync(ts.d_flag_bfs[1], 0, sizeof(int) * (size_t)ts.ntiles, s));
   if (!cut) JFC_E(cudaMemsetAsync(ts.d_grid_active, 0, sizeof(int) * ts.ngrids, s));
@@ -536,18 +541,22 @@ static int run_cycle(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, int interva
   return finish_bfs(ts, false, ctx->h_pin, passes, &active, nullptr, sweeps_done);
 }
 
-int engine_cut(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, std::vector<GridResult>& res, int& passes) {
+int engine_cut(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, std::vector<GridResult>& res, int& passes,
+               cudaEvent_t done) {
   cudaStream_t s = ctx->stream;
   res.assign(ts.ngrids, GridResult());
-  int bad = 0;
-  int rc = engine_bfs(ctx, ts, p, true, passes, nullptr, &bad, nullptr);
+  // counters and sums are read back together, with one wait
+  int rc = pin_reserve(ctx, pin_need(ts));
   if (rc) return rc;
-  JFC_CUDA(launch_grid_sums(ts, s));
-  rc = pin_reserve(ctx, pin_need(ts));
-  if (rc) return rc;
-  long long* hs = (long long*)ctx->h_pin;
+  JFC_CUDA(enqueue_bfs(ts, true, p.max_bfs_passes, s, ctx->h_pin));
+  if (ts.dims != 2) JFC_CUDA(launch_grid_sums(ts, s));   // (the 2D cut sums as it labels)
+  long long* hs = (long long*)((char*)ctx->h_pin + sizeof(DevCounters));
   JFC_CUDA(cudaMemcpyAsync(hs, ts.d_grid_sum, sizeof(long long) * 2 * ts.ngrids, cudaMemcpyDeviceToHost, s));
+  if (done) JFC_CUDA(cudaEventRecord(done, s));
   JFC_CUDA(cudaStreamSynchronize(s));
+  int bad = 0;
+  rc = finish_bfs(ts, true, ctx->h_pin, passes, nullptr, &bad, nullptr);
+  if (rc) return rc;
   for (int g = 0; g < ts.ngrids; ++g) {
     res[g].neg_sum = hs[2 * g];
     res[g].labels = hs[2 * g + 1];
@@ -715,16 +724,12 @@ int engine_solve(jfc_ctx* ctx, TileSet& ts, const jfc_params& p_in, std::vector<
   JFC_CUDA(cudaEventRecord(ev[2], s));
   int passes = st.bfs_passes;
   std::vector<GridResult> cut;
-  rc = engine_cut(ctx, ts, p, cut, passes);
+  rc = engine_cut(ctx, ts, p, cut, passes, ev[1]);
   if (rc && rc != JFC_ERR_NOT_CONVERGED) return rc;
   st.bfs_passes = passes;
-  JFC_CUDA(cudaEventRecord(ev[3], s));
-  // device-clock phase times and visit counters
-  unsigned long long* hv = (unsigned long long*)ctx->h_pin;
-  JFC_CUDA(cudaMemcpyAsync(hv, &ts.d_ctr->visits, 15 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-  JFC_CUDA(cudaEventRecord(ev[1], s));
-  JFC_CUDA(cudaStreamSynchronize(s));
-  st.ms_cut = elapsed_ms(ev[2], ev[3]);
+  // device-clock phase times and visit counters (the cut read them back)
+  const unsigned long long* hv = &((const DevCounters*)ctx->h_pin)->visits;
+  st.ms_cut = elapsed_ms(ev[2], ev[1]);
   st.ms_total = elapsed_ms(ev[0], ev[1]);
   st.tile_visits = (long long)hv[0];
   st.bfs_visits = (long long)hv[1];

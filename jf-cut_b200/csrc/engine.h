@@ -63,8 +63,11 @@ int engine_solve(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, std::vector<Gri
 // push-relabel phase that ran before it.
 int engine_bfs(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, bool cut, int& passes,
                std::vector<int>* active, int* cut_bad, int* sweeps_done);
-// Cut BFS + per-grid sums (min(e, 0), source-side count) of every grid of ts.
-int engine_cut(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, std::vector<GridResult>& res, int& passes);
+// Cut BFS + per-grid sums (min(e, 0), source-side count) of every grid of ts;
+// the last kernel on the set was its global relabel.  The control block is read
+// back into the context's pinned memory.  done (may be null) is recorded behind it.
+int engine_cut(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, std::vector<GridResult>& res, int& passes,
+               cudaEvent_t done = nullptr);
 // Build / free a tile set over grids (all of one dimensionality).  The control
 // block is reused while it is large enough.  With a stream the grid and tile
 // tables are uploaded asynchronously from pinned staging (rewrite it only

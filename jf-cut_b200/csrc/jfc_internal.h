@@ -161,6 +161,10 @@ cudaError_t launch_bfs(const TileSet& ts, bool cut, int max_passes, cudaStream_t
 // (kernels_wave.cu) the global relabel of a 2D tile set; resets its own queues
 // and counters
 cudaError_t launch_wave_relabel(const TileSet& ts, cudaStream_t s);
+// (kernels_wave.cu) the cut of a 2D tile set whose last kernel was its global
+// relabel: labels into the label planes, per-grid sums of min(e, 0) and of the
+// labels into d_grid_sum; resets what it uses
+cudaError_t launch_wave_cut(const TileSet& ts, int max_passes, cudaStream_t s);
 // regions of a 2D grid in that relabel
 inline int wave_regions(int tiles_x, int Hp) {
   return (tiles_x + JFC_WAVE_WORDS - 1) / JFC_WAVE_WORDS * ((Hp + JFC_WAVE_ROWS - 1) / JFC_WAVE_ROWS);

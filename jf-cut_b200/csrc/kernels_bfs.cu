@@ -1204,13 +1204,14 @@ int persistent_blocks_cached(int* cache, const void* kernel, int threads, size_t
 }
 
 static cudaError_t bfs_dispatch(const TileSet& ts, int mode, int max_passes, const uint8_t* seeds, cudaStream_t s) {
-#define JFC_BFS(D, Y, Z)                                                       \
-  (mode == 1 ? bfs_t<D, Y, Z, 1>(ts, max_passes, seeds, s) : bfs_t<D, Y, Z, 2>(ts, max_passes, seeds, s))
-#define JFC_BFS3(Y, Z) (mode == 0 ? bfs_t<3, Y, Z, 0>(ts, max_passes, seeds, s) : JFC_BFS(3, Y, Z))
+#define JFC_BFS3(Y, Z)                                                         \
+  (mode == 0 ? bfs_t<3, Y, Z, 0>(ts, max_passes, seeds, s)                     \
+             : mode == 1 ? bfs_t<3, Y, Z, 1>(ts, max_passes, seeds, s) : bfs_t<3, Y, Z, 2>(ts, max_passes, seeds, s))
   if (ts.dims == 2) {
     if (mode == 0) return launch_wave_relabel(ts, s);
-    if (ts.TR == 8) return JFC_BFS(2, 8, 1);
-    if (ts.TR == 16) return JFC_BFS(2, 16, 1);
+    if (mode == 1) return launch_wave_cut(ts, max_passes, s);
+    if (ts.TR == 8) return bfs_t<2, 8, 1, 2>(ts, max_passes, seeds, s);
+    if (ts.TR == 16) return bfs_t<2, 16, 1, 2>(ts, max_passes, seeds, s);
     return cudaErrorInvalidValue;
   }
   if (ts.TY == 4 && ts.TZ == 4) return JFC_BFS3(4, 4);
@@ -1219,7 +1220,6 @@ static cudaError_t bfs_dispatch(const TileSet& ts, int mode, int max_passes, con
   if (ts.TY == 8 && ts.TZ == 2) return JFC_BFS3(8, 2);
   if (ts.TY == 8 && ts.TZ == 1) return JFC_BFS3(8, 1);
 #undef JFC_BFS3
-#undef JFC_BFS
   return cudaErrorInvalidValue;
 }
 
@@ -1248,6 +1248,11 @@ cudaError_t launch_grid_sums(const TileSet& ts, cudaStream_t s) {
 }
 
 cudaError_t launch_mark_dirty(const TileSet& ts, cudaStream_t s) {
+  // (no region of an earlier, failed run takes part in a cut on its own)
+  for (int k = 0; k < 2 && ts.nreg > 0; ++k) {
+    const cudaError_t e = cudaMemsetAsync(ts.d_rflag[k], 0, (size_t)ts.nreg, s);
+    if (e != cudaSuccess) return e;
+  }
   return cudaMemsetAsync(ts.d_dirty, 1, (size_t)ts.ntiles, s);
 }
 

@@ -47,10 +47,7 @@ constexpr size_t kOffDesc = kOffLabel + al(kMaxNodes);
 constexpr size_t kOffInfo = kOffDesc + al(sizeof(GridDev));
 constexpr size_t kOffFlagPr = kOffInfo + al(sizeof(int4) * (size_t)kMaxTiles);
 constexpr size_t kOffQPr = kOffFlagPr + kTileI;     // 4 queues
-constexpr size_t kOffFlagBfs = kOffQPr + 4 * kTileI; // 2 flag arrays
-constexpr size_t kOffQBfs = kOffFlagBfs + 2 * kTileI; // 2 frontiers
-constexpr size_t kOffAct = kOffQBfs + 2 * kTileI;
-constexpr size_t kOffGact = kOffAct + al(kMaxTiles);
+constexpr size_t kOffGact = kOffQPr + 4 * kTileI;
 constexpr size_t kOffSum = kOffGact + 256;
 constexpr size_t kOffCtr = kOffSum + 256;
 // regions of the global relabel: the most a grid of kMaxNodes padded nodes has
@@ -129,14 +126,7 @@ int na_read(void* host, const void* dev, size_t bytes, cudaStream_t s) {
 }
 
 int na_bfs(TileSet& ts, const jfc_params& p, bool cut, cudaStream_t s, int* active, int* cut_bad) {
-  if (cut) {
-    JFC_CUDA(cudaMemsetAsync(ts.d_flag_bfs[0], 0, sizeof(int) * (size_t)ts.ntiles, s));
-    JFC_CUDA(cudaMemsetAsync(ts.d_flag_bfs[1], 0, sizeof(int) * (size_t)ts.ntiles, s));
-    JFC_CUDA(cudaMemsetAsync(ts.d_ctr->ticket, 0, sizeof(ts.d_ctr->ticket), s));
-    JFC_CUDA(cudaMemsetAsync(ts.d_ctr->qn_bfs, 0, sizeof(ts.d_ctr->qn_bfs), s));
-    JFC_CUDA(cudaMemsetAsync(&ts.d_ctr->bfs_status, 0, sizeof(int), s));
-    JFC_CUDA(cudaMemsetAsync(&ts.d_ctr->cut_bad, 0, sizeof(int), s));
-  }
+  if (cut) JFC_CUDA(cudaMemsetAsync(&ts.d_ctr->bfs_status, 0, sizeof(int), s));
   JFC_CUDA(launch_bfs(ts, cut, p.max_bfs_passes, s));
   DevCounters hc;
   int rc = na_read(&hc, ts.d_ctr, sizeof(hc), s);
@@ -205,11 +195,6 @@ extern "C" int jfc_solve_grid2d_noalloc(int device, void* stream, const jfc_para
   ts.d_info = (int4*)(base + kOffInfo);
   ts.d_flag_pr = (int*)(base + kOffFlagPr);
   for (int q = 0; q < 4; ++q) ts.d_q_pr[q >> 1][q & 1] = (int*)(base + kOffQPr + q * kTileI);
-  ts.d_flag_bfs[0] = (int*)(base + kOffFlagBfs);
-  ts.d_flag_bfs[1] = (int*)(base + kOffFlagBfs + kTileI);
-  ts.d_q_bfs[0] = (int*)(base + kOffQBfs);
-  ts.d_q_bfs[1] = (int*)(base + kOffQBfs + kTileI);
-  ts.d_act = (uint8_t*)(base + kOffAct);
   ts.d_grid_active = (int*)(base + kOffGact);
   ts.d_grid_sum = (long long*)(base + kOffSum);
   ts.d_ctr = (DevCounters*)(base + kOffCtr);
@@ -268,7 +253,6 @@ extern "C" int jfc_solve_grid2d_noalloc(int device, void* stream, const jfc_para
   rc = na_bfs(ts, p, true, s, nullptr, &cut_bad);
   if (rc) return rc;
   if (cut_bad) return set_error(JFC_ERR_NOT_CONVERGED, "cut BFS reached a deficit node");
-  JFC_CUDA(launch_grid_sums(ts, s));
   rc = na_read(sums, ts.d_grid_sum, sizeof(sums), s);
   if (rc) return rc;
   JFC_CUDA(na_copy(g.label, d_labels, 1, w, h, pitch, Hp, true, s));

@@ -1,4 +1,4 @@
-"""The 2D global relabel on grids whose sides fall on, just inside and just
+"""The 2D global relabel and cut on grids whose sides fall on, just inside and just
 outside its region edges (64 rows x 6 words of 32 columns, 32 levels a phase)
 and with distance caps around a phase's length: after a solve the heights are
 the exact residual BFS distances, and flow and cut are the oracle's.  Sparse
