@@ -206,17 +206,20 @@ cudaError_t launch_seed_stats(const GridDev& g, const void* d_img, int pixfmt, c
                               int* d_minmax /*[2][3][2]*/, unsigned long long* d_count /*[2]*/,
                               uint32_t* d_list_f, uint32_t* d_list_b, unsigned int* d_fill /*[2]*/,
                               bool fill, cudaStream_t s);
-// k-means state of both seed classes, resident on the device across the
-// queued iterations (class 0 = foreground list first, class 1 after it).
+// k-means state of both seed classes (class 0 = foreground list first, class 1
+// after it).
 struct KmeansDev {
   int mu[2][JFC_MAX_K * 3];            // centres, fixed point 1/16
   int k[2];
-  int live[2];                         // class still moving
+  int live[2];                         // class takes part
   unsigned long long n[2];             // list lengths
-  unsigned long long acc[2][JFC_MAX_K * 4];   // per centre: channel sums, count
-  unsigned int done;                   // blocks finished in the current launch
+  // grid-wide form (all zero at launch)
+  unsigned long long acc[3][2][JFC_MAX_K * 4];   // per centre: channel sums, count
+  unsigned long long bar;              // barrier arrivals
+  int error;                           // a barrier wait gave up
 };
-cudaError_t launch_kmeans(const uint32_t* d_list, KmeansDev* d_km, int pixfmt, unsigned long long nmax,
+// All iterations in one launch; ntotal: seeds of both classes.
+cudaError_t launch_kmeans(const uint32_t* d_list, KmeansDev* d_km, int pixfmt, unsigned long long ntotal,
                           int iters, cudaStream_t s);
 // Expand a monotone table given by its runs (value val[j] from entry start[j]
 // on, start[0] = 0, m runs) into fwd[n]; rev (may be null) gets it mirrored.

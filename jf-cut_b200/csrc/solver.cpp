@@ -216,7 +216,7 @@ int build_core(jfc_graph* G, const void* img, int pixfmt, const uint8_t* seeds, 
                           d_bs->fill, true, s));
 
   // 3. k-means per class (fixed point 1/16, integer distances, order-free
-  // sums), all iterations queued on the device; centres start evenly spaced
+  // sums), all iterations in one launch; centres start evenly spaced
   // between the per-channel seed minimum and maximum
   const int C = jfc_pix_channels(pixfmt);
   KmeansDev& km = hbs.km;
@@ -233,7 +233,7 @@ int build_core(jfc_graph* G, const void* img, int pixfmt, const uint8_t* seeds, 
         km.mu[cls][j * 3 + c] = (int)(16 * mn + (16 * (mx - mn) * (2 * j + 1)) / (2 * km.k[cls]));
       }
   JFC_B(cudaMemcpyAsync(&d_bs->km, &km, sizeof(km), cudaMemcpyHostToDevice, s));
-  JFC_B(launch_kmeans(d_list, &d_bs->km, pixfmt, std::max(nf, nb), m.kmeans_iters, s));
+  JFC_B(launch_kmeans(d_list, &d_bs->km, pixfmt, nf + nb, m.kmeans_iters, s));
 
   // 4. while the device iterates: n-link tables (data-dependent sigma) and,
   // when lambda_t changed, the t-link tables over the quantised probability
@@ -253,8 +253,9 @@ int build_core(jfc_graph* G, const void* img, int pixfmt, const uint8_t* seeds, 
     JFC_B(expand_runs(tlink_runs(m.lambda_t), JFC_TQ + 1, M.d_lut_s, M.d_lut_t, s));
     M.lut_lambda_t = m.lambda_t;
   }
-  JFC_B(cudaMemcpyAsync(km.mu, d_bs->km.mu, sizeof(km.mu), cudaMemcpyDeviceToHost, s));
+  JFC_B(cudaMemcpyAsync(&km, &d_bs->km, sizeof(km), cudaMemcpyDeviceToHost, s));
   JFC_B(cudaStreamSynchronize(s));
+  if (km.error) { cleanup(); return set_error(JFC_ERR_CUDA, "a device-side wait timed out in the colour models"); }
   const int (&mu)[2][JFC_MAX_K * 3] = km.mu;
   const int k[2] = {km.k[0], km.k[1]};
 
