@@ -22,9 +22,11 @@ struct DevModel {
   BuildModelDev m{};
   void* d_img = nullptr;
   uint8_t* d_seeds = nullptr;
-  int* d_lut_s = nullptr;        // t-link tables [JFC_TQ + 1]
-  int* d_lut_t = nullptr;
+  int* d_lut_t = nullptr;        // t-link costs [JFC_TQ + 1]; the two below share its allocation
+  int* d_mu = nullptr;           // centres [2][JFC_MAX_K * 3]
+  uint8_t* d_lut_t8 = nullptr;   // the costs as bytes, when they fit (lut_t_max < 256)
   int lut_lambda_t = -1;         // lambda_t the t-link tables hold (-1: none)
+  int lut_t_max = 0;             // largest cost
   size_t img_bytes = 0;
 };
 

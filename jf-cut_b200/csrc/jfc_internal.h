@@ -197,8 +197,6 @@ struct BuildModelDev {
   int pixfmt, channels;
   int kf, kb;
   int seed_cap;
-  int mu_f[JFC_MAX_K * 3];
-  int mu_b[JFC_MAX_K * 3];
 };
 cudaError_t launch_contrast_sum(const GridDev& g, const void* d_img, int pixfmt,
                                 unsigned long long* d_sum, cudaStream_t s);
@@ -222,15 +220,26 @@ struct KmeansDev {
 cudaError_t launch_kmeans(const uint32_t* d_list, KmeansDev* d_km, int pixfmt, unsigned long long ntotal,
                           int iters, cudaStream_t s);
 // Expand a monotone table given by its runs (value val[j] from entry start[j]
-// on, start[0] = 0, m runs) into fwd[n]; rev (may be null) gets it mirrored.
-cudaError_t launch_expand_runs(const int* d_start, const int* d_val, int m, int n, int* d_fwd, int* d_rev,
+// on, start[0] = 0, m runs) into n ints and / or bytes (either may be null).
+cudaError_t launch_expand_runs(const int* d_start, const int* d_val, int m, int n, int* d_out, uint8_t* d_out8,
                                cudaStream_t s);
+// n-link weights over the contrast index: whole int tables, or (xy8 set) bytes
+// whose last entry stands for all after it, when every weight and t-link cost
+// fits one and the tables fit shared memory (build_tables_fit).
+struct NlinkTables {
+  const int* xy = nullptr;
+  const int* z = nullptr;
+  const uint8_t* xy8 = nullptr;
+  const uint8_t* z8 = nullptr;
+  int nxy = 0, nz = 0;   // entries of xy8, z8
+};
+bool build_tables_fit(int dims, int nxy, int nz);
 cudaError_t launch_build_graph(const GridDev& g, const void* d_img, const uint8_t* d_seeds,
-                               const BuildModelDev& m, const int* d_lut_xy, const int* d_lut_z,
-                               const int* d_lut_s, const int* d_lut_t,
+                               const BuildModelDev& m, const int* d_mu /*[2][JFC_MAX_K * 3]*/,
+                               const NlinkTables& nl, const int* d_lut_t /*[JFC_TQ + 1]*/, const uint8_t* d_lut_t8,
                                unsigned long long* d_sink, cudaStream_t s);
 cudaError_t launch_edit_seeds(const GridDev& g, const void* d_img, uint8_t* d_seeds,
-                              const BuildModelDev& m, const int* d_lut_s, const int* d_lut_t,
+                              const BuildModelDev& m, const int* d_mu, const int* d_lut_t,
                               const uint32_t* d_idx, const uint8_t* d_new, size_t n,
                               long long* d_dsink, cudaStream_t s);
 

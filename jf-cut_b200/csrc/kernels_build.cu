@@ -47,19 +47,20 @@ __device__ __forceinline__ unsigned pack_feat(const int* f) {
 
 // contrast-table index and squared difference of a neighbour pair
 template <int PF>
-__device__ __forceinline__ long long contrast_index(const int* a, const int* b) {
+__device__ __forceinline__ int contrast_index(const int* a, const int* b) {
   if constexpr (PF == JFC_PIX_RGB8) {
     const int d0 = a[0] - b[0], d1 = a[1] - b[1], d2 = a[2] - b[2];
-    return (long long)d0 * d0 + (long long)d1 * d1 + (long long)d2 * d2;
+    return d0 * d0 + d1 * d1 + d2 * d2;
   } else {
     const int d = a[0] - b[0];
     return d < 0 ? -d : d;
   }
 }
 template <int PF>
-__device__ __forceinline__ unsigned long long contrast_sq(const int* a, const int* b) {
-  if constexpr (PF == JFC_PIX_RGB8) return (unsigned long long)contrast_index<PF>(a, b);
-  else { const long long d = contrast_index<PF>(a, b); return (unsigned long long)(d * d); }
+__device__ __forceinline__ unsigned contrast_sq(const int* a, const int* b) {   // (65535^2 fits 32 bits unsigned)
+  const unsigned d = (unsigned)contrast_index<PF>(a, b);
+  if constexpr (PF == JFC_PIX_RGB8) return d;
+  else return d * d;
 }
 
 __device__ __forceinline__ void dense_xyz(const GridDev& g, long long i, int& x, int& y, int& z) {
@@ -87,27 +88,76 @@ __device__ __forceinline__ void block_sum_to(unsigned long long v, unsigned long
   }
 }
 
-// Sum of squared neighbour differences over every +x / +y (/ +z) pair.  One
-// warp per image row at a time (rows stride over all warps of the grid).
+// Sum over i in [0, n - off) of (v[i] - v[i + off])^2, v the image's values
+// (bytes or int16) in memory order, as this thread's share of the grid.  Pairs at
+// one distance need no pixel arithmetic: 16 bytes a thread and step, the
+// partner's bytes from the aligned words around them by funnel shifts, four
+// byte differences and their squares in two instructions.
+template <typename V>
+__device__ __forceinline__ unsigned long long pair_sum(const V* __restrict__ v, long long n, long long off) {
+  constexpr int E = 16 / (int)sizeof(V);   // values a step
+  const long long pairs = n - off;
+  const unsigned* words = reinterpret_cast<const unsigned*>(v);
+  const long long wo = off * (long long)sizeof(V) / 4;
+  const unsigned sh = 8u * (unsigned)(off * (long long)sizeof(V) & 3);
+  unsigned long long acc = 0;
+  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c * E < pairs;
+       c += (long long)gridDim.x * blockDim.x) {
+    const long long i = c * E;
+    if (i + E + off + 4 / (long long)sizeof(V) <= n) {
+      const uint4 a4 = *reinterpret_cast<const uint4*>(words + 4 * c);
+      const unsigned a[4] = {a4.x, a4.y, a4.z, a4.w};
+      unsigned b[5];
+#pragma unroll
+      for (int k = 0; k < 5; ++k) b[k] = words[4 * c + wo + k];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const unsigned p = __funnelshift_r(b[k], b[k + 1], sh);
+        if constexpr (sizeof(V) == 1) {
+          const unsigned d = __vabsdiffu4(a[k], p);
+          acc += (unsigned long long)__dp4a(d, d, 0u);
+        } else {
+          const unsigned d = __vabsdiffs2(a[k], p);
+          acc += (unsigned long long)(d & 0xffffu) * (d & 0xffffu) + (unsigned long long)(d >> 16) * (d >> 16);
+        }
+      }
+    } else {
+      for (long long j = i; j < i + E && j < pairs; ++j) {
+        const long long d = (long long)v[j] - v[j + off];
+        acc += (unsigned long long)(d * d);
+      }
+    }
+  }
+  return acc;
+}
+
+// Sum of squared neighbour differences over every +x / +y (/ +z) pair: all pairs
+// of values one pixel, one row (and one slice) apart in memory, less those that
+// join the end of a row or slice to the start of the next (sums are modulo
+// 2^64, the result is their true value).  Pixel by pixel with its neighbours
+// loaded as bytes it took 506 us on 15000 x 10000 RGB and 33 us on 1920 x 1080;
+// this 240 and 7 (70 at the HBM rate).
 template <int PF, int DIMS>
 __global__ void __launch_bounds__(256) k_contrast_sum(GridDev g, const void* __restrict__ img,
                                                       unsigned long long* sum) {
-  const long long rows = (long long)g.H * g.D;
-  const long long wh = (long long)g.W * g.H;
-  unsigned long long acc = 0;
-  const int warps = (int)(blockDim.x >> 5);
-  for (long long r = (long long)blockIdx.x * warps + (threadIdx.x >> 5); r < rows; r += (long long)gridDim.x * warps) {
-    const int y = (int)(r % g.H), z = (int)(r / g.H);
-    const long long row = r * g.W;
-    for (int x = threadIdx.x & 31; x < g.W; x += 32) {
-      const long long i = row + x;
-      int a[3], b[3];
-      feat<PF>(img, i, a);
-      if (x + 1 < g.W) { feat<PF>(img, i + 1, b); acc += contrast_sq<PF>(a, b); }
-      if (y + 1 < g.H) { feat<PF>(img, i + g.W, b); acc += contrast_sq<PF>(a, b); }
-      if (DIMS == 3 && z + 1 < g.D) { feat<PF>(img, i + wh, b); acc += contrast_sq<PF>(a, b); }
+  using V = typename std::conditional<PF == JFC_PIX_I16, int16_t, uint8_t>::type;
+  constexpr int C = PF == JFC_PIX_RGB8 ? 3 : 1;
+  const V* v = (const V*)img;
+  const long long W = (long long)g.W * C, rows = (long long)g.H * g.D, n = W * rows, slab = W * g.H;
+  unsigned long long acc = pair_sum<V>(v, n, C) + pair_sum<V>(v, n, W);
+  if (DIMS == 3) acc += pair_sum<V>(v, n, slab);
+  const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x, tn = (long long)gridDim.x * blockDim.x;
+  auto less = [&](long long i, long long j) {
+    const long long d = (long long)v[i] - v[j];
+    acc -= (unsigned long long)(d * d);
+  };
+  for (long long r = t0; r + 1 < rows; r += tn)   // row r's last pixel and row r + 1's first
+    for (int c = 0; c < C; ++c) less((r + 1) * W - C + c, (r + 1) * W + c);
+  if (DIMS == 3)
+    for (long long i = t0; i < W * (g.D - 1); i += tn) {   // slice z's last row and slice z + 1's first
+      const long long j = (i / W + 1) * slab + i % W;
+      less(j - W, j);
     }
-  }
   block_sum_to(acc, sum);
 }
 
@@ -412,43 +462,117 @@ __global__ void __launch_bounds__(kKmThreads, 1) k_kmeans(const uint32_t* __rest
     for (int i = t; i < 2 * JFC_MAX_K * 3; i += kKmThreads) (&km->mu[0][0])[i] = (&s_mu[0][0])[i];
 }
 
-// t-link costs of one node.  q = floor(Q dF / (dF + dB)): for 8-bit features
-// (dF + dB < 2^27) a float quotient lands within 1 of q and one exact integer
-// step either way corrects it; 16-bit features divide in 64 bits.
+// Colour models as the t-link pass reads them, in shared memory: for centre mu
+// the squared distance of a feature f (scaled by 16) is |16 f|^2 + (|mu|^2 -
+// 32 f.mu), so a centre costs one multiply-add per channel and a minimum.
 template <int PF>
-__device__ __forceinline__ void tlinks(const BuildModelDev& m, const int* __restrict__ lut_s,
-                                       const int* __restrict__ lut_t, const int* f, int seed, int& cs,
-                                       int& ct) {
-  if (seed == JFC_SEED_FG) { cs = m.seed_cap; ct = 0; return; }
-  if (seed == JFC_SEED_BG) { cs = 0; ct = m.seed_cap; return; }
+struct TlinkModel {
+  static constexpr int C = PF == JFC_PIX_RGB8 ? 3 : 1;
   using T = typename Dist<PF>::T;
-  T dF = fdist<PF>(f, m.mu_f), dB = fdist<PF>(f, m.mu_b);
-  for (int j = 1; j < m.kf; ++j) dF = min(dF, fdist<PF>(f, m.mu_f + 3 * j));
-  for (int j = 1; j < m.kb; ++j) dB = min(dB, fdist<PF>(f, m.mu_b + 3 * j));
-  unsigned q;
-  if constexpr (PF == JFC_PIX_I16) {
-    const unsigned long long s = (unsigned long long)dF + (unsigned long long)dB;
-    q = (s == 0) ? JFC_TQ / 2 : (unsigned)(((unsigned long long)JFC_TQ * (unsigned long long)dF) / s);
-  } else {
-    const unsigned s = (unsigned)dF + (unsigned)dB;
-    if (s == 0) {
-      q = JFC_TQ / 2;
-    } else {
-      q = (unsigned)(__fdividef((float)dF, (float)s) * (float)JFC_TQ);
-      const unsigned long long num = (unsigned long long)JFC_TQ * (unsigned)dF;
-      const unsigned long long qs = (unsigned long long)q * s;
-      if (qs > num) --q;
-      else if (qs + s <= num) ++q;
+  struct alignas(16) Centre {
+    T sq;        // |mu|^2
+    int m[3];    // -32 mu
+  };
+  Centre c[2][JFC_MAX_K];
+  int k[2];
+};
+
+// Fill the block's model (all threads call it; a barrier follows).
+template <int PF>
+__device__ __forceinline__ void load_model(TlinkModel<PF>& s, const BuildModelDev& m, const int* __restrict__ mu) {
+  constexpr int C = TlinkModel<PF>::C;
+  for (int i = threadIdx.x; i < 2 * JFC_MAX_K; i += blockDim.x) {
+    const int cls = i / JFC_MAX_K, j = i % JFC_MAX_K;
+    typename TlinkModel<PF>::Centre c;
+    c.sq = 0;
+    for (int ch = 0; ch < 3; ++ch) {
+      const int v = ch < C ? mu[cls * JFC_MAX_K * 3 + 3 * j + ch] : 0;
+      c.sq += (typename TlinkModel<PF>::T)v * v;
+      c.m[ch] = -32 * v;
+    }
+    s.c[cls][j] = c;
+  }
+  if (threadIdx.x == 0) {
+    s.k[0] = m.kf;
+    s.k[1] = m.kb;
+  }
+}
+
+// min over the centres of |mu|^2 - 32 f.mu for N nodes; unrolled for up to 8
+// centres (a loop of one centre is as much branch as arithmetic).
+template <int PF, int K, int N>
+__device__ __forceinline__ void nearest_of(const typename TlinkModel<PF>::Centre* s, const int (&f)[N][3],
+                                           typename Dist<PF>::T (&best)[N], bool more = false) {
+  using T = typename Dist<PF>::T;
+#pragma unroll
+  for (int j = 0; j < K; ++j) {
+    const typename TlinkModel<PF>::Centre ce = s[j];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      T v = ce.sq;
+#pragma unroll
+      for (int c = 0; c < TlinkModel<PF>::C; ++c) v += (T)f[i][c] * ce.m[c];
+      best[i] = j == 0 && !more ? v : min(best[i], v);
     }
   }
-  cs = lut_s[q];
-  ct = lut_t[q];
+}
+template <int PF, int N>
+__device__ __forceinline__ void nearest_centre(const typename TlinkModel<PF>::Centre* s, int k, const int (&f)[N][3],
+                                               typename Dist<PF>::T (&best)[N]) {
+  switch (k) {
+    case 1: nearest_of<PF, 1, N>(s, f, best); return;
+    case 2: nearest_of<PF, 2, N>(s, f, best); return;
+    case 3: nearest_of<PF, 3, N>(s, f, best); return;
+    case 4: nearest_of<PF, 4, N>(s, f, best); return;
+    case 5: nearest_of<PF, 5, N>(s, f, best); return;
+    case 6: nearest_of<PF, 6, N>(s, f, best); return;
+    case 7: nearest_of<PF, 7, N>(s, f, best); return;
+    default: break;
+  }
+  nearest_of<PF, 8, N>(s, f, best);
+  for (int j = 8; j < k; ++j) nearest_of<PF, 1, N>(s + j, f, best, true);
+}
+
+// t-link costs of N nodes.  q = floor(Q dF / (dF + dB)): a float quotient lands
+// within 1 of q (its relative error is below 2^-21, q below 2^16) and one exact
+// integer step either way corrects it (8-bit features: dF + dB < 2^27; 16-bit:
+// < 2^42, the products below 2^59).
+// (tab: cost of the source link at q; the sink link's is the same table's at
+// the complementary probability, JFC_TQ - q)
+template <int PF, int N, typename Tab>
+__device__ __forceinline__ void tlinks(const TlinkModel<PF>& s, int seed_cap, const Tab* __restrict__ tab,
+                                       const int (&f)[N][3], const int (&seed)[N], int (&cs)[N], int (&ct)[N]) {
+  constexpr int C = TlinkModel<PF>::C;
+  using T = typename Dist<PF>::T;
+  using U = typename std::conditional<PF == JFC_PIX_I16, unsigned long long, unsigned>::type;
+  T dF[N], dB[N];
+  nearest_centre<PF, N>(s.c[0], s.k[0], f, dF);
+  nearest_centre<PF, N>(s.c[1], s.k[1], f, dB);
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    T ff = 0;
+#pragma unroll
+    for (int c = 0; c < C; ++c) ff += (T)(16 * f[i][c]) * (16 * f[i][c]);
+    const U d = (U)(dF[i] + ff), sum = d + (U)(dB[i] + ff);
+    unsigned q = JFC_TQ / 2;
+    if (sum != 0) {
+      q = (unsigned)(__fdividef((float)d, (float)sum) * (float)JFC_TQ);
+      const unsigned long long num = (unsigned long long)JFC_TQ * d, qs = (unsigned long long)q * sum;
+      if (qs > num) --q;
+      else if (qs + sum <= num) ++q;
+    }
+    cs[i] = tab[q];
+    ct[i] = tab[JFC_TQ - q];
+    if (seed[i] == JFC_SEED_FG) { cs[i] = seed_cap; ct[i] = 0; }
+    if (seed[i] == JFC_SEED_BG) { cs[i] = 0; ct[i] = seed_cap; }
+  }
 }
 
 // Table entry t takes the value of the last run that starts at or before it
-// (a bisection of the few hundred starts, which stay in L1).
+// (a bisection of the few hundred starts, which stay in L1), as an int and / or
+// as a byte.
 __global__ void __launch_bounds__(256) k_expand_runs(const int* __restrict__ start, const int* __restrict__ val, int m,
-                                                     int n, int* __restrict__ fwd, int* __restrict__ rev) {
+                                                     int n, int* __restrict__ out, uint8_t* __restrict__ out8) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   int lo = 0, hi = m;
@@ -458,68 +582,225 @@ __global__ void __launch_bounds__(256) k_expand_runs(const int* __restrict__ sta
     else hi = mid;
   }
   const int v = val[lo];
-  fwd[t] = v;
-  if (rev) rev[n - 1 - t] = v;
+  if (out) out[t] = v;
+  if (out8) out8[t] = (uint8_t)v;
+}
+
+// Features of 4 neighbouring pixels from pixel i on, one word each (RGB: bytes
+// r, g, b, 0; 16 bits: value + 32768), by aligned word loads and funnel shifts;
+// total: pixels of the image (what the words would reach past its end is not
+// read).
+template <int PF>
+__device__ __forceinline__ void feat4(const void* __restrict__ img, long long i, long long total, unsigned (&f)[4]) {
+  constexpr int B = PF == JFC_PIX_RGB8 ? 3 : PF == JFC_PIX_I16 ? 2 : 1;   // bytes a pixel = words of 4 pixels
+  const long long at = i * B;
+  if (at + 4 * B + 4 <= total * B) {
+    const unsigned* w = reinterpret_cast<const unsigned*>(img) + (at >> 2);
+    const unsigned sh = 8u * (unsigned)(at & 3);
+    unsigned v[B + 1], u[B];
+#pragma unroll
+    for (int k = 0; k <= B; ++k) v[k] = w[k];
+#pragma unroll
+    for (int k = 0; k < B; ++k) u[k] = __funnelshift_r(v[k], v[k + 1], sh);
+    if constexpr (PF == JFC_PIX_RGB8) {
+      f[0] = u[0] & 0xffffffu;
+      f[1] = __funnelshift_r(u[0], u[1], 24) & 0xffffffu;
+      f[2] = __funnelshift_r(u[1], u[2], 16) & 0xffffffu;
+      f[3] = u[2] >> 8;
+    } else if constexpr (PF == JFC_PIX_I16) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) f[k] = ((u[k / 2] >> (16 * (k & 1))) & 0xffffu) ^ 0x8000u;
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) f[k] = (u[0] >> (8 * k)) & 255u;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      int a[3] = {0, 0, 0};
+      if (i + k < total) feat<PF>(img, i + k, a);
+      f[k] = i + k < total ? pack_feat<PF>(a) : 0u;
+    }
+  }
+}
+
+// contrast-table index of two packed features
+template <int PF>
+__device__ __forceinline__ int contrast4(unsigned a, unsigned b) {
+  if constexpr (PF == JFC_PIX_RGB8) {
+    const unsigned d = __vabsdiffu4(a, b);
+    return (int)__dp4a(d, d, 0u);
+  } else {
+    return a > b ? (int)(a - b) : (int)(b - a);
+  }
 }
 
 // One pass over the padded grid: n-links (both directions of every pair, from
 // the contrast table), t-links, e = cs - ct, label = 0; padding is zeroed.
-template <int PF, int DIMS>
-__global__ void __launch_bounds__(256) k_build(GridDev g, const void* __restrict__ img,
-                                               const uint8_t* __restrict__ seeds, BuildModelDev m,
-                                               const int* __restrict__ lut_xy, const int* __restrict__ lut_z,
-                                               const int* __restrict__ lut_s, const int* __restrict__ lut_t,
-                                               unsigned long long* sink) {
-  // one warp per 32-node row segment; rows stride over gridDim.y so that the
-  // sum of ct takes one atomic per block instead of one per warp
-  const int x = blockIdx.x * 32 + (threadIdx.x & 31);
-  const long long rows = (long long)g.Hp * g.Dp;
+// A lane takes 4 neighbouring columns and walks down `rows` rows: pixels come as
+// words, planes leave as 128-bit stores, a centre is read once for 4 nodes, the
+// weight to the right is the next node's weight to the left, the weight down
+// the next row's weight up (across the ends of a strip they are computed
+// again; along z both are, each slice on its own).
+// BYTES: every weight and cost fits a byte (default scales: 100 and 118), so the
+// block holds the tables in shared memory (32 lanes' look-ups in tables of
+// 256-780 KB are up to 32 accesses of L1 each).
+// With a node a lane the pass was bound by instructions, 320 per 32 nodes:
+// 2.03 ms on 15000 x 10000 RGB (0.67 at the HBM rate) and, with a 64-bit division
+// per node, 0.40 ms on 317 x 301 x 181 int16; this 1.24 and 0.25 (60% of the
+// issue slots).
+struct BuildTables {
+  const int* xy;         // n-link weights over the contrast index (int), used when !BYTES
+  const int* z;
+  const int* t;          // t-link costs over the quantised probability
+  const uint8_t* xy8;    // the same as bytes (padded to 16): entries past the last are the last
+  const uint8_t* z8;
+  const uint8_t* t8;
+  int nxy, nz;           // entries of xy8, z8
+};
+constexpr int kBuildThreads = 384;
+__host__ __device__ constexpr int pad16(int v) { return (v + 15) / 16 * 16; }
+template <int PF, int DIMS, bool BYTES>
+__global__ void __launch_bounds__(kBuildThreads, 2) k_build(GridDev g, const void* __restrict__ img,
+                                                            const uint8_t* __restrict__ seeds, BuildModelDev m,
+                                                            const int* __restrict__ mu, BuildTables tb, int rows,
+                                                            unsigned long long* sink) {
+  __shared__ TlinkModel<PF> s_m;
+  extern __shared__ __align__(16) uint8_t s_tab[];   // t8, xy8, z8
+  load_model<PF>(s_m, m, mu);
+  uint8_t* const s_xy = s_tab + pad16(JFC_TQ + 1);
+  uint8_t* const s_z = s_xy + pad16(tb.nxy);
+  if constexpr (BYTES) {
+    auto copy = [](uint8_t* d, const uint8_t* src, int n) {
+      for (int i = threadIdx.x; i < n / 16; i += kBuildThreads)
+        reinterpret_cast<uint4*>(d)[i] = reinterpret_cast<const uint4*>(src)[i];
+    };
+    copy(s_tab, tb.t8, pad16(JFC_TQ + 1));
+    copy(s_xy, tb.xy8, pad16(tb.nxy));
+    if (DIMS == 3) copy(s_z, tb.z8, pad16(tb.nz));
+  }
+  __syncthreads();
+  auto w_xy = [&](unsigned a, unsigned b) -> int {
+    const int d = contrast4<PF>(a, b);
+    if constexpr (BYTES) return s_xy[min(d, tb.nxy - 1)];
+    else return tb.xy[d];
+  };
+  auto w_z = [&](unsigned a, unsigned b) -> int {
+    const int d = contrast4<PF>(a, b);
+    if constexpr (BYTES) return s_z[min(d, tb.nz - 1)];
+    else return tb.z[d];
+  };
+  const int lane = threadIdx.x & 31;
+  const int cols = (g.pitch + 127) / 128, bands = (g.Hp + rows - 1) / rows;
+  const long long items = (long long)cols * bands * g.Dp, wh = (long long)g.W * g.H, total = wh * g.D;
+  const int warps = kBuildThreads / 32 * gridDim.x;
   unsigned long long acc = 0;
-  for (long long yz = (long long)blockIdx.y * 8 + (threadIdx.x >> 5); yz < rows; yz += (long long)gridDim.y * 8) {
-  const int y = (int)(yz % g.Hp), z = (int)(yz / g.Hp);
-  if (x < g.pitch) {
-    const long long p = (long long)x + (long long)g.pitch * (y + (long long)g.Hp * z);
-    const bool real = x < g.W && y < g.H && z < g.D;
-    if (!real) {
-      g.e[p] = 0;
-      for (int k = 0; k < (DIMS == 2 ? 4 : 6); ++k) g.r[k][p] = 0;
-      g.label[p] = 0;
-      g.h[p] = JFC_INF;
-    } else {
-      const long long wh = (long long)g.W * g.H;
-      const long long i = (long long)x + (long long)g.W * y + wh * z;
-      int a[3], b[3];
-      feat<PF>(img, i, a);
-      int w_xp = 0, w_yp = 0, w_ym = 0, w_xm = 0, w_zp = 0, w_zm = 0;
-      if (x + 1 < g.W) { feat<PF>(img, i + 1, b); w_xp = lut_xy[contrast_index<PF>(a, b)]; }
-      if (x > 0) { feat<PF>(img, i - 1, b); w_xm = lut_xy[contrast_index<PF>(a, b)]; }
-      if (y + 1 < g.H) { feat<PF>(img, i + g.W, b); w_yp = lut_xy[contrast_index<PF>(a, b)]; }
-      if (y > 0) { feat<PF>(img, i - g.W, b); w_ym = lut_xy[contrast_index<PF>(a, b)]; }
-      if constexpr (DIMS == 3) {
-        if (z + 1 < g.D) { feat<PF>(img, i + wh, b); w_zp = lut_z[contrast_index<PF>(a, b)]; }
-        if (z > 0) { feat<PF>(img, i - wh, b); w_zm = lut_z[contrast_index<PF>(a, b)]; }
-        g.r[0][p] = w_xp; g.r[1][p] = w_yp; g.r[2][p] = w_zp;
-        g.r[3][p] = w_zm; g.r[4][p] = w_ym; g.r[5][p] = w_xm;
-      } else {
-        g.r[0][p] = w_xp; g.r[1][p] = w_yp; g.r[2][p] = w_ym; g.r[3][p] = w_xm;
+  for (long long it = blockIdx.x * (kBuildThreads / 32) + (threadIdx.x >> 5); it < items; it += warps) {
+    const int bx = (int)(it % cols);
+    const long long yz = it / cols;
+    const int y0 = (int)(yz % bands) * rows, z = (int)(yz / bands);
+    const int x = bx * 128 + 4 * lane, y1 = min(y0 + rows, g.Hp);
+    const bool store = x < g.pitch;
+    const bool col = x < g.W && z < g.D;                // the first of the 4 columns is real
+    const int nreal = col ? min(4, g.W - x) : 0;        // real columns
+    long long i = (long long)z * wh + (long long)y0 * g.W + x;
+    long long p = (long long)x + (long long)g.pitch * (y0 + (long long)g.Hp * z);
+    unsigned a[4] = {0, 0, 0, 0}, n[4] = {0, 0, 0, 0};   // this row's pixels, the next row's
+    int w_ym[4] = {0, 0, 0, 0};
+    if (col && y0 < g.H) {
+      feat4<PF>(img, i, total, a);
+      if (y0 > 0) {
+        feat4<PF>(img, i - g.W, total, n);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) w_ym[k] = k < nreal ? w_xy(a[k], n[k]) : 0;
       }
-      int cs, ct;
-      tlinks<PF>(m, lut_s, lut_t, a, seeds[i], cs, ct);
-      g.e[p] = cs - ct;
-      g.label[p] = 0;
-      acc += (unsigned long long)ct;
+    }
+    for (int y = y0; y < y1; ++y, i += g.W, p += g.pitch) {
+      const bool real = col && y < g.H, below = col && y + 1 < g.H;
+      if (below) feat4<PF>(img, i + g.W, total, n);
+      // seeds: one by one (rows start at any byte)
+      int seed[4] = {0, 0, 0, 0};
+      if (real) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (k < nreal) seed[k] = seeds[i + k];
+      }
+      // the pixel beside the warp's strip: lane 31 to the right, lane 0 to the left
+      unsigned beside = 0;
+      const bool has = real && ((lane == 31 && x + 4 < g.W) || (lane == 0 && x > 0));
+      if (has) {
+        int e[3] = {0, 0, 0};
+        feat<PF>(img, lane == 0 ? i - 1 : i + 4, e);
+        beside = pack_feat<PF>(e);
+      }
+      unsigned right = __shfl_down_sync(FULL, a[0], 1);
+      if (lane == 31) right = beside;
+      int w_xp[4], w_xm[4], w_yp[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        w_xp[k] = real && x + k + 1 < g.W ? w_xy(a[k], k < 3 ? a[k < 3 ? k + 1 : 3] : right) : 0;
+        w_yp[k] = below && k < nreal ? w_xy(a[k], n[k]) : 0;
+      }
+      w_xm[0] = __shfl_up_sync(FULL, w_xp[3], 1);
+      if (lane == 0) w_xm[0] = has ? w_xy(a[0], beside) : 0;
+      if (!real) w_xm[0] = 0;
+#pragma unroll
+      for (int k = 1; k < 4; ++k) w_xm[k] = w_xp[k - 1];
+      int cs[4] = {0, 0, 0, 0}, ct[4] = {0, 0, 0, 0};
+      if (real) {
+        int f[4][3];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) unpack_feat(a[k], PF == JFC_PIX_RGB8 ? 3 : 1, f[k]);
+        if constexpr (BYTES) tlinks<PF, 4>(s_m, m.seed_cap, s_tab, f, seed, cs, ct);
+        else tlinks<PF, 4>(s_m, m.seed_cap, tb.t, f, seed, cs, ct);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (!real || k >= nreal) cs[k] = ct[k] = 0;
+        acc += (unsigned long long)ct[k];
+      }
+      if (store) {
+        auto put = [&](int* plane, const int (&v)[4]) {
+          *reinterpret_cast<int4*>(plane + p) = make_int4(v[0], v[1], v[2], v[3]);
+        };
+        put(g.r[0], w_xp);
+        put(g.r[1], w_yp);
+        if constexpr (DIMS == 3) {
+          int w_zp[4] = {0, 0, 0, 0}, w_zm[4] = {0, 0, 0, 0};
+          unsigned b[4];
+          if (real && z + 1 < g.D) {
+            feat4<PF>(img, i + wh, total, b);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w_zp[k] = k < nreal ? w_z(a[k], b[k]) : 0;
+          }
+          if (real && z > 0) {
+            feat4<PF>(img, i - wh, total, b);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w_zm[k] = k < nreal ? w_z(a[k], b[k]) : 0;
+          }
+          put(g.r[2], w_zp);
+          put(g.r[3], w_zm);
+        }
+        if (!real) w_ym[0] = w_ym[1] = w_ym[2] = w_ym[3] = 0;
+        put(g.r[DIMS == 3 ? 4 : 2], w_ym);
+        put(g.r[DIMS == 3 ? 5 : 3], w_xm);
+        const int e[4] = {cs[0] - ct[0], cs[1] - ct[1], cs[2] - ct[2], cs[3] - ct[3]};
+        put(g.e, e);
+        *reinterpret_cast<unsigned*>(g.label + p) = 0u;
+        if (!real || nreal < 4) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (!real || k >= nreal) g.h[p + k] = JFC_INF;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        w_ym[k] = w_yp[k];
+        a[k] = n[k];
+      }
     }
   }
-  }
-  __shared__ unsigned long long s_acc[8];
-  acc = warp_sum_u64(acc);
-  if ((threadIdx.x & 31) == 0) s_acc[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned long long t = 0;
-    for (int w = 0; w < 8; ++w) t += s_acc[w];
-    if (t) atomicAdd(sink, t);
-  }
+  block_sum_to(acc, sink);
 }
 
 // Warm stroke edit: re-seed nodes with the colour model fixed; the residual
@@ -546,9 +827,12 @@ __global__ void k_edit_mark(GridDev g, const uint32_t* __restrict__ idx, long lo
 
 template <int PF>
 __global__ void k_edit_seeds(GridDev g, const void* __restrict__ img, uint8_t* __restrict__ seeds,
-                             BuildModelDev m, const int* __restrict__ lut_s, const int* __restrict__ lut_t,
-                             const uint32_t* __restrict__ idx, const uint8_t* __restrict__ nseed,
-                             long long n, long long* dsink) {
+                             BuildModelDev m, const int* __restrict__ mu, const int* __restrict__ lut_t,
+                             const uint32_t* __restrict__ idx, const uint8_t* __restrict__ nseed, long long n,
+                             long long* dsink) {
+  __shared__ TlinkModel<PF> s_m;
+  load_model<PF>(s_m, m, mu);
+  __syncthreads();
   long long acc = 0;
   for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < n;
        j += (long long)gridDim.x * blockDim.x) {
@@ -556,16 +840,16 @@ __global__ void k_edit_seeds(GridDev g, const void* __restrict__ img, uint8_t* _
     if (g.h[padded_of(g, i)] != (int)j) continue;   // a later entry edits this node
     const int s1 = nseed[j], s0 = seeds[i];
     if (s0 == s1) continue;
-    int f[3];
-    feat<PF>(img, i, f);
-    int cs0, ct0, cs1, ct1;
-    tlinks<PF>(m, lut_s, lut_t, f, s0, cs0, ct0);
-    tlinks<PF>(m, lut_s, lut_t, f, s1, cs1, ct1);
+    int f[1][3] = {{0, 0, 0}}, cs0[1], ct0[1], cs1[1], ct1[1];
+    feat<PF>(img, i, f[0]);
+    const int from[1] = {s0}, to[1] = {s1};
+    tlinks<PF, 1>(s_m, m.seed_cap, lut_t, f, from, cs0, ct0);
+    tlinks<PF, 1>(s_m, m.seed_cap, lut_t, f, to, cs1, ct1);
     int x, y, z;
     dense_xyz(g, i, x, y, z);
     const long long p = (long long)x + (long long)g.pitch * (y + (long long)g.Hp * z);
-    atomicAdd(g.e + p, (cs1 - ct1) - (cs0 - ct0));
-    acc += (long long)ct1 - ct0;
+    atomicAdd(g.e + p, (cs1[0] - ct1[0]) - (cs0[0] - ct0[0]));
+    acc += (long long)ct1[0] - ct0[0];
     seeds[i] = (uint8_t)s1;
   }
   for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
@@ -583,7 +867,8 @@ int flat_blocks(long long n) {
 
 cudaError_t launch_contrast_sum(const GridDev& g, const void* d_img, int pixfmt,
                                 unsigned long long* d_sum, cudaStream_t s) {
-  const int nb = (int)std::min<long long>(((long long)g.H * g.D + 7) / 8, 148 * 8);
+  const long long bytes = (long long)g.W * g.H * g.D * (long long)jfc_pix_bytes(pixfmt);
+  const int nb = (int)std::max<long long>(1, std::min<long long>((bytes + 16 * 256 - 1) / (16 * 256), 148 * 8));
   const bool d3 = g.dims == 3;
   jfc_note_launch();
   switch (pixfmt) {
@@ -662,36 +947,61 @@ cudaError_t launch_kmeans(const uint32_t* d_list, KmeansDev* d_km, int pixfmt, u
   }
 }
 
-cudaError_t launch_expand_runs(const int* d_start, const int* d_val, int m, int n, int* d_fwd, int* d_rev,
+cudaError_t launch_expand_runs(const int* d_start, const int* d_val, int m, int n, int* d_out, uint8_t* d_out8,
                                cudaStream_t s) {
   if (n <= 0 || m <= 0) return cudaErrorInvalidValue;
   jfc_note_launch();
-  k_expand_runs<<<(n + 255) / 256, 256, 0, s>>>(d_start, d_val, m, n, d_fwd, d_rev);
+  k_expand_runs<<<(n + 255) / 256, 256, 0, s>>>(d_start, d_val, m, n, d_out, d_out8);
   return cudaGetLastError();
 }
 
-cudaError_t launch_build_graph(const GridDev& g, const void* d_img, const uint8_t* d_seeds,
-                               const BuildModelDev& m, const int* d_lut_xy, const int* d_lut_z,
-                               const int* d_lut_s, const int* d_lut_t, unsigned long long* d_sink,
-                               cudaStream_t s) {
-  dim3 grid((g.pitch + 31) / 32, (unsigned)std::min<long long>((g.Hp * (long long)g.Dp + 7) / 8, 64));
-  const bool d3 = g.dims == 3;
+// Shared memory of k_build's byte tables; the pass uses them while two blocks
+// of it fit an SM (one block of 16 warps does not hide the look-ups' latency).
+static size_t build_table_bytes(int dims, int nxy, int nz) {
+  return (size_t)pad16(JFC_TQ + 1) + pad16(nxy) + (dims == 3 ? pad16(nz) : 0);
+}
+bool build_tables_fit(int dims, int nxy, int nz) { return build_table_bytes(dims, nxy, nz) <= 108 * 1024; }
+
+template <int PF, int DIMS, bool BYTES>
+static cudaError_t build_t(const GridDev& g, const void* d_img, const uint8_t* d_seeds, const BuildModelDev& m,
+                           const int* d_mu, const BuildTables& tb, unsigned long long* d_sink, cudaStream_t s) {
+  const void* fn = (const void*)k_build<PF, DIMS, BYTES>;
+  const size_t dyn = BYTES ? build_table_bytes(DIMS, tb.nxy, tb.nz) : 0;
+  if (BYTES) {
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 108 * 1024);
+    if (e != cudaSuccess) return e;
+  }
+  // strips of 16 rows, or of 4 or 1 while those would not give every SM 24 warps
+  const int cols = (g.pitch + 127) / 128, warps = kBuildThreads / 32;
+  auto strips = [&](int rows) { return (long long)cols * ((g.Hp + rows - 1) / rows) * g.Dp; };   // a warp each
+  const int rows = strips(16) >= 148 * 24 ? 16 : strips(4) >= 148 * 24 ? 4 : 1;
+  const int grid = (int)std::min<long long>((strips(rows) + warps - 1) / warps, 148 * 2);
   jfc_note_launch();
-#define JFC_BUILD(PF)                                                                                   \
-  (d3 ? k_build<PF, 3><<<grid, 256, 0, s>>>(g, d_img, d_seeds, m, d_lut_xy, d_lut_z, d_lut_s, d_lut_t, d_sink) \
-      : k_build<PF, 2><<<grid, 256, 0, s>>>(g, d_img, d_seeds, m, d_lut_xy, d_lut_z, d_lut_s, d_lut_t, d_sink))
+  k_build<PF, DIMS, BYTES><<<grid, kBuildThreads, dyn, s>>>(g, d_img, d_seeds, m, d_mu, tb, rows, d_sink);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_build_graph(const GridDev& g, const void* d_img, const uint8_t* d_seeds, const BuildModelDev& m,
+                               const int* d_mu, const NlinkTables& nl, const int* d_lut_t, const uint8_t* d_lut_t8,
+                               unsigned long long* d_sink, cudaStream_t s) {
+  BuildTables tb{nl.xy, nl.z, d_lut_t, nl.xy8, nl.z8, d_lut_t8, nl.nxy, nl.nz};
+  const bool d3 = g.dims == 3, bytes = nl.xy8 != nullptr;
+#define JFC_BUILD(PF)                                                                                       \
+  return d3 ? (bytes ? build_t<PF, 3, true>(g, d_img, d_seeds, m, d_mu, tb, d_sink, s)                      \
+                     : build_t<PF, 3, false>(g, d_img, d_seeds, m, d_mu, tb, d_sink, s))                    \
+            : (bytes ? build_t<PF, 2, true>(g, d_img, d_seeds, m, d_mu, tb, d_sink, s)                      \
+                     : build_t<PF, 2, false>(g, d_img, d_seeds, m, d_mu, tb, d_sink, s))
   switch (m.pixfmt) {
-    case JFC_PIX_GRAY8: JFC_BUILD(JFC_PIX_GRAY8); break;
-    case JFC_PIX_RGB8: JFC_BUILD(JFC_PIX_RGB8); break;
-    case JFC_PIX_I16: JFC_BUILD(JFC_PIX_I16); break;
+    case JFC_PIX_GRAY8: JFC_BUILD(JFC_PIX_GRAY8);
+    case JFC_PIX_RGB8: JFC_BUILD(JFC_PIX_RGB8);
+    case JFC_PIX_I16: JFC_BUILD(JFC_PIX_I16);
     default: return cudaErrorInvalidValue;
   }
 #undef JFC_BUILD
-  return cudaGetLastError();
 }
 
 cudaError_t launch_edit_seeds(const GridDev& g, const void* d_img, uint8_t* d_seeds, const BuildModelDev& m,
-                              const int* d_lut_s, const int* d_lut_t, const uint32_t* d_idx,
+                              const int* d_mu, const int* d_lut_t, const uint32_t* d_idx,
                               const uint8_t* d_new, size_t n, long long* d_dsink, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   const int nb = flat_blocks((long long)n);
@@ -701,15 +1011,15 @@ cudaError_t launch_edit_seeds(const GridDev& g, const void* d_img, uint8_t* d_se
   switch (m.pixfmt) {
     case JFC_PIX_GRAY8:
       jfc_note_launch();
-      k_edit_seeds<JFC_PIX_GRAY8><<<nb, 256, 0, s>>>(g, d_img, d_seeds, m, d_lut_s, d_lut_t, d_idx, d_new, (long long)n, d_dsink);
+      k_edit_seeds<JFC_PIX_GRAY8><<<nb, 256, 0, s>>>(g, d_img, d_seeds, m, d_mu, d_lut_t, d_idx, d_new, (long long)n, d_dsink);
       break;
     case JFC_PIX_RGB8:
       jfc_note_launch();
-      k_edit_seeds<JFC_PIX_RGB8><<<nb, 256, 0, s>>>(g, d_img, d_seeds, m, d_lut_s, d_lut_t, d_idx, d_new, (long long)n, d_dsink);
+      k_edit_seeds<JFC_PIX_RGB8><<<nb, 256, 0, s>>>(g, d_img, d_seeds, m, d_mu, d_lut_t, d_idx, d_new, (long long)n, d_dsink);
       break;
     case JFC_PIX_I16:
       jfc_note_launch();
-      k_edit_seeds<JFC_PIX_I16><<<nb, 256, 0, s>>>(g, d_img, d_seeds, m, d_lut_s, d_lut_t, d_idx, d_new, (long long)n, d_dsink);
+      k_edit_seeds<JFC_PIX_I16><<<nb, 256, 0, s>>>(g, d_img, d_seeds, m, d_mu, d_lut_t, d_idx, d_new, (long long)n, d_dsink);
       break;
     default: return cudaErrorInvalidValue;
   }

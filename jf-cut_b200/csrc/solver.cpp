@@ -126,8 +126,8 @@ TableRuns nlink_runs(int pixfmt, double scale, double sigma2) {
 }
 
 // t-link table over the quantised probability: round(lambda_t * -ln((q + 0.5) / (Q + 1))),
-// non-increasing in q; the sink side's table is the same one read from its
-// end (the quotient (Q + 0.5 - q) / (Q + 1) is that of entry Q - q).
+// non-increasing in q; the sink side reads the same table at Q - q (its
+// quotient (Q + 0.5 - q) / (Q + 1) is that entry's).
 TableRuns tlink_runs(int lambda_t) {
   return TableRuns(JFC_TQ + 1, [&](int q) {
     const double p = ((double)q + 0.5) / (double)(JFC_TQ + 1);
@@ -135,16 +135,16 @@ TableRuns tlink_runs(int lambda_t) {
   });
 }
 
-// Upload the runs and expand them into d_fwd (and mirrored into d_rev) on the
-// stream; the runs' buffer is freed on the stream.
-cudaError_t expand_runs(const TableRuns& r, int n, int* d_fwd, int* d_rev, cudaStream_t s) {
+// Upload the runs and expand them into n ints and / or bytes on the stream; the
+// runs' buffer is freed on the stream.
+cudaError_t expand_runs(const TableRuns& r, int n, int* d_out, uint8_t* d_out8, cudaStream_t s) {
   const size_t m = r.start.size();
   int* buf = nullptr;
   cudaError_t e = cudaMallocAsync((void**)&buf, 2 * m * sizeof(int), s);
   if (e != cudaSuccess) return e;
   e = cudaMemcpyAsync(buf, r.start.data(), m * sizeof(int), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(buf + m, r.val.data(), m * sizeof(int), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = launch_expand_runs(buf, buf + m, (int)m, n, d_fwd, d_rev, s);
+  if (e == cudaSuccess) e = launch_expand_runs(buf, buf + m, (int)m, n, d_out, d_out8, s);
   const cudaError_t f = cudaFreeAsync(buf, s);
   return e == cudaSuccess ? f : e;
 }
@@ -160,8 +160,12 @@ int ensure_model_buffers(jfc_graph* G, int pixfmt) {
   if (M.d_img && M.img_bytes != ib) { JFC_CUDA(cudaFreeAsync(M.d_img, s)); M.d_img = nullptr; }
   if (!M.d_img) { JFC_CUDA(cudaMallocAsync(&M.d_img, ib, s)); M.img_bytes = ib; }
   if (!M.d_seeds) JFC_CUDA(cudaMallocAsync((void**)&M.d_seeds, n, s));
-  if (!M.d_lut_s) JFC_CUDA(cudaMallocAsync((void**)&M.d_lut_s, sizeof(int) * (JFC_TQ + 1), s));
-  if (!M.d_lut_t) JFC_CUDA(cudaMallocAsync((void**)&M.d_lut_t, sizeof(int) * (JFC_TQ + 1), s));
+  if (!M.d_lut_t) {
+    const size_t ints = align256(sizeof(int) * (JFC_TQ + 1 + 2 * JFC_MAX_K * 3));
+    JFC_CUDA(cudaMallocAsync((void**)&M.d_lut_t, ints + align256(JFC_TQ + 1), s));
+    M.d_mu = M.d_lut_t + JFC_TQ + 1;
+    M.d_lut_t8 = (uint8_t*)M.d_lut_t + ints;
+  }
   return JFC_OK;
 }
 
@@ -237,38 +241,48 @@ int build_core(jfc_graph* G, const void* img, int pixfmt, const uint8_t* seeds, 
 
   // 4. while the device iterates: n-link tables (data-dependent sigma) and,
   // when lambda_t changed, the t-link tables over the quantised probability
-  const int nlut = nlink_entries(pixfmt);
-  int* d_lxy = nullptr;
-  int* d_lz = nullptr;
-  JFC_B(cudaMallocAsync((void**)&d_lxy, sizeof(int) * nlut, s));
-  temps.push_back(d_lxy);
-  JFC_B(expand_runs(nlink_runs(pixfmt, scale_xy, sigma2), nlut, d_lxy, nullptr, s));
-  if (G->dims == 3) {
-    JFC_B(cudaMallocAsync((void**)&d_lz, sizeof(int) * nlut, s));
-    temps.push_back(d_lz);
-    JFC_B(expand_runs(nlink_runs(pixfmt, scale_z, sigma2), nlut, d_lz, nullptr, s));
-  }
   if (M.lut_lambda_t != m.lambda_t) {
     M.lut_lambda_t = -1;
-    JFC_B(expand_runs(tlink_runs(m.lambda_t), JFC_TQ + 1, M.d_lut_s, M.d_lut_t, s));
+    const TableRuns rt = tlink_runs(m.lambda_t);
+    M.lut_t_max = rt.val.front();   // (non-increasing)
+    JFC_B(expand_runs(rt, JFC_TQ + 1, M.d_lut_t, M.lut_t_max < 256 ? M.d_lut_t8 : nullptr, s));
     M.lut_lambda_t = m.lambda_t;
   }
-  JFC_B(cudaMemcpyAsync(&km, &d_bs->km, sizeof(km), cudaMemcpyDeviceToHost, s));
-  JFC_B(cudaStreamSynchronize(s));
-  if (km.error) { cleanup(); return set_error(JFC_ERR_CUDA, "a device-side wait timed out in the colour models"); }
-  const int (&mu)[2][JFC_MAX_K * 3] = km.mu;
-  const int k[2] = {km.k[0], km.k[1]};
+  const TableRuns rxy = nlink_runs(pixfmt, scale_xy, sigma2);
+  const TableRuns rz = G->dims == 3 ? nlink_runs(pixfmt, scale_z, sigma2) : TableRuns(1, [](int) { return 0; });
+  NlinkTables nl;
+  nl.nxy = rxy.start.back() + 1;
+  nl.nz = rz.start.back() + 1;
+  const bool bytes = M.lut_t_max < 256 && rxy.val.front() < 256 && rz.val.front() < 256 &&
+                     build_tables_fit(G->dims, nl.nxy, nl.nz);
+  const int nlut = nlink_entries(pixfmt);
+  const size_t each = bytes ? align256(std::max(nl.nxy, nl.nz)) : align256(sizeof(int) * (size_t)nlut);
+  char* d_nl = nullptr;
+  JFC_B(cudaMallocAsync((void**)&d_nl, 2 * each, s));
+  temps.push_back(d_nl);
+  if (bytes) {
+    nl.xy8 = (uint8_t*)d_nl;
+    nl.z8 = (uint8_t*)d_nl + each;
+    JFC_B(expand_runs(rxy, nl.nxy, nullptr, (uint8_t*)nl.xy8, s));
+    if (G->dims == 3) JFC_B(expand_runs(rz, nl.nz, nullptr, (uint8_t*)nl.z8, s));
+  } else {
+    nl.xy = (int*)d_nl;
+    nl.z = (int*)(d_nl + each);
+    JFC_B(expand_runs(rxy, nlut, (int*)nl.xy, nullptr, s));
+    if (G->dims == 3) JFC_B(expand_runs(rz, nlut, (int*)nl.z, nullptr, s));
+  }
+  // the centres stay on the device (warm edits read them too)
+  JFC_B(cudaMemcpyAsync(M.d_mu, d_bs->km.mu, sizeof(km.mu), cudaMemcpyDeviceToDevice, s));
 
   BuildModelDev bm{};
-  bm.pixfmt = pixfmt; bm.channels = C; bm.kf = k[0]; bm.kb = k[1]; bm.seed_cap = m.seed_cap;
-  std::memcpy(bm.mu_f, mu[0], sizeof(bm.mu_f));
-  std::memcpy(bm.mu_b, mu[1], sizeof(bm.mu_b));
-  JFC_B(launch_build_graph(G->g, M.d_img, M.d_seeds, bm, d_lxy, d_lz ? d_lz : d_lxy, M.d_lut_s, M.d_lut_t,
-                           &d_bs->sink, s));
+  bm.pixfmt = pixfmt; bm.channels = C; bm.kf = km.k[0]; bm.kb = km.k[1]; bm.seed_cap = m.seed_cap;
+  JFC_B(launch_build_graph(G->g, M.d_img, M.d_seeds, bm, M.d_mu, nl, M.d_lut_t, M.d_lut_t8, &d_bs->sink, s));
   JFC_B(cudaMemcpyAsync(&hbs.sink, &d_bs->sink, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+  JFC_B(cudaMemcpyAsync(&km.error, &d_bs->km.error, sizeof(int), cudaMemcpyDeviceToHost, s));
   JFC_B(cudaStreamSynchronize(s));
 #undef JFC_B
   cleanup();
+  if (km.error) return set_error(JFC_ERR_CUDA, "a device-side wait timed out in the colour models");
   M.m = bm;
   M.valid = true;
   G->sink_total = (long long)hbs.sink;
@@ -461,7 +475,6 @@ void jfc_graph_destroy(jfc_graph* G) {
   if (G->d_state) cudaFree(G->d_state);
   if (G->model.d_img) cudaFree(G->model.d_img);
   if (G->model.d_seeds) cudaFree(G->model.d_seeds);
-  if (G->model.d_lut_s) cudaFree(G->model.d_lut_s);
   if (G->model.d_lut_t) cudaFree(G->model.d_lut_t);
   delete G;
 }
@@ -474,7 +487,6 @@ void graph_release(jfc_graph* G, cudaStream_t s) {
   if (G->d_state) cudaFreeAsync(G->d_state, s);
   if (G->model.d_img) cudaFreeAsync(G->model.d_img, s);
   if (G->model.d_seeds) cudaFreeAsync(G->model.d_seeds, s);
-  if (G->model.d_lut_s) cudaFreeAsync(G->model.d_lut_s, s);
   if (G->model.d_lut_t) cudaFreeAsync(G->model.d_lut_t, s);
   delete G;
 }
@@ -696,7 +708,7 @@ int jfc_graph_edit_seeds(jfc_graph* G, const uint32_t* idx, const uint8_t* new_s
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_new, new_seed, m, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_ds, 0, sizeof(long long), s);
   if (e == cudaSuccess)
-    e = launch_edit_seeds(G->g, G->model.d_img, G->model.d_seeds, G->model.m, G->model.d_lut_s,
+    e = launch_edit_seeds(G->g, G->model.d_img, G->model.d_seeds, G->model.m, G->model.d_mu,
                           G->model.d_lut_t, d_idx, d_new, m, d_ds, s);
   long long ds = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&ds, d_ds, sizeof(ds), cudaMemcpyDeviceToHost, s);
