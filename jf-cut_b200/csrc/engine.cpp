@@ -159,8 +159,8 @@ static bool encode_pr_maps(const GridDev& g, int ty, int tz, CUtensorMap* out) {
   return true;
 }
 
-// Carve the control block for cap_tiles tiles / cap_grids grids (and, in 2D
-// sets, cap_rw row words and cap_reg regions of the global relabel).
+// Carve the control block for cap_tiles tiles / cap_grids grids (and cap_rw
+// uint4 of row words, cap_reg regions of the global relabel).
 static void tileset_carve(TileSet& ts, char* blk, size_t* total) {
   const size_t nt = (size_t)ts.cap_tiles, ng = (size_t)ts.cap_grids;
   const size_t nr = (size_t)ts.cap_reg;
@@ -237,11 +237,11 @@ int tileset_build(TileSet& ts, int dims, int tile_rows, int tile_depth, const st
     base += g.tiles_x * g.tiles_y * g.tiles_z;
   }
   const int ntiles = base, ngrids = (int)grids.size();
-  // regions and row words of the 2D global relabel
+  // row words (2D: level-set state, 3D: twice that, the words themselves) and
+  // regions of the global relabel
   std::vector<int4> regs;
-  long long nrw = 0;
+  const long long nrw = dims == 2 ? (long long)ntiles * TY : 2ll * ntiles * TY * TZ;
   if (dims == 2) {
-    nrw = (long long)ntiles * TY;
     for (int gi = 0; gi < ngrids; ++gi) {
       const GridDev& g = grids[gi];
       const int rx = (g.tiles_x + JFC_WAVE_WORDS - 1) / JFC_WAVE_WORDS, first = (int)regs.size();
@@ -398,14 +398,15 @@ static cudaError_t enqueue_bfs(TileSet& ts, bool cut, int max_passes, cudaStream
     JFC_E(launch_wave_cut(ts, max_passes, s));
     return cudaMemcpyAsync(pin, ts.d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s);
   }
-  JFC_E(cudaMemsetAsync(ts.d_flag_bfs[0], 0, sizeof(int) * (size_t)ts.ntiles, s));
-  JFC_E(cudaMemsetAsync(ts.d_flag_bfs[1], 0, sizeof(int) * (size_t)ts.ntiles, s));
-  if (!cut) JFC_E(cudaMemsetAsync(ts.d_grid_active, 0, sizeof(int) * ts.ngrids, s));
-  // reset the BFS part of the control block: tickets, frontiers, status, cut flag
-  JFC_E(cudaMemsetAsync(ts.d_ctr->ticket, 0, sizeof(ts.d_ctr->ticket), s));
-  JFC_E(cudaMemsetAsync(ts.d_ctr->qn_bfs, 0, sizeof(ts.d_ctr->qn_bfs), s));
-  JFC_E(cudaMemsetAsync(&ts.d_ctr->bfs_status, 0, sizeof(int), s));
-  if (cut) JFC_E(cudaMemsetAsync(&ts.d_ctr->cut_bad, 0, sizeof(int), s));
+  if (cut) {
+    // reset the BFS part of the control block: tickets, frontiers, status, cut flag
+    JFC_E(cudaMemsetAsync(ts.d_flag_bfs[0], 0, sizeof(int) * (size_t)ts.ntiles, s));
+    JFC_E(cudaMemsetAsync(ts.d_flag_bfs[1], 0, sizeof(int) * (size_t)ts.ntiles, s));
+    JFC_E(cudaMemsetAsync(ts.d_ctr->ticket, 0, sizeof(ts.d_ctr->ticket), s));
+    JFC_E(cudaMemsetAsync(ts.d_ctr->qn_bfs, 0, sizeof(ts.d_ctr->qn_bfs), s));
+    JFC_E(cudaMemsetAsync(&ts.d_ctr->bfs_status, 0, sizeof(int), s));
+    JFC_E(cudaMemsetAsync(&ts.d_ctr->cut_bad, 0, sizeof(int), s));
+  }
   JFC_E(launch_bfs(ts, cut, max_passes, s));
   JFC_E(cudaMemcpyAsync(pin, ts.d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s));
   if (!cut)

@@ -98,8 +98,10 @@ struct TileSet {
   int* d_q_bfs[2] = {nullptr, nullptr};     // [buffer] BFS frontiers
   uint8_t* d_act = nullptr;          // [ntiles] bits 0-1: tile (half) held an active node at its last
                                      // relabel visit
-  // 2D global relabel (kernels_wave.cu; null in 3D sets)
-  uint4* d_vf = nullptr;             // [row words] two buffers of level-set state
+  // global relabel
+  uint4* d_vf = nullptr;             // 2D: [row words] two buffers of level-set state
+                                     // (kernels_wave.cu); 3D: [row words][2] arcs and excess
+                                     // signs (kernels_bfs.cu)
   int4* d_reg = nullptr;             // [nreg] {grid, region x, region y, first region of the grid}
   unsigned* d_rrec = nullptr;        // [nreg] phase << 1 | buffer that holds the region's state
   uint8_t* d_rflag[2] = {nullptr, nullptr};   // [phase & 1][nreg] the region takes part in the phase

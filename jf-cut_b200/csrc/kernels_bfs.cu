@@ -26,6 +26,8 @@
 // once with ballots, row closure by 5-step shift doubling, rows combined by
 // word AND/OR.  Reaching a deficit raises cut_bad (the reference's done[1]
 // divergence flag).
+#include <algorithm>
+
 #include "jfc_relax.cuh"
 #include "jfc_tma.cuh"
 
@@ -472,154 +474,197 @@ __device__ __forceinline__ void tile_close(int (&hv)[TY * TZ], const unsigned (&
   }
 }
 
-// First pass of the global relabel, one warp per tile: a bit-parallel BFS
-// from the deficit nodes.  Each tile row is a 32-bit word (bit = lane); the
-// level-d frontier expands through the residual-arc masks in a few word
-// operations per row, so a tile costs (levels x rows) word ops and no block
-// barrier.  Halo nodes count as sources only when they are deficits
-// (h = 0 in this pass); everything later passes refine.  (A min-plus closure
-// of the tile instead of the level steps measured slower here: the deficits
-// lie close, so few levels run, and the pass streams its loads.)
+// Row words of a 3D set, two uint4 per row segment of 32 nodes (bit = column):
+// {+x, +y, +z, -z residual arcs}, {-y, -x residual arcs, deficit (e < 0), excess
+// (e > 0)}; the cut keeps the reached nodes in the last word.
+__device__ __forceinline__ uint4* row_words(const TileSet& ts, const GridDev& g, long long first, int y, int z, int c) {
+  return ts.d_vf + 2 * (first + ((long long)z * g.Hp + y) * g.tiles_x + c);
+}
+
+// Row words and arc bytes of the tiles that something changed since the last
+// relabel (28 bytes per node read; later passes read 1), one warp per tile; the
+// relabel's counters reset.
 template <int TY, int TZ>
-__device__ __forceinline__ void relabel_first_warp(const TileSet& ts, int tid, const BfsQ& Q, int& cur_grid,
-                                                   int& delta) {
-  constexpr int DIMS = 3;
-  using D = Dirs<DIMS>;
+__global__ void __launch_bounds__(256, TY * TZ > 8 ? 1 : 2) k_bits3(TileSet ts) {
   constexpr int R = TY * TZ;
+  using D = Dirs<3>;
+  DevCounters* ctr = ts.d_ctr;
   const int lane = threadIdx.x & 31;
+  const long long gt = blockIdx.x * (long long)blockDim.x + threadIdx.x, gn = (long long)gridDim.x * blockDim.x;
+  if (gt == 0) {
+    ctr->t_gr_start = jfc::global_ns();
+    ctr->bfs_status = 0;
+    ctr->ticket[0] = ctr->ticket[1] = 0;
+    ctr->qn_bfs[0] = ctr->qn_bfs[1] = 0;
+  }
+  for (long long i = gt; i < ts.ngrids; i += gn) ts.d_grid_active[i] = 0;
+  for (long long t0 = gt - lane; t0 < ts.ntiles; t0 += gn) {
+    unsigned todo = __ballot_sync(FULL, t0 + lane < ts.ntiles && ts.d_dirty[t0 + lane] != 0);
+    while (todo) {
+      const long long tid = t0 + __ffs(todo) - 1;
+      todo &= todo - 1;
+      const int4 ti = ts.d_info[tid];
+      const GridDev& g = ts.d_desc[ti.x];
+      const Addr a = make_addr<3, TY, TZ>(g, ti, lane);
+      int e[R], r[6][R];
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        const long long n = roff<TY>(a, i);
+        e[i] = g.e[n];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) r[k][i] = g.r[k][n];
+      }
+      uint4 w0 = make_uint4(0, 0, 0, 0), w1 = w0;
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        unsigned m[6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) m[k] = __ballot_sync(FULL, r[k][i] > 0);
+        const unsigned neg = __ballot_sync(FULL, e[i] < 0), pos = __ballot_sync(FULL, e[i] > 0);
+        if (lane == i) {
+          w0 = make_uint4(m[D::XP], m[D::YP], m[D::ZP], m[D::ZM]);
+          w1 = make_uint4(m[D::YM], m[D::XM], neg, pos);
+        }
+        g.label[roff<TY>(a, i)] =
+            (uint8_t)((r[D::XP][i] > 0 ? jfc::A_XP : 0u) | (r[D::YP][i] > 0 ? jfc::A_YP : 0u) |
+                      (r[D::YM][i] > 0 ? jfc::A_YM : 0u) | (r[D::XM][i] > 0 ? jfc::A_XM : 0u) |
+                      (r[D::ZP][i] > 0 ? jfc::A_ZP : 0u) | (r[D::ZM][i] > 0 ? jfc::A_ZM : 0u) |
+                      (e[i] < 0 ? 64u : 0u) | (e[i] > 0 ? 128u : 0u));
+      }
+      if (lane < R) {
+        uint4* w = row_words(ts, g, (long long)g.tile_base * R, a.y0 + lane % TY, a.z0 + lane / TY, ti.y);
+        w[0] = w0;
+        w[1] = w1;
+      }
+      if (lane == 0) ts.d_dirty[tid] = 0;
+    }
+  }
+}
+
+// First pass of the global relabel: in every tile a bit-parallel level BFS from
+// its deficits (and from the deficits beside it), on the row words.  A lane
+// holds one row, so a warp expands 32 / R tiles at once, a dozen word operations
+// and four shuffles per level; 5 + 1 bits of level are kept per node and turned
+// into heights 4 columns a lane.  A row of heights is written only where it
+// differs from what the plane holds.  One byte of words and 4 bytes of heights
+// read per node: with a warp per tile and every lane holding every row's words
+// the pass took 2.2 ms on 2560 x 1440 x 50 (28 bytes read, 5 written per node,
+// 32 times the same word operations), with k_bits3 it takes 0.48 (few tiles
+// changed) to 0.78 ms (1.5 on a solve's first, which reads all planes).
+template <int TY, int TZ>
+__global__ void __launch_bounds__(256, 4) k_relabel_first(TileSet ts) {
+  constexpr int R = TY * TZ, G = 32 / R, kPlanes = R > 8 ? 10 : 9;   // tiles a warp; bits of a level (at most 32 R)
+  struct Row { unsigned v, def, p[kPlanes]; };
+  __shared__ Row s_row[8][32];
+  DevCounters* ctr = ts.d_ctr;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int tid = (int)min(w * G + lane / R, (long long)ts.ntiles - 1);
+  const bool ok = w * G + lane / R < ts.ntiles;
+  if (w * G >= ts.ntiles) return;
+  const int r = lane % R, y = r % TY, z = r / TY;
   const int4 ti = ts.d_info[tid];
   const GridDev& g = ts.d_desc[ti.x];
-  const Addr a = make_addr<DIMS, TY, TZ>(g, ti, lane);
-  unsigned AXP[R], AXM[R], AYP[R], AYM[R], AZP[DIMS == 3 ? R : 1], AZM[DIMS == 3 ? R : 1];
-  unsigned DEF[R], POS[R], V[R], F[R];
-  // each node as one byte (arc bits, bit 6 e < 0, bit 7 e > 0); the row
-  // masks come from it
+  const int gy = ti.z * TY + y, gz = ti.w * TZ + z;
+  const long long first = (long long)g.tile_base * R;
+  const bool xl = ti.y > 0, xr = ti.y + 1 < g.tiles_x, yt = gy > 0, yb = gy + 1 < g.Hp, zt = gz > 0, zb = gz + 1 < g.Dp;
+  uint4 w0 = make_uint4(0, 0, 0, 0), w1 = w0;
+  unsigned s1 = 0;   // nodes with a residual arc into a deficit outside the tile
+  if (ok) {
+    const uint4* rw = row_words(ts, g, first, gy, gz, ti.y);
+    w0 = rw[0];
+    w1 = rw[1];
+    auto neg = [&](int dy, int dz, int dc) { return row_words(ts, g, first, gy + dy, gz + dz, ti.y + dc)[1].z; };
+    if (xl) s1 |= neg(0, 0, -1) >> 31 & w1.y;
+    if (xr) s1 |= neg(0, 0, 1) << 31 & w0.x;
+    if (y == 0 && yt) s1 |= neg(-1, 0, 0) & w1.x;
+    if (y == TY - 1 && yb) s1 |= neg(1, 0, 0) & w0.y;
+    if (z == 0 && zt) s1 |= neg(0, -1, 0) & w0.w;
+    if (z == TZ - 1 && zb) s1 |= neg(0, 1, 0) & w0.z;
+  }
+  const unsigned def = w1.z, pos = w1.w;
+  unsigned V = def, F = def, P[kPlanes];
 #pragma unroll
-  for (int i = 0; i < R; ++i) {
-    const long long n = roff<TY>(a, i);
-    const int e = g.e[n];
-    unsigned b = (g.r[D::XP][n] > 0 ? jfc::A_XP : 0u) | (g.r[D::YP][n] > 0 ? jfc::A_YP : 0u) |
-                 (g.r[D::YM][n] > 0 ? jfc::A_YM : 0u) | (g.r[D::XM][n] > 0 ? jfc::A_XM : 0u) |
-                 (e < 0 ? 64u : 0u) | (e > 0 ? 128u : 0u);
-    if constexpr (DIMS == 3)
-      b |= (g.r[D::ZP][n] > 0 ? jfc::A_ZP : 0u) | (g.r[D::ZM][n] > 0 ? jfc::A_ZM : 0u);
-    AXP[i] = __ballot_sync(FULL, b & jfc::A_XP);
-    AXM[i] = __ballot_sync(FULL, b & jfc::A_XM);
-    AYP[i] = __ballot_sync(FULL, b & jfc::A_YP);
-    AYM[i] = __ballot_sync(FULL, b & jfc::A_YM);
-    if constexpr (DIMS == 3) {
-      AZP[i] = __ballot_sync(FULL, b & jfc::A_ZP);
-      AZM[i] = __ballot_sync(FULL, b & jfc::A_ZM);
+  for (int b = 0; b < kPlanes; ++b) P[b] = 0;
+  const int dmax = jfc::cap_of(g, ctr) - 1;   // (levels at or above the cap stay unreachable)
+  int d = 1;
+  for (; d <= 32 * R; ++d) {
+    const unsigned up = __shfl_up_sync(FULL, F, 1), dn = __shfl_down_sync(FULL, F, 1);
+    unsigned m = (F >> 1 & w0.x) | (F << 1 & w1.y);
+    if (y > 0) m |= up & w1.x;
+    if (y < TY - 1) m |= dn & w0.y;
+    if constexpr (TZ > 1) {
+      const unsigned fr = __shfl_down_sync(FULL, F, TY), bk = __shfl_up_sync(FULL, F, TY);
+      if (z < TZ - 1) m |= fr & w0.z;
+      if (z > 0) m |= bk & w0.w;
     }
-    DEF[i] = __ballot_sync(FULL, b & 64u);
-    POS[i] = __ballot_sync(FULL, b & 128u);
-    V[i] = DEF[i];
-    F[i] = DEF[i];
+    if (d == 1) m |= s1;
+    const unsigned N = d <= dmax ? m & ~V : 0u;
+    if (!__any_sync(FULL, N != 0u)) break;
+    V |= N;
+    F = N;
+#pragma unroll
+    for (int b = 0; b < kPlanes; ++b)
+      if (d >> b & 1) P[b] |= N;
   }
-  // level-1 seeds: nodes with a residual arc into a deficit halo node
-  unsigned S1[R];
+  const int bits = 32 - __clz(d);   // of the levels that occur
+  Row& o = s_row[warp][lane];
+  o.v = V;
+  o.def = def;
 #pragma unroll
-  for (int i = 0; i < R; ++i) S1[i] = 0u;
+  for (int b = 0; b < kPlanes; ++b) o.p[b] = P[b];
+  int* const hrow = ok ? g.h + (long long)ti.y * 32 + (long long)gy * g.pitch + (long long)gz * g.pitch * g.Hp : nullptr;
+  __syncwarp();
+#pragma unroll 2
+  for (int k = 0; k < 8; ++k) {
+    const int row = 4 * k + (lane >> 3), sh = 4 * (lane & 7);
+    int* h = reinterpret_cast<int*>(__shfl_sync(FULL, (unsigned long long)hrow, row));
+    const Row& q = s_row[warp][row];
+    if (!h) continue;
+    const int4 old = *reinterpret_cast<const int4*>(h + sh);
+    const unsigned vn = q.v >> sh & 15u, dn = q.def >> sh & 15u;
+    unsigned lo = 0, hi = 0;   // the 4 columns' levels, a byte each
 #pragma unroll
-  for (int z = 0; z < TZ; ++z) {
-    const long long n = roff<TY>(a, z * TY);
-    const bool t0 = a.has_yT && g.e[n - a.pitch] < 0;
-    const bool t1 = a.has_yB && g.e[n + (long long)TY * a.pitch] < 0;
-    S1[z * TY] |= __ballot_sync(FULL, t0) & AYM[z * TY];
-    S1[z * TY + TY - 1] |= __ballot_sync(FULL, t1) & AYP[z * TY + TY - 1];
-  }
-  if constexpr (DIMS == 3) {
+    for (int b = 0; b < 8; ++b)
+      if (b < bits) lo |= (((q.p[b] >> sh & 15u) * 0x00204081u) & 0x01010101u) << b;
+    if (bits > 8) {
 #pragma unroll
-    for (int y = 0; y < TY; ++y) {
-      const long long n = roff<TY>(a, y);
-      const bool t0 = a.has_zT && g.e[n - a.slab] < 0;
-      const bool t1 = a.has_zB && g.e[n + (long long)TZ * a.slab] < 0;
-      S1[y] |= __ballot_sync(FULL, t0) & AZM[y];
-      S1[(TZ - 1) * TY + y] |= __ballot_sync(FULL, t1) & AZP[(TZ - 1) * TY + y];
+      for (int b = 8; b < kPlanes; ++b) hi |= (((q.p[b] >> sh & 15u) * 0x00204081u) & 0x01010101u) << (b - 8);
     }
+    auto val = [&](int c) -> int {
+      const int l = (int)(lo >> (8 * c) & 255u) | (int)(hi >> (8 * c) & 255u) << 8;
+      return dn >> c & 1u ? 0 : vn >> c & 1u ? l : JFC_INF;
+    };
+    const int4 nw = make_int4(val(0), val(1), val(2), val(3));
+    if (nw.x != old.x || nw.y != old.y || nw.z != old.z || nw.w != old.w) *reinterpret_cast<int4*>(h + sh) = nw;
   }
-  {
-    const int row = lane & 15;
-    const bool left = lane < 16;
-    bool sdef = false;
-    if (row < R && (left ? a.has_xL : a.has_xR)) {
-      const long long n = (long long)(left ? a.x0 - 1 : a.x0 + 32) +
-                          (long long)(a.y0 + row % TY) * a.pitch + (long long)(a.z0 + row / TY) * a.slab;
-      sdef = g.e[n] < 0;
-    }
-    const unsigned sb = __ballot_sync(FULL, sdef);
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      S1[i] |= ((sb >> i) & 1u) & AXM[i];
-      S1[i] |= (((sb >> (16 + i)) & 1u) << 31) & AXP[i];
-    }
+  // ---- activity, and the neighbours whose halo holds news (finite and above 0)
+  const unsigned group = (R == 32 ? FULL : (1u << R) - 1u) << (lane / R * R);
+  const unsigned fin = ok ? V & ~def : 0u;
+  const bool act = (__ballot_sync(FULL, ok && (pos & V) != 0u) & group) != 0u;
+  const unsigned bx0 = __ballot_sync(FULL, (fin & 1u) != 0u), bx1 = __ballot_sync(FULL, fin >> 31 != 0u);
+  const unsigned by0 = __ballot_sync(FULL, y == 0 && fin), by1 = __ballot_sync(FULL, y == TY - 1 && fin);
+  const unsigned bz0 = __ballot_sync(FULL, z == 0 && fin), bz1 = __ballot_sync(FULL, z == TZ - 1 && fin);
+  const int txs = g.tiles_x, txy = g.tiles_x * g.tiles_y;
+  bool want = false;
+  int nb = tid;
+  switch (ok ? r : 7) {
+    case 0: want = (bx0 & group) && xl; nb = tid - 1; break;
+    case 1: want = (bx1 & group) && xr; nb = tid + 1; break;
+    case 2: want = (by0 & group) && ti.z > 0; nb = tid - txs; break;
+    case 3: want = (by1 & group) && ti.z + 1 < g.tiles_y; nb = tid + txs; break;
+    case 4: want = (bz0 & group) && ti.w > 0; nb = tid - txy; break;
+    case 5: want = (bz1 & group) && ti.w + 1 < g.tiles_z; nb = tid + txy; break;
+    default: break;
   }
-  // the frontier passes read one byte per node instead of e and the residual
-  // planes: bits 0-5 residual arcs (jfc::A_*), bit 6 e < 0, bit 7 e > 0 (the
-  // label plane is free until the cut BFS writes it)
-#pragma unroll
-  for (int i = 0; i < R; ++i) {
-    unsigned b = ((AXP[i] >> lane) & 1u) * jfc::A_XP | ((AYP[i] >> lane) & 1u) * jfc::A_YP |
-                 ((AYM[i] >> lane) & 1u) * jfc::A_YM | ((AXM[i] >> lane) & 1u) * jfc::A_XM |
-                 ((DEF[i] >> lane) & 1u) * 64u | ((POS[i] >> lane) & 1u) * 128u;
-    if constexpr (DIMS == 3) b |= ((AZP[i] >> lane) & 1u) * jfc::A_ZP | ((AZM[i] >> lane) & 1u) * jfc::A_ZM;
-    g.label[roff<TY>(a, i)] = (uint8_t)b;
+  jfc::warp_append(want, nb, ts.d_flag_bfs[1], ts.d_q_bfs[1], &ctr->qn_bfs[1]);
+  if (ok && r == 0) ts.d_act[tid] = act ? 1 : 0;
+  const unsigned lead = __ballot_sync(FULL, ok && r == 0 && act);
+  if (ts.ngrids == 1) {
+    if (lane == 0 && lead) atomicAdd(&ts.d_grid_active[0], __popc(lead));
+  } else if (ok && r == 0 && act) {
+    atomicAdd(&ts.d_grid_active[ti.x], 1);
   }
-  int h[R];
-#pragma unroll
-  for (int i = 0; i < R; ++i) h[i] = ((DEF[i] >> lane) & 1u) ? 0 : JFC_INF;
-  // level-synchronous expansion: u reaches level d+1 through an arc to a level-d node
-  // (levels at or above the relabel's distance cap stay unreachable)
-  const int dmax = min(32 * R, jfc::cap_of(g, ts.d_ctr) - 1);
-  for (int d = 0; d < dmax; ++d) {
-    unsigned any = 0;
-    unsigned N[R];
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const int y = i % TY, z = i / TY;
-      unsigned m = ((F[i] >> 1) & AXP[i]) | ((F[i] << 1) & AXM[i]);
-      if (y < TY - 1) m |= F[(i + 1 < R) ? i + 1 : i] & AYP[i];
-      if (y > 0) m |= F[(i > 0) ? i - 1 : 0] & AYM[i];
-      if constexpr (DIMS == 3) {
-        if (z < TZ - 1) m |= F[(i + TY < R) ? i + TY : i] & AZP[i];
-        if (z > 0) m |= F[(i >= TY) ? i - TY : 0] & AZM[i];
-      }
-      if (d == 0) m |= S1[i];
-      N[i] = m & ~V[i];
-      any |= N[i];
-    }
-    if (!any) break;
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      V[i] |= N[i];
-      F[i] = N[i];
-      if ((N[i] >> lane) & 1u) h[i] = d + 1;
-    }
-  }
-  unsigned rows_fin = 0, c0 = 0, c31 = 0, act = 0, act_hi = 0;
-#pragma unroll
-  for (int i = 0; i < R; ++i) {
-    g.h[roff<TY>(a, i)] = h[i];
-    const unsigned fin = V[i] & ~DEF[i];   // finite and above 0: news for the neighbours
-    if (fin) rows_fin |= 1u << i;
-    c0 |= fin & 1u;
-    c31 |= fin >> 31;
-    // activity per 8-row half of a 2D 32x16 tile (push-relabel work items)
-    if (DIMS == 2 && TY == 16 && i >= 8) act_hi |= POS[i] & V[i];
-    else act |= POS[i] & V[i];
-  }
-  if (lane == 0) {
-    const int old = 0;
-    ts.d_act[tid] = (uint8_t)((act ? 1 : 0) | (act_hi ? 2 : 0));
-    act |= act_hi;
-    if (ti.x != cur_grid) {
-      if (delta && cur_grid >= 0) atomicAdd(&ts.d_grid_active[cur_grid], delta);
-      delta = 0;
-      cur_grid = ti.x;
-    }
-    delta += (act ? 1 : 0) - old;
-  }
-  flag_neighbours<DIMS, TY, TZ>(g, a, tid, rows_fin, c0 != 0, c31 != 0, false, Q);
 }
 
 // Frontier visit, one warp per tile, min-plus form: the tile's heights in
@@ -813,26 +858,6 @@ __device__ __forceinline__ void refill_pr_queues(const TileSet& ts, DevCounters*
       jfc::warp_append(w[1][1], item0 + 1, nullptr, ts.d_q_pr[1][0], &ctr->qn_pr[1][0]);
     }
   }
-}
-
-// Global relabel, pass 0: every tile, one warp per tile (bit-parallel level
-// BFS from the deficits, fused initialisation).  A plain launch: its many
-// registers do not limit the occupancy of the frontier kernel.
-template <int TY, int TZ>
-__global__ void __launch_bounds__(256, TY * TZ > 8 ? 1 : 2)
-    k_relabel_first(TileSet ts) {
-  DevCounters* ctr = ts.d_ctr;
-  if (blockIdx.x == 0 && threadIdx.x == 0) ctr->t_gr_start = jfc::global_ns();
-  const int lane = threadIdx.x & 31;
-  const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (w >= ts.ntiles) return;
-  // (appends straight to the queue: gathering a CTA's appends behind a block
-  // barrier measured slower, the barrier holds the CTA's slot to its
-  // slowest warp)
-  BfsQ Q{ts.d_flag_bfs[1], ts.d_q_bfs[1], &ctr->qn_bfs[1]};
-  int wgrid = -1, wdelta = 0;
-  relabel_first_warp<TY, TZ>(ts, (int)w, Q, wgrid, wdelta);
-  if (lane == 0 && wdelta && wgrid >= 0) atomicAdd(&ts.d_grid_active[wgrid], wdelta);
 }
 
 // Global relabel, frontier passes (persistent, cooperative): one CTA per
@@ -1085,9 +1110,12 @@ cudaError_t bfs_t(const TileSet& ts, int max_passes, const uint8_t* seeds, cudaS
   static int cache[64] = {0};
   const int blocks = persistent_blocks_cached(cache, fn, nt, dyn);
   if constexpr (!CUT) {
-    const long long fb = ((long long)ts.ntiles * 32 + 255) / 256;
-    jfc_note_launch();
-    k_relabel_first<TY, TZ><<<(unsigned)fb, 256, 0, s>>>(ts);
+    static int cache_bits[64] = {0};
+    const int nb = persistent_blocks_cached(cache_bits, (const void*)k_bits3<TY, TZ>, 256);
+    jfc_note_launch(2);
+    k_bits3<TY, TZ><<<(unsigned)std::min<long long>(nb, ((long long)ts.ntiles + 255) / 256), 256, 0, s>>>(ts);
+    const long long warps = ((long long)ts.ntiles * (TY * TZ) + 31) / 32;
+    k_relabel_first<TY, TZ><<<(unsigned)((warps + 7) / 8), 256, 0, s>>>(ts);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
@@ -1248,6 +1276,11 @@ cudaError_t launch_grid_sums(const TileSet& ts, cudaStream_t s) {
 }
 
 cudaError_t launch_mark_dirty(const TileSet& ts, cudaStream_t s) {
+  // (a 3D relabel finds its frontier flags clear, unless the one before failed)
+  for (int k = 0; k < 2 && ts.dims == 3; ++k) {
+    const cudaError_t e = cudaMemsetAsync(ts.d_flag_bfs[k], 0, sizeof(int) * (size_t)ts.ntiles, s);
+    if (e != cudaSuccess) return e;
+  }
   // (no region of an earlier, failed run takes part in a cut on its own)
   for (int k = 0; k < 2 && ts.nreg > 0; ++k) {
     const cudaError_t e = cudaMemsetAsync(ts.d_rflag[k], 0, (size_t)ts.nreg, s);
