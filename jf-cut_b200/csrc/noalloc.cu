@@ -26,6 +26,7 @@
 //    (cudaGetSymbolAddress, once per device, with that device current); make
 //    that first call before any stream capture begins;
 //  * the caller's current device is restored before the call returns.
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 
@@ -47,14 +48,15 @@ constexpr size_t kOffDesc = kOffLabel + al(kMaxNodes);
 constexpr size_t kOffInfo = kOffDesc + al(sizeof(GridDev));
 constexpr size_t kOffFlagPr = kOffInfo + al(sizeof(int4) * (size_t)kMaxTiles);
 constexpr size_t kOffQPr = kOffFlagPr + kTileI;     // 4 queues
-constexpr size_t kOffGact = kOffQPr + 4 * kTileI;
-constexpr size_t kOffSum = kOffGact + 256;
+constexpr size_t kOffSum = kOffQPr + 4 * kTileI;
+// the control block and, behind it, the grid's active tiles: read back together
 constexpr size_t kOffCtr = kOffSum + 256;
+constexpr size_t kOffGact = kOffCtr + sizeof(DevCounters);
 // regions of the global relabel: the most a grid of kMaxNodes padded nodes has
 // (kMaxNodes / 32 row words; one column of regions 1 word wide, or one row of
 // regions 16 rows high)
 constexpr int kMaxReg = kMaxNodes / (32 * 16) / JFC_WAVE_WORDS + kMaxNodes / 32 / JFC_WAVE_ROWS + 2;
-constexpr size_t kOffDirty = kOffCtr + al(sizeof(DevCounters));
+constexpr size_t kOffDirty = kOffCtr + al(sizeof(DevCounters) + sizeof(int));
 constexpr size_t kOffVf = kOffDirty + al(kMaxTiles);
 constexpr size_t kOffReg = kOffVf + al(sizeof(uint4) * (size_t)(kMaxNodes / 32));
 constexpr size_t kOffRrec = kOffReg + al(sizeof(int4) * (size_t)kMaxReg);
@@ -125,21 +127,26 @@ int na_read(void* host, const void* dev, size_t bytes, cudaStream_t s) {
   return JFC_OK;
 }
 
-int na_bfs(TileSet& ts, const jfc_params& p, bool cut, cudaStream_t s, int* active, int* cut_bad) {
-  if (cut) JFC_CUDA(cudaMemsetAsync(&ts.d_ctr->bfs_status, 0, sizeof(int), s));
-  JFC_CUDA(launch_bfs(ts, cut, p.max_bfs_passes, s));
-  DevCounters hc;
-  int rc = na_read(&hc, ts.d_ctr, sizeof(hc), s);
-  if (rc) return rc;
-  if (hc.error) return set_error(JFC_ERR_CUDA, "a device-side wait timed out in a persistent kernel (grid barrier, worklist or tile staging)");
-  if (hc.bfs_status == 2) return set_error(JFC_ERR_NOT_CONVERGED, "BFS pass budget exhausted");
-  if (!cut) {
-    rc = na_read(active, ts.d_grid_active, sizeof(int), s);
-    if (rc) return rc;
-  } else {
-    *cut_bad = hc.cut_bad;
-  }
+// What a solve reads back, with one wait.
+struct NaRead {
+  DevCounters ctr;
+  int active;
+};
+
+int na_status(const NaRead& r) {
+  if (r.ctr.error) return set_error(JFC_ERR_CUDA, "a device-side wait timed out in a persistent kernel (grid barrier, worklist or tile staging)");
+  if (r.ctr.bfs_status == 2) return set_error(JFC_ERR_NOT_CONVERGED, "BFS pass budget exhausted");
   return JFC_OK;
+}
+
+// One global relabel (behind `sweeps` pairs of push-relabel sweeps when > 0) and
+// its outcome.
+int na_cycle(TileSet& ts, const jfc_params& p, int sweeps, int local_iters, cudaStream_t s, NaRead& r) {
+  if (sweeps > 0) JFC_CUDA(launch_pr_phase(ts, sweeps, local_iters, s));
+  JFC_CUDA(launch_bfs(ts, false, p.max_bfs_passes, s));
+  static_assert(sizeof(DevCounters) % alignof(int) == 0 && sizeof(NaRead) >= sizeof(DevCounters) + sizeof(int), "");
+  int rc = na_read(&r, ts.d_ctr, offsetof(NaRead, active) + sizeof(int), s);
+  return rc ? rc : na_status(r);
 }
 
 }  // namespace
@@ -223,40 +230,50 @@ extern "C" int jfc_solve_grid2d_noalloc(int device, void* stream, const jfc_para
   jfc_note_launch();
   k_na_regions<<<(ts.nreg + 255) / 256, 256, 0, s>>>(ts.d_reg, (g.tiles_x + JFC_WAVE_WORDS - 1) / JFC_WAVE_WORDS, ts.nreg);
   JFC_CUDA(cudaGetLastError());
-  int bad = 0;
-  rc = na_read(&bad, d_bad, sizeof(int), s);
-  if (rc) return rc;
-  if (bad) return set_error(JFC_ERR_INVALID_ARG, "negative n-link capacity");
-  long long sums[2];
   JFC_CUDA(launch_grid_sums(ts, s));
-  rc = na_read(sums, ts.d_grid_sum, sizeof(sums), s);
+  JFC_CUDA(cudaMemcpyAsync((char*)ts.d_grid_sum + 2 * sizeof(long long), d_bad, sizeof(int), cudaMemcpyDeviceToDevice, s));
+  struct { long long sums[2]; int bad; } in;
+  rc = na_read(&in, ts.d_grid_sum, 2 * sizeof(long long) + sizeof(int), s);
   if (rc) return rc;
-  const long long sink_total = (long long)flow_offset - sums[0];  // sum ct
+  if (in.bad) return set_error(JFC_ERR_INVALID_ARG, "negative n-link capacity");
+  const long long sink_total = (long long)flow_offset - in.sums[0];  // sum ct
 
-  // ---- solve: global relabel, push-relabel phases, device-side active count
+  // ---- solve, as engine_solve: relabels capped until no active tile is left,
+  //      then exact; each cycle waits once
   JFC_CUDA(launch_clear_counters(ts, s));
-  if (p.spin_limit > 0) JFC_CUDA(launch_set_limits(ts, (unsigned long long)p.spin_limit, 0, s));
-  int active = 0, sweeps = 0;
-  rc = na_bfs(ts, p, false, s, &active, nullptr);
+  int h_cap = relabel_cap_for(p, 2), sweeps = 0;
+  JFC_CUDA(launch_set_limits(ts, (unsigned long long)p.spin_limit, h_cap, s));
+  JFC_CUDA(launch_prepush(ts, s));
+  const int interval0 = interval_for(p, 2);
+  int interval = interval0;
+  NaRead r;
+  rc = na_cycle(ts, p, 0, 0, s, r);
   if (rc) return rc;
-  while (active > 0) {
-    if (sweeps >= p.max_sweeps) return set_error(JFC_ERR_NOT_CONVERGED, "sweep budget exhausted");
-    JFC_CUDA(launch_pr_phase(ts, interval_for(p, 2), p.local_iters, s));
-    rc = na_bfs(ts, p, false, s, &active, nullptr);
+  for (;;) {
+    while (r.active > 0) {
+      if (sweeps >= p.max_sweeps) return set_error(JFC_ERR_NOT_CONVERGED, "sweep budget exhausted");
+      rc = na_cycle(ts, p, interval, p.local_iters, s, r);
+      if (rc) return rc;
+      sweeps += r.ctr.sweeps_done > 0 ? r.ctr.sweeps_done : 1;
+      interval = (long long)r.active * 256 < ts.ntiles ? std::min(2 * interval, p.relabel_interval_max) : interval0;
+    }
+    if (h_cap == 0) break;
+    h_cap = 0;
+    JFC_CUDA(launch_set_limits(ts, (unsigned long long)p.spin_limit, 0, s));
+    rc = na_cycle(ts, p, 0, 0, s, r);
     if (rc) return rc;
-    int sw = 0;
-    rc = na_read(&sw, &ts.d_ctr->sweeps_done, sizeof(int), s);
-    if (rc) return rc;
-    sweeps += sw > 0 ? sw : 1;
   }
-  int cut_bad = 0;
-  rc = na_bfs(ts, p, true, s, nullptr, &cut_bad);
+  JFC_CUDA(cudaMemsetAsync(&ts.d_ctr->bfs_status, 0, sizeof(int), s));
+  JFC_CUDA(launch_bfs(ts, true, p.max_bfs_passes, s));
+  struct { long long sums[2]; } out;
+  JFC_CUDA(cudaMemcpyAsync(&out, ts.d_grid_sum, sizeof(out), cudaMemcpyDeviceToHost, s));
+  rc = na_read(&r, ts.d_ctr, sizeof(DevCounters), s);
   if (rc) return rc;
-  if (cut_bad) return set_error(JFC_ERR_NOT_CONVERGED, "cut BFS reached a deficit node");
-  rc = na_read(sums, ts.d_grid_sum, sizeof(sums), s);
+  rc = na_status(r);
   if (rc) return rc;
+  if (r.ctr.cut_bad) return set_error(JFC_ERR_NOT_CONVERGED, "cut BFS reached a deficit node");
   JFC_CUDA(na_copy(g.label, d_labels, 1, w, h, pitch, Hp, true, s));
   JFC_CUDA(cudaStreamSynchronize(s));
-  *flow = sink_total + sums[0];
+  *flow = sink_total + out.sums[0];
   return JFC_OK;
 }
