@@ -398,15 +398,6 @@ static cudaError_t enqueue_bfs(TileSet& ts, bool cut, int max_passes, cudaStream
     JFC_E(launch_wave_cut(ts, max_passes, s));
     return cudaMemcpyAsync(pin, ts.d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s);
   }
-  if (cut) {
-    // reset the BFS part of the control block: tickets, frontiers, status, cut flag
-    JFC_E(cudaMemsetAsync(ts.d_flag_bfs[0], 0, sizeof(int) * (size_t)ts.ntiles, s));
-    JFC_E(cudaMemsetAsync(ts.d_flag_bfs[1], 0, sizeof(int) * (size_t)ts.ntiles, s));
-    JFC_E(cudaMemsetAsync(ts.d_ctr->ticket, 0, sizeof(ts.d_ctr->ticket), s));
-    JFC_E(cudaMemsetAsync(ts.d_ctr->qn_bfs, 0, sizeof(ts.d_ctr->qn_bfs), s));
-    JFC_E(cudaMemsetAsync(&ts.d_ctr->bfs_status, 0, sizeof(int), s));
-    JFC_E(cudaMemsetAsync(&ts.d_ctr->cut_bad, 0, sizeof(int), s));
-  }
   JFC_E(launch_bfs(ts, cut, max_passes, s));
   JFC_E(cudaMemcpyAsync(pin, ts.d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s));
   if (!cut)
@@ -550,7 +541,6 @@ int engine_cut(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, std::vector<GridR
   int rc = pin_reserve(ctx, pin_need(ts));
   if (rc) return rc;
   JFC_CUDA(enqueue_bfs(ts, true, p.max_bfs_passes, s, ctx->h_pin));
-  if (ts.dims != 2) JFC_CUDA(launch_grid_sums(ts, s));   // (the 2D cut sums as it labels)
   long long* hs = (long long*)((char*)ctx->h_pin + sizeof(DevCounters));
   JFC_CUDA(cudaMemcpyAsync(hs, ts.d_grid_sum, sizeof(long long) * 2 * ts.ngrids, cudaMemcpyDeviceToHost, s));
   if (done) JFC_CUDA(cudaEventRecord(done, s));

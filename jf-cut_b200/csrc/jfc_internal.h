@@ -76,6 +76,7 @@ struct DevCounters {
   unsigned pr_tail;          // push-relabel worklist: ring positions reserved
   int pr_out;                // push-relabel worklist: items queued and not yet fully visited
   // 2D global relabel (kernels_wave.cu)
+  int cut_n[3];              // 3D cut: blocks queued for pass p, in entry p % 3
   unsigned long long wave_bar; // barrier arrivals (low 40 bits), CTAs that flagged a region (high bits)
   unsigned long long wave_q; // active items queued so far: parity 0 low, parity 1 high 32 bits
 };

@@ -1,31 +1,20 @@
-// kernels_bfs.cu — global relabel, convergence / cut BFS, reductions and
-// layout helpers.
+// kernels_bfs.cu — 3D global relabel and cut, tag BFS, reductions and layout
+// helpers (the 2D relabel and cut: kernels_wave.cu).
 //
 // Global relabel — reference graphcut_init_global_relabel / graphcut_global_relabel
-// (graphcut_global_relabel.cl:19-124 2D, :128-249 3D) driven by QGCWidget::globalRelabel
+// (graphcut_global_relabel.cl:128-249) driven by QGCWidget::globalRelabel
 // (QGCWidget.cpp:2208-2241): heights = exact BFS distance to the deficit nodes
 // (e < 0) over residual arcs, by in-tile fixpoint relaxation with tiles
 // revisited in level sweeps ordered by the jump-flooding tile BFS
 // (graphcut_bfs_block.cl).  Here the relaxation is monotone (heights only fall
-// from INF), so tiles need no parity and no order: a persistent cooperative
-// kernel runs a first pass over every tile (fused initialisation, one warp
-// per tile, bit-parallel level BFS) and then the frontier (a tile whose
-// boundary fell queues its neighbours).  In 2D the frontier starts with a
-// one-warp border check of the tiles the first pass queued and continues as
-// an asynchronous worklist: one CTA per queued tile closes the in-tile
-// distances with warp min-plus scans along rows and columns.  In 3D it runs in
-// passes separated by grid barriers, one warp per queued tile (level BFS
-// seeded by the halo heights).  Each visit records whether the tile holds an
-// active node (e > 0, h < INF): the device-side active-tile count
-// (graphcut_count_node, graphcut_count_block.cl:19-47) that decides
-// convergence, and the queue of tiles the next push-relabel phase visits.
-//
-// Cut — reference graphcut_init_cut / graphcut_compute_cut (graphcut_compute_cut.cl:19-140):
-// the source side is every node reachable from {e > 0} along residual arcs.
-// One warp per tile: R rows of 32-bit words (bit = lane), in-arc masks built
-// once with ballots, row closure by 5-step shift doubling, rows combined by
-// word AND/OR.  Reaching a deficit raises cut_bad (the reference's done[1]
-// divergence flag).
+// from INF), so tiles need no parity and no order: a first pass over every
+// tile (bit-parallel level BFS on row words), then a persistent cooperative
+// kernel drains the frontier (a tile whose boundary fell queues its
+// neighbours) in passes separated by grid barriers, one warp per queued tile.
+// Each visit records whether the tile holds an active node (e > 0, h < INF):
+// the device-side active-tile count (graphcut_count_node,
+// graphcut_count_block.cl:19-47) that decides convergence, and the queue of
+// tiles the next push-relabel phase visits.
 #include <algorithm>
 
 #include "jfc_relax.cuh"
@@ -128,9 +117,9 @@ __device__ __forceinline__ void flag_neighbours(const GridDev& g, const Addr& a,
   }
 }
 
-// ------------------------------------------------------------------ cut BFS
+// ------------------------------------------------------------------ tag BFS
+// bit x reached from bit x - 1 (x + 1) when m bit x is set; closure by doubling
 __device__ __forceinline__ unsigned close_right(unsigned p, unsigned m) {
-  // bit x reached from bit x-1 when m bit x is set; closure by doubling
   p |= (p << 1) & m; m &= m << 1;
   p |= (p << 2) & m; m &= m << 2;
   p |= (p << 4) & m; m &= m << 4;
@@ -147,201 +136,104 @@ __device__ __forceinline__ unsigned close_left(unsigned p, unsigned m) {
   return p;
 }
 
-// TAG: the reference's tag post-process (graphcut_compute_tag.cl) on the same
-// machinery: reachability from the foreground seeds through object nodes
-// (any direction), kept in bit 1 of the label byte; `seeds` is the dense
-// seed array (JFC_SEED_FG = 1).
-template <int DIMS, int TY, int TZ, bool FIRST, bool TAG = false>
-__device__ __forceinline__ void cut_tile(const GridDev& g, int4 ti, int tid, const BfsQ& Q,
-                                         int* __restrict__ bad, const uint8_t* __restrict__ seeds = nullptr) {
-  using D = Dirs<DIMS>;
+// The reference's tag post-process (graphcut_compute_tag.cl): reachability from
+// the foreground seeds through object nodes (any direction), kept in bit 1 of
+// the label byte; `seeds` is the dense seed array (JFC_SEED_FG = 1).  One warp
+// per tile: R rows of 32-bit words (bit = lane), row closure by 5-step shift
+// doubling, rows combined by word AND / OR.
+template <int DIMS, int TY, int TZ, bool FIRST>
+__device__ __forceinline__ void tag_tile(const GridDev& g, int4 ti, int tid, const BfsQ& Q,
+                                         const uint8_t* __restrict__ seeds) {
   constexpr int R = TY * TZ;
   const int lane = threadIdx.x & 31;
   const Addr a = make_addr<DIMS, TY, TZ>(g, ti, lane);
-  const int* __restrict__ E = g.e;
   uint8_t* __restrict__ Lb = g.label;
-  unsigned L[R], L0[R], IXL[R], IXR[R], IYU[R], IYD[R];
-  unsigned IZU[DIMS == 3 ? R : 1], IZD[DIMS == 3 ? R : 1];
-  unsigned NEG[R];
-  // dense index of this lane's node in row i (seed lookup of the tag pass)
-  auto dense = [&](int i) -> long long {
-    return (long long)(a.x0 + lane) + (long long)g.W * ((a.y0 + i % TY) + (long long)g.H * (a.z0 + i / TY));
+  unsigned L[R], L0[R], OBJ[R];   // tagged nodes, object nodes
+  auto is_seed = [&](int x, int y, int z) -> bool {
+    return x < g.W && y < g.H && z < g.D && seeds[x + (long long)g.W * (y + (long long)g.H * z)] == JFC_SEED_FG;
   };
-  auto is_seed = [&](int i) -> bool {
-    const int x = a.x0 + lane, y = a.y0 + i % TY, z = a.z0 + i / TY;
-    return x < g.W && y < g.H && z < g.D && seeds[dense(i)] == JFC_SEED_FG;
-  };
-  unsigned OBJ[TAG ? R : 1];   // object nodes (tag mode)
-  if constexpr (TAG) {
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const unsigned lb = Lb[roff<TY>(a, i)];
-      OBJ[i] = __ballot_sync(FULL, lb & 1u);
-      NEG[i] = 0u;
-      if constexpr (FIRST) L[i] = __ballot_sync(FULL, is_seed(i));
-      else L[i] = __ballot_sync(FULL, (lb & 2u) != 0);
-    }
-    // a node takes the tag from any tagged neighbour when it is an object node
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const int y = i % TY, z = i / TY;
-      IXL[i] = OBJ[i] & ~1u;
-      IXR[i] = OBJ[i] & 0x7fffffffu;
-      IYU[i] = y > 0 ? OBJ[i] : 0u;
-      IYD[i] = y < TY - 1 ? OBJ[i] : 0u;
-      if constexpr (DIMS == 3) {
-        IZU[i] = z > 0 ? OBJ[i] : 0u;
-        IZD[i] = z < TZ - 1 ? OBJ[i] : 0u;
-      }
-    }
-  } else {
-    int rxp[R], ryp[R], rym[R], rxm[R], rzp[DIMS == 3 ? R : 1], rzm[DIMS == 3 ? R : 1];
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const long long n = roff<TY>(a, i);
-      rxp[i] = g.r[D::XP][n]; ryp[i] = g.r[D::YP][n]; rym[i] = g.r[D::YM][n]; rxm[i] = g.r[D::XM][n];
-      if constexpr (DIMS == 3) { rzp[i] = g.r[D::ZP][n]; rzm[i] = g.r[D::ZM][n]; }
-      const int e = E[n];
-      NEG[i] = __ballot_sync(FULL, e < 0);
-      if constexpr (FIRST) L[i] = __ballot_sync(FULL, e > 0);
-      else L[i] = __ballot_sync(FULL, Lb[n] != 0);
-    }
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const int y = i % TY, z = i / TY;
-      const int fl = __shfl_up_sync(FULL, rxp[i], 1);
-      const int fr = __shfl_down_sync(FULL, rxm[i], 1);
-      IXL[i] = __ballot_sync(FULL, lane > 0 && fl > 0);
-      IXR[i] = __ballot_sync(FULL, lane < 31 && fr > 0);
-      IYU[i] = (y > 0) ? __ballot_sync(FULL, ryp[(i > 0) ? i - 1 : 0] > 0) : 0u;
-      IYD[i] = (y < TY - 1) ? __ballot_sync(FULL, rym[(i + 1 < R) ? i + 1 : i] > 0) : 0u;
-      if constexpr (DIMS == 3) {
-        IZU[i] = (z > 0) ? __ballot_sync(FULL, rzp[(i >= TY) ? i - TY : 0] > 0) : 0u;
-        IZD[i] = (z < TZ - 1) ? __ballot_sync(FULL, rzm[(i + TY < R) ? i + TY : i] > 0) : 0u;
-      }
-    }
+  for (int i = 0; i < R; ++i) {
+    const unsigned lb = Lb[roff<TY>(a, i)];
+    OBJ[i] = __ballot_sync(FULL, lb & 1u);
+    if constexpr (FIRST) L[i] = __ballot_sync(FULL, is_seed(a.x0 + lane, a.y0 + i % TY, a.z0 + i / TY));
+    else L[i] = __ballot_sync(FULL, (lb & 2u) != 0);
+    L0[i] = L[i];
   }
-#pragma unroll
-  for (int i = 0; i < R; ++i) L0[i] = L[i];
-  // sources entering through the halo: neighbour reached and its arc toward us
-  // residual (cut), or neighbour tagged (tag; the receiving node must be an
-  // object node, applied through the in-masks below)
-  auto halo_lab = [&](long long n) -> bool {
-    if constexpr (TAG) {
-      if constexpr (FIRST) {
-        const long long x = n % g.pitch, yz = n / g.pitch, y = yz % g.Hp, z = yz / g.Hp;
-        return x < g.W && y < g.H && z < g.D && seeds[x + (long long)g.W * (y + (long long)g.H * z)] == JFC_SEED_FG;
-      } else {
-        return (Lb[n] & 2u) != 0;
-      }
+  // a tagged node of the halo (an object node beside it takes the tag)
+  auto halo_tag = [&](long long n) -> bool {
+    if constexpr (FIRST) {
+      const long long yz = n / g.pitch;
+      return is_seed((int)(n % g.pitch), (int)(yz % g.Hp), (int)(yz / g.Hp));
     } else {
-      if constexpr (FIRST) return E[n] > 0;
-      else return Lb[n] != 0;
+      return (Lb[n] & 2u) != 0;
     }
-  };
-  // residual arc from halo node m toward the tile (cut); any neighbour (tag)
-  auto halo_arc = [&](int dir, long long m) -> bool {
-    if constexpr (TAG) return true;
-    else return g.r[dir][m] > 0;
-  };
-  // nodes a halo source may reach: all (cut: the arc decides) or objects (tag)
-  auto objm = [&](int i) -> unsigned {
-    if constexpr (TAG) return OBJ[i];
-    else return FULL;
   };
 #pragma unroll
   for (int z = 0; z < TZ; ++z) {
     const long long n = roff<TY>(a, z * TY);
-    bool s = false;
-    if (a.has_yT) { const long long m = n - a.pitch; s = halo_lab(m) && halo_arc(D::YP, m); }
-    L[z * TY] |= __ballot_sync(FULL, s) & objm(z * TY);
-    s = false;
-    if (a.has_yB) { const long long m = n + (long long)TY * a.pitch; s = halo_lab(m) && halo_arc(D::YM, m); }
-    L[z * TY + TY - 1] |= __ballot_sync(FULL, s) & objm(z * TY + TY - 1);
+    L[z * TY] |= __ballot_sync(FULL, a.has_yT && halo_tag(n - a.pitch)) & OBJ[z * TY];
+    L[z * TY + TY - 1] |= __ballot_sync(FULL, a.has_yB && halo_tag(n + (long long)TY * a.pitch)) & OBJ[z * TY + TY - 1];
   }
   if constexpr (DIMS == 3) {
 #pragma unroll
     for (int y = 0; y < TY; ++y) {
       const long long n = roff<TY>(a, y);
-      bool s = false;
-      if (a.has_zT) { const long long m = n - a.slab; s = halo_lab(m) && halo_arc(D::ZP, m); }
-      L[y] |= __ballot_sync(FULL, s) & objm(y);
-      s = false;
-      if (a.has_zB) { const long long m = n + (long long)TZ * a.slab; s = halo_lab(m) && halo_arc(D::ZM, m); }
-      L[(TZ - 1) * TY + y] |= __ballot_sync(FULL, s) & objm((TZ - 1) * TY + y);
+      L[y] |= __ballot_sync(FULL, a.has_zT && halo_tag(n - a.slab)) & OBJ[y];
+      L[(TZ - 1) * TY + y] |= __ballot_sync(FULL, a.has_zB && halo_tag(n + (long long)TZ * a.slab)) & OBJ[(TZ - 1) * TY + y];
     }
   }
   {
     const int row = lane & 15;
     const bool left = lane < 16;
     bool s = false;
-    if (row < R && (left ? a.has_xL : a.has_xR)) {
-      const long long n = (long long)(left ? a.x0 - 1 : a.x0 + 32) +
-                          (long long)(a.y0 + row % TY) * a.pitch + (long long)(a.z0 + row / TY) * a.slab;
-      s = halo_lab(n) && halo_arc(left ? D::XP : D::XM, n);
-    }
+    if (row < R && (left ? a.has_xL : a.has_xR))
+      s = halo_tag((long long)(left ? a.x0 - 1 : a.x0 + 32) + (long long)(a.y0 + row % TY) * a.pitch +
+                   (long long)(a.z0 + row / TY) * a.slab);
     const unsigned sb = __ballot_sync(FULL, s);
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-      L[i] |= ((sb >> i) & 1u) & objm(i);
-      L[i] |= (((sb >> (16 + i)) & 1u) << 31) & objm(i);
-    }
+    for (int i = 0; i < R; ++i) L[i] |= ((sb >> i & 1u) | (sb >> (16 + i) & 1u) << 31) & OBJ[i];
   }
   bool converged = false;
   for (int it = 0; it < 64; ++it) {
     unsigned ch = 0;
+    auto grow = [&](int i, unsigned p) { ch |= p ^ L[i]; L[i] = p; };
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const unsigned p = close_left(close_right(L[i], IXL[i]), IXR[i]);
-      ch |= p ^ L[i];
-      L[i] = p;
-    }
+    for (int i = 0; i < R; ++i) grow(i, close_left(close_right(L[i], OBJ[i] & ~1u), OBJ[i] & 0x7fffffffu));
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-      if (i % TY > 0) { const unsigned p = L[i] | (L[(i > 0) ? i - 1 : 0] & IYU[i]); ch |= p ^ L[i]; L[i] = p; }
-    }
+    for (int i = 1; i < R; ++i) if (i % TY > 0) grow(i, L[i] | (L[i - 1] & OBJ[i]));
 #pragma unroll
-    for (int i = R - 1; i >= 0; --i) {
-      if (i % TY < TY - 1) { const unsigned p = L[i] | (L[(i + 1 < R) ? i + 1 : i] & IYD[i]); ch |= p ^ L[i]; L[i] = p; }
-    }
+    for (int i = R - 2; i >= 0; --i) if (i % TY < TY - 1) grow(i, L[i] | (L[i + 1] & OBJ[i]));
     if constexpr (DIMS == 3) {
 #pragma unroll
-      for (int i = TY; i < R; ++i) { const unsigned p = L[i] | (L[i - TY] & IZU[i]); ch |= p ^ L[i]; L[i] = p; }
+      for (int i = TY; i < R; ++i) grow(i, L[i] | (L[i - TY] & OBJ[i]));
 #pragma unroll
-      for (int i = R - TY - 1; i >= 0; --i) { const unsigned p = L[i] | (L[i + TY] & IZD[i]); ch |= p ^ L[i]; L[i] = p; }
+      for (int i = R - TY - 1; i >= 0; --i) grow(i, L[i] | (L[i + TY] & OBJ[i]));
     }
     if (!ch) { converged = true; break; }
   }
   unsigned rows_changed = 0, col0 = 0, col31 = 0;
-  bool hit = false;
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     const unsigned c = L[i] ^ L0[i];
     if (c) rows_changed |= 1u << i;
     col0 |= c & 1u;
     col31 |= c >> 31;
-    hit |= (L[i] & NEG[i]) != 0u;
-    if constexpr (TAG) {
-      if (FIRST || c) {
-        uint8_t* p = Lb + roff<TY>(a, i);
-        *p = (uint8_t)((*p & 1u) | (((L[i] >> lane) & 1u) << 1));
-      }
-    } else {
-      if (FIRST || c) Lb[roff<TY>(a, i)] = (uint8_t)((L[i] >> lane) & 1u);
+    if (FIRST || c) {
+      uint8_t* p = Lb + roff<TY>(a, i);
+      *p = (uint8_t)((*p & 1u) | (((L[i] >> lane) & 1u) << 1));
     }
   }
-  if (lane == 0 && hit) *bad = 1;
-  // boundary labels that differ from what the neighbours last read (their
-  // halo read our labels, or our excess in the first pass)
+  // boundary tags that differ from what the neighbours last read
   flag_neighbours<DIMS, TY, TZ>(g, a, tid, rows_changed, col0 != 0, col31 != 0, !converged, Q);
 }
 
-// Persistent cut BFS: pass 0 visits every tile (labels start as e > 0),
-// later passes drain the frontier built by the previous one (one tile per
-// warp ticket), grid barriers in between, until a pass queues nothing or the
-// pass budget runs out.
-template <int DIMS, int TY, int TZ, bool TAG = false>
-__global__ void __launch_bounds__(256) k_cut(TileSet ts, int max_passes, const uint8_t* seeds) {
+// Persistent tag BFS: pass 0 visits every tile (tags start at the seeds), later
+// passes drain the frontier built by the previous one (one tile per warp
+// ticket), grid barriers in between, until a pass queues nothing or the pass
+// budget runs out.
+template <int DIMS, int TY, int TZ>
+__global__ void __launch_bounds__(256) k_tag(TileSet ts, int max_passes, const uint8_t* seeds) {
   DevCounters* ctr = ts.d_ctr;
   const int lane = threadIdx.x & 31;
   unsigned long long visits = 0;
@@ -357,7 +249,7 @@ __global__ void __launch_bounds__(256) k_cut(TileSet ts, int max_passes, const u
       for (int k = 0; k < cnt; ++k) {
         const int tt = (int)b + k;
         const int4 ti = ts.d_info[tt];
-        cut_tile<DIMS, TY, TZ, true, TAG>(ts.d_desc[ti.x], ti, tt, Q, &ctr->cut_bad, seeds);
+        tag_tile<DIMS, TY, TZ, true>(ts.d_desc[ti.x], ti, tt, Q, seeds);
         ++visits;
       }
     }
@@ -381,7 +273,7 @@ __global__ void __launch_bounds__(256) k_cut(TileSet ts, int max_passes, const u
       if (lane == 0) fcur[tt] = 0;
       __syncwarp();
       const int4 ti = ts.d_info[tt];
-      cut_tile<DIMS, TY, TZ, false, TAG>(ts.d_desc[ti.x], ti, tt, Q, &ctr->cut_bad, seeds);
+      tag_tile<DIMS, TY, TZ, false>(ts.d_desc[ti.x], ti, tt, Q, seeds);
       ++visits;
     }
     ok = jfc::grid_sync(ctr, [&]() {
@@ -483,7 +375,7 @@ __device__ __forceinline__ uint4* row_words(const TileSet& ts, const GridDev& g,
 
 // Row words and arc bytes of the tiles that something changed since the last
 // relabel (28 bytes per node read; later passes read 1), one warp per tile; the
-// relabel's counters reset.
+// counters of the relabel or cut that follows reset.
 template <int TY, int TZ>
 __global__ void __launch_bounds__(256, TY * TZ > 8 ? 1 : 2) k_bits3(TileSet ts) {
   constexpr int R = TY * TZ;
@@ -496,8 +388,14 @@ __global__ void __launch_bounds__(256, TY * TZ > 8 ? 1 : 2) k_bits3(TileSet ts) 
     ctr->bfs_status = 0;
     ctr->ticket[0] = ctr->ticket[1] = 0;
     ctr->qn_bfs[0] = ctr->qn_bfs[1] = 0;
+    ctr->cut_n[0] = ctr->cut_n[1] = ctr->cut_n[2] = 0;
+    ctr->cut_bad = 0;
+    ctr->wave_bar = 0;
   }
-  for (long long i = gt; i < ts.ngrids; i += gn) ts.d_grid_active[i] = 0;
+  for (long long i = gt; i < ts.ngrids; i += gn) {
+    ts.d_grid_active[i] = 0;
+    ts.d_grid_sum[2 * i] = ts.d_grid_sum[2 * i + 1] = 0;
+  }
   for (long long t0 = gt - lane; t0 < ts.ntiles; t0 += gn) {
     unsigned todo = __ballot_sync(FULL, t0 + lane < ts.ntiles && ts.d_dirty[t0 + lane] != 0);
     while (todo) {
@@ -1051,6 +949,200 @@ __global__ void __launch_bounds__(256, TY * TZ > 8 ? 2 : JFC_RL3D_MINB)
   }
 }
 
+// Cut of a 3D set (graphcut_init_cut / graphcut_compute_cut,
+// graphcut_compute_cut.cl:74-140): the source side is every node reachable from
+// {e > 0} along residual arcs; reaching a deficit raises cut_bad (the
+// reference's done[1] divergence flag).  On the row words: a warp holds a block
+// of BY x BZ = 32 rows (whole tiles, named by the first of them), a lane one
+// row, so a step closes all rows with a dozen word operations and exchanges the
+// reached nodes with four shuffles.  The reached nodes stay in the rows' last
+// word; only the block's warp writes them and they only grow, so the blocks
+// around may read them at any time.  The first pass visits every block; a block
+// whose border an arc from a newly reached node to an unreached one crosses
+// queues the block behind it for the next pass; a last pass writes the label
+// bytes and sums min(e, 0) and the labels per grid.  What bounds it is the
+// first pass's bytes (1 read per node, 5 in the last) and then the chain of
+// passes.  A pass of a warp per 8-row tile with every row's words in every
+// lane, from e and the arcs (29 bytes per node), and the separate sums took 0.45
+// ms on 317 x 301 x 181 and 4.2 ms on 2560 x 1440 x 50; this takes 0.12 and 0.77
+// (0.20 of it the excess and label planes at the HBM rate).
+template <int TY, int TZ>
+__global__ void __launch_bounds__(256, 4) k_cut3(TileSet ts, int max_passes) {
+  constexpr int BY = TY > 8 ? TY : 8, BZ = 32 / BY, MY = BY / TY, MZ = BZ / TZ;
+  constexpr int kList = 1024, kScan = 8;   // staged appends of a CTA; tiles a warp looks through at once
+  __shared__ int s_list[kList];
+  __shared__ int s_n, s_base;
+  __shared__ unsigned long long s_sum[2], s_vis;
+  DevCounters* ctr = ts.d_ctr;
+  const int t = threadIdx.x, lane = t & 31;
+  const int warp = (int)((blockIdx.x * blockDim.x + t) >> 5), nwarps = (int)(gridDim.x * blockDim.x >> 5);
+  if (t == 0) {
+    s_n = 0;
+    s_sum[0] = s_sum[1] = s_vis = 0;
+  }
+  __syncthreads();
+  struct Row { int y, z; bool ok; uint4* w; };
+  auto row_of = [&](const GridDev& g, int4 ti, int r) {
+    Row q;
+    q.y = ti.z * TY + r % BY;
+    q.z = ti.w * TZ + r / BY;
+    q.ok = q.y < g.Hp && q.z < g.Dp;
+    q.w = row_words(ts, g, (long long)g.tile_base * (TY * TZ), q.y, q.z, ti.y);
+    return q;
+  };
+  // f(tile, info) for every block of this warp
+  auto each_block = [&](auto f) {
+    for (long long t0 = (long long)warp * kScan; t0 < ts.ntiles; t0 += (long long)nwarps * kScan) {
+      const bool in = lane < kScan && t0 + lane < ts.ntiles;
+      const int4 mine = in ? ts.d_info[t0 + lane] : make_int4(0, 0, 0, 0);
+      unsigned todo = __ballot_sync(FULL, in && mine.z % MY == 0 && mine.w % MZ == 0);
+      while (todo) {
+        const int k = __ffs(todo) - 1;
+        todo &= todo - 1;
+        f((int)t0 + k, make_int4(__shfl_sync(FULL, mine.x, k), __shfl_sync(FULL, mine.y, k),
+                                 __shfl_sync(FULL, mine.z, k), __shfl_sync(FULL, mine.w, k)));
+      }
+    }
+  };
+  unsigned visits = 0;
+  int pass = 0;
+  auto visit = [&](int tid, int4 ti) {
+    const GridDev& g = ts.d_desc[ti.x];
+    const Row q = row_of(g, ti, lane);
+    const int y = lane % BY, z = lane / BY;
+    const long long sy = 2ll * g.tiles_x, sz = sy * g.Hp;   // words to the next row, slice
+    uint4 w0 = make_uint4(0, 0, 0, 0), w1 = w0;
+    // words beside the row, and their arcs toward it; what lies behind the block's border
+    unsigned lw = ~0u, rw = ~0u, yw = ~0u, zw = ~0u, la = 0, ra = 0, ya = 0, za = 0;
+    if (q.ok) {
+      w0 = q.w[0];
+      w1 = __ldcg(q.w + 1);
+      if (ti.y > 0) { lw = __ldcg(&q.w[-1].w); la = q.w[-2].x; }
+      if (ti.y + 1 < g.tiles_x) { rw = __ldcg(&q.w[3].w); ra = q.w[3].y; }
+      if (y == 0 && q.y > 0) { yw = __ldcg(&q.w[1 - sy].w); ya = q.w[-sy].y; }
+      if (y == BY - 1 && q.y + 1 < g.Hp) { yw = __ldcg(&q.w[1 + sy].w); ya = q.w[1 + sy].x; }
+      if (z == 0 && q.z > 0) { zw = __ldcg(&q.w[1 - sz].w); za = q.w[-sz].z; }
+      if (z == BZ - 1 && q.z + 1 < g.Dp) { zw = __ldcg(&q.w[1 + sz].w); za = q.w[sz].w; }
+    }
+    const unsigned L0 = w1.w;
+    unsigned L = L0 | (lw & la) >> 31 | (rw & ra) << 31 | (yw & ya) | (zw & za);
+    for (int it = 0; it < 32 * 32; ++it) {   // (a step but the last reaches a node)
+      const unsigned was = L;
+      L = close_left(close_right(L, w0.x << 1), w1.y >> 1);
+      const unsigned up = __shfl_up_sync(FULL, L & w0.y, 1), dn = __shfl_down_sync(FULL, L & w1.x, 1);
+      const unsigned fr = __shfl_up_sync(FULL, L & w0.z, BY), bk = __shfl_down_sync(FULL, L & w0.w, BY);
+      if (y > 0) L |= up;
+      if (y < BY - 1) L |= dn;
+      if (z > 0) L |= fr;
+      if (z < BZ - 1) L |= bk;
+      if (!__any_sync(FULL, L != was)) break;
+    }
+    const unsigned news = L & ~L0;
+    if (news) q.w[1].w = L;
+    if (L & w1.z) ctr->cut_bad = 1;
+    unsigned dirs = (news & w1.y & 1u & ~(lw >> 31)) | ((news & w0.x) >> 31 & ~rw) << 1;
+    if (y == 0 && (news & w1.x & ~yw)) dirs |= 4u;
+    if (y == BY - 1 && (news & w0.y & ~yw)) dirs |= 8u;
+    if (z == 0 && (news & w0.w & ~zw)) dirs |= 16u;
+    if (z == BZ - 1 && (news & w0.z & ~zw)) dirs |= 32u;
+    dirs = __reduce_or_sync(FULL, dirs);
+    if (lane < 6 && (dirs >> lane & 1u)) {
+      const int step = lane < 2 ? 1 : lane < 4 ? MY * g.tiles_x : MZ * g.tiles_x * g.tiles_y;
+      const int nb = lane & 1 ? tid + step : tid - step, b = (pass + 1) & 1;
+      if (atomicExch(ts.d_flag_bfs[b] + nb, 1) == 0) {
+        const int i = atomicAdd(&s_n, 1);
+        if (i < kList) s_list[i] = nb;
+        else ts.d_q_bfs[b][atomicAdd(&ctr->cut_n[(pass + 1) % 3], 1)] = nb;
+      }
+    }
+    ++visits;
+  };
+  bool ok = true;
+  for (;; ++pass) {
+    if (pass == 0) {
+      each_block(visit);
+    } else {
+      const int n = jfc::vload(&ctr->cut_n[pass % 3]);
+      if (n == 0) break;
+      if (pass > max_passes) {
+        if (blockIdx.x == 0 && t == 0) ctr->bfs_status = 2;
+        ok = false;
+        break;
+      }
+      for (int k = warp; k < n; k += nwarps) {
+        const int tid = __ldcg(ts.d_q_bfs[pass & 1] + k);
+        if (lane == 0) ts.d_flag_bfs[pass & 1][tid] = 0;
+        visit(tid, ts.d_info[tid]);
+      }
+      // (every CTA has read the count of the pass before; it is the one after next's)
+      if (blockIdx.x == 0 && t == 0) ctr->cut_n[(pass + 2) % 3] = 0;
+    }
+    __syncthreads();
+    const int staged = min(s_n, kList);
+    if (staged) {
+      if (t == 0) s_base = atomicAdd(&ctr->cut_n[(pass + 1) % 3], staged);
+      __syncthreads();
+      for (int i = t; i < staged; i += blockDim.x) ts.d_q_bfs[(pass + 1) & 1][s_base + i] = s_list[i];
+      __syncthreads();
+      if (t == 0) s_n = 0;
+    }
+    ok = jfc::arrive_wait(ctr, &ctr->wave_bar, (unsigned long long)(pass + 1) * gridDim.x);
+    if (!ok) break;
+  }
+  // ---- labels (4 nodes a lane) and sums
+  if (ok) {
+    long long neg = 0, lab = 0;
+    int cur = 0;
+    auto add = [&]() {
+      for (int o = 16; o; o >>= 1) {
+        neg += __shfl_xor_sync(FULL, neg, o);
+        lab += __shfl_xor_sync(FULL, lab, o);
+      }
+      if (lane == 0 && (neg || lab)) {
+        unsigned long long* sum = ts.ngrids == 1 ? s_sum : (unsigned long long*)ts.d_grid_sum + 2 * cur;
+        atomicAdd(sum, (unsigned long long)neg);
+        atomicAdd(sum + 1, (unsigned long long)lab);
+      }
+      neg = lab = 0;
+    };
+    each_block([&](int, int4 ti) {
+      if (ti.x != cur) {
+        add();
+        cur = ti.x;
+      }
+      const GridDev& g = ts.d_desc[ti.x];
+      const Row q = row_of(g, ti, lane);
+      const unsigned L = q.ok ? __ldcg(&q.w[1].w) : 0u;
+      lab += __popc(L);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int r = 4 * k + (lane >> 3), sh = 4 * (lane & 7);
+        const unsigned nib = __shfl_sync(FULL, L, r) >> sh & 15u;
+        const int ry = ti.z * TY + r % BY, rz = ti.w * TZ + r / BY;
+        if (ry >= g.Hp || rz >= g.Dp) continue;
+        const long long n = (long long)ti.y * 32 + sh + (long long)g.pitch * (ry + (long long)g.Hp * rz);
+        const int4 e = *reinterpret_cast<const int4*>(g.e + n);
+        *reinterpret_cast<unsigned*>(g.label + n) = (nib * 0x00204081u) & 0x01010101u;
+        neg += (long long)min(e.x, 0) + min(e.y, 0) + min(e.z, 0) + min(e.w, 0);
+      }
+    });
+    add();
+  }
+  if (lane == 0) atomicAdd(&s_vis, (unsigned long long)visits * (MY * MZ));
+  __syncthreads();
+  if (t == 0) {
+    if (ok && ts.ngrids == 1) {
+      atomicAdd((unsigned long long*)ts.d_grid_sum, s_sum[0]);
+      atomicAdd((unsigned long long*)ts.d_grid_sum + 1, s_sum[1]);
+    }
+    atomicAdd(&ctr->bfs_visits, s_vis);
+    if (blockIdx.x == 0) {
+      ctr->bfs_passes = pass;
+      if (ok) ctr->bfs_status = 1;
+    }
+  }
+}
+
 // per-grid sum of min(e, 0) and count of source-side nodes (reduce_flow,
 // bin/x64/cl/Infrastructures/reduce.cl:92-117, in int64 instead of int32 partials)
 template <int TY, int TZ>
@@ -1094,33 +1186,39 @@ __global__ void __launch_bounds__(256) k_grid_sums(const GridDev* __restrict__ g
 // MODE 0: global relabel, 1: cut, 2: tag
 template <int DIMS, int TY, int TZ, int MODE>
 cudaError_t bfs_t(const TileSet& ts, int max_passes, const uint8_t* seeds, cudaStream_t s) {
-  constexpr bool CUT = MODE != 0;
   const void* fn;
-  if constexpr (MODE == 1) fn = (const void*)k_cut<DIMS, TY, TZ, false>;
-  else if constexpr (MODE == 2) fn = (const void*)k_cut<DIMS, TY, TZ, true>;
+  if constexpr (MODE == 1) fn = (const void*)k_cut3<TY, TZ>;
+  else if constexpr (MODE == 2) fn = (const void*)k_tag<DIMS, TY, TZ>;
   else fn = (const void*)k_relabel_warp<TY, TZ>;
   const int nt = 256;
   // the 3D frontier's staging buffers: two per warp (dynamic shared memory)
-  const size_t dyn = (!CUT && JFC_RL3D_STAGE && TY * TZ <= 8)
+  const size_t dyn = (MODE == 0 && JFC_RL3D_STAGE && TY * TZ <= 8)
                          ? 2 * 8 * sizeof(RlStage<TY, TZ>) + 128 : 0;
   if (dyn > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
     if (e != cudaSuccess) return e;
   }
   static int cache[64] = {0};
-  const int blocks = persistent_blocks_cached(cache, fn, nt, dyn);
-  if constexpr (!CUT) {
+  int blocks = persistent_blocks_cached(cache, fn, nt, dyn);
+  // (no more CTAs than find blocks: the barrier's cost grows with them)
+  if constexpr (MODE == 1) blocks = std::max(1, std::min(blocks, (ts.ntiles + 63) / 64));
+  if constexpr (MODE != 2) {
     static int cache_bits[64] = {0};
     const int nb = persistent_blocks_cached(cache_bits, (const void*)k_bits3<TY, TZ>, 256);
-    jfc_note_launch(2);
+    jfc_note_launch();
     k_bits3<TY, TZ><<<(unsigned)std::min<long long>(nb, ((long long)ts.ntiles + 255) / 256), 256, 0, s>>>(ts);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  if constexpr (MODE == 0) {
+    jfc_note_launch();
     const long long warps = ((long long)ts.ntiles * (TY * TZ) + 31) / 32;
     k_relabel_first<TY, TZ><<<(unsigned)((warps + 7) / 8), 256, 0, s>>>(ts);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
   TileSet arg = ts;
-  void* params[] = {(void*)&arg, (void*)&max_passes, (void*)&seeds};   // relabel kernels take two
+  void* params[] = {(void*)&arg, (void*)&max_passes, (void*)&seeds};   // relabel and cut take two
   jfc_note_launch();
   return cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(nt), params, dyn, s);
 }
