@@ -394,7 +394,6 @@ static cudaError_t enqueue_bfs(TileSet& ts, bool cut, int max_passes, cudaStream
                            cudaMemcpyDeviceToHost, s);
   }
   if (cut && ts.dims == 2) {
-    JFC_E(cudaMemsetAsync(&ts.d_ctr->bfs_status, 0, sizeof(int), s));
     JFC_E(launch_wave_cut(ts, max_passes, s));
     return cudaMemcpyAsync(pin, ts.d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s);
   }

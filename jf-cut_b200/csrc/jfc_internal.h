@@ -52,11 +52,11 @@ struct DevCounters {
   unsigned bar_count;        // grid barrier arrivals
   unsigned bar_gen;          // grid barrier generation
   int error;                 // a barrier wait timed out: kernels leave, host reports
-  int cut_bad;               // cut BFS reached a deficit node (augmenting path left)
   int qn_pr[2][2];           // push-relabel queue lengths [parity][buffer]
   int cur_pr[2];             // pending buffer per parity
   int qn_bfs[2];             // BFS frontier lengths [buffer]
   int bfs_passes;            // passes of the last BFS
+  int cut_bad;               // cut BFS reached a deficit node (augmenting path left)
   int bfs_status;            // 1 converged, 2 pass budget exhausted
   int sweeps_done;           // sweeps run by the last push-relabel phase
   int pr_sweeps;             // sweep pairs of the next phase when launched with sweeps <= 0
@@ -77,7 +77,8 @@ struct DevCounters {
   int pr_out;                // push-relabel worklist: items queued and not yet fully visited
   // 2D global relabel (kernels_wave.cu)
   int cut_n[3];              // 3D cut: blocks queued for pass p, in entry p % 3
-  unsigned long long wave_bar; // barrier arrivals (low 40 bits), CTAs that flagged a region (high bits)
+  unsigned long long wave_bar[2]; // barrier arrivals (low 40 bits), CTAs that flagged a region (high bits)
+  unsigned wave_epoch;       // launches so far: which of the two the next one uses
   unsigned long long wave_q; // active items queued so far: parity 0 low, parity 1 high 32 bits
 };
 
@@ -153,7 +154,8 @@ void jfc_note_launch(int n = 1);
 // serves every interval
 // sched 2: the asynchronous worklist (needs ts.d_pr_ring) instead of the
 // parity sweeps
-// (the launcher zeroes the phase's tickets and barrier counter first)
+// (a global relabel comes before each: it zeroes the tickets and the barrier
+// counter)
 cudaError_t launch_pr_phase(const TileSet& ts, int sweeps, int local_iters, cudaStream_t s, int sched = 1);
 // Local pre-push inside every tile before the first relabel of a solve.
 cudaError_t launch_prepush(const TileSet& ts, cudaStream_t s);

@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(256, TY * TZ > 8 ? 1 : 2) k_bits3(TileSet ts) 
     ctr->qn_bfs[0] = ctr->qn_bfs[1] = 0;
     ctr->cut_n[0] = ctr->cut_n[1] = ctr->cut_n[2] = 0;
     ctr->cut_bad = 0;
-    ctr->wave_bar = 0;
+    ctr->pr_bar = 0;
   }
   for (long long i = gt; i < ts.ngrids; i += gn) {
     ts.d_grid_active[i] = 0;
@@ -1086,7 +1086,7 @@ __global__ void __launch_bounds__(256, 4) k_cut3(TileSet ts, int max_passes) {
       __syncthreads();
       if (t == 0) s_n = 0;
     }
-    ok = jfc::arrive_wait(ctr, &ctr->wave_bar, (unsigned long long)(pass + 1) * gridDim.x);
+    ok = jfc::arrive_wait(ctr, &ctr->pr_bar, (unsigned long long)(pass + 1) * gridDim.x);
     if (!ok) break;
   }
   // ---- labels (4 nodes a lane) and sums

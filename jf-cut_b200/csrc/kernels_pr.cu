@@ -457,7 +457,7 @@ __device__ __forceinline__ int pr_visit(const TileSet& ts, int tid, const int4& 
 // latencies, so the chain is kept short: which buffer a parity is on follows
 // from the sweep index; the queue's length and the CTA's own entry are one
 // round trip to L2; the barrier is one growing counter (pr_bar, zeroed with
-// the tickets before the phase) whose arrivals are also its release; the
+// the tickets by the relabel before) whose arrivals are also its release; the
 // counters that a sweep leaves are reset by block 0 during the next one.
 // 26 us a sweep before, 19.5 now (4096 x 3072, 200-1,000 active tiles).
 //
@@ -832,10 +832,6 @@ cudaError_t launch_t(const TileSet& ts, int sweeps, int local_iters, cudaStream_
     if (e != cudaSuccess) return e;
   }
   const int blocks = persistent_blocks_cached(async ? cache_async : cache_sweeps, fn, NT, dyn);
-  static_assert(offsetof(DevCounters, ticket) == 0 && offsetof(DevCounters, pr_bar) == sizeof(unsigned) * 2,
-                "tickets and barrier counter are zeroed together");
-  const cudaError_t z = cudaMemsetAsync(ts.d_ctr, 0, offsetof(DevCounters, pr_bar) + sizeof(unsigned long long), st);
-  if (z != cudaSuccess) return z;
   TileSet arg = ts;
   void* params[] = {(void*)&arg, (void*)&sweeps, (void*)&local_iters};
   jfc_note_launch();

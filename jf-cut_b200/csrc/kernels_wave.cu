@@ -11,7 +11,7 @@
 // segment of 32 nodes in its 32 bytes:
 //   0..3  residual arc +x, +y, -y, -x      4, 5  unused
 //   6     deficit (e < 0)                  7     excess (e > 0)
-// k_wave_bits writes them, from 20 bytes per node of e and the four residual
+// changed_tiles writes them, from 20 bytes per node of e and the four residual
 // planes, for the tiles that something changed since the last relabel (a
 // byte per tile, set by the push-relabel visits; every tile at the start of a
 // solve).  All further work of a relabel is on words: 0.75 bytes per node.
@@ -36,6 +36,7 @@
 // / 1.1 ms; a solve's last ones: 15000 x 10000 1.65 / 0.43 ms, 4096 x 3072 0.46
 // / 0.16 ms, 1023 x 767 0.139 / 0.045 ms.
 #include <algorithm>
+#include <cstddef>
 
 #include "jfc_sync.cuh"
 
@@ -58,56 +59,68 @@ __device__ __forceinline__ uint32_t* seg_words(const GridDev& g, int y, int c) {
 }
 
 // Row words of the changed tiles, their heights (0 at deficits, else INF) and
-// empty level-set state; the relabel's queues, flags and counters reset.
-// One warp per changed tile; lane i of the tile's rows writes row i's words.
+// empty level-set state; the queues, flags and counters of the relabel and of the
+// push-relabel phase behind it reset.  The first part of k_wave_relabel, one
+// warp per changed tile; lane i of the tile's rows writes row i's words.  A
+// warp looks at every nwarps-th tile, 32 at once: tiles change in clusters, and
+// neighbours fall to different warps.  (As a kernel of its own, a warp for 32
+// tiles in a row, it and the second launch took 15 us of every relabel of 640 x
+// 480 or 1023 x 767 instead of 6.)
 template <int TY>
-__global__ void __launch_bounds__(256) k_wave_bits(TileSet ts) {
+__device__ __forceinline__ void changed_tiles(const TileSet& ts) {
+  constexpr int kRows = 4;   // rows in flight: 20 loads a lane in the 64 registers that the levels leave
   DevCounters* ctr = ts.d_ctr;
   const int lane = threadIdx.x & 31;
   const long long gt = blockIdx.x * (long long)blockDim.x + threadIdx.x, gn = (long long)gridDim.x * blockDim.x;
   if (gt == 0) {
-    ctr->t_gr_start = jfc::global_ns();
     ctr->bfs_status = 0;
-    ctr->wave_bar = ctr->wave_q = 0;
+    ctr->wave_q = 0;
+    ctr->ticket[0] = ctr->ticket[1] = 0;
+    ctr->pr_bar = 0;
   }
   for (long long i = gt; i < ts.ngrids; i += gn) ts.d_grid_active[i] = 0;
   for (long long i = gt; i < ts.nreg; i += gn) ts.d_rflag[0][i] = ts.d_rflag[1][i] = 0;
   const long long nitems = ts.pr_split ? 2ll * ts.ntiles : ts.ntiles;
   for (long long i = gt; i < nitems; i += gn) ts.d_flag_pr[i] = 0;
-  for (long long t0 = gt - lane; t0 < ts.ntiles; t0 += gn) {
-    unsigned todo = __ballot_sync(FULL, t0 + lane < ts.ntiles && ts.d_dirty[t0 + lane] != 0);
+  const long long w = gt >> 5, nw = gn >> 5;
+  for (long long t0 = w; t0 < ts.ntiles; t0 += 32 * nw) {
+    const long long cand = t0 + lane * nw;
+    unsigned todo = __ballot_sync(FULL, cand < ts.ntiles && ts.d_dirty[cand] != 0);
     while (todo) {
-      const long long tid = t0 + __ffs(todo) - 1;
+      const long long tid = t0 + (__ffs(todo) - 1) * nw;
       todo &= todo - 1;
       const int4 ti = ts.d_info[tid];
       const GridDev& g = ts.d_desc[ti.x];
       const long long pitch = g.pitch;
       const int y0 = ti.z * TY;
       const long long n0 = (long long)ti.y * 32 + lane + (long long)y0 * pitch;
-      int e[TY], r[4][TY];
-#pragma unroll
-      for (int i = 0; i < TY; ++i) {
-        const long long n = n0 + i * pitch;
-        e[i] = g.e[n];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) r[k][i] = g.r[k][n];
-      }
       uint4 arcs = make_uint4(0, 0, 0, 0), sign = make_uint4(0, 0, 0, 0);
+#pragma unroll 1
+      for (int j = 0; j < TY; j += kRows) {
+        int e[kRows], r[4][kRows];
 #pragma unroll
-      for (int i = 0; i < TY; ++i) {
-        const unsigned xp = __ballot_sync(FULL, r[0][i] > 0), yp = __ballot_sync(FULL, r[1][i] > 0);
-        const unsigned ym = __ballot_sync(FULL, r[2][i] > 0), xm = __ballot_sync(FULL, r[3][i] > 0);
-        const unsigned neg = __ballot_sync(FULL, e[i] < 0), pos = __ballot_sync(FULL, e[i] > 0);
-        if (lane == i) {
-          arcs = make_uint4(xp, yp, ym, xm);
-          sign = make_uint4(0, 0, neg, pos);
+        for (int i = 0; i < kRows; ++i) {
+          const long long n = n0 + (j + i) * pitch;
+          e[i] = g.e[n];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) r[k][i] = g.r[k][n];
         }
-        g.h[n0 + i * pitch] = e[i] < 0 ? 0 : JFC_INF;
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+          const unsigned xp = __ballot_sync(FULL, r[0][i] > 0), yp = __ballot_sync(FULL, r[1][i] > 0);
+          const unsigned ym = __ballot_sync(FULL, r[2][i] > 0), xm = __ballot_sync(FULL, r[3][i] > 0);
+          const unsigned neg = __ballot_sync(FULL, e[i] < 0), pos = __ballot_sync(FULL, e[i] > 0);
+          if (lane == j + i) {
+            arcs = make_uint4(xp, yp, ym, xm);
+            sign = make_uint4(0, 0, neg, pos);
+          }
+          g.h[n0 + (j + i) * pitch] = e[i] < 0 ? 0 : JFC_INF;
+        }
       }
       if (lane < TY) {
-        uint4* w = reinterpret_cast<uint4*>(seg_words(g, y0 + lane, ti.y));
-        w[0] = arcs;
-        w[1] = sign;
+        uint4* q = reinterpret_cast<uint4*>(seg_words(g, y0 + lane, ti.y));
+        q[0] = arcs;
+        q[1] = sign;
         ts.d_vf[(long long)g.tile_base * TY + (long long)(y0 + lane) * g.tiles_x + ti.y] = make_uint4(0, 0, 0, 0);
       }
       if (lane == 0) ts.d_dirty[tid] = 0;
@@ -115,25 +128,28 @@ __global__ void __launch_bounds__(256) k_wave_bits(TileSet ts) {
   }
 }
 
-// Grid barrier of the relabel: one counter that only grows (zeroed by
-// k_wave_bits), so an arrival is also the release and nothing is reset; its
-// high bits count the CTAs that flagged a region for the next phase, which
+// Grid barrier of the relabel and the cut: one counter that only grows, so an
+// arrival is also the release and nothing is reset.  There are two, used by
+// launches in turn (wave_epoch counts them; the launch behind finds its own
+// zero).  The counter's high bits count the CTAs that flagged a region for the next phase, which
 // makes "is there a next phase" part of the same poll.  (A CTA that sees
 // arrivals of the phase after it sees them because that phase exists.)
 // Bounded like jfc::grid_sync.  Returns -1 on error, else whether any region
 // was flagged since `seen` (updated).
 constexpr int kArriveBits = 40;   // low bits of the counter: arrivals; the rest: CTAs that flagged
-__device__ __forceinline__ int wave_sync(DevCounters* ctr, unsigned long long target, bool any, unsigned& seen) {
+__device__ __forceinline__ int wave_sync(DevCounters* ctr, unsigned epoch, unsigned long long target, bool any,
+                                         unsigned& seen) {
   __shared__ int s_res;
   __shared__ unsigned s_seen;
   __syncthreads();
   if (threadIdx.x == 0) {
+    unsigned long long* const bar = ctr->wave_bar + (epoch & 1u);
     __threadfence();
-    atomicAdd(&ctr->wave_bar, 1ull + (any ? 1ull << kArriveBits : 0ull));
+    atomicAdd(bar, 1ull + (any ? 1ull << kArriveBits : 0ull));
     unsigned long long spins = 0, v;
     const unsigned long long cap = jfc::spin_cap(ctr);
     int res = 0;
-    while (((v = *(volatile unsigned long long*)&ctr->wave_bar) & ((1ull << kArriveBits) - 1)) < target) {
+    while (((v = *(volatile unsigned long long*)bar) & ((1ull << kArriveBits) - 1)) < target) {
       if (jfc::vload(&ctr->error)) { res = -1; break; }
       if (++spins > cap) { atomicExch(&ctr->error, 1); res = -1; break; }
       if (spins > 16) __nanosleep(40);
@@ -148,6 +164,14 @@ __device__ __forceinline__ int wave_sync(DevCounters* ctr, unsigned long long ta
   __syncthreads();
   if (s_res > 0) seen = s_seen;
   return s_res;
+}
+
+// This launch's epoch: read by every CTA before its first arrival; the first CTA
+// zeroes the next launch's counter, and names it behind the last barrier.
+__device__ __forceinline__ unsigned wave_epoch(DevCounters* ctr) {
+  const unsigned epoch = *(volatile unsigned*)&ctr->wave_epoch;
+  if (blockIdx.x == 0 && threadIdx.x == 0) ctr->wave_bar[(epoch & 1u) ^ 1u] = 0;
+  return epoch;
 }
 
 // What a phase writes to the height plane for one row word.
@@ -185,7 +209,16 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave_relabel(TileSet ts) {
   __shared__ unsigned s_mask, s_new[2], s_tiles;
   __shared__ unsigned long long s_base;
   DevCounters* ctr = ts.d_ctr;
-  const unsigned long long t1 = jfc::global_ns();
+  const unsigned epoch = wave_epoch(ctr);
+  unsigned seen = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) ctr->t_gr_start = jfc::global_ns();
+  changed_tiles<TY>(ts);
+  if (wave_sync(ctr, epoch, gridDim.x, false, seen) < 0) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const unsigned long long t1 = jfc::global_ns();
+    ctr->ns_gr_first += t1 - ctr->t_gr_start;
+    ctr->t_gr_start = t1;
+  }
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int c = t & (kC - 1), s = t >> 3, ws = s & 3;   // word column, strip of 4 rows, strip within the warp
   const bool inner = c >= 1 && c <= kIW && s >= kT / 4 && s < (kT + kIR) / 4;
@@ -197,7 +230,6 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave_relabel(TileSet ts) {
   const unsigned ml = c == 0 ? 0u : ~0u, mr = c == kC - 1 ? 0u : ~0u;
   RowOut* const mine = &s_out[inner ? (4 * (s - kT / 4)) * kIW + c - 1 : 0];   // (interior) rows kIW apart
   unsigned long long visits = 0;
-  unsigned seen = 0;
   int phase = 1;
   for (;; ++phase) {
     const bool first = phase == 1;
@@ -433,7 +465,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave_relabel(TileSet ts) {
         __syncthreads();   // the shared state is free for the next region
       }
     }
-    if (wave_sync(ctr, (unsigned long long)phase * gridDim.x, any_next, seen) <= 0) break;
+    if (wave_sync(ctr, epoch, (unsigned long long)(phase + 1) * gridDim.x, any_next, seen) <= 0) break;
   }
   if (t == 0) {
     atomicAdd(&ctr->bfs_visits, visits * (unsigned long long)(kIR / TY * kIW));
@@ -446,9 +478,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave_relabel(TileSet ts) {
       ctr->cur_pr[0] = ctr->cur_pr[1] = 0;
       ctr->bfs_passes = phase;
       ctr->bfs_status = 1;
-      const unsigned long long t2 = jfc::global_ns();
-      ctr->ns_gr_first += t1 - ctr->t_gr_start;
-      ctr->ns_gr_frontier += t2 - t1;
+      ctr->wave_epoch = epoch + 1;
+      ctr->ns_gr_frontier += jfc::global_ns() - ctr->t_gr_start;
     }
   }
 }
@@ -503,6 +534,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave_cut(TileSet ts, int max_pa
   const int aout = ws == 0 ? 2 * (warp + 1) * kC + c : ws == 3 ? (2 * (warp + 1) + 1) * kC + c : 192 + lane;
   const unsigned ml = c == 0 ? 0u : ~0u, mr = c == kC - 1 ? 0u : ~0u;
   unsigned long long visits = 0;
+  const unsigned epoch = wave_epoch(ctr);
   unsigned seen = 0;
   int phase = 1;
   bool ok_all = true;
@@ -637,7 +669,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave_cut(TileSet ts, int max_pa
         __syncthreads();
       }
     }
-    const int more = wave_sync(ctr, (unsigned long long)phase * gridDim.x, any_next, seen);
+    const int more = wave_sync(ctr, epoch, (unsigned long long)phase * gridDim.x, any_next, seen);
     if (more < 0) ok_all = false;
     if (more <= 0) break;
     if (phase > max_passes) {
@@ -684,6 +716,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave_cut(TileSet ts, int max_pa
     atomicAdd(&ctr->bfs_visits, visits * (unsigned long long)(kIR / TY * kIW));
     if (blockIdx.x == 0) {
       ctr->bfs_passes = phase;
+      ctr->wave_epoch = epoch + 1;
       if (ok_all) ctr->bfs_status = 1;
     }
   }
@@ -694,8 +727,8 @@ cudaError_t wave_cut_t(const TileSet& ts, int max_passes, cudaStream_t s) {
   static int cache[64] = {0};
   const void* fn = (const void*)k_wave_cut<TY>;
   cudaError_t e = cudaMemsetAsync(ts.d_grid_sum, 0, sizeof(long long) * 2 * ts.ngrids, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(&ts.d_ctr->wave_bar, 0, sizeof(unsigned long long), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(&ts.d_ctr->cut_bad, 0, sizeof(int), s);
+  static_assert(offsetof(DevCounters, bfs_status) == offsetof(DevCounters, cut_bad) + sizeof(int), "zeroed together");
+  if (e == cudaSuccess) e = cudaMemsetAsync(&ts.d_ctr->cut_bad, 0, 2 * sizeof(int), s);
   if (e != cudaSuccess) return e;
   const int blocks = std::min(persistent_blocks_cached(cache, fn, kThreads), ts.nreg);
   TileSet arg = ts;
@@ -706,14 +739,8 @@ cudaError_t wave_cut_t(const TileSet& ts, int max_passes, cudaStream_t s) {
 
 template <int TY>
 cudaError_t wave_t(const TileSet& ts, cudaStream_t s) {
-  static int cache_bits[64] = {0}, cache[64] = {0};
+  static int cache[64] = {0};
   const void* fn = (const void*)k_wave_relabel<TY>;
-  const int nb = persistent_blocks_cached(cache_bits, (const void*)k_wave_bits<TY>, 256);
-  const int need = (int)std::min<long long>(nb, (2ll * ts.ntiles + 255) / 256);
-  jfc_note_launch();
-  k_wave_bits<TY><<<need, 256, 0, s>>>(ts);
-  const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
   // no more CTAs than regions: the grid barrier's cost grows with them
   const int blocks = std::min(persistent_blocks_cached(cache, fn, kThreads), ts.nreg);
   TileSet arg = ts;

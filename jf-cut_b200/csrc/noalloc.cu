@@ -263,7 +263,6 @@ extern "C" int jfc_solve_grid2d_noalloc(int device, void* stream, const jfc_para
     rc = na_cycle(ts, p, 0, 0, s, r);
     if (rc) return rc;
   }
-  JFC_CUDA(cudaMemsetAsync(&ts.d_ctr->bfs_status, 0, sizeof(int), s));
   JFC_CUDA(launch_bfs(ts, true, p.max_bfs_passes, s));
   struct { long long sums[2]; } out;
   JFC_CUDA(cudaMemcpyAsync(&out, ts.d_grid_sum, sizeof(out), cudaMemcpyDeviceToHost, s));
