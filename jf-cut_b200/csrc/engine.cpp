@@ -374,36 +374,26 @@ static size_t pin_need(const TileSet& ts) {
   return sizeof(DevCounters) + sizeof(long long) * 2 * (size_t)ts.ngrids + 64;
 }
 
-// pinned slot holding the sweep pairs of the next push-relabel phase and the
-// distance cap of the relabel after it (after the read-back area); copied to
-// the control block (pr_sweeps, h_cap) by the cycle itself
-static int* pin_sweeps(jfc_ctx* ctx, const TileSet& ts) {
-  return (int*)((char*)ctx->h_pin + (pin_need(ts) + 255) / 256 * 256);
+// pinned slot of the schedule (after the read-back area); copied to the control
+// block (cyc) by the run of cycles itself
+static CycleState* pin_cycle(jfc_ctx* ctx, const TileSet& ts) {
+  return (CycleState*)((char*)ctx->h_pin + (pin_need(ts) + 255) / 256 * 256);
 }
-static size_t pin_need_cycle(const TileSet& ts) { return (pin_need(ts) + 255) / 256 * 256 + 64; }
+static size_t pin_need_cycle(const TileSet& ts) { return (pin_need(ts) + 255) / 256 * 256 + 256; }
 
-// Enqueue one BFS (global relabel when !cut, cut otherwise) and the read-back
-// of its counters (+ per-grid active tiles) into pinned memory `pin`.
-static cudaError_t enqueue_bfs(TileSet& ts, bool cut, int max_passes, cudaStream_t s, void* pin) {
-  cudaError_t e;
-#define JFC_E(call) do { e = (call); if (e != cudaSuccess) return e; } while (0)
-  if (!cut && ts.dims == 2) {
-    JFC_E(launch_wave_relabel(ts, s));
-    JFC_E(cudaMemcpyAsync(pin, ts.d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s));
-    return cudaMemcpyAsync((char*)pin + sizeof(DevCounters), ts.d_grid_active, sizeof(int) * ts.ngrids,
-                           cudaMemcpyDeviceToHost, s);
-  }
-  if (cut && ts.dims == 2) {
-    JFC_E(launch_wave_cut(ts, max_passes, s));
-    return cudaMemcpyAsync(pin, ts.d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s);
-  }
-  JFC_E(launch_bfs(ts, cut, max_passes, s));
-  JFC_E(cudaMemcpyAsync(pin, ts.d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s));
-  if (!cut)
-    JFC_E(cudaMemcpyAsync((char*)pin + sizeof(DevCounters), ts.d_grid_active, sizeof(int) * ts.ngrids,
-                          cudaMemcpyDeviceToHost, s));
-#undef JFC_E
-  return cudaSuccess;
+// Enqueue the read-back of the counters (+ per-grid active tiles) into pinned
+// memory `pin`.
+static cudaError_t enqueue_read(const TileSet& ts, bool active, cudaStream_t s, void* pin) {
+  const cudaError_t e = cudaMemcpyAsync(pin, ts.d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s);
+  if (e != cudaSuccess || !active) return e;
+  return cudaMemcpyAsync((char*)pin + sizeof(DevCounters), ts.d_grid_active, sizeof(int) * ts.ngrids,
+                         cudaMemcpyDeviceToHost, s);
+}
+
+// Enqueue one BFS (global relabel when !cut, cut otherwise) and its read-back.
+static cudaError_t enqueue_bfs(const TileSet& ts, bool cut, int max_passes, cudaStream_t s, void* pin) {
+  const cudaError_t e = launch_bfs(ts, cut, max_passes, s);
+  return e == cudaSuccess ? enqueue_read(ts, !cut, s, pin) : e;
 }
 
 // Outcome of a BFS from the pinned read-back (after the stream sync).
@@ -436,16 +426,18 @@ int engine_bfs(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, bool cut, int& pa
   return finish_bfs(ts, cut, ctx->h_pin, passes, active, cut_bad, sweeps_done);
 }
 
-// ---- CUDA graphs of the relabel cycle -------------------------------------
-// One cycle = { push-relabel phase (interval sweeps), global relabel, counter
-// read-back }: ~10 stream operations between two host syncs.  They are
-// captured once per (interval, local_iters, pass budget, read-back buffer)
-// and replayed with one graph launch.  The cache belongs to the tile set and
-// is dropped whenever the tile set changes.
+// ---- CUDA graphs of the relabel cycles ------------------------------------
+// A run of cycles { push-relabel phase, global relabel } is one graph launch and
+// one host wait: the schedule goes in, a loop node repeats the cycle while
+// jfc::end_cycle says so, the counters come back.  The first run of a solve
+// starts with the relabel alone.  Captured once per (kind, pass budget, schedule
+// kind, read-back buffer); the cache belongs to the tile set and is dropped
+// whenever the tile set changes.
 namespace {
 struct CycleGraphs {
   struct Entry {
-    int local_iters, max_passes, sched;
+    bool init;
+    int max_passes, sched;
     void* pin;
     cudaGraphExec_t exec;
   };
@@ -462,74 +454,123 @@ void tileset_drop_graphs(TileSet& ts) {
   ts.gcache = nullptr;
 }
 
-static cudaError_t enqueue_cycle(TileSet& ts, const int* pin_sw, int local_iters, int max_passes, int sched,
-                                 cudaStream_t s, void* pin) {
-  static_assert(offsetof(DevCounters, h_cap) == offsetof(DevCounters, pr_sweeps) + sizeof(int),
-                "pr_sweeps and h_cap are copied together");
-  cudaError_t e = cudaMemcpyAsync(&ts.d_ctr->pr_sweeps, pin_sw, 2 * sizeof(int), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = launch_pr_phase(ts, 0, local_iters, s, sched);
-  if (e == cudaSuccess) e = enqueue_bfs(ts, false, max_passes, s, pin);
-  return e;
+static cudaError_t enqueue_schedule(const TileSet& ts, const CycleState* pin_cyc, cudaStream_t s) {
+  return cudaMemcpyAsync(&ts.d_ctr->cyc, pin_cyc, sizeof(CycleState), cudaMemcpyHostToDevice, s);
 }
 
-static cudaGraphExec_t cycle_graph(TileSet& ts, const int* pin_sw, int local_iters, int max_passes, int sched,
+// One cycle, or the relabel alone (init).
+static cudaError_t enqueue_cycle(TileSet ts, bool init, int max_passes, int sched, unsigned long long cond,
+                                 cudaStream_t s) {
+  ts.cyc_mode = init ? 1 : 2;
+  ts.cyc_cond = cond;
+  const cudaError_t e = init ? cudaSuccess : launch_pr_phase(ts, 0, 0, s, sched);
+  return e == cudaSuccess ? launch_bfs(ts, false, max_passes, s) : e;
+}
+
+// Capture what f enqueues on s into graph g behind node dep (null: none); `last`
+// gets the node behind which the next one goes.
+template <typename F>
+static cudaError_t capture_into(cudaGraph_t g, cudaGraphNode_t* dep, cudaStream_t s, cudaGraphNode_t* last, F f) {
+  cudaError_t e = cudaStreamBeginCaptureToGraph(s, g, dep, nullptr, dep ? 1 : 0, cudaStreamCaptureModeThreadLocal);
+  if (e != cudaSuccess) return e;
+  g_capturing = true;
+  const cudaError_t e1 = f();
+  g_capturing = false;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  const cudaGraphNode_t* deps = nullptr;
+  size_t n = 0;
+  const cudaError_t e2 = cudaStreamGetCaptureInfo_v2(s, &st, nullptr, nullptr, &deps, &n);
+  if (e2 == cudaSuccess && last && n == 1) *last = deps[0];
+  e = cudaStreamEndCapture(s, &g);
+  if (e1 != cudaSuccess || e2 != cudaSuccess) return e1 != cudaSuccess ? e1 : e2;
+  return e == cudaSuccess && last && n != 1 ? cudaErrorUnknown : e;
+}
+
+static cudaError_t build_cycle_graph(const TileSet& ts, bool init, const CycleState* pin_cyc, int max_passes,
+                                     int sched, cudaStream_t s, void* pin, cudaGraph_t g) {
+  cudaGraphConditionalHandle cond;
+  // (no cycle to decide about it before the first: the run starts with one)
+  cudaError_t e = cudaGraphConditionalHandleCreate(&cond, g, init ? 0u : 1u, cudaGraphCondAssignDefault);
+  if (e != cudaSuccess) return e;
+  cudaGraphNode_t last{}, loop{};
+  e = capture_into(g, nullptr, s, &last, [&]() {
+    const cudaError_t c = enqueue_schedule(ts, pin_cyc, s);
+    return c == cudaSuccess && init ? enqueue_cycle(ts, true, max_passes, sched, cond, s) : c;
+  });
+  if (e != cudaSuccess) return e;
+  cudaGraphNodeParams np{};
+  np.type = cudaGraphNodeTypeConditional;
+  np.conditional.handle = cond;
+  np.conditional.type = cudaGraphCondTypeWhile;
+  np.conditional.size = 1;
+  e = cudaGraphAddNode(&loop, g, &last, 1, &np);
+  if (e != cudaSuccess) return e;
+  e = capture_into(np.conditional.phGraph_out[0], nullptr, s, nullptr,
+                   [&]() { return enqueue_cycle(ts, false, max_passes, sched, cond, s); });
+  if (e != cudaSuccess) return e;
+  return capture_into(g, &loop, s, nullptr, [&]() { return enqueue_read(ts, true, s, pin); });
+}
+
+static cudaGraphExec_t cycle_graph(TileSet& ts, bool init, const CycleState* pin_cyc, int max_passes, int sched,
                                    cudaStream_t s, void* pin) {
   if (!ts.gcache) ts.gcache = new CycleGraphs();
   CycleGraphs* c = (CycleGraphs*)ts.gcache;
   if (c->broken) return nullptr;
   for (auto& e : c->v)
-    if (e.local_iters == local_iters && e.max_passes == max_passes && e.sched == sched && e.pin == pin)
-      return e.exec;
+    if (e.init == init && e.max_passes == max_passes && e.sched == sched && e.pin == pin) return e.exec;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
     c->broken = true;   // the caller is capturing this stream itself
     return nullptr;
   }
-  if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-    cudaGetLastError();
-    c->broken = true;
-    return nullptr;
-  }
-  g_capturing = true;
-  const cudaError_t e1 = enqueue_cycle(ts, pin_sw, local_iters, max_passes, sched, s, pin);
-  g_capturing = false;
   cudaGraph_t g = nullptr;
-  const cudaError_t e2 = cudaStreamEndCapture(s, &g);
   cudaGraphExec_t x = nullptr;
-  if (e1 == cudaSuccess && e2 == cudaSuccess && g) {
-    if (cudaGraphInstantiate(&x, g, 0) != cudaSuccess) x = nullptr;
-  }
+  if (cudaGraphCreate(&g, 0) == cudaSuccess &&
+      build_cycle_graph(ts, init, pin_cyc, max_passes, sched, s, pin, g) == cudaSuccess &&
+      cudaGraphInstantiate(&x, g, 0) != cudaSuccess)
+    x = nullptr;
   if (g) cudaGraphDestroy(g);
   cudaGetLastError();   // a refused capture leaves no sticky error
   if (!x) {
     c->broken = true;
     return nullptr;
   }
-  c->v.push_back({local_iters, max_passes, sched, pin, x});
+  c->v.push_back({init, max_passes, sched, pin, x});
   return x;
 }
 
-// One relabel cycle, replayed from a graph when enabled; returns the outcome
-// of its global relabel.
-static int run_cycle(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, int interval, int h_cap, int local_iters,
-                     int sched, int& passes, std::vector<int>& active, int* sweeps_done, bool* used_graph) {
+// A run of cycles by schedule cyc (advanced to its state behind the run),
+// replayed from a graph when enabled, else one cycle; returns the outcome of the
+// last global relabel.  init: the run starts with a relabel alone.
+static int run_cycles(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, bool init, CycleState& cyc, int sched,
+                      int& passes, std::vector<int>& active, bool* used_graph) {
   cudaStream_t s = ctx->stream;
   int rc = pin_reserve(ctx, pin_need_cycle(ts));
   if (rc) return rc;
-  int* pin_sw = pin_sweeps(ctx, ts);
-  pin_sw[0] = interval;   // the previous cycle's copies finished at its sync
-  pin_sw[1] = h_cap;
-  cudaGraphExec_t x = p.use_graph ? cycle_graph(ts, pin_sw, local_iters, p.max_bfs_passes, sched, s, ctx->h_pin)
-                                  : nullptr;
+  CycleState* pin_cyc = pin_cycle(ctx, ts);
+  cyc.cycles = cyc.sweeps = cyc.passes = 0;
+  *pin_cyc = cyc;   // the previous run's copies finished at its wait
+  const bool alone = init && cyc.max_cycles == 1;   // the relabel, no cycle behind it
+  cudaGraphExec_t x = p.use_graph && !alone
+                          ? cycle_graph(ts, init, pin_cyc, p.max_bfs_passes, sched, s, ctx->h_pin)
+                          : nullptr;
   if (x) {
     JFC_CUDA(cudaGraphLaunch(x, s));
-    jfc_note_launch(2);
-    if (used_graph) *used_graph = true;
   } else {
-    JFC_CUDA(enqueue_cycle(ts, pin_sw, local_iters, p.max_bfs_passes, sched, s, ctx->h_pin));
+    JFC_CUDA(enqueue_schedule(ts, pin_cyc, s));
+    JFC_CUDA(enqueue_cycle(ts, init, p.max_bfs_passes, sched, 0, s));
+    JFC_CUDA(enqueue_read(ts, true, s, ctx->h_pin));
   }
   JFC_CUDA(cudaStreamSynchronize(s));
-  return finish_bfs(ts, false, ctx->h_pin, passes, &active, nullptr, sweeps_done);
+  cyc = ((const DevCounters*)ctx->h_pin)->cyc;
+  if (x) {
+    const int per = ts.dims == 2 ? 1 : 4;   // kernels of a relabel
+    jfc_note_launch(per * cyc.cycles + cyc.cycles - (init ? 1 : 0));
+    if (used_graph && cyc.cycles > (init ? 1 : 0)) *used_graph = true;
+  }
+  passes += cyc.passes;
+  int last = 0;
+  return finish_bfs(ts, false, ctx->h_pin, last, &active, nullptr, nullptr);
 }
 
 int engine_cut(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, std::vector<GridResult>& res, int& passes,
@@ -577,18 +618,38 @@ int engine_solve(jfc_ctx* ctx, TileSet& ts, const jfc_params& p_in, std::vector<
   // relabel certifies the result
   int h_cap = relabel_cap_for(p, ts.dims);   // cap of the next relabel
   int last_cap = h_cap;                       // cap the last relabel ran with
-  if (p.spin_limit > 0 || h_cap > 0)
-    JFC_CUDA(launch_set_limits(ts, (unsigned long long)p.spin_limit, h_cap, s));
+  if (p.spin_limit > 0) JFC_CUDA(launch_set_limits(ts, (unsigned long long)p.spin_limit, h_cap, s));
 #ifndef JFC_NO_PREPUSH
   if (p.pr_mode != 1) JFC_CUDA(launch_prepush(ts, s));   // the Fast-Cut comparison stays as it was
 #endif
   std::vector<int> active;
   int rc;
 
-  // initial global relabel (exact sink distances; fills the work queues)
-  rc = engine_bfs(ctx, ts, p, false, st.bfs_passes, &active, nullptr, nullptr);
+  bool graphs = false;
+  CycleState cyc{};
+  cyc.interval0 = cyc.pr_sweeps = interval_for(p, ts.dims);
+  cyc.interval_max = p.relabel_interval_max;
+  cyc.h_cap = h_cap;
+  // in the long-path tail (a sliver of the tiles active) visits are longer, so
+  // excess crosses a whole tile per visit instead of per several sweeps
+  cyc.iters = p.local_iters;
+  cyc.iters_tail = p.local_iters_tail > 0 ? p.local_iters_tail
+                   : p.local_iters_tail < 0 ? p.local_iters : std::min(2 * p.local_iters, 64);
+  // (a run comes back to the host now and then: no launch holds the device for
+  // an unbounded time; verbose solves report every relabel)
+  cyc.max_cycles = p.verbose ? 1 : 256;
+  cyc.max_sweeps = p.max_sweeps;
+  // pr_sched 3: parity sweeps in the bulk, the worklist in the tail, so a run
+  // stays in either; the Fast-Cut comparison has no cycles
+  const bool fast = p.pr_mode == 1 && fast_grid;
+  cyc.tail = pr_sched_for(p) == 3 || fast ? 0 : -1;
+  if (fast) cyc.max_cycles = 1;
+  // initial global relabel (fills the work queues), and the cycles behind it
+  rc = run_cycles(ctx, ts, p, true, cyc, pr_sched_for(p) == 3 ? 1 : pr_sched_for(p), st.bfs_passes, active, &graphs);
   if (rc) return rc;
-  st.global_relabels = 1;
+  st.global_relabels = cyc.cycles;
+  st.pr_phases = cyc.cycles - 1;
+  st.sweeps += cyc.sweeps;
 
   auto total = [&]() { long long t = 0; for (int v : active) t += v; return t; };
   const DevCounters* hc = (const DevCounters*)ctx->h_pin;
@@ -605,77 +666,53 @@ int engine_solve(jfc_ctx* ctx, TileSet& ts, const jfc_params& p_in, std::vector<
             c0->bfs_visits);
   }
   int status = JFC_OK;
-  // Adaptive schedule: while a large part of the grid is active, frequent
-  // global relabels pay off; once only a sliver is active (long transport
-  // paths, few tiles), the dense relabel dominates, so the interval doubles
-  // (the push-relabel phase still stops as soon as its queues drain).
-  //  The interval also doubles while the last relabel cost more than twice
-  // the push-relabel phase before it (device clocks) and that phase used all
-  // its sweeps: the relabel is then the bottleneck and is amortised.
-  const int interval0 = interval_for(p, ts.dims);
-  int interval = interval0;
-  const int tail_iters = p.local_iters_tail > 0 ? p.local_iters_tail
-                         : p.local_iters_tail < 0 ? p.local_iters : std::min(2 * p.local_iters, 64);
-  bool graphs = false;
   double fast_ms = 0.0;   // Fast-Cut iterations (event-timed: many small launches)
-  unsigned long long last_pr = 0, last_gr = 0;
   bool post_exact = false;   // the exact relabel ran and found reachable excess
-  {
-    const DevCounters* c0 = (const DevCounters*)ctx->h_pin;
-    last_pr = c0->ns_pr;
-    last_gr = c0->ns_gr_first + c0->ns_gr_frontier;
-  }
   for (;;) {
   while (total() > 0) {
     if (st.sweeps >= p.max_sweeps) {
       status = set_error(JFC_ERR_NOT_CONVERGED, "sweep budget exhausted");
       break;
     }
-    // relabel_interval x (even sweep, odd sweep), global relabel, active-tile
-    // count: one host read-back per cycle
-    int sw = 0;
-    if (p.pr_mode == 1 && fast_grid) {
+    const bool tail = cycle_tail(total(), ts.ntiles);
+    if (fast) {
       // Fast-Cut comparison: `interval` line-sweep iterations, then the
       // exact global relabel and convergence test
       cudaEvent_t f0 = ev[2], f1 = ev[3];
       JFC_CUDA(cudaEventRecord(f0, s));
-      for (int it = 0; it < interval; ++it) JFC_CUDA(launch_fast_iteration(*fast_grid, &ts.d_ctr->fast_moved, s));
+      for (int it = 0; it < cyc.pr_sweeps; ++it) JFC_CUDA(launch_fast_iteration(*fast_grid, &ts.d_ctr->fast_moved, s));
       JFC_CUDA(launch_mark_dirty(ts, s));
       JFC_CUDA(cudaEventRecord(f1, s));
       rc = engine_bfs(ctx, ts, p, false, st.bfs_passes, &active, nullptr, nullptr);
       if (rc) return rc;
       const double fms = elapsed_ms(f0, f1);
       fast_ms += fms;
-      last_pr -= (unsigned long long)(fms * 1e6);   // the cost rule below sees the sweeps' time
-      sw = 2 * interval;
+      const DevCounters* c1 = (const DevCounters*)ctx->h_pin;
+      const unsigned long long gr = c1->ns_gr_first + c1->ns_gr_frontier;
+      st.sweeps += 2 * cyc.pr_sweeps;
+      cyc.pr_sweeps = next_interval(cyc, cycle_tail(total(), ts.ntiles), (unsigned long long)(fms * 1e6),
+                                    gr - cyc.last_gr, 2 * cyc.pr_sweeps);
+      cyc.last_gr = gr;
+      ++st.global_relabels;
     } else {
-      // the long-path tail (a sliver of the tiles active): longer visits, so
-      // excess crosses a whole tile per visit instead of per several sweeps
-      const bool tail = total() * 256 < (long long)ts.ntiles;
-      const int li = tail ? tail_iters : p.local_iters;
-      // pr_sched 3: parity sweeps in the bulk, the worklist in the tail;
-      // automatic: the worklist once the exact relabel found excess farther
-      // than the cap from every deficit (a few tiles whose excess crosses
-      // many tiles, where the sweeps would idle at their barriers)
+      // cycles of relabel_interval x (even sweep, odd sweep), global relabel and
+      // active-tile count, with one host wait per run of them.  pr_sched 3:
+      // parity sweeps in the bulk, the worklist in the tail; automatic: the
+      // worklist once the exact relabel found excess farther than the cap from
+      // every deficit (a few tiles whose excess crosses many tiles, where the
+      // sweeps would idle at their barriers)
       const int sched = pr_sched_for(p) == 3 ? (tail ? 2 : 1) : (p.pr_sched == 0 && post_exact) ? 2
                                                                                                : pr_sched_for(p);
-      rc = run_cycle(ctx, ts, p, interval, h_cap, li, sched, st.bfs_passes, active, &sw, &graphs);
-      last_cap = h_cap;
-      ++st.pr_phases;
+      cyc.h_cap = last_cap = h_cap;
+      cyc.local_iters = tail ? cyc.iters_tail : cyc.iters;
+      if (pr_sched_for(p) == 3) cyc.tail = tail ? 1 : 0;
+      cyc.max_sweeps = p.max_sweeps - st.sweeps;
+      rc = run_cycles(ctx, ts, p, false, cyc, sched, st.bfs_passes, active, &graphs);
+      st.pr_phases += cyc.cycles;
+      st.global_relabels += cyc.cycles;
       if (rc) return rc;
+      st.sweeps += cyc.sweeps;
     }
-    st.sweeps += sw;
-    {
-      const DevCounters* c1 = (const DevCounters*)ctx->h_pin;
-      const unsigned long long pr = c1->ns_pr - last_pr, gr = c1->ns_gr_first + c1->ns_gr_frontier - last_gr;
-      last_pr = c1->ns_pr;
-      last_gr = c1->ns_gr_first + c1->ns_gr_frontier;
-      const bool sliver = total() * 256 < (long long)ts.ntiles;
-      const bool relabel_bound = gr > 2 * pr && sw >= 2 * interval;
-      if (sliver || relabel_bound) interval = std::min(interval * 2, p.relabel_interval_max);
-      else interval = interval0;
-    }
-    ++st.global_relabels;
     if (p.verbose) {
       hc = (const DevCounters*)ctx->h_pin;
       const double pr = hc->ns_pr * 1e-6, gr = (hc->ns_gr_first + hc->ns_gr_frontier) * 1e-6;

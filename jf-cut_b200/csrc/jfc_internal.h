@@ -45,6 +45,37 @@ struct GridDev {
   uint8_t* label;
 };
 
+// Schedule of the relabel cycles { push-relabel phase, global relabel } of a
+// solve: written by the host before a run of cycles, advanced on the device at
+// the end of each (jfc::end_cycle), read back behind the run.
+struct CycleState {
+  int pr_sweeps;             // sweep pairs of the next phase launched with sweeps <= 0
+  int h_cap;                 // global relabels: distances >= h_cap count as unreachable (0: no cap)
+  int local_iters;           // local relabel iterations of the next phase launched with sweeps <= 0
+  int iters, iters_tail;     // its values in the bulk and in the tail
+  int interval0, interval_max;
+  int tail;                  // stay in the bulk (0) or the tail (1) only; -1: either
+  int max_cycles, max_sweeps;  // the run ends with the cycle that reaches either
+  int cycles, sweeps, passes;  // relabels, sweeps and BFS passes of the run so far
+  unsigned long long last_pr, last_gr;  // ns_pr, ns_gr_first + ns_gr_frontier behind the last cycle
+};
+
+// The tail of a solve: a sliver of the tiles active (long transport paths).
+__host__ __device__ inline bool cycle_tail(long long active, long long ntiles) { return active * 256 < ntiles; }
+
+// Sweep pairs of the next phase.  While a large part of the grid is active,
+// frequent global relabels pay off; in the tail the dense relabel dominates, so
+// the interval doubles (the phase still stops as soon as its queues drain).  It
+// also doubles while the last relabel cost more than twice the push-relabel
+// phase before it (device clocks) and that phase used all its sweeps: the
+// relabel is then the bottleneck and is amortised.
+__host__ __device__ inline int next_interval(const CycleState& c, bool tail, unsigned long long ns_pr,
+                                             unsigned long long ns_gr, int sweeps) {
+  const bool relabel_bound = ns_gr > 2 * ns_pr && sweeps >= 2 * c.pr_sweeps;
+  if (!tail && !relabel_bound) return c.interval0;
+  return 2 * c.pr_sweeps < c.interval_max ? 2 * c.pr_sweeps : c.interval_max;
+}
+
 // Device-side control state of one tile set (persistent phase kernels).
 struct DevCounters {
   unsigned ticket[2];        // work tickets (alternate between phases)
@@ -59,9 +90,7 @@ struct DevCounters {
   int cut_bad;               // cut BFS reached a deficit node (augmenting path left)
   int bfs_status;            // 1 converged, 2 pass budget exhausted
   int sweeps_done;           // sweeps run by the last push-relabel phase
-  int pr_sweeps;             // sweep pairs of the next phase when launched with sweeps <= 0
-  int h_cap;                 // global relabels: distances >= h_cap count as unreachable (0: no cap)
-                             // (pr_sweeps and h_cap: a relabel cycle copies both at once)
+  CycleState cyc;
   int fast_moved;            // a Fast-Cut push moved flow (comparison mode)
   unsigned long long visits; // push-relabel tile visits
   unsigned long long bfs_visits;
@@ -121,6 +150,9 @@ struct TileSet {
   DevCounters* d_ctr = nullptr;
   void* d_block = nullptr;           // single allocation backing the above
   size_t block_bytes = 0;
+  int cyc_mode = 0;                  // global relabels advance d_ctr->cyc: 0 no, 1 as the first of a run
+                                     // (no phase before it), 2 as the end of a cycle
+  unsigned long long cyc_cond = 0;   // and say whether the graph's loop goes on (0: none)
   int cap_tiles = 0, cap_grids = 0;  // capacity of d_block (reused while it fits)
   long long cap_rw = 0;              // row words
   int cap_reg = 0;                   // regions
@@ -150,8 +182,8 @@ void jfc_note_launch(int n = 1);
 // ----------------------------------------------------------- kernel launchers
 // (kernels_pr.cu) `sweeps` parity sweeps (even tiles, then odd tiles, ...)
 // in one persistent launch, draining the device work queues; sweeps <= 0
-// reads the count from the control block (pr_sweeps), so one captured graph
-// serves every interval
+// reads the count and the local iterations from the control block (cyc), so one
+// captured graph serves the whole schedule
 // sched 2: the asynchronous worklist (needs ts.d_pr_ring) instead of the
 // parity sweeps
 // (a global relabel comes before each: it zeroes the tickets and the barrier

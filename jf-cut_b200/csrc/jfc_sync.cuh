@@ -79,11 +79,11 @@ __device__ __forceinline__ bool arrive_wait(DevCounters* ctr, unsigned long long
 }
 
 // Distance cap of the running global relabel: distances at or above it are
-// stored as unreachable (JFC_INF); no cap when ctr->h_cap is 0.
+// stored as unreachable (JFC_INF); no cap when ctr->cyc.h_cap is 0.
 // (set before the kernel that reads it runs, constant during it: an ordinary
 // cached load, not a poll of L2 on every tile visit)
 __device__ __forceinline__ int height_cap(const DevCounters* ctr) {
-  const int v = ctr->h_cap;
+  const int v = ctr->cyc.h_cap;
   return v > 0 ? v : JFC_INF;
 }
 // The cap for grid g: its own when set, else the tile set's.
@@ -96,6 +96,44 @@ __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
+}
+
+// A loop that this relabel ends a turn of stops unless end_cycle says otherwise
+// (one thread, at the relabel's start: a relabel that gives up ends the loop).
+__device__ __forceinline__ void begin_cycle(const TileSet& ts) {
+  if (ts.cyc_cond) cudaGraphSetConditional((cudaGraphConditionalHandle)ts.cyc_cond, 0u);
+}
+
+// End of a relabel cycle, one warp, behind the relabel's last barrier and its
+// thread 0's counters: advance the schedule, and let the loop go on while tiles
+// are active and no limit is reached.  A cycle decided by the host costs 28 us
+// besides its kernels (read-back, wait, launch), a turn of the graph's loop 10
+// (1023 x 767: 14 relabels, 2.12 / 1.94 ms).
+__device__ __forceinline__ void end_cycle(const TileSet& ts) {
+  if (ts.cyc_mode == 0) return;
+  DevCounters* ctr = ts.d_ctr;
+  const int lane = threadIdx.x & 31;
+  long long active = 0;
+  for (int i = lane; i < ts.ngrids; i += 32) active += __ldcg(ts.d_grid_active + i);
+  for (int o = 16; o; o >>= 1) active += __shfl_xor_sync(FULL, active, o);
+  if (lane != 0) return;
+  CycleState c = ctr->cyc;
+  const bool tail = cycle_tail(active, ts.ntiles);
+  const unsigned long long gr = ctr->ns_gr_first + ctr->ns_gr_frontier, pr = ctr->ns_pr;
+  if (ts.cyc_mode == 2) {
+    const int sw = ctr->sweeps_done;
+    c.pr_sweeps = next_interval(c, tail, pr - c.last_pr, gr - c.last_gr, sw);
+    c.sweeps += sw;
+  }
+  c.local_iters = tail ? c.iters_tail : c.iters;
+  c.last_pr = pr;
+  c.last_gr = gr;
+  c.cycles += 1;
+  c.passes += ctr->bfs_passes;
+  ctr->cyc = c;
+  const bool go = active > 0 && vload(&ctr->error) == 0 && ctr->bfs_status == 1 && c.cycles < c.max_cycles &&
+                  c.sweeps < c.max_sweeps && (c.tail < 0 || (c.tail != 0) == tail);
+  if (go && ts.cyc_cond) cudaGraphSetConditional((cudaGraphConditionalHandle)ts.cyc_cond, 1u);
 }
 
 // Phase-clock instrumentation (builds with -DJFC_PHASE_CLOCK): thread 0 adds

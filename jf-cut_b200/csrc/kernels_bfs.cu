@@ -385,6 +385,7 @@ __global__ void __launch_bounds__(256, TY * TZ > 8 ? 1 : 2) k_bits3(TileSet ts) 
   const long long gt = blockIdx.x * (long long)blockDim.x + threadIdx.x, gn = (long long)gridDim.x * blockDim.x;
   if (gt == 0) {
     ctr->t_gr_start = jfc::global_ns();
+    jfc::begin_cycle(ts);
     ctr->bfs_status = 0;
     ctr->ticket[0] = ctr->ticket[1] = 0;
     ctr->qn_bfs[0] = ctr->qn_bfs[1] = 0;
@@ -1143,6 +1144,10 @@ __global__ void __launch_bounds__(256, 4) k_cut3(TileSet ts, int max_passes) {
   }
 }
 
+// (a launch of its own: in k_relabel_warp it changed the visits' registers and made
+// the frontier 15% slower)
+__global__ void k_end_cycle(TileSet ts) { jfc::end_cycle(ts); }
+
 // per-grid sum of min(e, 0) and count of source-side nodes (reduce_flow,
 // bin/x64/cl/Infrastructures/reduce.cl:92-117, in int64 instead of int32 partials)
 template <int TY, int TZ>
@@ -1220,7 +1225,11 @@ cudaError_t bfs_t(const TileSet& ts, int max_passes, const uint8_t* seeds, cudaS
   TileSet arg = ts;
   void* params[] = {(void*)&arg, (void*)&max_passes, (void*)&seeds};   // relabel and cut take two
   jfc_note_launch();
-  return cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(nt), params, dyn, s);
+  const cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(nt), params, dyn, s);
+  if (MODE != 0 || e != cudaSuccess || ts.cyc_mode == 0) return e;
+  jfc_note_launch();
+  k_end_cycle<<<1, 32, 0, s>>>(ts);
+  return cudaGetLastError();
 }
 
 template <int TY, int TZ>
@@ -1395,7 +1404,7 @@ cudaError_t launch_clear_counters(const TileSet& ts, cudaStream_t s) {
 namespace {
 __global__ void k_set_limits(DevCounters* ctr, unsigned long long polls, int h_cap) {
   ctr->spin_limit = polls;
-  ctr->h_cap = h_cap;
+  ctr->cyc.h_cap = h_cap;
 }
 }  // namespace
 

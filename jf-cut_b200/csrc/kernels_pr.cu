@@ -73,6 +73,7 @@ struct PrSmem {
   int face[6];            // any flow left through face: x-, x+, y-, y+, z-, z+
   int q_nb[6];            // after a visit: the work item behind each face that received flow, or -1
   int active;             // after a visit: the item still holds an active node
+  int local_iters;        // rounds of a visit, at most
 };
 
 template <int DIMS, int TY, int TZ>
@@ -248,7 +249,7 @@ __device__ __forceinline__ bool local_distance(Smem& s, const int* sh, int hi, c
 // s.q_nb[f] the item behind each face f that received flow (-1: none).  The
 // caller queues them.
 template <int DIMS, int TY, int TZ, bool SPLIT>
-__device__ __forceinline__ int pr_visit(const TileSet& ts, int tid, const int4& ti, int local_iters, bool local_relabel,
+__device__ __forceinline__ int pr_visit(const TileSet& ts, int tid, const int4& ti, bool local_relabel,
                                         PrSmem<DIMS, TY, TZ>& s, PrStage<DIMS, TY, TZ>& st, bool staged, bool failed) {
   using T = PrTile<DIMS, TY, TZ>;
   const int t = threadIdx.x;
@@ -337,7 +338,7 @@ __device__ __forceinline__ int pr_visit(const TileSet& ts, int tid, const int4& 
   constexpr int kOrder[6] = {T::XP, T::YP, T::YM, DIMS == 3 ? T::ZP : T::XM, T::ZM, T::XM};
   constexpr int NP = T::K;
   int it = 0;
-  for (; it < local_iters; ++it) {
+  for (; it < s.local_iters; ++it) {
     // relabel every active node without an admissible arc
     // (graphcut_push_relabel.cl:80-99 relabels two colours in turn): 1 + the
     // lowest residual neighbour; heights only grow, so the labelling stays
@@ -393,7 +394,7 @@ __device__ __forceinline__ int pr_visit(const TileSet& ts, int tid, const int4& 
       r[k] += in[k] - d[k];
     }
   }
-  const int rounds = it < local_iters ? it + 1 : local_iters;
+  const int rounds = it < s.local_iters ? it + 1 : s.local_iters;
   JFC_PCLK(ts.d_ctr, 2);
 
   // ---- write back the 32-byte sectors of each row that hold a changed word
@@ -497,7 +498,8 @@ __global__ void __launch_bounds__(Tile<DIMS, TY, TZ>::NT,
   int acquired_grid = -1;   // thread 0: grid whose tensor maps it acquired
   int next_buf = 0;         // thread 0: buffer of the next fill
   int s = 0;
-  const int npairs = sweeps > 0 ? sweeps : jfc::vload(&ctr->pr_sweeps);
+  const int npairs = sweeps > 0 ? sweeps : jfc::vload(&ctr->cyc.pr_sweeps);
+  if (threadIdx.x == 0) sm.local_iters = sweeps > 0 ? local_iters : jfc::vload(&ctr->cyc.local_iters);
   const int own = min((int)blockIdx.x, ts.ntiles - 1);   // (a parity's queue holds at most ntiles items)
   int cur[2] = {0, 0};   // pending buffer per parity (0 after a global relabel)
   bool failed = false;   // a staging copy never completed (error raised): leave
@@ -571,7 +573,7 @@ __global__ void __launch_bounds__(Tile<DIMS, TY, TZ>::NT,
       // first sweep of a phase: nothing moved since the exact global relabel
       // (the halo tiles have the other parity), so the local relabel would
       // reproduce the heights it finds
-      const int rd = pr_visit<DIMS, TY, TZ, SPLIT>(ts, tid, ti, local_iters, s > 0, sm, stage[buf], tma, late);
+      const int rd = pr_visit<DIMS, TY, TZ, SPLIT>(ts, tid, ti, s > 0, sm, stage[buf], tma, late);
       if (rd < 0) {
         if (threadIdx.x == 0) {
           atomicExch(&ctr->error, 1);
@@ -678,7 +680,8 @@ __global__ void __launch_bounds__(Tile<DIMS, TY, TZ>::NT)
       *reinterpret_cast<PrStage<DIMS, TY, TZ>*>(s_dyn + ((128u - (jfc::smem_addr(s_dyn) & 127u)) & 127u));
   DevCounters* ctr = ts.d_ctr;
   const unsigned long long t0 = jfc::global_ns();
-  const int npairs = sweeps > 0 ? sweeps : jfc::vload(&ctr->pr_sweeps);
+  const int npairs = sweeps > 0 ? sweeps : jfc::vload(&ctr->cyc.pr_sweeps);
+  if (threadIdx.x == 0) sm.local_iters = sweeps > 0 ? local_iters : jfc::vload(&ctr->cyc.local_iters);
   const int gens = 2 * npairs;
   const unsigned cap = (unsigned)(SPLIT ? 2 * ts.ntiles : ts.ntiles);
   unsigned long long* ring = ts.d_pr_ring;
@@ -771,7 +774,7 @@ __global__ void __launch_bounds__(Tile<DIMS, TY, TZ>::NT)
     // generation 0: nothing around the item moved since the exact global
     // relabel unless a neighbour was visited first; the local relabel is an
     // improvement only, so skipping it is safe either way
-    rounds += pr_visit<DIMS, TY, TZ, SPLIT>(ts, item, sm.ti, local_iters, gen > 0, sm, stage, false, false);
+    rounds += pr_visit<DIMS, TY, TZ, SPLIT>(ts, item, sm.ti, gen > 0, sm, stage, false, false);
     ++visits;
     maxgen = max(maxgen, gen);
     // release the item (its writes visible first), then queue what it fed

@@ -211,7 +211,10 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave_relabel(TileSet ts) {
   DevCounters* ctr = ts.d_ctr;
   const unsigned epoch = wave_epoch(ctr);
   unsigned seen = 0;
-  if (blockIdx.x == 0 && threadIdx.x == 0) ctr->t_gr_start = jfc::global_ns();
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    ctr->t_gr_start = jfc::global_ns();
+    jfc::begin_cycle(ts);
+  }
   changed_tiles<TY>(ts);
   if (wave_sync(ctr, epoch, gridDim.x, false, seen) < 0) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -482,6 +485,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave_relabel(TileSet ts) {
       ctr->ns_gr_frontier += jfc::global_ns() - ctr->t_gr_start;
     }
   }
+  if (blockIdx.x == 0 && warp == 0) jfc::end_cycle(ts);
 }
 
 // bit x reached from bit x - 1 (x + 1) when m bit x is set; closure by doubling
