@@ -371,7 +371,11 @@ static int pin_reserve(jfc_ctx* ctx, size_t bytes) {
 }
 
 static size_t pin_need(const TileSet& ts) {
-  return sizeof(DevCounters) + sizeof(long long) * 2 * (size_t)ts.ngrids + 64;
+  return sizeof(DevCounters) + (sizeof(long long) * 2 + sizeof(int)) * (size_t)ts.ngrids + 64;
+}
+// the per-grid sums of a cut in that buffer, behind the counters and the active tiles
+static long long* pin_sums(const TileSet& ts, void* pin) {
+  return (long long*)((char*)pin + (sizeof(DevCounters) + sizeof(int) * (size_t)ts.ngrids + 7) / 8 * 8);
 }
 
 // pinned slot of the schedule (after the read-back area); copied to the control
@@ -388,6 +392,10 @@ static cudaError_t enqueue_read(const TileSet& ts, bool active, cudaStream_t s, 
   if (e != cudaSuccess || !active) return e;
   return cudaMemcpyAsync((char*)pin + sizeof(DevCounters), ts.d_grid_active, sizeof(int) * ts.ngrids,
                          cudaMemcpyDeviceToHost, s);
+}
+
+static cudaError_t enqueue_read_sums(const TileSet& ts, cudaStream_t s, void* pin) {
+  return cudaMemcpyAsync(pin_sums(ts, pin), ts.d_grid_sum, sizeof(long long) * 2 * ts.ngrids, cudaMemcpyDeviceToHost, s);
 }
 
 // Enqueue one BFS (global relabel when !cut, cut otherwise) and its read-back.
@@ -429,8 +437,10 @@ int engine_bfs(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, bool cut, int& pa
 // ---- CUDA graphs of the relabel cycles ------------------------------------
 // A run of cycles { push-relabel phase, global relabel } is one graph launch and
 // one host wait: the schedule goes in, a loop node repeats the cycle while
-// jfc::end_cycle says so, the counters come back.  The first run of a solve
-// starts with the relabel alone.  Captured once per (kind, pass budget, schedule
+// jfc::end_cycle says so, the exact relabel and the cut follow if they are due,
+// and all their results come back.  The first run of a solve starts with the
+// relabel alone.  (With the exact relabel and the cut
+// launched by the host, each behind a wait, a 640 x 480 image took 0.68 ms, so 0.64.)  Captured once per (kind, pass budget, schedule
 // kind, read-back buffer); the cache belongs to the tile set and is dropped
 // whenever the tile set changes.
 namespace {
@@ -465,6 +475,16 @@ static cudaError_t enqueue_cycle(TileSet ts, bool init, int max_passes, int sche
   ts.cyc_cond = cond;
   const cudaError_t e = init ? cudaSuccess : launch_pr_phase(ts, 0, 0, s, sched);
   return e == cudaSuccess ? launch_bfs(ts, false, max_passes, s) : e;
+}
+
+// The exact relabel and the cut behind the cycles of a run, and what is read back.
+static cudaError_t enqueue_finish(TileSet ts, int max_passes, cudaStream_t s, void* pin) {
+  ts.cyc_mode = 3;
+  cudaError_t e = launch_bfs(ts, false, max_passes, s);
+  ts.cyc_mode = 4;
+  if (e == cudaSuccess) e = launch_bfs(ts, true, max_passes, s);
+  if (e == cudaSuccess) e = enqueue_read(ts, true, s, pin);
+  return e == cudaSuccess ? enqueue_read_sums(ts, s, pin) : e;
 }
 
 // Capture what f enqueues on s into graph g behind node dep (null: none); `last`
@@ -508,7 +528,7 @@ static cudaError_t build_cycle_graph(const TileSet& ts, bool init, const CycleSt
   e = capture_into(np.conditional.phGraph_out[0], nullptr, s, nullptr,
                    [&]() { return enqueue_cycle(ts, false, max_passes, sched, cond, s); });
   if (e != cudaSuccess) return e;
-  return capture_into(g, &loop, s, nullptr, [&]() { return enqueue_read(ts, true, s, pin); });
+  return capture_into(g, &loop, s, nullptr, [&]() { return enqueue_finish(ts, max_passes, s, pin); });
 }
 
 static cudaGraphExec_t cycle_graph(TileSet& ts, bool init, const CycleState* pin_cyc, int max_passes, int sched,
@@ -541,16 +561,18 @@ static cudaGraphExec_t cycle_graph(TileSet& ts, bool init, const CycleState* pin
 
 // A run of cycles by schedule cyc (advanced to its state behind the run),
 // replayed from a graph when enabled, else one cycle; returns the outcome of the
-// last global relabel.  init: the run starts with a relabel alone.
+// last global relabel.  init: the run starts with a relabel alone.  Behind
+// cyc.done = 2 the cut has run.
 static int run_cycles(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, bool init, CycleState& cyc, int sched,
-                      int& passes, std::vector<int>& active, bool* used_graph) {
+                      int& passes, std::vector<int>& active, bool* used_graph, cudaEvent_t done) {
   cudaStream_t s = ctx->stream;
   int rc = pin_reserve(ctx, pin_need_cycle(ts));
   if (rc) return rc;
   CycleState* pin_cyc = pin_cycle(ctx, ts);
-  cyc.cycles = cyc.sweeps = cyc.passes = 0;
+  cyc.cycles = cyc.sweeps = cyc.passes = cyc.done = cyc.exact = 0;
+  cyc.go = !init;
   *pin_cyc = cyc;   // the previous run's copies finished at its wait
-  const bool alone = init && cyc.max_cycles == 1;   // the relabel, no cycle behind it
+  const bool alone = cyc.max_cycles == 1;   // one relabel or cycle, nothing behind it
   cudaGraphExec_t x = p.use_graph && !alone
                           ? cycle_graph(ts, init, pin_cyc, p.max_bfs_passes, sched, s, ctx->h_pin)
                           : nullptr;
@@ -559,35 +581,34 @@ static int run_cycles(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, bool init,
   } else {
     JFC_CUDA(enqueue_schedule(ts, pin_cyc, s));
     JFC_CUDA(enqueue_cycle(ts, init, p.max_bfs_passes, sched, 0, s));
-    JFC_CUDA(enqueue_read(ts, true, s, ctx->h_pin));
+    JFC_CUDA(alone ? enqueue_read(ts, true, s, ctx->h_pin) : enqueue_finish(ts, p.max_bfs_passes, s, ctx->h_pin));
   }
+  JFC_CUDA(cudaEventRecord(done, s));
   JFC_CUDA(cudaStreamSynchronize(s));
   cyc = ((const DevCounters*)ctx->h_pin)->cyc;
+  if (alone) cyc.done = 0;
+  const int phases = cyc.cycles - cyc.exact - (init ? 1 : 0);
   if (x) {
     const int per = ts.dims == 2 ? 1 : 4;   // kernels of a relabel
-    jfc_note_launch(per * cyc.cycles + cyc.cycles - (init ? 1 : 0));
-    if (used_graph && cyc.cycles > (init ? 1 : 0)) *used_graph = true;
+    jfc_note_launch(per * cyc.cycles + phases + (cyc.done == 2 ? (ts.dims == 2 ? 1 : 2) : 0));
+    if (used_graph && phases > 0) *used_graph = true;
   }
   passes += cyc.passes;
   int last = 0;
-  return finish_bfs(ts, false, ctx->h_pin, last, &active, nullptr, nullptr);
+  rc = finish_bfs(ts, false, ctx->h_pin, last, &active, nullptr, nullptr);
+  if (cyc.done == 2 && rc == JFC_ERR_NOT_CONVERGED) {   // the cut's budget, reported with the cut
+    active.assign(ts.ngrids, 0);
+    rc = JFC_OK;
+  }
+  return rc;
 }
 
-int engine_cut(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, std::vector<GridResult>& res, int& passes,
-               cudaEvent_t done) {
-  cudaStream_t s = ctx->stream;
-  res.assign(ts.ngrids, GridResult());
-  // counters and sums are read back together, with one wait
-  int rc = pin_reserve(ctx, pin_need(ts));
-  if (rc) return rc;
-  JFC_CUDA(enqueue_bfs(ts, true, p.max_bfs_passes, s, ctx->h_pin));
-  long long* hs = (long long*)((char*)ctx->h_pin + sizeof(DevCounters));
-  JFC_CUDA(cudaMemcpyAsync(hs, ts.d_grid_sum, sizeof(long long) * 2 * ts.ngrids, cudaMemcpyDeviceToHost, s));
-  if (done) JFC_CUDA(cudaEventRecord(done, s));
-  JFC_CUDA(cudaStreamSynchronize(s));
+// Outcome of a cut from the pinned read-back (after the stream sync).
+static int finish_cut(const TileSet& ts, void* pin, std::vector<GridResult>& res, int& passes) {
   int bad = 0;
-  rc = finish_bfs(ts, true, ctx->h_pin, passes, nullptr, &bad, nullptr);
+  int rc = finish_bfs(ts, true, pin, passes, nullptr, &bad, nullptr);
   if (rc) return rc;
+  const long long* hs = pin_sums(ts, pin);
   for (int g = 0; g < ts.ngrids; ++g) {
     res[g].neg_sum = hs[2 * g];
     res[g].labels = hs[2 * g + 1];
@@ -597,6 +618,20 @@ int engine_cut(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, std::vector<GridR
     for (auto& r : res) r.status = rc;
   }
   return rc;
+}
+
+int engine_cut(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, std::vector<GridResult>& res, int& passes,
+               cudaEvent_t done) {
+  cudaStream_t s = ctx->stream;
+  res.assign(ts.ngrids, GridResult());
+  // counters and sums are read back together, with one wait
+  const int rc = pin_reserve(ctx, pin_need(ts));
+  if (rc) return rc;
+  JFC_CUDA(enqueue_bfs(ts, true, p.max_bfs_passes, s, ctx->h_pin));
+  JFC_CUDA(enqueue_read_sums(ts, s, ctx->h_pin));
+  if (done) JFC_CUDA(cudaEventRecord(done, s));
+  JFC_CUDA(cudaStreamSynchronize(s));
+  return finish_cut(ts, ctx->h_pin, res, passes);
 }
 
 int engine_solve(jfc_ctx* ctx, TileSet& ts, const jfc_params& p_in, std::vector<GridResult>& res,
@@ -644,12 +679,21 @@ int engine_solve(jfc_ctx* ctx, TileSet& ts, const jfc_params& p_in, std::vector<
   const bool fast = p.pr_mode == 1 && fast_grid;
   cyc.tail = pr_sched_for(p) == 3 || fast ? 0 : -1;
   if (fast) cyc.max_cycles = 1;
-  // initial global relabel (fills the work queues), and the cycles behind it
-  rc = run_cycles(ctx, ts, p, true, cyc, pr_sched_for(p) == 3 ? 1 : pr_sched_for(p), st.bfs_passes, active, &graphs);
+  // initial global relabel (fills the work queues), the cycles behind it, and the
+  // exact relabel and the cut
+  rc = run_cycles(ctx, ts, p, true, cyc, pr_sched_for(p) == 3 ? 1 : pr_sched_for(p), st.bfs_passes, active, &graphs, ev[1]);
   if (rc) return rc;
   st.global_relabels = cyc.cycles;
-  st.pr_phases = cyc.cycles - 1;
+  st.pr_phases = cyc.cycles - cyc.exact - 1;
   st.sweeps += cyc.sweeps;
+  bool post_exact = false;   // the exact relabel ran and found reachable excess
+  // the run's exact relabel, if it came to one, stands for the host's below
+  auto ran_exact = [&]() {
+    if (!cyc.exact) return;
+    h_cap = last_cap = 0;
+    if (cyc.done != 2) post_exact = true;
+  };
+  ran_exact();
 
   auto total = [&]() { long long t = 0; for (int v : active) t += v; return t; };
   const DevCounters* hc = (const DevCounters*)ctx->h_pin;
@@ -667,7 +711,6 @@ int engine_solve(jfc_ctx* ctx, TileSet& ts, const jfc_params& p_in, std::vector<
   }
   int status = JFC_OK;
   double fast_ms = 0.0;   // Fast-Cut iterations (event-timed: many small launches)
-  bool post_exact = false;   // the exact relabel ran and found reachable excess
   for (;;) {
   while (total() > 0) {
     if (st.sweeps >= p.max_sweeps) {
@@ -707,11 +750,12 @@ int engine_solve(jfc_ctx* ctx, TileSet& ts, const jfc_params& p_in, std::vector<
       cyc.local_iters = tail ? cyc.iters_tail : cyc.iters;
       if (pr_sched_for(p) == 3) cyc.tail = tail ? 1 : 0;
       cyc.max_sweeps = p.max_sweeps - st.sweeps;
-      rc = run_cycles(ctx, ts, p, false, cyc, sched, st.bfs_passes, active, &graphs);
-      st.pr_phases += cyc.cycles;
+      rc = run_cycles(ctx, ts, p, false, cyc, sched, st.bfs_passes, active, &graphs, ev[1]);
+      st.pr_phases += cyc.cycles - cyc.exact;
       st.global_relabels += cyc.cycles;
       if (rc) return rc;
       st.sweeps += cyc.sweeps;
+      ran_exact();
     }
     if (p.verbose) {
       hc = (const DevCounters*)ctx->h_pin;
@@ -748,15 +792,15 @@ int engine_solve(jfc_ctx* ctx, TileSet& ts, const jfc_params& p_in, std::vector<
   }
 
   // canonical cut: nodes reachable from excess in the final residual graph
-  JFC_CUDA(cudaEventRecord(ev[2], s));
   int passes = st.bfs_passes;
-  std::vector<GridResult> cut;
-  rc = engine_cut(ctx, ts, p, cut, passes, ev[1]);
+  std::vector<GridResult> cut(ts.ngrids);
+  rc = status == JFC_OK && cyc.done == 2 ? finish_cut(ts, ctx->h_pin, cut, passes) 
+                                         : engine_cut(ctx, ts, p, cut, passes, ev[1]);
   if (rc && rc != JFC_ERR_NOT_CONVERGED) return rc;
   st.bfs_passes = passes;
   // device-clock phase times and visit counters (the cut read them back)
   const unsigned long long* hv = &((const DevCounters*)ctx->h_pin)->visits;
-  st.ms_cut = elapsed_ms(ev[2], ev[1]);
+  st.ms_cut = ((const DevCounters*)ctx->h_pin)->ns_cut * 1e-6;
   st.ms_total = elapsed_ms(ev[0], ev[1]);
   st.tile_visits = (long long)hv[0];
   st.bfs_visits = (long long)hv[1];

@@ -57,6 +57,10 @@ struct CycleState {
   int tail;                  // stay in the bulk (0) or the tail (1) only; -1: either
   int max_cycles, max_sweeps;  // the run ends with the cycle that reaches either
   int cycles, sweeps, passes;  // relabels, sweeps and BFS passes of the run so far
+  int go;                    // the run's next cycle is due
+  int done;                  // 1: no active tile under the cap, the exact relabel is due; 2: none at all, the
+                             // cut is due
+  int exact;                 // exact relabels of the run
   unsigned long long last_pr, last_gr;  // ns_pr, ns_gr_first + ns_gr_frontier behind the last cycle
 };
 
@@ -100,6 +104,7 @@ struct DevCounters {
   unsigned long long ns_pr;           // push-relabel phases, device ns
   unsigned long long t_gr_start;      // device clock at the start of the last relabel
   unsigned long long prof[8];         // SM-cycle split of push-relabel visits (JFC_PHASE_CLOCK builds)
+  unsigned long long ns_cut;          // last cut, device ns
   unsigned long long spin_limit;  // polls before a device-side wait gives up (0: 2^26)
   unsigned pr_head;          // push-relabel worklist: tickets taken
   unsigned pr_tail;          // push-relabel worklist: ring positions reserved
@@ -150,8 +155,9 @@ struct TileSet {
   DevCounters* d_ctr = nullptr;
   void* d_block = nullptr;           // single allocation backing the above
   size_t block_bytes = 0;
-  int cyc_mode = 0;                  // global relabels advance d_ctr->cyc: 0 no, 1 as the first of a run
-                                     // (no phase before it), 2 as the end of a cycle
+  int cyc_mode = 0;                  // part of a run of cycles (d_ctr->cyc) that a launch is: 0 none, 1 first
+                                     // relabel, 2 cycle, 3 exact relabel, 4 cut; 2 to 4 return at once
+                                     // unless due
   unsigned long long cyc_cond = 0;   // and say whether the graph's loop goes on (0: none)
   int cap_tiles = 0, cap_grids = 0;  // capacity of d_block (reused while it fits)
   long long cap_rw = 0;              // row words

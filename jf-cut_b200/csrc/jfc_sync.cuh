@@ -98,6 +98,14 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
+// A launch of a run of cycles that is not due (the same for all of its CTAs: only
+// a relabel's end changes it).
+__device__ __forceinline__ bool cycle_skips(const TileSet& ts) {
+  const CycleState& c = ts.d_ctr->cyc;
+  return ts.cyc_mode == 2 ? !vload(&c.go) : ts.cyc_mode == 3 ? vload(&c.done) != 1
+       : ts.cyc_mode == 4 ? vload(&c.done) != 2 : false;
+}
+
 // A loop that this relabel ends a turn of stops unless end_cycle says otherwise
 // (one thread, at the relabel's start: a relabel that gives up ends the loop).
 __device__ __forceinline__ void begin_cycle(const TileSet& ts) {
@@ -106,7 +114,9 @@ __device__ __forceinline__ void begin_cycle(const TileSet& ts) {
 
 // End of a relabel cycle, one warp, behind the relabel's last barrier and its
 // thread 0's counters: advance the schedule, and let the loop go on while tiles
-// are active and no limit is reached.  A cycle decided by the host costs 28 us
+// are active and no limit is reached.  Without active tiles under the cap the
+// exact relabel is due, without any the cut: both are behind the loop in the
+// same run.  A cycle decided by the host costs 28 us
 // besides its kernels (read-back, wait, launch), a turn of the graph's loop 10
 // (1023 x 767: 14 relabels, 2.12 / 1.94 ms).
 __device__ __forceinline__ void end_cycle(const TileSet& ts) {
@@ -130,10 +140,14 @@ __device__ __forceinline__ void end_cycle(const TileSet& ts) {
   c.last_gr = gr;
   c.cycles += 1;
   c.passes += ctr->bfs_passes;
+  const bool ok = vload(&ctr->error) == 0 && ctr->bfs_status == 1;
+  c.go = ok && ts.cyc_mode != 3 && active > 0 && c.cycles < c.max_cycles && c.sweeps < c.max_sweeps &&
+         (c.tail < 0 || (c.tail != 0) == tail);
+  c.done = ok && active == 0 ? (c.h_cap > 0 ? 1 : 2) : 0;
+  if (ts.cyc_mode == 3) c.exact += 1;
+  if (c.done == 1) c.h_cap = 0;
   ctr->cyc = c;
-  const bool go = active > 0 && vload(&ctr->error) == 0 && ctr->bfs_status == 1 && c.cycles < c.max_cycles &&
-                  c.sweeps < c.max_sweeps && (c.tail < 0 || (c.tail != 0) == tail);
-  if (go && ts.cyc_cond) cudaGraphSetConditional((cudaGraphConditionalHandle)ts.cyc_cond, 1u);
+  if (c.go && ts.cyc_cond) cudaGraphSetConditional((cudaGraphConditionalHandle)ts.cyc_cond, 1u);
 }
 
 // Phase-clock instrumentation (builds with -DJFC_PHASE_CLOCK): thread 0 adds

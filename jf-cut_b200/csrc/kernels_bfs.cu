@@ -380,6 +380,7 @@ template <int TY, int TZ>
 __global__ void __launch_bounds__(256, TY * TZ > 8 ? 1 : 2) k_bits3(TileSet ts) {
   constexpr int R = TY * TZ;
   using D = Dirs<3>;
+  if (jfc::cycle_skips(ts)) return;
   DevCounters* ctr = ts.d_ctr;
   const int lane = threadIdx.x & 31;
   const long long gt = blockIdx.x * (long long)blockDim.x + threadIdx.x, gn = (long long)gridDim.x * blockDim.x;
@@ -455,6 +456,7 @@ __global__ void __launch_bounds__(256, 4) k_relabel_first(TileSet ts) {
   constexpr int R = TY * TZ, G = 32 / R, kPlanes = R > 8 ? 10 : 9;   // tiles a warp; bits of a level (at most 32 R)
   struct Row { unsigned v, def, p[kPlanes]; };
   __shared__ Row s_row[8][32];
+  if (jfc::cycle_skips(ts)) return;
   DevCounters* ctr = ts.d_ctr;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -779,6 +781,7 @@ __device__ __forceinline__ void refill_pr_queues(const TileSet& ts, DevCounters*
 template <int TY, int TZ>
 __global__ void __launch_bounds__(256, TY * TZ > 8 ? 2 : JFC_RL3D_MINB)
     k_relabel_warp(TileSet ts, int max_passes) {
+  if (jfc::cycle_skips(ts)) return;
   __shared__ int s_items[8][64];   // per-warp staged queue appends (at most 38 before a flush)
   __shared__ int s_cnt[8];
   // 3D tiles of up to 8 rows with tensor maps: each warp stages its tiles by
@@ -974,6 +977,7 @@ __global__ void __launch_bounds__(256, 4) k_cut3(TileSet ts, int max_passes) {
   __shared__ int s_list[kList];
   __shared__ int s_n, s_base;
   __shared__ unsigned long long s_sum[2], s_vis;
+  if (jfc::cycle_skips(ts)) return;
   DevCounters* ctr = ts.d_ctr;
   const int t = threadIdx.x, lane = t & 31;
   const int warp = (int)((blockIdx.x * blockDim.x + t) >> 5), nwarps = (int)(gridDim.x * blockDim.x >> 5);
@@ -1139,6 +1143,7 @@ __global__ void __launch_bounds__(256, 4) k_cut3(TileSet ts, int max_passes) {
     atomicAdd(&ctr->bfs_visits, s_vis);
     if (blockIdx.x == 0) {
       ctr->bfs_passes = pass;
+      ctr->ns_cut = jfc::global_ns() - ctr->t_gr_start;
       if (ok) ctr->bfs_status = 1;
     }
   }
@@ -1146,7 +1151,9 @@ __global__ void __launch_bounds__(256, 4) k_cut3(TileSet ts, int max_passes) {
 
 // (a launch of its own: in k_relabel_warp it changed the visits' registers and made
 // the frontier 15% slower)
-__global__ void k_end_cycle(TileSet ts) { jfc::end_cycle(ts); }
+__global__ void k_end_cycle(TileSet ts) {
+  if (!jfc::cycle_skips(ts)) jfc::end_cycle(ts);
+}
 
 // per-grid sum of min(e, 0) and count of source-side nodes (reduce_flow,
 // bin/x64/cl/Infrastructures/reduce.cl:92-117, in int64 instead of int32 partials)

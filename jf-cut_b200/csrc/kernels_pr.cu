@@ -499,6 +499,7 @@ __global__ void __launch_bounds__(Tile<DIMS, TY, TZ>::NT,
   int next_buf = 0;         // thread 0: buffer of the next fill
   int s = 0;
   const int npairs = sweeps > 0 ? sweeps : jfc::vload(&ctr->cyc.pr_sweeps);
+  if (jfc::cycle_skips(ts)) return;
   if (threadIdx.x == 0) sm.local_iters = sweeps > 0 ? local_iters : jfc::vload(&ctr->cyc.local_iters);
   const int own = min((int)blockIdx.x, ts.ntiles - 1);   // (a parity's queue holds at most ntiles items)
   int cur[2] = {0, 0};   // pending buffer per parity (0 after a global relabel)
@@ -681,6 +682,7 @@ __global__ void __launch_bounds__(Tile<DIMS, TY, TZ>::NT)
   DevCounters* ctr = ts.d_ctr;
   const unsigned long long t0 = jfc::global_ns();
   const int npairs = sweeps > 0 ? sweeps : jfc::vload(&ctr->cyc.pr_sweeps);
+  if (jfc::cycle_skips(ts)) return;
   if (threadIdx.x == 0) sm.local_iters = sweeps > 0 ? local_iters : jfc::vload(&ctr->cyc.local_iters);
   const int gens = 2 * npairs;
   const unsigned cap = (unsigned)(SPLIT ? 2 * ts.ntiles : ts.ntiles);

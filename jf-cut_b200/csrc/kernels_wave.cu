@@ -77,8 +77,12 @@ __device__ __forceinline__ void changed_tiles(const TileSet& ts) {
     ctr->wave_q = 0;
     ctr->ticket[0] = ctr->ticket[1] = 0;
     ctr->pr_bar = 0;
+    ctr->cut_bad = 0;
   }
-  for (long long i = gt; i < ts.ngrids; i += gn) ts.d_grid_active[i] = 0;
+  for (long long i = gt; i < ts.ngrids; i += gn) {
+    ts.d_grid_active[i] = 0;
+    ts.d_grid_sum[2 * i] = ts.d_grid_sum[2 * i + 1] = 0;
+  }
   for (long long i = gt; i < ts.nreg; i += gn) ts.d_rflag[0][i] = ts.d_rflag[1][i] = 0;
   const long long nitems = ts.pr_split ? 2ll * ts.ntiles : ts.ntiles;
   for (long long i = gt; i < nitems; i += gn) ts.d_flag_pr[i] = 0;
@@ -209,6 +213,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave_relabel(TileSet ts) {
   __shared__ unsigned s_mask, s_new[2], s_tiles;
   __shared__ unsigned long long s_base;
   DevCounters* ctr = ts.d_ctr;
+  if (jfc::cycle_skips(ts)) return;
   const unsigned epoch = wave_epoch(ctr);
   unsigned seen = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -538,8 +543,10 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave_cut(TileSet ts, int max_pa
   const int aout = ws == 0 ? 2 * (warp + 1) * kC + c : ws == 3 ? (2 * (warp + 1) + 1) * kC + c : 192 + lane;
   const unsigned ml = c == 0 ? 0u : ~0u, mr = c == kC - 1 ? 0u : ~0u;
   unsigned long long visits = 0;
+  if (jfc::cycle_skips(ts)) return;
   const unsigned epoch = wave_epoch(ctr);
   unsigned seen = 0;
+  if (blockIdx.x == 0 && t == 0) ctr->t_gr_start = jfc::global_ns();
   int phase = 1;
   bool ok_all = true;
   for (;; ++phase) {
@@ -721,6 +728,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave_cut(TileSet ts, int max_pa
     if (blockIdx.x == 0) {
       ctr->bfs_passes = phase;
       ctr->wave_epoch = epoch + 1;
+      ctr->ns_cut = jfc::global_ns() - ctr->t_gr_start;
       if (ok_all) ctr->bfs_status = 1;
     }
   }
@@ -730,9 +738,10 @@ template <int TY>
 cudaError_t wave_cut_t(const TileSet& ts, int max_passes, cudaStream_t s) {
   static int cache[64] = {0};
   const void* fn = (const void*)k_wave_cut<TY>;
-  cudaError_t e = cudaMemsetAsync(ts.d_grid_sum, 0, sizeof(long long) * 2 * ts.ngrids, s);
+  // (in a run of cycles the relabel before it cleared them, and may have set the status)
+  cudaError_t e = ts.cyc_mode ? cudaSuccess : cudaMemsetAsync(ts.d_grid_sum, 0, sizeof(long long) * 2 * ts.ngrids, s);
   static_assert(offsetof(DevCounters, bfs_status) == offsetof(DevCounters, cut_bad) + sizeof(int), "zeroed together");
-  if (e == cudaSuccess) e = cudaMemsetAsync(&ts.d_ctr->cut_bad, 0, 2 * sizeof(int), s);
+  if (e == cudaSuccess && !ts.cyc_mode) e = cudaMemsetAsync(&ts.d_ctr->cut_bad, 0, 2 * sizeof(int), s);
   if (e != cudaSuccess) return e;
   const int blocks = std::min(persistent_blocks_cached(cache, fn, kThreads), ts.nreg);
   TileSet arg = ts;
