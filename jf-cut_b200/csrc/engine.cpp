@@ -560,9 +560,9 @@ static cudaGraphExec_t cycle_graph(TileSet& ts, bool init, const CycleState* pin
 }
 
 // A run of cycles by schedule cyc (advanced to its state behind the run),
-// replayed from a graph when enabled, else one cycle; returns the outcome of the
-// last global relabel.  init: the run starts with a relabel alone.  Behind
-// cyc.done = 2 the cut has run.
+// replayed from a graph when enabled, else one relabel (init) or cycle; returns the
+// outcome of the last global relabel.  init: the run starts with a relabel
+// alone.  Behind cyc.done = 2 the cut has run.
 static int run_cycles(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, bool init, CycleState& cyc, int sched,
                       int& passes, std::vector<int>& active, bool* used_graph, cudaEvent_t done) {
   cudaStream_t s = ctx->stream;
@@ -572,8 +572,7 @@ static int run_cycles(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, bool init,
   cyc.cycles = cyc.sweeps = cyc.passes = cyc.done = cyc.exact = 0;
   cyc.go = !init;
   *pin_cyc = cyc;   // the previous run's copies finished at its wait
-  const bool alone = cyc.max_cycles == 1;   // one relabel or cycle, nothing behind it
-  cudaGraphExec_t x = p.use_graph && !alone
+  cudaGraphExec_t x = p.use_graph && cyc.max_cycles > 1
                           ? cycle_graph(ts, init, pin_cyc, p.max_bfs_passes, sched, s, ctx->h_pin)
                           : nullptr;
   if (x) {
@@ -581,12 +580,12 @@ static int run_cycles(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, bool init,
   } else {
     JFC_CUDA(enqueue_schedule(ts, pin_cyc, s));
     JFC_CUDA(enqueue_cycle(ts, init, p.max_bfs_passes, sched, 0, s));
-    JFC_CUDA(alone ? enqueue_read(ts, true, s, ctx->h_pin) : enqueue_finish(ts, p.max_bfs_passes, s, ctx->h_pin));
+    JFC_CUDA(enqueue_read(ts, true, s, ctx->h_pin));
   }
   JFC_CUDA(cudaEventRecord(done, s));
   JFC_CUDA(cudaStreamSynchronize(s));
   cyc = ((const DevCounters*)ctx->h_pin)->cyc;
-  if (alone) cyc.done = 0;
+  if (!x) cyc.done = 0;   // (nothing behind one relabel or cycle)
   const int phases = cyc.cycles - cyc.exact - (init ? 1 : 0);
   if (x) {
     const int per = ts.dims == 2 ? 1 : 4;   // kernels of a relabel

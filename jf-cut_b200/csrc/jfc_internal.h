@@ -110,7 +110,7 @@ struct DevCounters {
   unsigned pr_tail;          // push-relabel worklist: ring positions reserved
   int pr_out;                // push-relabel worklist: items queued and not yet fully visited
   // 2D global relabel (kernels_wave.cu)
-  int cut_n[3];              // 3D cut: blocks queued for pass p, in entry p % 3
+  int q3_n[3];               // 3D relabel and cut: tiles or blocks queued for pass p, in entry p % 3
   unsigned long long wave_bar[2]; // barrier arrivals (low 40 bits), CTAs that flagged a region (high bits)
   unsigned wave_epoch;       // launches so far: which of the two the next one uses
   unsigned long long wave_q; // active items queued so far: parity 0 low, parity 1 high 32 bits
@@ -132,8 +132,7 @@ struct TileSet {
   int* d_q_pr[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [parity][buffer]
   int* d_flag_bfs[2] = {nullptr, nullptr};  // [buffer][ntiles] tile waits in a BFS frontier
   int* d_q_bfs[2] = {nullptr, nullptr};     // [buffer] BFS frontiers
-  uint8_t* d_act = nullptr;          // [ntiles] bits 0-1: tile (half) held an active node at its last
-                                     // relabel visit
+  uint8_t* d_act = nullptr;          // [ntiles] 3D: the tile held an active node at its last relabel visit
   // global relabel
   uint4* d_vf = nullptr;             // 2D: [row words] two buffers of level-set state
                                      // (kernels_wave.cu); 3D: [row words][2] arcs and excess

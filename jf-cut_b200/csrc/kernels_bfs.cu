@@ -321,48 +321,46 @@ __device__ __forceinline__ int row_close(int v, unsigned axp, unsigned axm, int 
 // over residual arcs u -> v inside the tile, to the fixpoint.  Row closures
 // by doubling shuffles, y and z runs in registers (a backward and a forward
 // sweep per line); bounded by the tile's nodes (every pass but the last
-// lowers some height, and heights are bounded below by 0).
+// lowers some height, and heights are bounded below by 0).  The row closures
+// are what a visit costs (10 shuffles and 80 instructions a row), so only rows
+// that something lowered since their last one get one, 4 at a time (their
+// chains overlap); `rows`: the rows lowered before the call (the same in every
+// lane).  With every row closed in every pass, and a last pass to see that
+// nothing falls, the frontier took 48.2 ms of a 2560 x 1440 x 50 solve instead of
+// 44.9.
 template <int DIMS, int TY, int TZ>
 __device__ __forceinline__ void tile_close(int (&hv)[TY * TZ], const unsigned (&lab)[TY * TZ],
-                                           const unsigned (&AXP)[TY * TZ], const unsigned (&AXM)[TY * TZ], int lane) {
+                                           const unsigned (&AXP)[TY * TZ], const unsigned (&AXM)[TY * TZ], int lane,
+                                           unsigned rows) {
   constexpr int R = TY * TZ;
-  for (int pass = 0; pass < 32 * R; ++pass) {
-    bool ch = false;
+  for (int pass = 0; rows != 0u && pass < 32 * R; ++pass) {
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const int v = row_close(hv[i], AXP[i], AXM[i], lane);
-      ch |= v < hv[i];
-      hv[i] = v;
+    for (int i0 = 0; i0 < R; i0 += 4) {
+      if ((rows >> i0 & 15u) == 0u) continue;
+#pragma unroll
+      for (int i = i0; i < i0 + 4; ++i) hv[i] = row_close(hv[i], AXP[i], AXM[i], lane);
     }
+    unsigned low = 0;   // rows lowered in this lane
+    auto run = [&](int i, int from, unsigned arc) {
+      if ((lab[i] & arc) && hv[from] + 1 < hv[i]) { hv[i] = hv[from] + 1; low |= 1u << i; }
+    };
 #pragma unroll
     for (int z = 0; z < TZ; ++z) {
 #pragma unroll
-      for (int y = TY - 2; y >= 0; --y) {
-        const int i = z * TY + y;
-        if ((lab[i] & jfc::A_YP) && hv[i + 1] + 1 < hv[i]) { hv[i] = hv[i + 1] + 1; ch = true; }
-      }
+      for (int y = TY - 2; y >= 0; --y) run(z * TY + y, z * TY + y + 1, jfc::A_YP);
 #pragma unroll
-      for (int y = 1; y < TY; ++y) {
-        const int i = z * TY + y;
-        if ((lab[i] & jfc::A_YM) && hv[i - 1] + 1 < hv[i]) { hv[i] = hv[i - 1] + 1; ch = true; }
-      }
+      for (int y = 1; y < TY; ++y) run(z * TY + y, z * TY + y - 1, jfc::A_YM);
     }
     if constexpr (DIMS == 3) {
 #pragma unroll
       for (int y = 0; y < TY; ++y) {
 #pragma unroll
-        for (int z = TZ - 2; z >= 0; --z) {
-          const int i = z * TY + y;
-          if ((lab[i] & jfc::A_ZP) && hv[i + TY] + 1 < hv[i]) { hv[i] = hv[i + TY] + 1; ch = true; }
-        }
+        for (int z = TZ - 2; z >= 0; --z) run(z * TY + y, z * TY + y + TY, jfc::A_ZP);
 #pragma unroll
-        for (int z = 1; z < TZ; ++z) {
-          const int i = z * TY + y;
-          if ((lab[i] & jfc::A_ZM) && hv[i - TY] + 1 < hv[i]) { hv[i] = hv[i - TY] + 1; ch = true; }
-        }
+        for (int z = 1; z < TZ; ++z) run(z * TY + y, z * TY + y - TY, jfc::A_ZM);
       }
     }
-    if (!__any_sync(FULL, ch)) break;
+    rows = __reduce_or_sync(FULL, low);
   }
 }
 
@@ -389,8 +387,10 @@ __global__ void __launch_bounds__(256, TY * TZ > 8 ? 1 : 2) k_bits3(TileSet ts) 
     jfc::begin_cycle(ts);
     ctr->bfs_status = 0;
     ctr->ticket[0] = ctr->ticket[1] = 0;
-    ctr->qn_bfs[0] = ctr->qn_bfs[1] = 0;
-    ctr->cut_n[0] = ctr->cut_n[1] = ctr->cut_n[2] = 0;
+    ctr->qn_pr[0][0] = ctr->qn_pr[0][1] = ctr->qn_pr[1][0] = ctr->qn_pr[1][1] = 0;
+    ctr->cur_pr[0] = ctr->cur_pr[1] = 0;
+    ctr->wave_bar[0] = 0;
+    ctr->q3_n[0] = ctr->q3_n[1] = ctr->q3_n[2] = 0;
     ctr->cut_bad = 0;
     ctr->pr_bar = 0;
   }
@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(256, 4) k_relabel_first(TileSet ts) {
     case 5: want = (bz1 & group) && ti.w + 1 < g.tiles_z; nb = tid + txy; break;
     default: break;
   }
-  jfc::warp_append(want, nb, ts.d_flag_bfs[1], ts.d_q_bfs[1], &ctr->qn_bfs[1]);
+  jfc::warp_append(want, nb, ts.d_flag_bfs[1], ts.d_q_bfs[1], &ctr->q3_n[1]);
   if (ok && r == 0) ts.d_act[tid] = act ? 1 : 0;
   const unsigned lead = __ballot_sync(FULL, ok && r == 0 && act);
   if (ts.ngrids == 1) {
@@ -664,34 +664,34 @@ __device__ __forceinline__ void relabel_frontier_minplus(const TileSet& ts, int 
   // the tile's interior is at its fixpoint (the dense pass or its last
   // visit closed it, and only its own visits write it), so only a halo seed
   // that lowers a border node can change anything
-  bool seeded = false;
-  auto seed = [&](int& v, bool arc, int hn) {
-    if (arc && hn + 1 < v) { v = hn + 1; seeded = true; }
+  unsigned seeded = 0;   // rows lowered by the halo in this lane
+  auto seed = [&](int i, bool arc, int hn) {
+    if (arc && hn + 1 < hv[i]) { hv[i] = hn + 1; seeded |= 1u << i; }
   };
 #pragma unroll
   for (int z = 0; z < TZ; ++z) {
     const int it = z * TY, ib = z * TY + TY - 1;
-    seed(hv[it], lab[it] & jfc::A_YM, HT[z]);
-    seed(hv[ib], lab[ib] & jfc::A_YP, HB[z]);
+    seed(it, lab[it] & jfc::A_YM, HT[z]);
+    seed(ib, lab[ib] & jfc::A_YP, HB[z]);
   }
   if constexpr (DIMS == 3) {
 #pragma unroll
     for (int y = 0; y < TY; ++y) {
       const int it = y, ib = (TZ - 1) * TY + y;
-      seed(hv[it], lab[it] & jfc::A_ZM, HZT[y]);
-      seed(hv[ib], lab[ib] & jfc::A_ZP, HZB[y]);
+      seed(it, lab[it] & jfc::A_ZM, HZT[y]);
+      seed(ib, lab[ib] & jfc::A_ZP, HZB[y]);
     }
   }
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     const int hl = __shfl_sync(FULL, hx, i), hr = __shfl_sync(FULL, hx, 16 + i);
-    seed(hv[i], lane == 0 && (lab[i] & jfc::A_XM), hl);
-    seed(hv[i], lane == 31 && (lab[i] & jfc::A_XP), hr);
+    seed(i, lane == 0 && (lab[i] & jfc::A_XM), hl);
+    seed(i, lane == 31 && (lab[i] & jfc::A_XP), hr);
   }
-  if (__any_sync(FULL, seeded)) tile_close<DIMS, TY, TZ>(hv, lab, AXP, AXM, lane);
+  tile_close<DIMS, TY, TZ>(hv, lab, AXP, AXM, lane, __reduce_or_sync(FULL, seeded));
   const int cap = jfc::cap_of(g, ts.d_ctr);
   unsigned rows_changed = 0;
-  bool c0 = false, c31 = false, act_lo = false, act_hi = false;
+  bool c0 = false, c31 = false, act = false;
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     if (hv[i] >= cap) hv[i] = h0[i];   // at or above the cap: stays as it was (unreachable)
@@ -703,18 +703,12 @@ __device__ __forceinline__ void relabel_frontier_minplus(const TileSet& ts, int 
       c31 |= (m >> 31) != 0;
     }
     if (chg) g.h[roff<TY>(a, i)] = hv[i];
-    // activity per 8-row half of a 2D 32x16 tile (bit 0 rows 0-7, bit 1
-    // rows 8-15: the push-relabel work items of split tile sets), else bit 0
-    const bool live = ((posm >> i) & 1u) && hv[i] < JFC_INF;
-    if (DIMS == 2 && TY == 16 && i >= 8) act_hi |= live;
-    else act_lo |= live;
+    act |= ((posm >> i) & 1u) && hv[i] < JFC_INF;
   }
-  act_lo = __any_sync(FULL, act_lo);
-  act_hi = __any_sync(FULL, act_hi);
-  const bool act = act_lo || act_hi;
+  act = __any_sync(FULL, act);
   if (lane == 0) {
-    const int old = (act_old & 3u) != 0 ? 1 : 0;
-    ts.d_act[tid] = (uint8_t)((act_lo ? 1 : 0) | (act_hi ? 2 : 0));
+    const int old = act_old != 0 ? 1 : 0;
+    ts.d_act[tid] = act ? 1 : 0;
     if (ti.x != cur_grid) {
       if (delta && cur_grid >= 0) atomicAdd(&ts.d_grid_active[cur_grid], delta);
       delta = 0;
@@ -726,51 +720,34 @@ __device__ __forceinline__ void relabel_frontier_minplus(const TileSet& ts, int 
 }
 
 // Refill of the push-relabel queues (buffer 0 of each parity) from the
-// active-tile bits, warp-aggregated.  Split tile sets queue the active 8-row
-// halves as work items 2 * tile + half, half 0 with the tile's checkerboard
-// parity in the 32x8 tiling and half 1 with the other.
-__device__ __forceinline__ void refill_pr_queues(const TileSet& ts, DevCounters* ctr, int lane) {
-  for (;;) {
-    const unsigned c = jfc::warp_ticket(&ctr->ticket[0]);
-    const long long b = (long long)c * 32;
-    if (b >= ts.ntiles) break;
+// active-tile flags, warp-aggregated.
+__device__ __forceinline__ void refill_pr_queues(const TileSet& ts, DevCounters* ctr, int warp, int nwarps, int lane) {
+  for (long long b = 32ll * warp; b < ts.ntiles; b += 32ll * nwarps) {
     const long long t = b + lane;
-    bool w[2][2] = {{false, false}, {false, false}};   // [half][parity queue]
-    if (t < ts.ntiles) {
-      const unsigned bits = ts.d_act[t] & 3u;
-      int par = 0;
-      if (bits) { const int4 ti = ts.d_info[t]; par = (ti.y + (ts.pr_split ? 2 * ti.z : ti.z) + ti.w) & 1; }
-      if (ts.pr_split) {
-        const bool a0 = (bits & 1u) != 0, a1 = (bits & 2u) != 0;
-        ts.d_flag_pr[2 * t] = a0 ? 1 : 0;
-        ts.d_flag_pr[2 * t + 1] = a1 ? 1 : 0;
-        w[0][par] = a0;
-        w[1][par ^ 1] = a1;
-      } else {
-        ts.d_flag_pr[t] = bits ? 1 : 0;
-        w[0][par] = bits != 0;
-      }
-    }
-    const int item0 = ts.pr_split ? (int)(2 * t) : (int)t;
-    jfc::warp_append(w[0][0], item0, nullptr, ts.d_q_pr[0][0], &ctr->qn_pr[0][0]);
-    jfc::warp_append(w[0][1], item0, nullptr, ts.d_q_pr[1][0], &ctr->qn_pr[1][0]);
-    if (ts.pr_split) {
-      jfc::warp_append(w[1][0], item0 + 1, nullptr, ts.d_q_pr[0][0], &ctr->qn_pr[0][0]);
-      jfc::warp_append(w[1][1], item0 + 1, nullptr, ts.d_q_pr[1][0], &ctr->qn_pr[1][0]);
-    }
+    const bool act = t < ts.ntiles && __ldcg(ts.d_act + t) != 0;
+    int par = 0;
+    if (act) { const int4 ti = ts.d_info[t]; par = (ti.y + ti.z + ti.w) & 1; }
+    if (t < ts.ntiles) ts.d_flag_pr[t] = act ? 1 : 0;
+    jfc::warp_append(act && par == 0, (int)t, nullptr, ts.d_q_pr[0][0], &ctr->qn_pr[0][0]);
+    jfc::warp_append(act && par == 1, (int)t, nullptr, ts.d_q_pr[1][0], &ctr->qn_pr[1][0]);
   }
 }
 
-// Global relabel, frontier passes (persistent, cooperative): one CTA per
-// queued tile, grid barrier between passes, until a pass queues nothing; then
-// the push-relabel queues are refilled with every tile holding an active node
-// (the reference's graphcut_count_node + clogs scan + graphcut_scatter_node,
+// Global relabel, frontier passes (persistent, cooperative): one warp per queued
+// tile, a grid barrier between passes, until a pass queues nothing; then the
+// push-relabel queues are refilled with every tile holding an active node (the
+// reference's graphcut_count_node + clogs scan + graphcut_scatter_node,
 // graphcut_count_block.cl:19-65, as one warp-aggregated append).
-// Warp form of the frontier passes: one warp per queued tile (3D: many
-// tiles per pass, so the visit throughput counts).
-// (2 CTAs per SM, the registers the two-ahead ticket pipeline holds without spills: 3
-// CTAs per SM spilled and measured slower, 116.5 vs 104-108.5 ms of frontier
-// per video solve)
+// A pass holds a few tiles per warp and its time is a chain of latencies, so
+// every nwarps-th queue entry is a warp's own, consecutive ones on different
+// SMs: a warp reads up to 32 entries and their tiles at once.  (By tickets, with
+// the next two tiles' tickets, entries and coordinates fetched one after the
+// other before each visit, and barriers of 3 us, the frontier took
+// 27.2 ms of a 2560 x 1440 x 50 solve instead of 23.5, 3.25 of a 640 x 400 x 20 one
+// instead of 2.38.)
+// (2 CTAs per SM, the registers the staging holds without spills: 3 CTAs per
+// SM spilled and measured slower, 116.5 vs 104-108.5 ms of frontier per video
+// solve)
 #ifndef JFC_RL3D_MINB
 #define JFC_RL3D_MINB 2
 #endif
@@ -786,13 +763,14 @@ __global__ void __launch_bounds__(256, TY * TZ > 8 ? 2 : JFC_RL3D_MINB)
   __shared__ int s_cnt[8];
   // 3D tiles of up to 8 rows with tensor maps: each warp stages its tiles by
   // tensor copies into two buffers of its own (dynamic shared memory), the
-  // next ticket's tile copied while the current one is visited
+  // next entry's tile copied while the current one is visited
   using Stage = RlStage<TY, TZ>;
   constexpr bool kStage = JFC_RL3D_STAGE && TY * TZ <= 8;
   __shared__ uint64_t s_bar[8][2];
   extern __shared__ __align__(128) unsigned char s_dyn[];
   DevCounters* ctr = ts.d_ctr;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int gw = warp * (int)gridDim.x + (int)blockIdx.x, nw = (int)(gridDim.x * (blockDim.x >> 5));
   const bool tma = kStage && ts.d_tmap != nullptr;
   Stage* stage = reinterpret_cast<Stage*>(s_dyn + ((128u - (jfc::smem_addr(s_dyn) & 127u)) & 127u)) + 2 * warp;
   if (lane == 0) s_cnt[warp] = 0;
@@ -827,113 +805,80 @@ __global__ void __launch_bounds__(256, TY * TZ > 8 ? 2 : JFC_RL3D_MINB)
   const unsigned long long t1 = jfc::global_ns();
   for (pass = 1; ok; ++pass) {
     const int cb = pass & 1;
-    const int n = jfc::vload(&ctr->qn_bfs[cb]);
+    const int n = jfc::vload(&ctr->q3_n[pass % 3]);
     if (n == 0) break;
     if (pass > max_passes) {
       if (blockIdx.x == 0 && threadIdx.x == 0) ctr->bfs_status = 2;
       break;
     }
-    BfsQ Q{ts.d_flag_bfs[cb ^ 1], ts.d_q_bfs[cb ^ 1], &ctr->qn_bfs[cb ^ 1], s_items[warp], &s_cnt[warp]};
+    BfsQ Q{ts.d_flag_bfs[cb ^ 1], ts.d_q_bfs[cb ^ 1], &ctr->q3_n[(pass + 1) % 3], s_items[warp], &s_cnt[warp]};
     const int* queue = ts.d_q_bfs[cb];
     int* fcur = ts.d_flag_bfs[cb];
-    // Tickets come in chunks of kChunk while the pass holds a full round of
-    // chunks beyond the warp's (one counter update per chunk: the ticket
-    // and queue counters are single addresses every warp updates, which
-    // serialises them), singly near the end of the pass.  The next ticket,
-    // its queue entry and its tile are fetched while the current tile is
-    // visited.  Queue appends are staged per warp and published 32 or more
-    // at a time.
-    constexpr unsigned kChunk = 4;
-    const long long round = (long long)gridDim.x * (blockDim.x >> 5);
-    unsigned k = 0, kend = 0;   // tickets [k, kend) held by the warp
-    auto take = [&]() -> int {
-      if (k >= kend) {
-        unsigned v = 0;
-        // chunk size from the warp's last ticket (a lower bound on the
-        // counter): no extra read of the counter on the way to its update
-        const unsigned c = (long long)k + round * kChunk < n ? kChunk : 1u;
-        if (lane == 0) v = atomicAdd(&ctr->ticket[cb], c);
-        k = __shfl_sync(FULL, v, 0);
-        kend = k + c;
-      }
-      const unsigned kk = k++;
-      return (int)kk < n ? queue[kk] : -1;
-    };
+    // (every CTA has read the count of the pass before; it is the one after next's)
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctr->q3_n[(pass + 2) % 3] = 0;
     // the previous pass's writes (seen through the grid barrier) come before
     // this pass's tensor reads
     if (tma && lane == 0) jfc::fence_async_global();
-    // Two tickets ahead: the current tile tt is staged in `buf`, the next
-    // one tn is being copied into the other buffer, and the ticket and tile
-    // of the one after (tnn) are fetched while tt is visited; tnn's copy goes
-    // into `buf` once tt's visit has read it.
-    int tt = take();
-    int4 ti = tt >= 0 ? ts.d_info[tt] : make_int4(0, 0, 0, 0);
-    int buf = 0;
-    if (tma && tt >= 0) issue(ti, buf);
-    int tn = tt >= 0 ? take() : -1;
-    int4 tin = tn >= 0 ? ts.d_info[tn] : make_int4(0, 0, 0, 0);
-    if (tma && tn >= 0) issue(tin, buf ^ 1);
-    while (tt >= 0) {
-      const int tnn = tn >= 0 ? take() : -1;
-      const int4 tinn = tnn >= 0 ? ts.d_info[tnn] : make_int4(0, 0, 0, 0);
-      if (lane == 0) fcur[tt] = 0;
-      __syncwarp();
+    const int mine = n > gw ? (n - gw + nw - 1) / nw : 0;   // entries gw, gw + nw, ...
+    bool got = true;
+    for (int b = 0; b < mine && got; b += 32) {
+      const int cnt = min(32, mine - b);
+      const int my_t = lane < cnt ? __ldcg(queue + gw + (b + lane) * nw) : 0;
+      const int4 my_ti = lane < cnt ? ts.d_info[my_t] : make_int4(0, 0, 0, 0);
+      if (lane < cnt) fcur[my_t] = 0;
+      auto tile = [&](int j) {
+        return make_int4(__shfl_sync(FULL, my_ti.x, j), __shfl_sync(FULL, my_ti.y, j), __shfl_sync(FULL, my_ti.z, j),
+                         __shfl_sync(FULL, my_ti.w, j));
+      };
+      // entry j is staged in buffer j & 1, the next one being copied into the other
       if (tma) {
-        const unsigned ph = (parity >> buf) & 1u;
-        const bool got = __all_sync(FULL, jfc::mbar_wait(&s_bar[warp][buf], ph, spin));
-        parity ^= 1u << buf;
-        if (!got) {
-          if (lane == 0) {
-            atomicExch(&ctr->error, 1);
-            // copies in flight land before the warp leaves (fixed bound)
-            constexpr unsigned long long kDrainPolls = 1ull << 26;
-            jfc::mbar_wait(&s_bar[warp][buf], ph, kDrainPolls);
-            if (tn >= 0) jfc::mbar_wait(&s_bar[warp][buf ^ 1], (parity >> (buf ^ 1)) & 1u, kDrainPolls);
+        issue(tile(0), 0);
+        if (cnt > 1) issue(tile(1), 1);
+      }
+      for (int j = 0; j < cnt; ++j) {
+        const int tt = __shfl_sync(FULL, my_t, j), buf = j & 1;
+        const int4 ti = tile(j);
+        __syncwarp();
+        if (tma) {
+          const unsigned ph = (parity >> buf) & 1u;
+          got = __all_sync(FULL, jfc::mbar_wait(&s_bar[warp][buf], ph, spin));
+          parity ^= 1u << buf;
+          if (!got) {
+            if (lane == 0) {
+              atomicExch(&ctr->error, 1);
+              // copies in flight land before the warp leaves (fixed bound)
+              constexpr unsigned long long kDrainPolls = 1ull << 26;
+              jfc::mbar_wait(&s_bar[warp][buf], ph, kDrainPolls);
+              if (j + 1 < cnt) jfc::mbar_wait(&s_bar[warp][buf ^ 1], (parity >> (buf ^ 1)) & 1u, kDrainPolls);
+            }
+            __syncwarp();
+            break;   // the grid barrier below sees the error: every CTA leaves
           }
-          __syncwarp();
-          break;   // the grid barrier below sees the error: every CTA leaves
+          relabel_frontier_minplus<TY, TZ, true>(ts, tt, ti, Q, cur_grid, delta, stage[buf].hb, stage[buf].lb);
+          __syncwarp();   // every lane has read `buf` before it is refilled
+          if (j + 2 < cnt) issue(tile(j + 2), buf);
+        } else {
+          relabel_frontier_minplus<TY, TZ>(ts, tt, ti, Q, cur_grid, delta);
         }
-        relabel_frontier_minplus<TY, TZ, true>(ts, tt, ti, Q, cur_grid, delta, stage[buf].hb, stage[buf].lb);
-        __syncwarp();   // every lane has read `buf` before it is refilled
-        if (tnn >= 0) issue(tinn, buf);
-      } else {
-        relabel_frontier_minplus<TY, TZ>(ts, tt, ti, Q, cur_grid, delta);
-      }
-      buf ^= 1;
-      ++visits;
-      __syncwarp();
-      if (*(volatile int*)Q.scnt >= 32) {
-        flush_staged(Q, lane);
+        ++visits;
         __syncwarp();
-        if (lane == 0) *Q.scnt = 0;
-        __syncwarp();
+        if (*(volatile int*)Q.scnt >= 32) {
+          flush_staged(Q, lane);
+          __syncwarp();
+          if (lane == 0) *Q.scnt = 0;
+          __syncwarp();
+        }
       }
-      tt = tn;
-      ti = tin;
-      tn = tnn;
-      tin = tinn;
     }
     __syncwarp();
     flush_staged(Q, lane);
     __syncwarp();
     if (lane == 0) *Q.scnt = 0;
     __syncwarp();
-    ok = jfc::grid_sync(ctr, [&]() {
-      ctr->ticket[cb] = 0;
-      ctr->qn_bfs[cb] = 0;
-    });
+    ok = jfc::arrive_wait(ctr, ctr->wave_bar, (unsigned long long)pass * gridDim.x);
   }
   if (lane == 0 && delta && cur_grid >= 0) atomicAdd(&ts.d_grid_active[cur_grid], delta);
-  // refill the push-relabel queues (buffer 0 of each parity) from the
-  // active-tile flags
-  if (ok) ok = jfc::grid_sync(ctr, [&]() {
-    ctr->qn_pr[0][0] = ctr->qn_pr[0][1] = ctr->qn_pr[1][0] = ctr->qn_pr[1][1] = 0;
-    ctr->cur_pr[0] = ctr->cur_pr[1] = 0;
-  });
-  if (ok) {
-    refill_pr_queues(ts, ctr, lane);
-    ok = jfc::grid_sync(ctr, [&]() { ctr->ticket[0] = 0; });
-  }
+  if (ok) refill_pr_queues(ts, ctr, gw, nw, lane);
   // frontier visits are counted per warp (lane 0); pass 0 visited every tile
   __shared__ unsigned long long s_vis;
   if (threadIdx.x == 0) s_vis = 0;
@@ -1057,7 +1002,7 @@ __global__ void __launch_bounds__(256, 4) k_cut3(TileSet ts, int max_passes) {
       if (atomicExch(ts.d_flag_bfs[b] + nb, 1) == 0) {
         const int i = atomicAdd(&s_n, 1);
         if (i < kList) s_list[i] = nb;
-        else ts.d_q_bfs[b][atomicAdd(&ctr->cut_n[(pass + 1) % 3], 1)] = nb;
+        else ts.d_q_bfs[b][atomicAdd(&ctr->q3_n[(pass + 1) % 3], 1)] = nb;
       }
     }
     ++visits;
@@ -1067,7 +1012,7 @@ __global__ void __launch_bounds__(256, 4) k_cut3(TileSet ts, int max_passes) {
     if (pass == 0) {
       each_block(visit);
     } else {
-      const int n = jfc::vload(&ctr->cut_n[pass % 3]);
+      const int n = jfc::vload(&ctr->q3_n[pass % 3]);
       if (n == 0) break;
       if (pass > max_passes) {
         if (blockIdx.x == 0 && t == 0) ctr->bfs_status = 2;
@@ -1080,12 +1025,12 @@ __global__ void __launch_bounds__(256, 4) k_cut3(TileSet ts, int max_passes) {
         visit(tid, ts.d_info[tid]);
       }
       // (every CTA has read the count of the pass before; it is the one after next's)
-      if (blockIdx.x == 0 && t == 0) ctr->cut_n[(pass + 2) % 3] = 0;
+      if (blockIdx.x == 0 && t == 0) ctr->q3_n[(pass + 2) % 3] = 0;
     }
     __syncthreads();
     const int staged = min(s_n, kList);
     if (staged) {
-      if (t == 0) s_base = atomicAdd(&ctr->cut_n[(pass + 1) % 3], staged);
+      if (t == 0) s_base = atomicAdd(&ctr->q3_n[(pass + 1) % 3], staged);
       __syncthreads();
       for (int i = t; i < staged; i += blockDim.x) ts.d_q_bfs[(pass + 1) & 1][s_base + i] = s_list[i];
       __syncthreads();

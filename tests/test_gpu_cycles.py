@@ -63,3 +63,28 @@ def test_sweep_budget_ends_a_run(ctx, budget, use_graph):
     assert g.flow() == flow and np.array_equal(g.labels().ravel(), lab)
     assert st.global_relabels >= 3 and st.used_graph == use_graph
     g.close()
+
+
+@pytest.mark.parametrize("interval,cap,local", [(1, 3, 1), (1, -1, 16), (2, 0, 4), (64, 40, 16)])
+@pytest.mark.parametrize("shape", [(1, 1), (70, 210), (300, 333)])
+def test_allocation_free_cycles(ctx, shape, interval, cap, local):
+    # a run of the allocation-free solve ends after 8 cycles: short intervals need many runs
+    import torch
+    rng = np.random.default_rng(17 + shape[0])
+    n = shape[0] * shape[1]
+    caps = [np.where(rng.random(n) < 0.7, rng.integers(1, 25, n), 0).astype(np.int32) for _ in range(4)]
+    zero_boundary(shape, caps)
+    e = rng.integers(-3, 3, n).astype(np.int32)
+    e[rng.integers(0, n, max(1, n // 300))] -= 400
+    e[rng.integers(0, n, max(1, n // 200))] += 300
+    params = jfcut.default_params(relabel_interval=interval, relabel_interval_max=interval, relabel_cap=cap,
+                                  local_iters=local)
+    d_e = torch.from_numpy(e).cuda()
+    d_c = [torch.from_numpy(c).cuda() for c in caps]
+    d_lab = torch.empty(n, dtype=torch.uint8, device="cuda")
+    flow, _, _, lab = oracle.maxflow(shape, e, caps)
+    for turn in range(2):
+        d_lab.fill_(7)
+        f = jfcut.solve_grid2d_noalloc(shape[1], shape[0], d_e.data_ptr(), [c.data_ptr() for c in d_c],
+                                       d_lab.data_ptr(), params=params)
+        assert f == flow and np.array_equal(d_lab.cpu().numpy(), lab)
