@@ -92,8 +92,8 @@ typedef struct jfc_params {
                             (graphcut_push_relabel_fast.cl), for comparison; plain solves only,
                             relabel_interval iterations between global relabels; 2: block-wise
                             on whole 32 x 16 tiles */
-  int spin_limit;        /* polls before a device-side wait gives up (grid barrier, relabel
-                            worklist): 0 = default (2^26 polls, seconds); on expiry the
+  int spin_limit;        /* polls before a device-side wait gives up (grid barriers, tile
+                            staging, push-relabel worklist): 0 = default (2^26 polls, seconds); on expiry the
                             kernels leave, the call returns JFC_ERR_CUDA ("timed out") and the
                             context stays usable */
   int relabel_cap;       /* distance cap of the global relabels while solving: nodes farther
