@@ -111,7 +111,7 @@ struct DevCounters {
   int pr_out;                // push-relabel worklist: items queued and not yet fully visited
   // 2D global relabel (kernels_wave.cu)
   int q3_n[3];               // 3D relabel and cut: tiles or blocks queued for pass p, in entry p % 3
-  unsigned long long wave_bar[2]; // barrier arrivals (low 40 bits), CTAs that flagged a region (high bits)
+  unsigned long long wave_bar[2]; // barrier words (jfc_flagbar.h)
   unsigned wave_epoch;       // launches so far: which of the two the next one uses
   unsigned long long wave_q; // active items queued so far: parity 0 low, parity 1 high 32 bits
 };

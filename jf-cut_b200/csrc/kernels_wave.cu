@@ -38,6 +38,7 @@
 #include <algorithm>
 #include <cstddef>
 
+#include "jfc_flagbar.h"
 #include "jfc_sync.cuh"
 
 namespace {
@@ -132,41 +133,37 @@ __device__ __forceinline__ void changed_tiles(const TileSet& ts) {
   }
 }
 
-// Grid barrier of the relabel and the cut: one counter that only grows, so an
-// arrival is also the release and nothing is reset.  There are two, used by
-// launches in turn (wave_epoch counts them; the launch behind finds its own
-// zero).  The counter's high bits count the CTAs that flagged a region for the next phase, which
-// makes "is there a next phase" part of the same poll.  (A CTA that sees
-// arrivals of the phase after it sees them because that phase exists.)
-// Bounded like jfc::grid_sync.  Returns -1 on error, else whether any region
-// was flagged since `seen` (updated).
-constexpr int kArriveBits = 40;   // low bits of the counter: arrivals; the rest: CTAs that flagged
-__device__ __forceinline__ int wave_sync(DevCounters* ctr, unsigned epoch, unsigned long long target, bool any,
-                                         unsigned& seen) {
+// Grid barrier number `b` (0, 1, ...) of a launch of the relabel or the cut, on a
+// word whose arrivals only grow, so an arrival is also the release and nothing is
+// reset.  There are two words, used by launches in turn (wave_epoch counts them;
+// the launch behind finds its own zero).  The word also counts the CTAs that
+// flagged a region for the next phase (FlagBar), which makes "is there a
+// next phase" part of the same poll.  Bounded like jfc::grid_sync.  Returns -1 on
+// error, else whether any CTA passed `any` (thread 0's) at this barrier.
+__device__ __forceinline__ int wave_sync(DevCounters* ctr, unsigned epoch, unsigned b, bool any) {
   __shared__ int s_res;
-  __shared__ unsigned s_seen;
+  __shared__ unsigned s_mine;   // (thread 0)
   __syncthreads();
   if (threadIdx.x == 0) {
     unsigned long long* const bar = ctr->wave_bar + (epoch & 1u);
+    unsigned mine = b == 0 ? 0u : s_mine;
+    const unsigned long long add = jfc::FlagBar::arrival(b, any, mine);
+    s_mine = mine;
     __threadfence();
-    atomicAdd(bar, 1ull + (any ? 1ull << kArriveBits : 0ull));
+    atomicAdd(bar, add);
     unsigned long long spins = 0, v;
     const unsigned long long cap = jfc::spin_cap(ctr);
     int res = 0;
-    while (((v = *(volatile unsigned long long*)bar) & ((1ull << kArriveBits) - 1)) < target) {
+    while (!jfc::FlagBar::complete(v = *(volatile unsigned long long*)bar, b, gridDim.x)) {
       if (jfc::vload(&ctr->error)) { res = -1; break; }
       if (++spins > cap) { atomicExch(&ctr->error, 1); res = -1; break; }
       if (spins > 16) __nanosleep(40);
     }
     __threadfence();
-    if (res == 0) {
-      res = (unsigned)(v >> kArriveBits) != seen;
-      s_seen = (unsigned)(v >> kArriveBits);
-    }
+    if (res == 0) res = jfc::FlagBar::asked(v, b);
     s_res = res;
   }
   __syncthreads();
-  if (s_res > 0) seen = s_seen;
   return s_res;
 }
 
@@ -215,13 +212,12 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave_relabel(TileSet ts) {
   DevCounters* ctr = ts.d_ctr;
   if (jfc::cycle_skips(ts)) return;
   const unsigned epoch = wave_epoch(ctr);
-  unsigned seen = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     ctr->t_gr_start = jfc::global_ns();
     jfc::begin_cycle(ts);
   }
   changed_tiles<TY>(ts);
-  if (wave_sync(ctr, epoch, gridDim.x, false, seen) < 0) return;
+  if (wave_sync(ctr, epoch, 0, false) < 0) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     const unsigned long long t1 = jfc::global_ns();
     ctr->ns_gr_first += t1 - ctr->t_gr_start;
@@ -473,7 +469,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave_relabel(TileSet ts) {
         __syncthreads();   // the shared state is free for the next region
       }
     }
-    if (wave_sync(ctr, epoch, (unsigned long long)(phase + 1) * gridDim.x, any_next, seen) <= 0) break;
+    if (wave_sync(ctr, epoch, phase, any_next) <= 0) break;
   }
   if (t == 0) {
     atomicAdd(&ctr->bfs_visits, visits * (unsigned long long)(kIR / TY * kIW));
@@ -545,7 +541,6 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave_cut(TileSet ts, int max_pa
   unsigned long long visits = 0;
   if (jfc::cycle_skips(ts)) return;
   const unsigned epoch = wave_epoch(ctr);
-  unsigned seen = 0;
   if (blockIdx.x == 0 && t == 0) ctr->t_gr_start = jfc::global_ns();
   int phase = 1;
   bool ok_all = true;
@@ -680,7 +675,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave_cut(TileSet ts, int max_pa
         __syncthreads();
       }
     }
-    const int more = wave_sync(ctr, epoch, (unsigned long long)phase * gridDim.x, any_next, seen);
+    const int more = wave_sync(ctr, epoch, phase - 1, any_next);
     if (more < 0) ok_all = false;
     if (more <= 0) break;
     if (phase > max_passes) {
@@ -743,7 +738,7 @@ cudaError_t wave_cut_t(const TileSet& ts, int max_passes, cudaStream_t s) {
   static_assert(offsetof(DevCounters, bfs_status) == offsetof(DevCounters, cut_bad) + sizeof(int), "zeroed together");
   if (e == cudaSuccess && !ts.cyc_mode) e = cudaMemsetAsync(&ts.d_ctr->cut_bad, 0, 2 * sizeof(int), s);
   if (e != cudaSuccess) return e;
-  const int blocks = std::min(persistent_blocks_cached(cache, fn, kThreads), ts.nreg);
+  const int blocks = std::min({persistent_blocks_cached(cache, fn, kThreads), ts.nreg, (int)jfc::kFlagBarBlocks});
   TileSet arg = ts;
   void* params[] = {(void*)&arg, (void*)&max_passes};
   jfc_note_launch();
@@ -755,7 +750,7 @@ cudaError_t wave_t(const TileSet& ts, cudaStream_t s) {
   static int cache[64] = {0};
   const void* fn = (const void*)k_wave_relabel<TY>;
   // no more CTAs than regions: the grid barrier's cost grows with them
-  const int blocks = std::min(persistent_blocks_cached(cache, fn, kThreads), ts.nreg);
+  const int blocks = std::min({persistent_blocks_cached(cache, fn, kThreads), ts.nreg, (int)jfc::kFlagBarBlocks});
   TileSet arg = ts;
   void* params[] = {(void*)&arg};
   jfc_note_launch();
