@@ -139,12 +139,15 @@ __device__ __forceinline__ void changed_tiles(const TileSet& ts) {
 // the launch behind finds its own zero).  The word also counts the CTAs that
 // flagged a region for the next phase (FlagBar), which makes "is there a
 // next phase" part of the same poll.  Bounded like jfc::grid_sync.  Returns -1 on
-// error, else whether any CTA passed `any` (thread 0's) at this barrier.
-__device__ __forceinline__ int wave_sync(DevCounters* ctr, unsigned epoch, unsigned b, bool any) {
+// error, else whether any CTA passed `any` (thread 0's) at this barrier.  dead
+// (thread 0's): leave without an arrival.
+__device__ __forceinline__ int wave_sync(DevCounters* ctr, unsigned epoch, unsigned b, bool any, bool dead = false) {
   __shared__ int s_res;
   __shared__ unsigned s_mine;   // (thread 0)
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0 && dead) {
+    s_res = -1;
+  } else if (threadIdx.x == 0) {
     unsigned long long* const bar = ctr->wave_bar + (epoch & 1u);
     unsigned mine = b == 0 ? 0u : s_mine;
     const unsigned long long add = jfc::FlagBar::arrival(b, any, mine);
@@ -216,8 +219,12 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave_relabel(TileSet ts) {
     ctr->t_gr_start = jfc::global_ns();
     jfc::begin_cycle(ts);
   }
+  // a wait of an earlier launch gave up (a run without a graph queues launches
+  // behind it): that launch may have left arrivals in this epoch's word, so no
+  // barrier would hold
+  if (threadIdx.x == 0) s_tiles = (unsigned)jfc::vload(&ctr->error);
   changed_tiles<TY>(ts);
-  if (wave_sync(ctr, epoch, 0, false) < 0) return;
+  if (wave_sync(ctr, epoch, 0, false, threadIdx.x == 0 && s_tiles != 0) < 0) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     const unsigned long long t1 = jfc::global_ns();
     ctr->ns_gr_first += t1 - ctr->t_gr_start;
