@@ -334,6 +334,7 @@ __device__ __forceinline__ int pr_visit(const TileSet& ts, int tid, const int4& 
     }
   };
   heights();
+  __syncthreads();   // (the first round's relabels write what the other warps read here)
   // push order: +x, +y, -y, (+z, -z,) -x
   constexpr int kOrder[6] = {T::XP, T::YP, T::YM, DIMS == 3 ? T::ZP : T::XM, T::ZM, T::XM};
   constexpr int NP = T::K;
