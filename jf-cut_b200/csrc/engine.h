@@ -24,9 +24,9 @@ struct DevModel {
   uint8_t* d_seeds = nullptr;
   int* d_lut_t = nullptr;        // t-link costs [JFC_TQ + 1]; the two below share its allocation
   int* d_mu = nullptr;           // centres [2][JFC_MAX_K * 3]
-  uint8_t* d_lut_t8 = nullptr;   // the costs as bytes, when they fit (lut_t_max < 256)
+  uint8_t* d_lut_t8 = nullptr;   // the costs as bytes, when they fit (lut_t_bytes)
   int lut_lambda_t = -1;         // lambda_t the t-link tables hold (-1: none)
-  int lut_t_max = 0;             // largest cost
+  bool lut_t_bytes = false;      // every cost fits a byte
   size_t img_bytes = 0;
 };
 

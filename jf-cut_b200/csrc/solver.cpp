@@ -135,6 +135,10 @@ TableRuns tlink_runs(int lambda_t) {
   });
 }
 
+// Every entry fits a byte.  (A non-increasing table's first is its largest; scales
+// past 2^31 turn the first entries into INT_MIN.)
+bool byte_table(const TableRuns& r) { return r.val.front() >= 0 && r.val.front() < 256; }
+
 // Upload the runs and expand them into n ints and / or bytes on the stream; the
 // runs' buffer is freed on the stream.
 cudaError_t expand_runs(const TableRuns& r, int n, int* d_out, uint8_t* d_out8, cudaStream_t s) {
@@ -244,8 +248,8 @@ int build_core(jfc_graph* G, const void* img, int pixfmt, const uint8_t* seeds, 
   if (M.lut_lambda_t != m.lambda_t) {
     M.lut_lambda_t = -1;
     const TableRuns rt = tlink_runs(m.lambda_t);
-    M.lut_t_max = rt.val.front();   // (non-increasing)
-    JFC_B(expand_runs(rt, JFC_TQ + 1, M.d_lut_t, M.lut_t_max < 256 ? M.d_lut_t8 : nullptr, s));
+    M.lut_t_bytes = byte_table(rt);
+    JFC_B(expand_runs(rt, JFC_TQ + 1, M.d_lut_t, M.lut_t_bytes ? M.d_lut_t8 : nullptr, s));
     M.lut_lambda_t = m.lambda_t;
   }
   const TableRuns rxy = nlink_runs(pixfmt, scale_xy, sigma2);
@@ -253,8 +257,7 @@ int build_core(jfc_graph* G, const void* img, int pixfmt, const uint8_t* seeds, 
   NlinkTables nl;
   nl.nxy = rxy.start.back() + 1;
   nl.nz = rz.start.back() + 1;
-  const bool bytes = M.lut_t_max < 256 && rxy.val.front() < 256 && rz.val.front() < 256 &&
-                     build_tables_fit(G->dims, nl.nxy, nl.nz);
+  const bool bytes = M.lut_t_bytes && byte_table(rxy) && byte_table(rz) && build_tables_fit(G->dims, nl.nxy, nl.nz);
   const int nlut = nlink_entries(pixfmt);
   const size_t each = bytes ? align256(std::max(nl.nxy, nl.nz)) : align256(sizeof(int) * (size_t)nlut);
   char* d_nl = nullptr;
