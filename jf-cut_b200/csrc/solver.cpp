@@ -81,26 +81,51 @@ struct BuildScratch {
 };
 
 // A monotone integer table as runs of equal entries: value val[j] from entry
-// start[j] on.
+// start[j] on.  A table of more than an eighth of its entries (and 4,096) in runs,
+// as large scales give, is kept entry by entry in `whole` instead, each evaluated
+// once: finding its runs took up to twice as many evaluations as it has entries
+// (RGB at lambda_n of a million 4.6 ms of host time, 1.9 now; at 100 16 us as
+// before).
 struct TableRuns {
-  std::vector<int> start, val;
-  // Runs of the table t -> f(t), t in [0, n), f monotone: gallop from each run's
-  // start until the value changes, then bisect for the first entry that differs.
+  std::vector<int> start, val, whole;
+  // The table t -> f(t), t in [0, n), f monotone: gallop from each run's start
+  // until the value changes, then bisect for the first entry that differs, whose
+  // value is then known.
   template <typename F>
   TableRuns(int n, F f) {
+    const size_t most = std::max(4096, n / 8);
+    int v = f(0);
     for (int t = 0; t < n;) {
-      const int v = f(t);
+      if (val.size() == most) {
+        whole.resize(n);
+        for (size_t j = 0; j < most; ++j)
+          std::fill(whole.begin() + start[j], whole.begin() + (j + 1 < most ? start[j + 1] : t), val[j]);
+        for (whole[t] = v; ++t < n;) whole[t] = f(t);
+        return;
+      }
       start.push_back(t);
       val.push_back(v);
-      int lo = t, step = 1;                    // f(lo) == v
-      while (lo + step < n && f(lo + step) == v) { lo += step; step *= 2; }
-      int hi = std::min(n, lo + step);         // f(hi) != v, or the table's end
+      int lo = t, hi = n, next = v;            // f(lo) == v; f(hi) == next != v, or hi is the table's end
+      for (int step = 1; lo + step < n; step *= 2) {
+        const int w = f(lo + step);
+        if (w != v) {
+          hi = lo + step;
+          next = w;
+          break;
+        }
+        lo += step;
+      }
       while (hi - lo > 1) {
-        const int mid = lo + (hi - lo) / 2;
-        if (f(mid) == v) lo = mid;
-        else hi = mid;
+        const int mid = lo + (hi - lo) / 2, w = f(mid);
+        if (w == v) {
+          lo = mid;
+        } else {
+          hi = mid;
+          next = w;
+        }
       }
       t = hi;
+      v = next;
     }
   }
 };
@@ -109,7 +134,7 @@ struct TableRuns {
 // for RGB (t = ||dI||^2) and t^2 for scalar images (t = |dI|).  Non-increasing
 // (in floating point too: neighbouring arguments of exp lie apart by at least
 // 1 / (2 * 65535^2), many times its error), so it is found by its runs: about
-// 2,000 evaluations of exp at the default scale of 100 instead of the 195,076
+// 1,400 evaluations of exp at the default scale of 100 instead of the 195,076
 // entries of an RGB table, which took 1.9 ms of host time per build; the
 // device expands the runs.  (64 builds and one batch solve of images with
 // sides 128-1024: 119.6 -> 35.4 ms; 1920 x 1080 RGB, host to host: 9.7 -> 8.1;
@@ -135,13 +160,16 @@ TableRuns tlink_runs(int lambda_t) {
   });
 }
 
-// Every entry fits a byte.  (A non-increasing table's first is its largest; scales
-// past 2^31 turn the first entries into INT_MIN.)
+// Every entry fits a byte (then the table is in runs, at most 256).  (A
+// non-increasing table's first is its largest; scales past 2^31 turn the first
+// entries into INT_MIN.)
 bool byte_table(const TableRuns& r) { return r.val.front() >= 0 && r.val.front() < 256; }
 
 // Upload the runs and expand them into n ints and / or bytes on the stream; the
-// runs' buffer is freed on the stream.
+// runs' buffer is freed on the stream.  A whole table has no byte form and is
+// copied as it is.
 cudaError_t expand_runs(const TableRuns& r, int n, int* d_out, uint8_t* d_out8, cudaStream_t s) {
+  if (!r.whole.empty()) return cudaMemcpyAsync(d_out, r.whole.data(), n * sizeof(int), cudaMemcpyHostToDevice, s);
   const size_t m = r.start.size();
   int* buf = nullptr;
   cudaError_t e = cudaMallocAsync((void**)&buf, 2 * m * sizeof(int), s);
