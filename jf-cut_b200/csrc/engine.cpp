@@ -214,9 +214,7 @@ static void tileset_carve(TileSet& ts, char* blk, size_t* total) {
   ts.d_rflag[1] = (uint8_t*)(blk + o_rf1);
 }
 
-int tileset_build(TileSet& ts, int dims, int tile_rows, int tile_depth, const std::vector<GridDev>& grids_in,
-                  cudaStream_t s, bool pr_split) {
-  int TY, TZ;
+static void tile_shape(int dims, int tile_rows, int tile_depth, int& TY, int& TZ) {
   if (dims == 2) {
     TY = tile_rows; TZ = 1;
   } else {
@@ -225,6 +223,42 @@ int tileset_build(TileSet& ts, int dims, int tile_rows, int tile_depth, const st
     TZ = tile_depth > 0 ? tile_depth : 2;
     TY = tile_depth > 0 ? tile_rows / tile_depth : 4;
   }
+}
+
+// uint4 of row words of a tile set (2D: level-set state, 3D: twice that, the
+// words themselves)
+static long long row_word_count(int dims, long long ntiles, int TY, int TZ) {
+  return (dims == 2 ? 1 : 2) * ntiles * TY * TZ;
+}
+
+// The headroom of a block that is staged asynchronously (the server's, re-formed
+// between relabels).
+static void tileset_caps(TileSet& ts, int ntiles, int ngrids, long long nrw, int nreg, bool headroom) {
+  ts.cap_tiles = headroom ? ntiles + ntiles / 4 + 64 : ntiles;
+  ts.cap_grids = headroom ? ngrids + ngrids / 4 + 8 : ngrids;
+  ts.cap_rw = headroom ? nrw + nrw / 4 : nrw;
+  ts.cap_reg = headroom ? nreg + nreg / 4 : nreg;
+  if (ts.cap_tiles < 1) ts.cap_tiles = 1;
+  if (ts.cap_grids < 1) ts.cap_grids = 1;
+}
+
+size_t tileset_bytes(int dims, int tile_rows, int tile_depth, int w, int h, int d) {
+  int TY, TZ, pitch, Hp, Dp;
+  tile_shape(dims, tile_rows, tile_depth, TY, TZ);
+  grid_layout(dims, w, h, d, pitch, Hp, Dp);
+  const long long ntiles = (long long)(pitch / JFC_TW) * (Hp / TY) * (Dp / TZ);
+  TileSet ts;
+  tileset_caps(ts, (int)ntiles, 1, row_word_count(dims, ntiles, TY, TZ),
+               dims == 2 ? wave_regions(pitch / JFC_TW, Hp) : 0, true);
+  size_t total = 0;
+  tileset_carve(ts, nullptr, &total);
+  return total;
+}
+
+int tileset_build(TileSet& ts, int dims, int tile_rows, int tile_depth, const std::vector<GridDev>& grids_in,
+                  cudaStream_t s, bool pr_split) {
+  int TY, TZ;
+  tile_shape(dims, tile_rows, tile_depth, TY, TZ);
   std::vector<GridDev> grids = grids_in;
   int base = 0, npar[2] = {0, 0};
   for (size_t gi = 0; gi < grids.size(); ++gi) {
@@ -237,10 +271,9 @@ int tileset_build(TileSet& ts, int dims, int tile_rows, int tile_depth, const st
     base += g.tiles_x * g.tiles_y * g.tiles_z;
   }
   const int ntiles = base, ngrids = (int)grids.size();
-  // row words (2D: level-set state, 3D: twice that, the words themselves) and
-  // regions of the global relabel
+  // row words and regions of the global relabel
   std::vector<int4> regs;
-  const long long nrw = dims == 2 ? (long long)ntiles * TY : 2ll * ntiles * TY * TZ;
+  const long long nrw = row_word_count(dims, ntiles, TY, TZ);
   if (dims == 2) {
     for (int gi = 0; gi < ngrids; ++gi) {
       const GridDev& g = grids[gi];
@@ -264,12 +297,7 @@ int tileset_build(TileSet& ts, int dims, int tile_rows, int tile_depth, const st
     } else {
       tileset_free(ts);
     }
-    ts.cap_tiles = s ? ntiles + ntiles / 4 + 64 : ntiles;
-    ts.cap_grids = s ? ngrids + ngrids / 4 + 8 : ngrids;
-    ts.cap_rw = s ? nrw + nrw / 4 : nrw;
-    ts.cap_reg = s ? nreg + nreg / 4 : nreg;
-    if (ts.cap_tiles < 1) ts.cap_tiles = 1;
-    if (ts.cap_grids < 1) ts.cap_grids = 1;
+    tileset_caps(ts, ntiles, ngrids, nrw, nreg, s != nullptr);
     size_t total = 0;
     tileset_carve(ts, nullptr, &total);
     char* blk = nullptr;

@@ -77,6 +77,8 @@ int engine_cut(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, std::vector<GridR
 int tileset_build(TileSet& ts, int dims, int tile_rows, int tile_depth, const std::vector<GridDev>& grids,
                   cudaStream_t s = nullptr, bool pr_split = false);
 void tileset_free(TileSet& ts);
+// Bytes of the control block, with its headroom, of a set that holds one grid.
+size_t tileset_bytes(int dims, int tile_rows, int tile_depth, int w, int h, int d);
 // Drop the tile set's captured relabel-cycle graphs.
 void tileset_drop_graphs(TileSet& ts);
 int shape_code(int dims, int tile_rows, int tile_depth, bool pr_split);
@@ -120,6 +122,7 @@ void fill_defaults(jfc_params& p);
 // solver.cpp: graph layout, capacity build and plane copies
 size_t align256(size_t v);
 size_t state_bytes(int dims, int w, int h, int d);
+void grid_layout(int dims, int w, int h, int d, int& pitch, int& Hp, int& Dp);
 void model_defaults(jfc_model& m);
 int build_core(jfc_graph* G, const void* img, int pixfmt, const uint8_t* seeds, const jfc_model* mdl,
                cudaMemcpyKind kind);

@@ -66,6 +66,7 @@ struct Session {
   jfc_graph* G = nullptr;
   size_t charge = 0;                // bytes the session needs on the device
   size_t held = 0;                  // bytes held against the budget (after admission)
+  size_t sets = 0, sets_held = 0;   // the same of its share of the tile sets, held against the device
   Phase phase = WAIT_BUILD;
   std::deque<Request> reqs;         // front = the request being served
   jfc_request_info last{};
@@ -92,6 +93,7 @@ struct jfc_server {
   unsigned long long pool_threshold0 = 0;   // its release threshold before the server
   std::mutex read_mu;
   size_t budget = 0, used = 0;
+  size_t device_bytes = 0, sets_used = 0;   // what the device has for sessions; the sessions' shares of tile sets
   int max_slots = 64;
 
   std::mutex mu;
@@ -120,6 +122,32 @@ size_t session_bytes(int dims, int w, int h, int d, int pixfmt, size_t nseeds) {
          2 * align256(sizeof(int) * (JFC_TQ + 1)) +
          // capacity-build temporaries: seed lists, n-link tables, scratch
          align256(4 * nseeds) + 2 * align256(sizeof(int) * nlut) + 4096;
+}
+
+// Bytes of the device that are free now, with what its pool keeps mapped unused.
+size_t free_bytes(int device) {
+  size_t fr = 0, tot = 0;
+  if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) fr = 0;
+  cudaMemPool_t pool = nullptr;
+  unsigned long long kept = 0, inuse = 0;
+  if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &kept) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &inuse) == cudaSuccess && kept > inuse)
+    fr += kept - inuse;
+  cudaGetLastError();
+  return fr;
+}
+
+// A session may go from admission to its build (lock held): the sessions' own
+// bytes fit the budget, and with their tile sets they fit the device (a tile
+// set that finds no memory stops the server).  A session alone always goes.
+bool fits(jfc_server* S, const Session* s) {
+  if (S->used + s->charge > S->budget) return false;
+  const size_t need = S->used + S->sets_used + s->charge + s->sets;
+  if (S->used == 0 || need <= S->device_bytes) return true;
+  // (others may have given memory back since it was looked at)
+  S->device_bytes = std::max(S->device_bytes, free_bytes(S->device) + S->used);
+  return need <= S->device_bytes;
 }
 
 // Finish the front request of a session (lock held).
@@ -161,7 +189,8 @@ void free_session(jfc_server* S, Session* s) {
   }
   std::lock_guard<std::mutex> lk(S->mu);
   S->used -= s->held;
-  s->held = 0;
+  S->sets_used -= s->sets_held;
+  s->held = s->sets_held = 0;
   S->cv_build.notify_all();
 }
 
@@ -175,7 +204,7 @@ void builder_loop(jfc_server* S) {
         if (S->stop) return true;
         if (S->build_q.empty()) return false;
         const Session* f = S->sessions.at(S->build_q.front()).get();
-        return S->used + f->charge <= S->budget;
+        return fits(S, f);
       });
       if (S->stop) return;
       s = S->sessions.at(S->build_q.front()).get();
@@ -183,6 +212,8 @@ void builder_loop(jfc_server* S) {
       S->used += s->charge;
       S->peak_used = std::max(S->peak_used, S->used);
       s->held = s->charge;
+      S->sets_used += s->sets;
+      s->sets_held = s->sets;
       s->phase = BUILDING;
       s->reqs.front().t_admit = Clock::now();
     }
@@ -602,6 +633,7 @@ int jfc_server_create(jfc_ctx* ctx, size_t hbm_budget_bytes, int max_slots, jfc_
   S->params = ctx->params;
   fill_defaults(S->params);
   S->budget = hbm_budget_bytes;
+  S->device_bytes = free_bytes(ctx->device);
   S->max_slots = max_slots;
   int rc = jfc_create(ctx->device, &S->params, &S->solve_ctx);
   if (rc == JFC_OK) rc = jfc_create(ctx->device, &S->params, &S->build_ctx);
@@ -686,6 +718,9 @@ int jfc_server_submit(jfc_server* S, int dims, int w, int h, int d, const void* 
   if (model) s->model = *model;
   model_defaults(s->model);
   s->charge = session_bytes(dims, w, h, d, pixfmt, nseeds);
+  // its grid is in up to three sets' blocks, which keep the size they grew to: the
+  // lane of its cold request, the lane of its edits and the cut's
+  s->sets = 3 * tileset_bytes(dims, S->params.tile_rows, S->params.tile_depth, w, h, d);
   if (s->charge > S->budget) return set_error(JFC_ERR_OOM, "session needs more device memory than the server budget");
   // the copies (up to hundreds of MB) are made before the server lock is
   // taken: the solver thread takes it between every two relabel cycles
