@@ -616,8 +616,9 @@ static int run_cycles(jfc_ctx* ctx, TileSet& ts, const jfc_params& p, bool init,
   if (!x) cyc.done = 0;   // (nothing behind one relabel or cycle)
   const int phases = cyc.cycles - cyc.exact - (init ? 1 : 0);
   if (x) {
-    const int per = ts.dims == 2 ? 1 : 4;   // kernels of a relabel
-    jfc_note_launch(per * cyc.cycles + phases + (cyc.done == 2 ? (ts.dims == 2 ? 1 : 2) : 0));
+    // (the exact relabel and the cut are launched whether they are due or not)
+    const int per = ts.dims == 2 ? 1 : 4, cut = ts.dims == 2 ? 1 : 2;   // kernels of a relabel, of a cut
+    jfc_note_launch(per * (cyc.cycles - cyc.exact) + phases + per + cut);
     if (used_graph && phases > 0) *used_graph = true;
   }
   passes += cyc.passes;
