@@ -78,7 +78,10 @@ typedef struct jfc_params {
   int relabel_interval;  /* sweep pairs between global relabels at the start (default 0 =
                             automatic: 2 for 2D grids, 5 for 3D grids) */
   int max_sweeps;        /* budget of sweeps -> JFC_ERR_NOT_CONVERGED (default 1<<20) */
-  int max_bfs_passes;    /* budget of tile passes per BFS (default 1<<20) */
+  int max_bfs_passes;    /* budget of passes behind a BFS's first -> JFC_ERR_NOT_CONVERGED (default
+                            1<<20): frontier passes of a 3D global relabel, passes over regions
+                            (2D) or blocks (3D) of the cut, tile passes of the tag.  A 2D global
+                            relabel has none: it ends with the last reachable node */
   int use_graph;         /* 1: replay each relabel cycle (push-relabel phase + global
                             relabel + read-back) as one CUDA graph launch (default) */
   int verbose;           /* 1: one JSON line per global relabel on stderr */
@@ -92,10 +95,11 @@ typedef struct jfc_params {
                             (graphcut_push_relabel_fast.cl), for comparison; plain solves only,
                             relabel_interval iterations between global relabels; 2: block-wise
                             on whole 32 x 16 tiles */
-  int spin_limit;        /* polls before a device-side wait gives up (grid barriers, tile
-                            staging, push-relabel worklist): 0 = default (2^26 polls, seconds); on expiry the
-                            kernels leave, the call returns JFC_ERR_CUDA ("timed out") and the
-                            context stays usable */
+  int spin_limit;        /* polls before a device-side wait of a solve or tag gives up (grid
+                            barriers, tile staging, push-relabel worklist): 0 = default (2^26
+                            polls, seconds); on expiry the kernels leave, the call returns
+                            JFC_ERR_CUDA ("timed out") and the context stays usable.  The
+                            capacity build's k-means barrier always has the default */
   int relabel_cap;       /* distance cap of the global relabels while solving: nodes farther
                             than this from every deficit count as unreachable until no active
                             tile is left, then one exact (uncapped) relabel certifies the maximum
