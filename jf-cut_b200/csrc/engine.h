@@ -86,12 +86,9 @@ int shape_code(int dims, int tile_rows, int tile_depth, bool pr_split);
 bool pr_split_for(const jfc_params& p, int dims);
 // Sweep pairs between global relabels: relabel_interval, or when it is 0 the
 // measured best per dimensionality (2D: relabels are cheap next to the
-// push-relabel sweeps; 3D: the relabel dominates and runs less often).  Against 2,
-// 42 2D solves (7 image sizes, 6 seeds) are 6% slower in the mean with 1, 5% with 3
-// and 11% with 4; against 5, 16 videos (2 sizes, 8 seeds) are 6% slower with 3, 4%
-// with 4 and 1% with 6.
+// push-relabel sweeps; 3D: the relabel dominates and runs less often).
 inline int interval_for(const jfc_params& p, int dims) {
-  return p.relabel_interval > 0 ? p.relabel_interval : (dims == 2 ? 2 : 5);
+  return p.relabel_interval > 0 ? p.relabel_interval : (dims == 2 ? 2 : 3);
 }
 // Push-relabel visit scheduling (1 sweeps, 2 worklist, 3 sweeps while many
 // tiles are active and the worklist in the tail): pr_sched, or the sweeps when
