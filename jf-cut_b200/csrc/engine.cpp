@@ -260,7 +260,7 @@ int tileset_build(TileSet& ts, int dims, int tile_rows, int tile_depth, const st
   int TY, TZ;
   tile_shape(dims, tile_rows, tile_depth, TY, TZ);
   std::vector<GridDev> grids = grids_in;
-  int base = 0, npar[2] = {0, 0};
+  int base = 0;
   for (size_t gi = 0; gi < grids.size(); ++gi) {
     GridDev& g = grids[gi];
     if (g.dims != dims) return set_error(JFC_ERR_INVALID_ARG, "tile set mixes 2D and 3D grids");
@@ -354,19 +354,13 @@ int tileset_build(TileSet& ts, int dims, int tile_rows, int tile_depth, const st
   bool tma = JFC_PR_TMA && ngrids > 0;
   for (int gi = 0; gi < ngrids && tma; ++gi)
     tma = encode_pr_maps(grids[gi], ts.pr_split ? 8 : TY, TZ, maps + 3 * gi);
-  npar[0] = npar[1] = 0;
   size_t k = 0;
   for (size_t gi = 0; gi < grids.size(); ++gi) {
     const GridDev& g = grids[gi];
     for (int tz = 0; tz < g.tiles_z; ++tz)
       for (int ty = 0; ty < g.tiles_y; ++ty)
-        for (int tx = 0; tx < g.tiles_x; ++tx) {
-          info[k++] = make_int4((int)gi, tx, ty, tz);
-          ++npar[(tx + ty + tz) & 1];
-        }
+        for (int tx = 0; tx < g.tiles_x; ++tx) info[k++] = make_int4((int)gi, tx, ty, tz);
   }
-  ts.nlist[0] = npar[0];
-  ts.nlist[1] = npar[1];
   ts.d_tmap = tma ? ts.tmap_slot : nullptr;
   if (s) {
     // the staging buffer is rewritten only after the next host sync on `s`

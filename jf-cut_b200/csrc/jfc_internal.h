@@ -127,7 +127,6 @@ struct TileSet {
   int ntiles = 0;
   GridDev* d_desc = nullptr;         // [ngrids]
   int4* d_info = nullptr;            // [ntiles] {grid, tx, ty, tz}
-  int nlist[2] = {0, 0};             // tiles of parity 0 / 1
   int* d_flag_pr = nullptr;          // [2 * ntiles] work item waits in a push-relabel queue
   int* d_q_pr[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [parity][buffer]
   int* d_flag_bfs[2] = {nullptr, nullptr};  // [buffer][ntiles] tile waits in a BFS frontier
@@ -251,7 +250,6 @@ cudaError_t launch_seed_stats(const GridDev& g, const void* d_img, int pixfmt, c
 struct KmeansDev {
   int mu[2][JFC_MAX_K * 3];            // centres, fixed point 1/16
   int k[2];
-  int live[2];                         // class takes part
   unsigned long long n[2];             // list lengths
   // grid-wide form (all zero at launch)
   unsigned long long acc[3][2][JFC_MAX_K * 4];   // per centre: channel sums, count

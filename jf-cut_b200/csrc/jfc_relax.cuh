@@ -1,4 +1,4 @@
-// jfc_relax.cuh — CTA tile geometry and the arc bits of the global relabel.
+// jfc_relax.cuh — CTA tile geometry, the arc bits of the 3D global relabel, closures of row words.
 #pragma once
 
 #include "jfc_sync.cuh"
@@ -47,5 +47,23 @@ struct CtaTile {
 
 // Arc bits used by the relaxation: bit 0 +x, 1 +y, 2 -y, 3 -x, 4 +z, 5 -z.
 constexpr unsigned A_XP = 1u, A_YP = 2u, A_YM = 4u, A_XM = 8u, A_ZP = 16u, A_ZM = 32u;
+
+// bit x reached from bit x - 1 (x + 1) when m bit x is set; closure by doubling
+__device__ __forceinline__ unsigned close_right(unsigned p, unsigned m) {
+  p |= (p << 1) & m; m &= m << 1;
+  p |= (p << 2) & m; m &= m << 2;
+  p |= (p << 4) & m; m &= m << 4;
+  p |= (p << 8) & m; m &= m << 8;
+  p |= (p << 16) & m;
+  return p;
+}
+__device__ __forceinline__ unsigned close_left(unsigned p, unsigned m) {
+  p |= (p >> 1) & m; m &= m >> 1;
+  p |= (p >> 2) & m; m &= m >> 2;
+  p |= (p >> 4) & m; m &= m >> 4;
+  p |= (p >> 8) & m; m &= m >> 8;
+  p |= (p >> 16) & m;
+  return p;
+}
 
 }  // namespace jfc

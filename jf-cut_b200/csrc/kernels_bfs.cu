@@ -49,15 +49,6 @@ __device__ __forceinline__ void flush_staged(const BfsQ& Q, int lane) {
   for (int i = lane; i < cnt; i += 32) Q.q[base + i] = Q.sbuf[i];
 }
 
-template <int DIMS>
-struct Dirs {
-  static constexpr int XP = 0, YP = 1;
-  static constexpr int ZP = DIMS == 2 ? 0 : 2;
-  static constexpr int ZM = DIMS == 2 ? 0 : 3;
-  static constexpr int YM = DIMS == 2 ? 2 : 4;
-  static constexpr int XM = DIMS == 2 ? 3 : 5;
-};
-
 struct Addr {
   long long base, pitch, slab;
   bool has_yT, has_yB, has_zT, has_zB, has_xL, has_xR;
@@ -118,24 +109,6 @@ __device__ __forceinline__ void flag_neighbours(const GridDev& g, const Addr& a,
 }
 
 // ------------------------------------------------------------------ tag BFS
-// bit x reached from bit x - 1 (x + 1) when m bit x is set; closure by doubling
-__device__ __forceinline__ unsigned close_right(unsigned p, unsigned m) {
-  p |= (p << 1) & m; m &= m << 1;
-  p |= (p << 2) & m; m &= m << 2;
-  p |= (p << 4) & m; m &= m << 4;
-  p |= (p << 8) & m; m &= m << 8;
-  p |= (p << 16) & m;
-  return p;
-}
-__device__ __forceinline__ unsigned close_left(unsigned p, unsigned m) {
-  p |= (p >> 1) & m; m &= m >> 1;
-  p |= (p >> 2) & m; m &= m >> 2;
-  p |= (p >> 4) & m; m &= m >> 4;
-  p |= (p >> 8) & m; m &= m >> 8;
-  p |= (p >> 16) & m;
-  return p;
-}
-
 // The reference's tag post-process (graphcut_compute_tag.cl): reachability from
 // the foreground seeds through object nodes (any direction), kept in bit 1 of
 // the label byte; `seeds` is the dense seed array (JFC_SEED_FG = 1).  One warp
@@ -199,7 +172,7 @@ __device__ __forceinline__ void tag_tile(const GridDev& g, int4 ti, int tid, con
     unsigned ch = 0;
     auto grow = [&](int i, unsigned p) { ch |= p ^ L[i]; L[i] = p; };
 #pragma unroll
-    for (int i = 0; i < R; ++i) grow(i, close_left(close_right(L[i], OBJ[i] & ~1u), OBJ[i] & 0x7fffffffu));
+    for (int i = 0; i < R; ++i) grow(i, jfc::close_left(jfc::close_right(L[i], OBJ[i] & ~1u), OBJ[i] & 0x7fffffffu));
 #pragma unroll
     for (int i = 1; i < R; ++i) if (i % TY > 0) grow(i, L[i] | (L[i - 1] & OBJ[i]));
 #pragma unroll
@@ -328,7 +301,7 @@ __device__ __forceinline__ int row_close(int v, unsigned axp, unsigned axm, int 
 // lane).  With every row closed in every pass, and a last pass to see that
 // nothing falls, the frontier took 48.2 ms of a 2560 x 1440 x 50 solve instead of
 // 44.9.
-template <int DIMS, int TY, int TZ>
+template <int TY, int TZ>
 __device__ __forceinline__ void tile_close(int (&hv)[TY * TZ], const unsigned (&lab)[TY * TZ],
                                            const unsigned (&AXP)[TY * TZ], const unsigned (&AXM)[TY * TZ], int lane,
                                            unsigned rows) {
@@ -351,14 +324,12 @@ __device__ __forceinline__ void tile_close(int (&hv)[TY * TZ], const unsigned (&
 #pragma unroll
       for (int y = 1; y < TY; ++y) run(z * TY + y, z * TY + y - 1, jfc::A_YM);
     }
-    if constexpr (DIMS == 3) {
 #pragma unroll
-      for (int y = 0; y < TY; ++y) {
+    for (int y = 0; y < TY; ++y) {
 #pragma unroll
-        for (int z = TZ - 2; z >= 0; --z) run(z * TY + y, z * TY + y + TY, jfc::A_ZP);
+      for (int z = TZ - 2; z >= 0; --z) run(z * TY + y, z * TY + y + TY, jfc::A_ZP);
 #pragma unroll
-        for (int z = 1; z < TZ; ++z) run(z * TY + y, z * TY + y - TY, jfc::A_ZM);
-      }
+      for (int z = 1; z < TZ; ++z) run(z * TY + y, z * TY + y - TY, jfc::A_ZM);
     }
     rows = __reduce_or_sync(FULL, low);
   }
@@ -377,7 +348,7 @@ __device__ __forceinline__ uint4* row_words(const TileSet& ts, const GridDev& g,
 template <int TY, int TZ>
 __global__ void __launch_bounds__(256, TY * TZ > 8 ? 1 : 2) k_bits3(TileSet ts) {
   constexpr int R = TY * TZ;
-  using D = Dirs<3>;
+  using D = jfc::CtaTile<3, TY, TZ>;
   if (jfc::cycle_skips(ts)) return;
   DevCounters* ctr = ts.d_ctr;
   const int lane = threadIdx.x & 31;
@@ -595,12 +566,11 @@ template <int TY, int TZ, bool STAGED = false>
 __device__ __forceinline__ void relabel_frontier_minplus(const TileSet& ts, int tid, int4 ti, const BfsQ& Q,
                                                          int& cur_grid, int& delta, const int* hb = nullptr,
                                                          const uint8_t* lb = nullptr) {
-  constexpr int DIMS = 3;
   constexpr int R = TY * TZ;
   using ST = jfc::CtaTile<3, TY, TZ, 40, 4>;
   const int lane = threadIdx.x & 31;
   const GridDev& g = ts.d_desc[ti.x];
-  const Addr a = make_addr<DIMS, TY, TZ>(g, ti, lane);
+  const Addr a = make_addr<3, TY, TZ>(g, ti, lane);
   // the tile's activity byte as the last visit left it (another SM's write of
   // an earlier pass: read from L2, and early, so its latency overlaps the
   // closure)
@@ -630,7 +600,7 @@ __device__ __forceinline__ void relabel_frontier_minplus(const TileSet& ts, int 
   // the halo, fixed during the visit: y faces per z slice (lane = x), z
   // faces per row y, x faces in lanes r (left of row r) and 16 + r (right);
   // loaded together with the tile (no load waits for the arc bytes)
-  int HT[TZ], HB[TZ], HZT[DIMS == 3 ? TY : 1], HZB[DIMS == 3 ? TY : 1];
+  int HT[TZ], HB[TZ], HZT[TY], HZB[TY];
 #pragma unroll
   for (int z = 0; z < TZ; ++z) {
     if constexpr (STAGED) {
@@ -642,17 +612,15 @@ __device__ __forceinline__ void relabel_frontier_minplus(const TileSet& ts, int 
       HB[z] = a.has_yB ? g.h[n + (long long)TY * a.pitch] : JFC_INF;
     }
   }
-  if constexpr (DIMS == 3) {
 #pragma unroll
-    for (int y = 0; y < TY; ++y) {
-      if constexpr (STAGED) {
-        HZT[y] = a.has_zT ? hb[ST::hidx(lane, y, -1)] : JFC_INF;
-        HZB[y] = a.has_zB ? hb[ST::hidx(lane, y, TZ)] : JFC_INF;
-      } else {
-        const long long n = roff<TY>(a, y);
-        HZT[y] = a.has_zT ? g.h[n - a.slab] : JFC_INF;
-        HZB[y] = a.has_zB ? g.h[n + (long long)TZ * a.slab] : JFC_INF;
-      }
+  for (int y = 0; y < TY; ++y) {
+    if constexpr (STAGED) {
+      HZT[y] = a.has_zT ? hb[ST::hidx(lane, y, -1)] : JFC_INF;
+      HZB[y] = a.has_zB ? hb[ST::hidx(lane, y, TZ)] : JFC_INF;
+    } else {
+      const long long n = roff<TY>(a, y);
+      HZT[y] = a.has_zT ? g.h[n - a.slab] : JFC_INF;
+      HZB[y] = a.has_zB ? g.h[n + (long long)TZ * a.slab] : JFC_INF;
     }
   }
   const int xrow = lane & 15;
@@ -674,13 +642,11 @@ __device__ __forceinline__ void relabel_frontier_minplus(const TileSet& ts, int 
     seed(it, lab[it] & jfc::A_YM, HT[z]);
     seed(ib, lab[ib] & jfc::A_YP, HB[z]);
   }
-  if constexpr (DIMS == 3) {
 #pragma unroll
-    for (int y = 0; y < TY; ++y) {
-      const int it = y, ib = (TZ - 1) * TY + y;
-      seed(it, lab[it] & jfc::A_ZM, HZT[y]);
-      seed(ib, lab[ib] & jfc::A_ZP, HZB[y]);
-    }
+  for (int y = 0; y < TY; ++y) {
+    const int it = y, ib = (TZ - 1) * TY + y;
+    seed(it, lab[it] & jfc::A_ZM, HZT[y]);
+    seed(ib, lab[ib] & jfc::A_ZP, HZB[y]);
   }
 #pragma unroll
   for (int i = 0; i < R; ++i) {
@@ -688,7 +654,7 @@ __device__ __forceinline__ void relabel_frontier_minplus(const TileSet& ts, int 
     seed(i, lane == 0 && (lab[i] & jfc::A_XM), hl);
     seed(i, lane == 31 && (lab[i] & jfc::A_XP), hr);
   }
-  tile_close<DIMS, TY, TZ>(hv, lab, AXP, AXM, lane, __reduce_or_sync(FULL, seeded));
+  tile_close<TY, TZ>(hv, lab, AXP, AXM, lane, __reduce_or_sync(FULL, seeded));
   const int cap = jfc::cap_of(g, ts.d_ctr);
   unsigned rows_changed = 0;
   bool c0 = false, c31 = false, act = false;
@@ -716,7 +682,7 @@ __device__ __forceinline__ void relabel_frontier_minplus(const TileSet& ts, int 
     }
     delta += (act ? 1 : 0) - old;
   }
-  flag_neighbours<DIMS, TY, TZ>(g, a, tid, rows_changed, c0, c31, false, Q);
+  flag_neighbours<3, TY, TZ>(g, a, tid, rows_changed, c0, c31, false, Q);
 }
 
 // Refill of the push-relabel queues (buffer 0 of each parity) from the
@@ -978,7 +944,7 @@ __global__ void __launch_bounds__(256, 4) k_cut3(TileSet ts, int max_passes) {
     unsigned L = L0 | (lw & la) >> 31 | (rw & ra) << 31 | (yw & ya) | (zw & za);
     for (int it = 0; it < 32 * 32; ++it) {   // (a step but the last reaches a node)
       const unsigned was = L;
-      L = close_left(close_right(L, w0.x << 1), w1.y >> 1);
+      L = jfc::close_left(jfc::close_right(L, w0.x << 1), w1.y >> 1);
       const unsigned up = __shfl_up_sync(FULL, L & w0.y, 1), dn = __shfl_down_sync(FULL, L & w1.x, 1);
       const unsigned fr = __shfl_up_sync(FULL, L & w0.z, BY), bk = __shfl_down_sync(FULL, L & w0.w, BY);
       if (y > 0) L |= up;

@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(kKmThreads, 1) k_kmeans(const uint32_t* __rest
   const int t = threadIdx.x, lane = t & 31;
   const long long stride = (long long)gridDim.x * kKmThreads, start = (long long)blockIdx.x * kKmThreads + t;
   for (int i = t; i < 2 * JFC_MAX_K * 3; i += kKmThreads) (&s_mu[0][0])[i] = (&km->mu[0][0])[i];
-  bool live[2] = {km->live[0] != 0, km->live[1] != 0};
+  bool live[2] = {true, true};   // the class still moves
   bool ok = true;
   for (int it = 0; it < iters && ok && (live[0] || live[1]); ++it) {
     unsigned long long(*acc)[JFC_MAX_K * 4] = s_acc[it & 1];

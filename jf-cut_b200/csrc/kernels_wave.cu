@@ -39,7 +39,7 @@
 #include <cstddef>
 
 #include "jfc_flagbar.h"
-#include "jfc_sync.cuh"
+#include "jfc_relax.cuh"
 
 namespace {
 
@@ -496,24 +496,6 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave_relabel(TileSet ts) {
   if (blockIdx.x == 0 && warp == 0) jfc::end_cycle(ts);
 }
 
-// bit x reached from bit x - 1 (x + 1) when m bit x is set; closure by doubling
-__device__ __forceinline__ unsigned close_right(unsigned p, unsigned m) {
-  p |= (p << 1) & m; m &= m << 1;
-  p |= (p << 2) & m; m &= m << 2;
-  p |= (p << 4) & m; m &= m << 4;
-  p |= (p << 8) & m; m &= m << 8;
-  p |= (p << 16) & m;
-  return p;
-}
-__device__ __forceinline__ unsigned close_left(unsigned p, unsigned m) {
-  p |= (p >> 1) & m; m &= m >> 1;
-  p |= (p >> 2) & m; m &= m >> 2;
-  p |= (p >> 4) & m; m &= m >> 4;
-  p |= (p >> 8) & m; m &= m >> 8;
-  p |= (p >> 16) & m;
-  return p;
-}
-
 // Cut (graphcut_init_cut / graphcut_compute_cut, graphcut_compute_cut.cl:19-140):
 // the source side is every node reachable from {e > 0} along residual arcs;
 // reaching a deficit raises cut_bad (the reference's done[1] divergence flag).
@@ -623,7 +605,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_wave_cut(TileSet ts, int max_pa
 #pragma unroll
             for (int turn = 0; turn < 2; ++turn) {
 #pragma unroll
-              for (int i = 0; i < 4; ++i) L[i] = close_left(close_right(L[i], arc[i].x << 1), arc[i].w >> 1);
+              for (int i = 0; i < 4; ++i) L[i] = jfc::close_left(jfc::close_right(L[i], arc[i].x << 1), arc[i].w >> 1);
 #pragma unroll
               for (int i = 1; i < 4; ++i) L[i] |= L[i - 1] & arc[i - 1].y;
 #pragma unroll

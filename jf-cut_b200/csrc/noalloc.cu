@@ -216,10 +216,6 @@ extern "C" int jfc_solve_grid2d_noalloc(int device, void* stream, const jfc_para
   ts.dims = 2; ts.TR = TR; ts.TY = TR; ts.TZ = 1;
   ts.ngrids = 1;
   ts.ntiles = g.tiles_x * g.tiles_y;
-  int npar0 = 0;
-  for (int ty = 0; ty < g.tiles_y; ++ty) npar0 += (g.tiles_x + 1 - (ty & 1)) / 2;
-  ts.nlist[0] = npar0;
-  ts.nlist[1] = ts.ntiles - npar0;
   ts.d_desc = (GridDev*)(base + kOffDesc);
   ts.d_info = (int4*)(base + kOffInfo);
   ts.d_flag_pr = (int*)(base + kOffFlagPr);

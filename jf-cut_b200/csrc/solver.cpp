@@ -261,7 +261,6 @@ int build_core(jfc_graph* G, const void* img, int pixfmt, const uint8_t* seeds, 
   km.k[1] = std::min<int>(std::min(m.k_bg, JFC_MAX_K), (int)std::min<unsigned long long>(nb, JFC_MAX_K));
   km.n[0] = nf;
   km.n[1] = nb;
-  km.live[0] = km.live[1] = 1;
   for (int cls = 0; cls < 2; ++cls)
     for (int j = 0; j < km.k[cls]; ++j)
       for (int c = 0; c < C; ++c) {
