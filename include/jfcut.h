@@ -76,7 +76,7 @@ typedef struct jfc_params {
                             see tile_depth */
   int local_iters;       /* push/relabel rounds per tile visit (default 12) */
   int relabel_interval;  /* sweep pairs between global relabels at the start (default 0 =
-                            automatic: 2 for 2D grids, 3 for 3D grids) */
+                            automatic: 2 for 2D grids, 5 for 3D grids) */
   int max_sweeps;        /* budget of sweeps -> JFC_ERR_NOT_CONVERGED (default 1<<20) */
   int max_bfs_passes;    /* budget of passes behind a BFS's first -> JFC_ERR_NOT_CONVERGED (default
                             1<<20): frontier passes of a 3D global relabel, passes over regions

@@ -88,12 +88,14 @@ bool pr_split_for(const jfc_params& p, int dims);
 // measured best per dimensionality (2D: relabels are cheap next to the
 // push-relabel sweeps; 3D: the relabel dominates and runs less often).  Against 2,
 // 42 2D solves (7 image sizes, 6 seeds) are 6% slower in the mean with 1, 5% with 3
-// and 11% with 4.  Against 3, 44 videos (5 sizes, 8 or 12 seeds, the middle of 3
-// single solves) take 4% longer with 2 and 1% less with 4 and with 5, but with 4
-// one takes 19% and with 5 one 55% longer, and the 12 of 2560 x 1440 x 50 take as
-// long with 4 and 1% longer with 5.
+// and 11% with 4.  Against 3, by single solves of 348 videos: the 92 of 2560 x 1440 x
+// 50 take as long with 4 and with 5 (means 0.999 and 1.001 of the time, +-0.004),
+// the 256 others (320 to 1600 wide, 6 to 48 frames) 2.5% less with 4 and 3.5% less
+// with 5.  On single inputs the intervals differ either way: with 5, 12 took over
+// 10% longer than with 3 (most: 55%, an exact relabel that found far excess) and
+// 54 over 10% less.
 inline int interval_for(const jfc_params& p, int dims) {
-  return p.relabel_interval > 0 ? p.relabel_interval : (dims == 2 ? 2 : 3);
+  return p.relabel_interval > 0 ? p.relabel_interval : (dims == 2 ? 2 : 5);
 }
 // Push-relabel visit scheduling (1 sweeps, 2 worklist, 3 sweeps while many
 // tiles are active and the worklist in the tail): pr_sched, or the sweeps when
