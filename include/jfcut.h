@@ -276,7 +276,10 @@ typedef struct jfc_request_info {
 } jfc_request_info;
 
 /* max_slots: requests solving at once (0: 64); cold requests take at most
- * max_slots - max_slots / 4 of them, the rest stay free for warm edits. */
+ * max_slots - max_slots / 4 of them, the rest stay free for warm edits.  A
+ * session waits for its build while the sessions' own bytes with it exceed
+ * the budget, or those and their shares of the shared working sets exceed what
+ * the device has (a session alone does not wait for the latter). */
 int  jfc_server_create(jfc_ctx* ctx, size_t hbm_budget_bytes, int max_slots, jfc_server** out);
 void jfc_server_destroy(jfc_server* s);
 /* Submit a new session from host image + seeds; returns a session id >= 0 in *sid. */
